@@ -175,14 +175,16 @@ int lapis_b200_spmv_f64(lapis_b200_csr_t h, const double *d_x, double *d_y, int 
  * faster depends on the matrix: the persistent one when x is served from cache (banded
  * matrices), the other when the gathers of x dominate.  lapis_b200_csr_tune times the
  * candidates on the matrix (a few SpMV launches into scratch buffers it allocates and frees;
- * synchronises `stream`) and stores the winner in the handle; untuned handles use (256,4).
+ * synchronises `stream`) and stores the winner in the handle; untuned handles use (256,4), or
+ * the kind for short rows below.
  * lapis_b200_spmv_select_kernel forces one variant process-wide (threads = 0 returns to the
  * handles' own choice); the environment variable LAPIS_B200_SPMV="threads,blocks,l2_hint" does
  * the same from outside.  l2_hint marks x evict-last in L2.
- * A third kind, threads = 1 and blocks_per_sm = 0, gives every row to one thread; the tuner considers it
- * (and the launch honours it) only for matrices whose longest row has at most 32 entries -- up to there it
- * returns the same bits as the others -- and such matrices (stencils, bounded-degree graphs) are where it
- * wins.  On other matrices, and on handles that were never tuned, a request for it runs (256,4).
+ * A third kind, threads = 1 and blocks_per_sm = 0, has one thread add up every row (one thread per row, or a block
+ * per 32 or 64 rows that stages their products); the tuner considers it (and the launch honours it) only for
+ * matrices whose longest row has at most 32 entries -- up to there it returns the same bits as the others.  Such
+ * matrices (stencils, bounded-degree graphs) are where it wins, and handles that were never tuned use it for them;
+ * on other matrices a request for it runs (256,4).  l2_hint 2, 3 or 4 names one of its three kernels.
  * A fourth kind, threads = 2 (256 threads, blocks_per_sm in {4, 5}) or threads = 3 (512 threads,
  * blocks_per_sm in {2, 3, 4}), is the chunk kernel with the row sums done by a
  * segmented scan in registers instead of one lane per row over shared memory (less shared-memory traffic

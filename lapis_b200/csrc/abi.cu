@@ -49,6 +49,52 @@ int sm_count() {
   return cached[dev];
 }
 
+// ---- device memory pool -----------------------------------------------------
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pools[64] = {nullptr};
+
+static int pool_of_device(cudaMemPool_t *out) {
+  int dev = 0;
+  LAPIS_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return fail(LAPIS_EBADARG, "device index %d not supported", dev);
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (g_pools[dev] == nullptr) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool;
+    LAPIS_CUDA_TRY(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = POOL_KEEP_BYTES;
+    LAPIS_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_pools[dev] = pool;
+  }
+  *out = g_pools[dev];
+  return LAPIS_OK;
+}
+
+int pool_alloc(void **p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = nullptr;
+  LAPIS_TRY(pool_of_device(&pool));
+  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 16, pool, st);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    return fail(LAPIS_ECUDA, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  }
+  return LAPIS_OK;
+}
+
+void pool_free(void *p, cudaStream_t st) {
+  if (p != nullptr) cudaFreeAsync(p, st);
+}
+
+void pool_trim() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  for (cudaMemPool_t pool : g_pools)
+    if (pool != nullptr) cudaMemPoolTrimTo(pool, 0);
+}
+
 // ---- module state -----------------------------------------------------------
 static int g_init_count = 0;
 static std::vector<void *> g_alive_host;  // result buffers handed to the caller (LAPISSupport.hpp:93-120)
@@ -521,6 +567,7 @@ extern "C" void lapis_finalize(void) {
     for (void *p : g_alive_host) std::free(p);
     g_alive_host.clear();
     cudaDeviceSynchronize();
+    pool_trim();
   }
 }
 

@@ -197,7 +197,8 @@ spmv_chunk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const do
   __shared__ double s_red[THREADS / 32];
   using Pair = typename IndexPair<I>::type;
 
-  asm volatile("griddepcontrol.launch_dependents;");  // the fix-up kernel may start launching; it waits for our completion
+  pdl_release();  // only the small fix-up kernel follows at once
+  pdl_wait();
   if (skip_flag != nullptr && *skip_flag != 0) return;
 
   const int tid = threadIdx.x;
@@ -319,7 +320,8 @@ spmv_scan_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   __shared__ double s_red[THREADS / 32];
   using Pair = typename IndexPair<I>::type;
 
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_release();  // only the small fix-up kernel follows at once
+  pdl_wait();
   if (skip_flag != nullptr && *skip_flag != 0) return;
 
   const int tid = threadIdx.x, lane = tid & 31;
@@ -485,7 +487,8 @@ spmv_pipe_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   double *s_red = reinterpret_cast<double *>(s_nlong + 2);
   uint64_t *full = reinterpret_cast<uint64_t *>(s_red + THREADS / 32);
 
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_release();  // only the small fix-up kernel follows at once
+  pdl_wait();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   const int tid = threadIdx.x;
   if (tid == 0) {
@@ -675,7 +678,8 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
                  const int *__restrict__ skip_flag) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int S = SPMV_WALK_STEP;
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_release();  // only the small fix-up kernel follows at once
+  pdl_wait();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * (SPMV_WALK_THREADS / 32) + (threadIdx.x >> 5);
@@ -883,7 +887,8 @@ __global__ void spmv_fixup_kernel(const I *__restrict__ pos, const int64_t *__re
                                   double *__restrict__ y, const int *__restrict__ skip_flag, int tile) {
   // Launched with programmatic stream serialization: the blocks may already be resident while the SpMV
   // kernel drains; nothing is read before that kernel has completed and its writes are visible.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
+  pdl_release();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk - 1) return;
@@ -937,6 +942,7 @@ spmv_rowthread_kernel(const I *__restrict__ pos, const I *__restrict__ crd, cons
                       double *__restrict__ blk_partial, const int *__restrict__ skip_flag, PcgExchange ex) {
   __shared__ double s_red[8];
   __shared__ int s_flag;
+  pdl_wait();
   if (skip_flag != nullptr && *skip_flag != 0) return;
   if (PCG_FUSED && ex.mbox != nullptr && !pcg_wait_halo(ex, &s_flag)) return;
   double dot_local = 0.0;
@@ -965,11 +971,93 @@ spmv_rowthread_kernel(const I *__restrict__ pos, const I *__restrict__ crd, cons
       if (FUSE_DOT) dot_local = __dadd_rn(dot_local, __dmul_rn(__dadd_rn(carried, s_last), dv));
     }
   }
+  pdl_release();
   if (FUSE_DOT) {
     const double t = block_sum(dot_local, s_red);
     if (threadIdx.x == 0) blk_partial[blockIdx.x] = t;
     if (PCG_FUSED && pcg_last_block(pcg_tickets(ex.sc) + 0, gridDim.x, &s_flag)) pcg_tail_pass_a(ex, blk_partial, gridDim.x, s_red);
   }
+}
+
+// ---------------------------------------------------------------------------
+// One block per ROWS consecutive short rows, one launch: the block's entries are contiguous, so all threads stream
+// them with coalesced loads, gather x and park the products in shared memory, and one thread per row adds them in
+// entry order (and in the pieces of the chunk boundaries, as spmv_rowthread_kernel does: same bits).  No plan, no
+// carries, no second kernel.
+// Bound by the chain pos -> entries -> x -> sums at small sizes (10,000 rows of 10: 2.9 us a call, where the chunk
+// kernel and its fix-up take 4.9), by the gathers of x at large ones (1e6 x 10: 51 us, chunk kernel 63; 1e6 x 5: 27,
+// chunk 36).  Few rows per block keep its shared memory small, which leaves L1 to the gathers: with 128 rows of 32
+// entries per block (32 KB) the same kernel takes 522 us where 32 rows (8 KB) take 232.  Only on stencils of millions
+// of rows is one thread per row faster (2000^2 grid: 71 us, 78 here), which the tuner finds out.
+// ---------------------------------------------------------------------------
+template <typename I, int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS)
+spmv_rowblock_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, int64_t abase,
+                     int64_t nrows, const double *__restrict__ x, double *__restrict__ y, int accumulate,
+                     const int *__restrict__ skip_flag) {
+  static_assert(ROWS <= THREADS, "one thread per row");
+  extern __shared__ double s_rowprod[];
+  pdl_wait();
+  if (skip_flag != nullptr && *skip_flag != 0) return;
+  const int64_t r0 = (int64_t)blockIdx.x * ROWS;
+  const int nr = (int)(nrows - r0 < ROWS ? nrows - r0 : ROWS);
+  const int64_t e0 = (int64_t)pos[r0];
+  const int n = (int)((int64_t)pos[r0 + nr] - e0);
+  int64_t lo = 0, hi = 0;
+  double yin = 0.0;
+  if (threadIdx.x < nr) {
+    lo = (int64_t)pos[r0 + threadIdx.x];
+    hi = (int64_t)pos[r0 + threadIdx.x + 1];
+    if (accumulate) yin = y[r0 + threadIdx.x];
+  }
+  const I *c = crd + e0;
+  const double *v = val + e0;
+  int j = threadIdx.x;
+  for (; j + 3 * THREADS < n; j += 4 * THREADS) {
+    double a[4], xv[4];
+    I ci[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      ci[u] = __ldcs(c + j + u * THREADS);
+      a[u] = __ldcs(v + j + u * THREADS);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) xv[u] = __ldg(x + (int64_t)ci[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s_rowprod[j + u * THREADS] = __dmul_rn(a[u], xv[u]);
+  }
+  if (j < n) {  // up to three more per thread, again all loads first
+    double a[3], xv[3];
+    I ci[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      const bool in = j + u * THREADS < n;
+      ci[u] = in ? __ldcs(c + j + u * THREADS) : (I)0;
+      a[u] = in ? __ldcs(v + j + u * THREADS) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) xv[u] = j + u * THREADS < n ? __ldg(x + (int64_t)ci[u]) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (j + u * THREADS < n) s_rowprod[j + u * THREADS] = __dmul_rn(a[u], xv[u]);
+  }
+  __syncthreads();
+  pdl_release();
+  if (threadIdx.x >= nr) return;
+  auto piece = [&](int64_t from, int64_t to) {
+    double acc = 0.0;
+    for (int q = (int)(from - e0); q < (int)(to - e0); ++q) acc = __dadd_rn(acc, s_rowprod[q]);
+    return acc;
+  };
+  const int64_t bnd = abase + ((lo - abase) / SPMV_TILE + 1) * (int64_t)SPMV_TILE;  // first chunk boundary after lo
+  double out;
+  if (bnd >= hi) {
+    out = __dadd_rn(piece(lo, hi), yin);
+  } else {  // rows of at most 32 entries cross one boundary
+    const double first = piece(lo, bnd), last = piece(bnd, hi);
+    out = __dadd_rn(__dadd_rn(last, yin), first);
+  }
+  y[r0 + threadIdx.x] = out;
 }
 
 // ---------------------------------------------------------------------------
@@ -1107,8 +1195,9 @@ pcg_spmv_direction_kernel(const I *__restrict__ pos, const I *__restrict__ crd, 
   if (go) pcg_tail_pass_a(ex, blk_partial, gridDim.x, s_red);  // reads the iteration counter advanced above
 }
 
+// What the host needs to know of a matrix to plan for it: {longest row, pos[0], pos[nrows]}; facts[0] starts at zero.
 template <typename I>
-__global__ void max_row_len_kernel(const I *__restrict__ pos, int64_t nrows, unsigned long long *out) {
+__global__ void csr_facts_kernel(const I *__restrict__ pos, int64_t nrows, unsigned long long *facts) {
   unsigned long long m = 0;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += (int64_t)gridDim.x * blockDim.x) {
     const unsigned long long len = (unsigned long long)((int64_t)pos[r + 1] - (int64_t)pos[r]);
@@ -1119,7 +1208,11 @@ __global__ void max_row_len_kernel(const I *__restrict__ pos, int64_t nrows, uns
     const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
     m = o > m ? o : m;
   }
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
+  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(facts, m);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    facts[1] = (unsigned long long)(int64_t)pos[0];
+    facts[2] = (unsigned long long)(int64_t)pos[nrows];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1249,7 +1342,7 @@ spmm_row_direct_kernel(const I *__restrict__ pos, const I *__restrict__ crd, con
 // Host side
 // ---------------------------------------------------------------------------
 // Kernel variant: {threads, blocks per SM, L2 hint}.  threads >= 256: one chunk per block; threads == 2 / 3: the
-// segmented-scan chunk kernel with 256 / 512 threads (minb blocks per SM); threads == 1: one thread per row;
+// segmented-scan chunk kernel with 256 / 512 threads (minb blocks per SM); threads == 1: the kernels for short rows;
 // threads < 0: the persistent bulk-copy kernel with |threads| threads.  Which one is faster
 // depends on the matrix (the persistent kernel wins when x is served from L1/L2, as for banded
 // matrices; the one-chunk kernel when the gathers of x dominate), so lapis_b200_csr_tune times
@@ -1259,6 +1352,9 @@ struct SpmvVariant {
   int threads, minb, hint;
 };
 constexpr SpmvVariant SPMV_DEFAULT{256, 4, 1};
+// hint of the threads == 1 variant (matrices of short rows, all with the same bits): which kernel; below 2: by the
+// mean row length
+enum { SHORT_ROW_PER_THREAD = 2, SHORT_64_ROWS = 3, SHORT_32_ROWS = 4 };
 static SpmvVariant &spmv_override() {  // threads == 0: no override
   static SpmvVariant v = [] {
     SpmvVariant d{0, 0, 0};
@@ -1287,11 +1383,11 @@ static void launch_chunks(const lapis_b200_csr *h, const double *x, double *y, i
   const I *crd = static_cast<const I *>(h->crd);
   const int64_t abase = h->base & ~(int64_t)3, nnz_end = h->base + h->nnz;
   if (dotvec != nullptr)
-    spmv_chunk_kernel<I, THREADS, MINB, true, HINT><<<(unsigned)h->nblk, THREADS, 0, st>>>(
+    launch_pdl(spmv_chunk_kernel<I, THREADS, MINB, true, HINT>, (unsigned)h->nblk, THREADS, 0, st,
         pos, crd, h->val, h->blk_row, abase, nnz_end, h->nrows, x, y, accumulate, h->carry, dotvec, blk_partial,
         skip_flag);
   else
-    spmv_chunk_kernel<I, THREADS, MINB, false, HINT><<<(unsigned)h->nblk, THREADS, 0, st>>>(
+    launch_pdl(spmv_chunk_kernel<I, THREADS, MINB, false, HINT>, (unsigned)h->nblk, THREADS, 0, st,
         pos, crd, h->val, h->blk_row, abase, nnz_end, h->nrows, x, y, accumulate, h->carry, nullptr, nullptr,
         skip_flag);
 }
@@ -1350,28 +1446,25 @@ template <typename I>
 static int launch_fixup(const lapis_b200_csr *h, const int64_t *plan, const double *carry, int64_t nblk, int tile, double *y,
                         const int *skip_flag, cudaStream_t st) {
   if (nblk <= 1) return LAPIS_OK;
-  const I *pos = static_cast<const I *>(h->pos);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((nblk - 1 + 255) / 256));
-  cfg.blockDim = dim3(256);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;  // lets the fix-up blocks become resident while the SpMV kernel drains
-  LAPIS_CUDA_TRY(cudaLaunchKernelEx(&cfg, spmv_fixup_kernel<I>, pos, plan, (int64_t)(h->base & ~(int64_t)3), nblk,
-                                    (int64_t)h->nrows, carry, y, skip_flag, tile));
+  LAPIS_CUDA_TRY(launch_pdl(spmv_fixup_kernel<I>, (unsigned)((nblk - 1 + 255) / 256), 256, 0, st, static_cast<const I *>(h->pos), plan,
+                            h->base & ~(int64_t)3, nblk, h->nrows, carry, y, skip_flag, tile));
   return LAPIS_OK;
 }
 
-// Whether spmv_launch will run the one-thread-per-row kernel for this handle (the variant that can carry the
-// head and tail of a PCG iteration's first pass).
-static bool uses_rowthread(const lapis_b200_csr *h) {
+static bool has_short_rows(const lapis_b200_csr *h) { return h->max_row_len >= 0 && h->max_row_len <= SPMV_ROWTHREAD_MAX_LEN; }
+
+// The variant a launch on this handle runs: the override, the tuned one, or the default for the matrix.
+static SpmvVariant spmv_variant(const lapis_b200_csr *h) {
   SpmvVariant v = spmv_override();
-  if (v.threads == 0) v = h->tuned_threads != 0 ? SpmvVariant{h->tuned_threads, h->tuned_minb, h->tuned_hint} : SPMV_DEFAULT;
-  return v.threads == 1 && h->max_row_len >= 0 && h->max_row_len <= SPMV_ROWTHREAD_MAX_LEN;
+  if (v.threads == 0 && h->tuned_threads != 0) v = SpmvVariant{h->tuned_threads, h->tuned_minb, h->tuned_hint};
+  else if (v.threads == 0) v = has_short_rows(h) ? SpmvVariant{1, 0, 1} : SPMV_DEFAULT;
+  if (v.threads == 1 && !has_short_rows(h)) v = SPMV_DEFAULT;
+  return v;
 }
+
+// Whether spmv_launch will run the kernels for short rows on this handle (one thread per row: the variant that can
+// carry the head and tail of a PCG iteration's first pass).
+static bool uses_rowthread(const lapis_b200_csr *h) { return spmv_variant(h).threads == 1; }
 
 // Grid of the SpMV pass of a PCG iteration in both of its forms (spmv_rowthread_kernel with head and tail,
 // pcg_spmv_direction_kernel): the blocks that are resident at once for either kernel, looping over the row
@@ -1400,35 +1493,39 @@ template <typename I>
 static int launch_spmv(const lapis_b200_csr *h, const double *x, double *y, int accumulate,
                        const double *dotvec, double *blk_partial, const int *skip_flag,
                        cudaStream_t st, const PcgExchange *ex) {
-  SpmvVariant v = spmv_override();
-  if (v.threads == 0) v = h->tuned_threads != 0 ? SpmvVariant{h->tuned_threads, h->tuned_minb, h->tuned_hint} : SPMV_DEFAULT;
+  SpmvVariant v = spmv_variant(h);
   if (v.threads == 1) {
-    // one thread per row: only where it returns the chunk kernels' bits (rows of at most 32 entries, which the
-    // tuner has checked); otherwise the default kernel runs
-    if (h->max_row_len >= 0 && h->max_row_len <= SPMV_ROWTHREAD_MAX_LEN) {
-      const I *pos = static_cast<const I *>(h->pos);
-      const I *crd = static_cast<const I *>(h->crd);
-      const int64_t abase = h->base & ~(int64_t)3, ntiles = (h->nrows + 255) / 256;
-      const PcgExchange none = {};
-      if (dotvec != nullptr && ex != nullptr) {
-        // as pass A of a PCG iteration: a grid of exactly the blocks that are resident at once, looping over the
-        // row tiles, so that the block that finishes last has about a thousand partial sums to add, not one per
-        // chunk of the plan (a grid larger than what is resident would run its last blocks on a nearly empty GPU)
-        unsigned grid = 1;
-        LAPIS_TRY(pcg_pass_grid<I>(h, &grid));
-        spmv_rowthread_kernel<I, true, true><<<grid, 256, 0, st>>>(pos, crd, h->val, abase, h->nrows, ntiles, x, y,
-                                                                                  accumulate, dotvec, blk_partial, skip_flag, *ex);
-      }
-      else if (dotvec != nullptr)
-        spmv_rowthread_kernel<I, true, false><<<(unsigned)h->nblk, 256, 0, st>>>(pos, crd, h->val, abase, h->nrows, ntiles, x, y,
-                                                                                 accumulate, dotvec, blk_partial, skip_flag, none);
+    const I *pos = static_cast<const I *>(h->pos);
+    const I *crd = static_cast<const I *>(h->crd);
+    const int64_t abase = h->base & ~(int64_t)3, ntiles = (h->nrows + 255) / 256;
+    const PcgExchange none = {};
+    if (dotvec != nullptr && ex != nullptr) {
+      // as pass A of a PCG iteration: a grid of exactly the blocks that are resident at once, looping over the
+      // row tiles, so that the block that finishes last has about a thousand partial sums to add, not one per
+      // chunk of the plan (a grid larger than what is resident would run its last blocks on a nearly empty GPU)
+      unsigned grid = 1;
+      LAPIS_TRY(pcg_pass_grid<I>(h, &grid));
+      spmv_rowthread_kernel<I, true, true><<<grid, 256, 0, st>>>(pos, crd, h->val, abase, h->nrows, ntiles, x, y, accumulate, dotvec,
+                                                                 blk_partial, skip_flag, *ex);
+    } else if (dotvec != nullptr) {
+      spmv_rowthread_kernel<I, true, false><<<(unsigned)h->nblk, 256, 0, st>>>(pos, crd, h->val, abase, h->nrows, ntiles, x, y,
+                                                                               accumulate, dotvec, blk_partial, skip_flag, none);
+    } else {
+      // rows of few entries: more rows per block and two threads each; longer ones: four threads each
+      const int shape = v.hint >= 2 ? v.hint : h->nnz <= 6 * h->nrows ? SHORT_64_ROWS : SHORT_32_ROWS;
+      const size_t row_bytes = (size_t)std::max<int64_t>(h->max_row_len, 1) * sizeof(double);
+      if (shape == SHORT_ROW_PER_THREAD)
+        launch_pdl(spmv_rowthread_kernel<I, false, false>, (unsigned)h->nblk, 256, 0, st, pos, crd, h->val, abase, h->nrows, ntiles, x,
+                   y, accumulate, nullptr, nullptr, skip_flag, none);
+      else if (shape == SHORT_64_ROWS)
+        launch_pdl(spmv_rowblock_kernel<I, 128, 64>, (unsigned)((h->nrows + 63) / 64), 128, 64 * row_bytes, st, pos, crd, h->val, abase,
+                   h->nrows, x, y, accumulate, skip_flag);
       else
-        spmv_rowthread_kernel<I, false, false><<<(unsigned)h->nblk, 256, 0, st>>>(pos, crd, h->val, abase, h->nrows, ntiles, x, y,
-                                                                                  accumulate, nullptr, nullptr, skip_flag, none);
-      LAPIS_CUDA_TRY(cudaGetLastError());
-      return LAPIS_OK;
+        launch_pdl(spmv_rowblock_kernel<I, 128, 32>, (unsigned)((h->nrows + 31) / 32), 128, 32 * row_bytes, st, pos, crd, h->val, abase,
+                   h->nrows, x, y, accumulate, skip_flag);
     }
-    v = SPMV_DEFAULT;
+    LAPIS_CUDA_TRY(cudaGetLastError());
+    return LAPIS_OK;
   }
   if (ex != nullptr) return fail(LAPIS_EBADARG, "spmv: the fused PCG pass needs the one-thread-per-row kernel");
   if (v.threads == 4) {
@@ -1444,19 +1541,16 @@ static int launch_spmv(const lapis_b200_csr *h, const double *x, double *y, int 
       // chunks of the shared plan (the consumers of the fused dot product expect one partial per chunk)
       const unsigned grid = (unsigned)((h->nblk + WPB - 1) / WPB);
       if (dotvec != nullptr)
-        spmv_walk_kernel<I, true><<<grid, SPMV_WALK_THREADS, 0, st>>>(pos, crd, h->val, h->blk_row, abase, h->base, nnz_end,
-                                                                      h->nrows, h->nblk, SPMV_TILE, x, y, accumulate, h->carry,
-                                                                      dotvec, blk_partial, skip_flag);
+        launch_pdl(spmv_walk_kernel<I, true>, grid, SPMV_WALK_THREADS, 0, st, pos, crd, h->val, h->blk_row, abase, h->base, nnz_end,
+                   h->nrows, h->nblk, SPMV_TILE, x, y, accumulate, h->carry, dotvec, blk_partial, skip_flag);
       else
-        spmv_walk_kernel<I, false><<<grid, SPMV_WALK_THREADS, 0, st>>>(pos, crd, h->val, h->blk_row, abase, h->base, nnz_end,
-                                                                       h->nrows, h->nblk, SPMV_TILE, x, y, accumulate, h->carry,
-                                                                       nullptr, nullptr, skip_flag);
+        launch_pdl(spmv_walk_kernel<I, false>, grid, SPMV_WALK_THREADS, 0, st, pos, crd, h->val, h->blk_row, abase, h->base, nnz_end,
+                   h->nrows, h->nblk, SPMV_TILE, x, y, accumulate, h->carry, nullptr, nullptr, skip_flag);
     } else {
       // a small matrix: shorter ranges per warp (the handle's second plan), so that the warps fill the SMs evenly
       const unsigned grid = (unsigned)((h->walk_nblk + WPB - 1) / WPB);
-      spmv_walk_kernel<I, false><<<grid, SPMV_WALK_THREADS, 0, st>>>(pos, crd, h->val, h->walk_plan, abase, h->base, nnz_end,
-                                                                     h->nrows, h->walk_nblk, h->walk_tile, x, y, accumulate,
-                                                                     h->walk_carry, nullptr, nullptr, skip_flag);
+      launch_pdl(spmv_walk_kernel<I, false>, grid, SPMV_WALK_THREADS, 0, st, pos, crd, h->val, h->walk_plan, abase, h->base, nnz_end,
+                 h->nrows, h->walk_nblk, h->walk_tile, x, y, accumulate, h->walk_carry, nullptr, nullptr, skip_flag);
       LAPIS_CUDA_TRY(cudaGetLastError());
       return launch_fixup<I>(h, h->walk_plan, h->walk_carry, h->walk_nblk, h->walk_tile, y, skip_flag, st);
     }
@@ -1598,22 +1692,24 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
   int dev = 0;
   LAPIS_CUDA_TRY(cudaGetDevice(&dev));
 
-  // pos[0] and pos[nrows] define the nnz range addressed by this matrix.
-  int64_t ends[2] = {0, 0};
-  if (idx_bytes == 4) {
-    int32_t e32[2];
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(&e32[0], d_pos, 4, cudaMemcpyDeviceToHost, st));
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(&e32[1], static_cast<const int32_t *>(d_pos) + nrows, 4,
-                                   cudaMemcpyDeviceToHost, st));
-    LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
-    ends[0] = e32[0];
-    ends[1] = e32[1];
-  } else {
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(&ends[0], d_pos, 8, cudaMemcpyDeviceToHost, st));
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(&ends[1], static_cast<const int64_t *>(d_pos) + nrows, 8,
-                                   cudaMemcpyDeviceToHost, st));
+  // pos[0] and pos[nrows] define the nnz range addressed by this matrix; the longest row decides which SpMV kernels
+  // serve it
+  int64_t facts[3] = {0, 0, 0};
+  {
+    PoolBuf scratch;
+    LAPIS_TRY(scratch.alloc(sizeof(facts), st));
+    LAPIS_CUDA_TRY(cudaMemsetAsync(scratch.p, 0, sizeof(facts), st));
+    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nrows + 255) / 256, (int64_t)sm_count() * 8));
+    unsigned long long *d_facts = static_cast<unsigned long long *>(scratch.p);
+    if (idx_bytes == 4)
+      csr_facts_kernel<int32_t><<<g, 256, 0, st>>>(static_cast<const int32_t *>(d_pos), nrows, d_facts);
+    else
+      csr_facts_kernel<int64_t><<<g, 256, 0, st>>>(static_cast<const int64_t *>(d_pos), nrows, d_facts);
+    LAPIS_CUDA_TRY(cudaGetLastError());
+    LAPIS_CUDA_TRY(cudaMemcpyAsync(facts, scratch.p, sizeof(facts), cudaMemcpyDeviceToHost, st));
     LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
   }
+  const int64_t *ends = facts + 1;
   if (ends[1] < ends[0] || ends[0] < 0) return fail(LAPIS_EBADSHAPE, "csr_create: pos is not non-decreasing");
   const int64_t nnz = ends[1] - ends[0];
   if (nnz > 0 && (d_crd == nullptr || d_val == nullptr)) return fail(LAPIS_EBADARG, "csr_create: crd/val null");
@@ -1635,7 +1731,7 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
   h->blk_partial = nullptr;
   h->carry = nullptr;
   h->tuned_threads = h->tuned_minb = h->tuned_hint = 0;
-  h->max_row_len = -1;
+  h->max_row_len = facts[0];
   h->device = dev;
   h->walk_plan = nullptr;
   h->walk_carry = nullptr;
@@ -1649,19 +1745,19 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
     h->walk_tile = SPMV_WALK_FINE_TILE;
     h->walk_nblk = (ends[1] - (ends[0] & ~(int64_t)3) + h->walk_tile - 1) / h->walk_tile;
   }
-  cudaError_t e = cudaMalloc(&h->blk_row, (size_t)(nblk + 1) * sizeof(int64_t));
-  if (e == cudaSuccess) e = cudaMalloc(&h->blk_partial, (size_t)nblk * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&h->carry, (size_t)nblk * sizeof(double));
-  if (e == cudaSuccess && h->walk_nblk > 0) e = cudaMalloc(&h->walk_plan, (size_t)(h->walk_nblk + 1) * sizeof(int64_t));
-  if (e == cudaSuccess && h->walk_nblk > 0) e = cudaMalloc(&h->walk_carry, (size_t)h->walk_nblk * sizeof(double));
-  if (e != cudaSuccess) {
-    cudaFree(h->blk_row);
-    cudaFree(h->blk_partial);
-    cudaFree(h->carry);
-    cudaFree(h->walk_plan);
-    cudaFree(h->walk_carry);
+  // one allocation: plan, partial sums, carries, and the second plan with its carries
+  const size_t words = (size_t)(nblk + 1) + 2 * (size_t)nblk + (h->walk_nblk > 0 ? 2 * (size_t)h->walk_nblk + 1 : 0);
+  void *scratch = nullptr;
+  if (pool_alloc(&scratch, words * 8, st) != LAPIS_OK) {
     delete h;
-    return fail(LAPIS_ECUDA, "csr_create: cudaMalloc failed: %s", cudaGetErrorString(e));
+    return lapis_last_error();
+  }
+  h->blk_row = static_cast<int64_t *>(scratch);
+  h->blk_partial = reinterpret_cast<double *>(h->blk_row + nblk + 1);
+  h->carry = h->blk_partial + nblk;
+  if (h->walk_nblk > 0) {
+    h->walk_plan = reinterpret_cast<int64_t *>(h->carry + nblk);
+    h->walk_carry = reinterpret_cast<double *>(h->walk_plan + h->walk_nblk + 1);
   }
   const unsigned pgrid = (unsigned)((nblk + 1 + 255) / 256);
   if (idx_bytes == 4)
@@ -1677,13 +1773,9 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
       spmv_plan_kernel<int64_t><<<wgrid, 256, 0, st>>>(static_cast<const int64_t *>(d_pos), nrows, h->walk_nblk, h->walk_plan,
                                                        h->walk_tile);
   }
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
-    cudaFree(h->blk_row);
-    cudaFree(h->blk_partial);
-    cudaFree(h->carry);
-    cudaFree(h->walk_plan);
-    cudaFree(h->walk_carry);
+    pool_free(scratch, st);
     delete h;
     return fail(LAPIS_ECUDA, "csr_create: plan kernel launch failed: %s", cudaGetErrorString(e));
   }
@@ -1698,7 +1790,8 @@ extern "C" int lapis_b200_spmv_select_kernel(int threads, int blocks_per_sm, int
     return LAPIS_OK;
   }
   if (!spmv_variant_known(threads, blocks_per_sm)) return fail(LAPIS_EBADARG, "spmv_select_kernel: unknown kernel variant");
-  spmv_override() = SpmvVariant{threads, blocks_per_sm, l2_hint ? 1 : 0};
+  const bool shape = threads == 1 && l2_hint >= SHORT_ROW_PER_THREAD && l2_hint <= SHORT_32_ROWS;
+  spmv_override() = SpmvVariant{threads, blocks_per_sm, shape ? l2_hint : l2_hint ? 1 : 0};
   return LAPIS_OK;
 }
 
@@ -1710,28 +1803,15 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
   if (h == nullptr) return fail(LAPIS_EBADARG, "csr_tune: null matrix handle");
   if (h->nrows == 0 || h->nnz == 0) return LAPIS_OK;
   cudaStream_t st = as_stream(stream);
-  double *x = nullptr, *y = nullptr;
-  LAPIS_CUDA_TRY(cudaMalloc(&x, (size_t)(h->ncols > 0 ? h->ncols : 1) * 8));
-  cudaError_t e = cudaMalloc(&y, (size_t)h->nrows * 8);
-  if (e != cudaSuccess) {
-    cudaFree(x);
-    return fail(LAPIS_ECUDA, "csr_tune: cudaMalloc failed: %s", cudaGetErrorString(e));
-  }
+  PoolBuf bx, by;
+  LAPIS_TRY(bx.alloc((size_t)(h->ncols > 0 ? h->ncols : 1) * 8, st));
+  LAPIS_TRY(by.alloc((size_t)h->nrows * 8, st));
+  double *x = static_cast<double *>(bx.p), *y = static_cast<double *>(by.p);
   cudaMemsetAsync(x, 0, (size_t)(h->ncols > 0 ? h->ncols : 1) * 8, st);
-  if (h->max_row_len < 0) {  // the longest row decides whether the one-thread-per-row kernel is a candidate
-    unsigned long long *d_max = reinterpret_cast<unsigned long long *>(y), h_max = 0;
-    cudaMemsetAsync(d_max, 0, 8, st);
-    const unsigned g = (unsigned)std::min<int64_t>((h->nrows + 255) / 256, (int64_t)sm_count() * 8);
-    if (h->idx_bytes == 4)
-      max_row_len_kernel<int32_t><<<g, 256, 0, st>>>(static_cast<const int32_t *>(h->pos), h->nrows, d_max);
-    else
-      max_row_len_kernel<int64_t><<<g, 256, 0, st>>>(static_cast<const int64_t *>(h->pos), h->nrows, d_max);
-    if (cudaMemcpyAsync(&h_max, d_max, 8, cudaMemcpyDeviceToHost, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess)
-      h->max_row_len = (int64_t)h_max;
-  }
   const int pipe_blocks = h->idx_bytes == 4 ? 4 : 3;  // what fits in shared memory
-  const bool short_rows = h->max_row_len >= 0 && h->max_row_len <= SPMV_ROWTHREAD_MAX_LEN;
-  const SpmvVariant cand[] = {{256, 4, 1}, {256, 6, 1}, {512, 3, 1}, {-256, pipe_blocks, 1}, {1, 0, 1},
+  const bool short_rows = has_short_rows(h);
+  const SpmvVariant cand[] = {{256, 4, 1}, {256, 6, 1}, {512, 3, 1}, {-256, pipe_blocks, 1},
+                              {1, 0, SHORT_ROW_PER_THREAD}, {1, 0, SHORT_64_ROWS}, {1, 0, SHORT_32_ROWS},
                               {2, 5, 1}, {2, 5, 0}, {3, 4, 1}, {3, 4, 0}, {4, 0, 0}};
   const SpmvVariant saved = spmv_override();
   cudaEvent_t e0, e1;
@@ -1766,8 +1846,6 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
   spmv_override() = saved;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(x);
-  cudaFree(y);
   return status;
 }
 
@@ -1798,11 +1876,13 @@ extern "C" int lapis_b200_spmv_status(void *stream) {
 extern "C" int lapis_b200_csr_destroy(lapis_b200_csr_t h) {
   // does not touch the recorded status: it runs while an error of the enclosing call unwinds
   if (h == nullptr) return LAPIS_OK;
-  cudaFree(h->blk_row);
-  cudaFree(h->blk_partial);
-  cudaFree(h->carry);
-  cudaFree(h->walk_plan);
-  cudaFree(h->walk_carry);
+  int dev = -1;
+  cudaGetDevice(&dev);
+  if (dev != h->device) cudaSetDevice(h->device);
+  // launches on any stream may still use the scratch: wait for them, as cudaFree would
+  cudaDeviceSynchronize();
+  pool_free(h->blk_row, nullptr);
+  if (dev >= 0 && dev != h->device) cudaSetDevice(dev);
   delete h;
   return LAPIS_OK;
 }

@@ -14,9 +14,14 @@ import torch
 
 from ._lib import c_dbl, c_int, c_u64, c_vp, check, load
 
+try:
+    from . import _calls  # csrc/torch_calls.cpp; torch must be imported first
+except ImportError as exc:
+    raise ImportError("lapis_b200/_calls is missing: build it with `python -m lapis_b200._build`") from exc
+
 
 def _stream():
-    return c_vp(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t):
@@ -55,6 +60,7 @@ class CsrMatrix:
             check(self._lib.lapis_b200_csr_create(ctypes.byref(h), c_int(pos.element_size()), self.nrows, self.ncols,
                                                   _ptr(pos), _ptr(crd), _ptr(val), _stream()))
         self._h = h
+        self._addr = h.value
         self.nnz = int(self._lib.lapis_b200_csr_nnz(h))
         if tune:
             self.tune()
@@ -94,19 +100,22 @@ class CsrMatrix:
 
     def spmv(self, x: torch.Tensor, y: torch.Tensor, accumulate: bool = True) -> torch.Tensor:
         """y = (y if accumulate else 0) + A x, in place."""
-        _f64(x, "x"), _f64(y, "y")
-        if x.numel() != self.ncols or y.numel() != self.nrows:
-            raise ValueError("spmv: x/y length mismatch")
-        check(self._lib.lapis_b200_spmv_f64(self._h, _ptr(x), _ptr(y), c_int(1 if accumulate else 0), _stream()))
+        status = _calls.spmv(self._addr, self.nrows, self.ncols, x, y, accumulate)
+        if status:
+            if status < 0:
+                _f64(x, "x"), _f64(y, "y")
+                raise ValueError("spmv: x/y length mismatch")
+            check(status)
         return y
 
     def spmm(self, B: torch.Tensor, C: torch.Tensor, accumulate: bool = True) -> torch.Tensor:
         """C = (C if accumulate else 0) + A B, in place; B [ncols, k], C [nrows, k] row-major."""
-        _f64(B, "B"), _f64(C, "C")
-        if B.shape[0] != self.ncols or C.shape[0] != self.nrows or B.shape[1] != C.shape[1]:
-            raise ValueError("spmm: B/C shape mismatch")
-        check(self._lib.lapis_b200_spmm_f64(self._h, int(B.shape[1]), _ptr(B), _ptr(C), c_int(1 if accumulate else 0),
-                                            _stream()))
+        status = _calls.spmm(self._addr, self.nrows, self.ncols, B, C, accumulate)
+        if status:
+            if status < 0:
+                _f64(B, "B"), _f64(C, "C")
+                raise ValueError("spmm: B/C shape mismatch")
+            check(status)
         return C
 
     def pcg(self, b: torch.Tensor, dinv: torch.Tensor, tol: float, maxiter: int):
@@ -154,8 +163,10 @@ def bspmm_csrv(pos: torch.Tensor, crd: torch.Tensor, val: torch.Tensor, B: torch
         C = torch.empty((n1, dh, nh), dtype=torch.float32, device=B.device)
     elif tuple(C.shape) != (n1, dh, nh) or C.dtype != torch.float32 or not C.is_contiguous():
         raise ValueError("bspmm: C must be a contiguous float32 [n1, dh, nh] tensor")
-    check(load().lapis_b200_bspmm_csrv_f32(c_int(pos.element_size()), n1, n2, nh, dh, _ptr(pos), _ptr(crd), _ptr(val),
-                                           _ptr(B), _ptr(C), c_int(1 if accumulate else 0), _stream()))
+    status = _calls.bspmm(pos, crd, val, B, C, n2, accumulate)
+    if status < 0:
+        raise TypeError("bspmm: operands must be contiguous CUDA tensors")
+    check(status)
     return C
 
 
@@ -163,13 +174,16 @@ def spmm_dcsr(i1: torch.Tensor, p2: torch.Tensor, i2: torch.Tensor, val: torch.T
               ncols: int) -> torch.Tensor:
     """C[i1[r], :] += sum_j val[j] * B[i2[j], :] for the stored rows r of a DCSR matrix
     (examples/spmm_dcsr_opdsl.py:59-101 in the LAPIS project), in place; ``i1`` must ascend (a row number may repeat)."""
-    if not (i1.dtype == p2.dtype == i2.dtype) or p2.dtype not in (torch.int32, torch.int64):
-        raise TypeError("i1/p2/i2 must all be int32 or all int64")
-    _f64(val, "val"), _f64(B, "B"), _f64(C, "C")
-    if B.dim() != 2 or C.dim() != 2 or B.shape[0] != ncols or B.shape[1] != C.shape[1] or p2.numel() != i1.numel() + 1:
-        raise ValueError("spmm_dcsr: shape mismatch")
-    check(load().lapis_b200_spmm_dcsr_f64(c_int(p2.element_size()), int(C.shape[0]), ncols, i1.numel(), int(B.shape[1]),
-                                          _ptr(i1), _ptr(p2), _ptr(i2), _ptr(val), _ptr(B), _ptr(C), _stream()))
+    status = _calls.spmm_dcsr(i1, p2, i2, val, B, C, ncols)
+    if status:
+        if status < 0:
+            if not (i1.dtype == p2.dtype == i2.dtype) or p2.dtype not in (torch.int32, torch.int64):
+                raise TypeError("i1/p2/i2 must all be int32 or all int64")
+            _f64(val, "val"), _f64(B, "B"), _f64(C, "C")
+            if not all(t.is_cuda and t.is_contiguous() for t in (i1, p2, i2)):
+                raise TypeError("i1/p2/i2 must be contiguous CUDA tensors")
+            raise ValueError("spmm_dcsr: shape mismatch")
+        check(status)
     return C
 
 
@@ -185,21 +199,16 @@ def normalize_mom2(mom1: torch.Tensor, mom2: torch.Tensor) -> torch.Tensor:
 
 def bgemm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
     """C = C + A @ B in place; fp32, [M,K]x[K,N] or batched [b,M,K]x[b,K,N]."""
-    for t in (A, B, C):
-        if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
-            raise TypeError("bgemm operands must be contiguous float32 CUDA tensors")
-    if A.dim() == 2:
-        batch, (M, K), (K2, N) = 1, A.shape, B.shape
-    else:
-        batch, M, K = A.shape
-        b2, K2, N = B.shape
-        if b2 != batch:
-            raise ValueError("mismatching contracting dimension")
-    if K != K2:
-        raise ValueError("mismatching contracting dimension")
-    if tuple(C.shape) != (tuple(A.shape[:-1]) + (N,)):
-        raise ValueError("bgemm: output shape mismatch")
-    check(load().lapis_b200_bgemm_f32(batch, M, N, K, _ptr(A), _ptr(B), _ptr(C), _stream()))
+    status = _calls.bgemm(A, B, C)
+    if status:
+        if status < 0:
+            for t in (A, B, C):
+                if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
+                    raise TypeError("bgemm operands must be contiguous float32 CUDA tensors")
+            if A.dim() != B.dim() or A.shape[-1] != B.shape[-2] or A.shape[:-2] != B.shape[:-2]:
+                raise ValueError("mismatching contracting dimension")
+            raise ValueError("bgemm: output shape mismatch")
+        check(status)
     return C
 
 
