@@ -25,6 +25,7 @@ from __future__ import annotations
 import ctypes
 import os
 import re
+import struct
 
 import numpy as np
 
@@ -233,8 +234,27 @@ def _classify(fn: dict, all_funcs: dict, module_text: str = ""):
 # ---------------------------------------------------------------------------
 # The module object returned by compile()
 # ---------------------------------------------------------------------------
+_MEMREF = {rank: struct.Struct("PPq%dq" % (2 * rank)) for rank in (1, 2, 3)}
+_CSR_SPEC = struct.Struct("5q")
+
+
 def _desc(arr):
-    return ctypes.pointer(rt.get_ranked_memref_descriptor(arr))
+    """The memref descriptor of a C-contiguous array as bytes (passed by address; ``arr`` must stay alive)."""
+    address, shape = arr.__array_interface__["data"][0], arr.shape
+    if len(shape) == 1:
+        return _MEMREF[1].pack(address, address, 0, shape[0], 1)
+    if len(shape) == 2:
+        return _MEMREF[2].pack(address, address, 0, shape[0], shape[1], shape[1], 1)
+    return _MEMREF[3].pack(address, address, 0, *shape, shape[1] * shape[2], shape[2], 1)
+
+
+def _c_array(a, dtype, rank):
+    """``a`` as a C-contiguous numpy array of ``dtype`` and the rank the function was compiled for."""
+    if type(a) is not np.ndarray or a.dtype != dtype or not a.flags.c_contiguous:
+        a = np.require(a, dtype=dtype, requirements=["C"])
+    if a.ndim != rank:
+        raise ValueError(f"expected an array of rank {rank}, got rank {a.ndim}")
+    return a
 
 
 def _ret_slot(rank):
@@ -252,7 +272,10 @@ def _flatten_spec(spec):
 
 def _resident(*args) -> bool:
     from .dualview import DualView
-    return any(isinstance(a, DualView) for a in args)
+    for a in args:
+        if isinstance(a, DualView):
+            return True
+    return False
 
 
 class LAPISModule:
@@ -438,11 +461,9 @@ class LAPISModule:
         symbol = "py_" + _shim.export_name(name)  # the emitter's export name, from the module's own library
 
         def csr_args(pos, crd, val, spec):
-            pos = np.require(pos, dtype=idx_dtype, requirements=["C"])
-            crd = np.require(crd, dtype=idx_dtype, requirements=["C"])
-            val = np.require(val, dtype=np.float64, requirements=["C"])
-            flat = _flatten_spec(spec)
-            return (pos, crd, val, flat), (_desc(pos), _desc(crd), _desc(val), flat.ctypes.data_as(ctypes.c_void_p))
+            pos, crd, val = _c_array(pos, idx_dtype, 1), _c_array(crd, idx_dtype, 1), _c_array(val, np.float64, 1)
+            (rows, cols), (npos, ncrd, nval) = spec
+            return (pos, crd, val), (_desc(pos), _desc(crd), _desc(val), _CSR_SPEC.pack(rows, cols, npos, ncrd, nval))
 
         if kind == "spmv":
             fn = getattr(lib, symbol)
@@ -466,10 +487,8 @@ class LAPISModule:
                     y.modifyDevice()
                     return y
                 keep, cargs = csr_args(pos, crd, val, spec)
-                x = np.require(x, dtype=np.float64, requirements=["C"])
-                y = np.require(y, dtype=np.float64, requirements=["C"])
-                ret0 = _ret_slot(1)
-                fn(ret0, *cargs, _desc(x), _desc(y))
+                x, y = _c_array(x, np.float64, 1), _c_array(y, np.float64, 1)
+                fn(None, *cargs, _desc(x), _desc(y))  # no result slot: the result is the caller's y
                 check_last()
                 del keep
                 return y  # the function returns its outs argument
@@ -492,10 +511,8 @@ class LAPISModule:
                     C.modifyDevice()
                     return C
                 keep, cargs = csr_args(pos, crd, val, spec)
-                B = np.require(B, dtype=np.float64, requirements=["C"])
-                C = np.require(C, dtype=np.float64, requirements=["C"])
-                ret0 = _ret_slot(2)
-                fn(ret0, *cargs, _desc(B), _desc(C))
+                B, C = _c_array(B, np.float64, 2), _c_array(C, np.float64, 2)
+                fn(None, *cargs, _desc(B), _desc(C))
                 check_last()
                 del keep
                 return C
@@ -512,11 +529,8 @@ class LAPISModule:
                     D.bgemm(A.device_view(), B.device_view(), C.device_view())
                     C.modifyDevice()
                     return C
-                A = np.require(A, dtype=np.float32, requirements=["C"])
-                B = np.require(B, dtype=np.float32, requirements=["C"])
-                C = np.require(C, dtype=np.float32, requirements=["C"])
-                ret0 = _ret_slot(rank)
-                fn(ret0, _desc(A), _desc(B), _desc(C))
+                A, B, C = (_c_array(t, np.float32, rank) for t in (A, B, C))
+                fn(None, _desc(A), _desc(B), _desc(C))
                 check_last()
                 return C
 
@@ -532,8 +546,7 @@ class LAPISModule:
                     x, iters, relres = A.pcg(b.device_view(), dinv.device_view(), float(tol), int(maxiter))
                     return DualView.from_device(x), iters, relres
                 keep, cargs = csr_args(pos, crd, val, spec)
-                b = np.require(b, dtype=np.float64, requirements=["C"])
-                dinv = np.require(dinv, dtype=np.float64, requirements=["C"])
+                b, dinv = _c_array(b, np.float64, 1), _c_array(dinv, np.float64, 1)
                 ret0 = _ret_slot(1)
                 ret1 = ctypes.c_size_t(0)
                 ret2 = ctypes.c_double(0.0)
@@ -586,10 +599,8 @@ class LAPISModule:
                     C = D.bspmm_csrv(pos.device_view(), crd.device_view(), val.device_view(), B.device_view(),
                                      int(flat[1]), None)
                     return DualView.from_device(C)
-                pos = np.require(pos, dtype=idx_dtype, requirements=["C"])
-                crd = np.require(crd, dtype=idx_dtype, requirements=["C"])
-                val = np.require(val, dtype=np.float32, requirements=["C"])
-                B = np.require(B, dtype=np.float32, requirements=["C"])
+                pos, crd, val = _c_array(pos, idx_dtype, 1), _c_array(crd, idx_dtype, 1), _c_array(val, np.float32, 1)
+                B = _c_array(B, np.float32, 3)
                 ret0 = _ret_slot(3)
                 fn(ret0, _desc(pos), _desc(crd), _desc(val), flat.ctypes.data_as(ctypes.c_void_p), _desc(B))
                 check_last()
@@ -613,12 +624,9 @@ class LAPISModule:
                                 B.device_view(), C.device_view(), int(flat[1]))
                     C.modifyDevice()
                     return C
-                arrs = [np.require(t, dtype=idx_dtype, requirements=["C"]) for t in (p1, i1, p2, i2)]
-                val = np.require(val, dtype=np.float64, requirements=["C"])
-                B = np.require(B, dtype=np.float64, requirements=["C"])
-                C = np.require(C, dtype=np.float64, requirements=["C"])
-                ret0 = _ret_slot(2)
-                fn(ret0, *[_desc(t) for t in arrs], _desc(val), flat.ctypes.data_as(ctypes.c_void_p), _desc(B), _desc(C))
+                arrs = [_c_array(t, idx_dtype, 1) for t in (p1, i1, p2, i2)]
+                val, B, C = _c_array(val, np.float64, 1), _c_array(B, np.float64, 2), _c_array(C, np.float64, 2)
+                fn(None, *[_desc(t) for t in arrs], _desc(val), flat.ctypes.data_as(ctypes.c_void_p), _desc(B), _desc(C))
                 check_last()
                 return C
 
@@ -634,8 +642,7 @@ class LAPISModule:
                     m1, m2 = A.mht(mask.device_view(), d.device_view(), float(alpha), float(tol), int(maxiter))
                     return DualView.from_device(m1), DualView.from_device(m2)
                 keep, cargs = csr_args(pos, crd, val, spec)
-                mask = np.require(mask, dtype=np.float64, requirements=["C"])
-                d = np.require(d, dtype=np.float64, requirements=["C"])
+                mask, d = _c_array(mask, np.float64, 1), _c_array(d, np.float64, 1)
                 ret0, ret1 = _ret_slot(1), _ret_slot(1)
                 fn(ret0, ret1, *cargs, _desc(mask), _desc(d), ctypes.c_double(alpha), ctypes.c_double(tol),
                    ctypes.c_size_t(maxiter))
@@ -653,8 +660,7 @@ class LAPISModule:
                     from .dualview import DualView
                     mom1, mom2 = self._dv(mom1, np.float64), self._dv(mom2, np.float64)
                     return DualView.from_device(D.normalize_mom2(mom1.device_view(), mom2.device_view()))
-                mom1 = np.require(mom1, dtype=np.float64, requirements=["C"])
-                mom2 = np.require(mom2, dtype=np.float64, requirements=["C"])
+                mom1, mom2 = _c_array(mom1, np.float64, 1), _c_array(mom2, np.float64, 1)
                 ret0 = _ret_slot(1)
                 fn(ret0, _desc(mom1), _desc(mom2))
                 check_last()

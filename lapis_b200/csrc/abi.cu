@@ -5,7 +5,7 @@
 // `ret` slots, device work fenced before returning.  Where the emitted wrapper
 // wraps host pointers in unmanaged Kokkos views and lets LAPIS::DualView copy them
 // to the device (LAPISSupport.hpp:193-282), this file stages the operands in device
-// buffers with cudaMemcpyAsync, runs the kernels and copies the result back.
+// buffers (stage.h), runs the kernels and copies the result back.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "common.h"
+#include "stage.h"
 
 extern "C" int64_t lapis_b200_pcg_workspace_bytes(int64_t n, int64_t n_p);
 
@@ -98,20 +99,6 @@ void pool_trim() {
 // ---- module state -----------------------------------------------------------
 static int g_init_count = 0;
 static std::vector<void *> g_alive_host;  // result buffers handed to the caller (LAPISSupport.hpp:93-120)
-
-// Scoped device buffer.
-struct DevBuf {
-  void *p = nullptr;
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
-  int alloc(size_t bytes) {
-    if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) return fail(LAPIS_ECUDA, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
-    return LAPIS_OK;
-  }
-};
 
 static int require_init() {
   if (g_init_count <= 0) return fail(LAPIS_ENOTINIT, "lapis_initialize has not been called");
@@ -206,35 +193,79 @@ static int check_crd_host(const I *crd, int64_t nnz, int64_t ncols) {
   return LAPIS_OK;
 }
 
-// Uploads a CSR matrix and builds its handle.
-struct DeviceCsr {
-  DevBuf pos, crd, val;
-  lapis_b200_csr_t h = nullptr;
-  ~DeviceCsr() { lapis_b200_csr_destroy(h); }
+// A result vector owned by the module until lapis_finalize (LAPISSupport.hpp:93-120), filled from the device.
+static int result_vector(const void *d_src, int64_t n, lapis_memref1 *out, cudaStream_t st) {
+  double *hx = static_cast<double *>(std::malloc(n > 0 ? (size_t)n * 8 : 8));
+  if (hx == nullptr) return fail(LAPIS_ECUDA, "host allocation failed");
+  g_alive_host.push_back(hx);
+  LAPIS_TRY(stage_download(hx, d_src, (size_t)n * 8, st));
+  out->basePtr = hx;
+  out->data = hx;
+  out->offset = 0;
+  out->sizes[0] = n;
+  out->strides[0] = 1;
+  return LAPIS_OK;
+}
+
+// Operands of a call: laid out in one device allocation and sent there.  A failure leaves nothing in flight that still
+// reads the caller's arrays.
+struct Operands {
+  Upload up;
+  PoolBuf dev;
+  int send(cudaStream_t st, Upload::Facts *facts, size_t extra = 0) {
+    const size_t bytes = up.layout();
+    extra_at = bytes;
+    LAPIS_TRY(dev.alloc(bytes + extra, st));
+    const int rc = up.run(dev.p, st, facts);
+    if (rc != LAPIS_OK) cudaStreamSynchronize(st);
+    return rc;
+  }
+  template <typename T>
+  T *at(int part) const {
+    return up.at<T>(dev.p, part);
+  }
+  template <typename T>
+  T *extra(size_t offset = 0) const {
+    return reinterpret_cast<T *>(static_cast<char *>(dev.p) + extra_at + offset);
+  }
+  size_t extra_at = 0;
 };
 
+// What the upload found out about the index arrays, as a status.
 template <typename I>
-static int upload_csr(const lapis_memref1 *pos, const lapis_memref1 *crd, const lapis_memref1 *val, const CsrArgs &a,
-                      DeviceCsr *d, cudaStream_t st) {
-  const I *hpos = elem_ptr<I>(pos);
-  LAPIS_TRY(d->pos.alloc((size_t)a.npos * sizeof(I)));
-  LAPIS_TRY(d->crd.alloc((size_t)a.nnz * sizeof(I)));
-  LAPIS_TRY(d->val.alloc((size_t)a.nnz * sizeof(double)));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(d->pos.p, hpos, (size_t)a.npos * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(d->crd.p, elem_ptr<I>(crd), (size_t)a.nnz * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(d->val.p, elem_ptr<double>(val), (size_t)a.nnz * sizeof(double), cudaMemcpyHostToDevice, st));
-  // validated on the host while the copies are in flight (they are asynchronous from pinned memory);
-  // no kernel has been given the offsets yet
-  if (check_pos_host<I>(hpos, a.nrows, a.nnz) != LAPIS_OK || check_crd_host<I>(elem_ptr<I>(crd), a.nnz, a.ncols) != LAPIS_OK) {
-    const int code = lapis_last_error();
-    char msg[512];
-    snprintf(msg, sizeof(msg), "%s", lapis_last_error_message());
-    cudaStreamSynchronize(st);
-    return fail(code, "%s", msg);
-  }
-  return lapis_b200_csr_create(&d->h, (int)sizeof(I), a.nrows, a.ncols, d->pos.p, d->crd.p,
-                               static_cast<const double *>(d->val.p), st);
+static int check_facts(const Upload::Facts &f, const I *pos, const I *crd, int64_t nrows, int64_t nnz, int64_t ncols, cudaStream_t st) {
+  int rc = LAPIS_OK;
+  if (pos[0] != 0)
+    rc = fail(LAPIS_EBADSHAPE, "pos[0] must be 0");
+  else if (f.bad_row >= 0)
+    rc = fail(LAPIS_EBADSHAPE, "pos is not non-decreasing at row %lld", (long long)f.bad_row);
+  else if ((int64_t)pos[nrows] != nnz)
+    rc = fail(LAPIS_EBADSHAPE, "pos[rows] != number of stored entries");
+  else if (!f.crd_in_range)
+    rc = check_crd_host<I>(crd, nnz, ncols);  // finds the values for the message
+  if (rc != LAPIS_OK) cudaStreamSynchronize(st);
+  return rc;
 }
+
+// A CSR operand of a call: its three arrays among the uploaded parts, and the handle over them.
+struct CsrOperand {
+  int pos = 0, crd = 0, val = 0;
+  lapis_b200_csr h;
+  PoolBuf scratch;
+  template <typename I>
+  void add(Upload &up, const lapis_memref1 *mpos, const lapis_memref1 *mcrd, const lapis_memref1 *mval, const CsrArgs &a) {
+    pos = up.add_pos(elem_ptr<I>(mpos), a.npos);
+    crd = up.add_crd(elem_ptr<I>(mcrd), a.nnz, a.ncols);
+    val = up.add(elem_ptr<double>(mval), (size_t)a.nnz * 8);
+  }
+  template <typename I>
+  int setup(const Operands &ops, const Upload::Facts &f, const lapis_memref1 *mpos, const lapis_memref1 *mcrd, const CsrArgs &a,
+            bool plan_on_demand, cudaStream_t st) {
+    LAPIS_TRY((check_facts<I>(f, elem_ptr<I>(mpos), elem_ptr<I>(mcrd), a.nrows, a.nnz, a.ncols, st)));
+    return csr_setup(&h, (int)sizeof(I), a.nrows, a.ncols, 0, a.nnz, f.max_row_len, ops.at<void>(pos), ops.at<void>(crd),
+                     ops.at<double>(val), plan_on_demand, &scratch, st);
+  }
+};
 
 template <typename I>
 static int spmv_host(lapis_memref1 **ret0, lapis_memref1 *pos, lapis_memref1 *crd, lapis_memref1 *val,
@@ -247,16 +278,15 @@ static int spmv_host(lapis_memref1 **ret0, lapis_memref1 *pos, lapis_memref1 *cr
   LAPIS_TRY((check_contig<lapis_memref1, 1>(y, "y")));
   if (x->sizes[0] != a.ncols || y->sizes[0] != a.nrows) return fail(LAPIS_EBADSHAPE, "spmv: x/y length mismatch");
   cudaStream_t st = nullptr;
-  DeviceCsr d;
-  LAPIS_TRY(upload_csr<I>(pos, crd, val, a, &d, st));
-  DevBuf dx, dy;
-  LAPIS_TRY(dx.alloc((size_t)a.ncols * 8));
-  LAPIS_TRY(dy.alloc((size_t)a.nrows * 8));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dx.p, elem_ptr<double>(x), (size_t)a.ncols * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dy.p, elem_ptr<double>(y), (size_t)a.nrows * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_spmv_f64(d.h, static_cast<const double *>(dx.p), static_cast<double *>(dy.p), 1, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(elem_ptr<double>(y), dy.p, (size_t)a.nrows * 8, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));  // results host-visible on return (emitted fence, :2682)
+  Operands ops;
+  CsrOperand A;
+  A.add<I>(ops.up, pos, crd, val, a);
+  const int px = ops.up.add(elem_ptr<double>(x), (size_t)a.ncols * 8), py = ops.up.add(elem_ptr<double>(y), (size_t)a.nrows * 8);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts));
+  LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, true, st));
+  LAPIS_TRY(lapis_b200_spmv_f64(&A.h, ops.at<double>(px), ops.at<double>(py), 1, st));
+  LAPIS_TRY(stage_download(elem_ptr<double>(y), ops.at<double>(py), (size_t)a.nrows * 8, st));  // emitted fence, :2682
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *y;  // the function returns its outs argument
   return LAPIS_OK;
 }
@@ -274,37 +304,30 @@ static int spmm_host(lapis_memref2 **ret0, lapis_memref1 *pos, lapis_memref1 *cr
   if (B->sizes[0] != a.ncols || C->sizes[0] != a.nrows || C->sizes[1] != k)
     return fail(LAPIS_EBADSHAPE, "spmm: B/C shape mismatch");
   cudaStream_t st = nullptr;
-  DeviceCsr d;
-  LAPIS_TRY(upload_csr<I>(pos, crd, val, a, &d, st));
-  DevBuf dB, dC;
-  const size_t bB = (size_t)a.ncols * k * 8, bC = (size_t)a.nrows * k * 8;
-  LAPIS_TRY(dB.alloc(bB));
-  LAPIS_TRY(dC.alloc(bC));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dB.p, elem_ptr<double>(B), bB, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dC.p, elem_ptr<double>(C), bC, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_spmm_f64(d.h, k, static_cast<const double *>(dB.p), static_cast<double *>(dC.p), 1, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(elem_ptr<double>(C), dC.p, bC, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  Operands ops;
+  CsrOperand A;
+  A.add<I>(ops.up, pos, crd, val, a);
+  const size_t bC = (size_t)a.nrows * k * 8;
+  const int pB = ops.up.add(elem_ptr<double>(B), (size_t)a.ncols * k * 8), pC = ops.up.add(elem_ptr<double>(C), bC);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts));
+  LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, true, st));
+  LAPIS_TRY(lapis_b200_spmm_f64(&A.h, k, ops.at<double>(pB), ops.at<double>(pC), 1, st));
+  LAPIS_TRY(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st));
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *C;
   return LAPIS_OK;
 }
 
 static int gemm_host(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C) {
   cudaStream_t st = nullptr;
-  DevBuf dA, dB, dC;
-  const size_t bA = (size_t)batch * M * K * 4, bB = (size_t)batch * K * N * 4, bC = (size_t)batch * M * N * 4;
-  LAPIS_TRY(dA.alloc(bA));
-  LAPIS_TRY(dB.alloc(bB));
-  LAPIS_TRY(dC.alloc(bC));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dA.p, A, bA, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dB.p, B, bB, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dC.p, C, bC, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_bgemm_f32(batch, M, N, K, static_cast<const float *>(dA.p), static_cast<const float *>(dB.p),
-                                 static_cast<float *>(dC.p), st));
+  Operands ops;
+  const size_t bC = (size_t)batch * M * N * 4;
+  const int pA = ops.up.add(A, (size_t)batch * M * K * 4), pB = ops.up.add(B, (size_t)batch * K * N * 4), pC = ops.up.add(C, bC);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts));
+  LAPIS_TRY(lapis_b200_bgemm_f32(batch, M, N, K, ops.at<float>(pA), ops.at<float>(pB), ops.at<float>(pC), st));
   LAPIS_TRY(lapis_b200_bgemm_status(st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(C, dC.p, bC, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
-  return LAPIS_OK;
+  return stage_download(C, ops.at<float>(pC), bC, st);
 }
 
 template <typename I>
@@ -321,47 +344,20 @@ static int pcg_host(lapis_memref1 **ret0, size_t *ret1, double *ret2, lapis_memr
   if (a.nrows != n || a.ncols != n || dinv->sizes[0] != n) return fail(LAPIS_EBADSHAPE, "pcg: A, b, dinv sizes differ");
   if (ret0 == nullptr || *ret0 == nullptr) return fail(LAPIS_EBADARG, "pcg: null result slot");
   cudaStream_t st = nullptr;
-  DeviceCsr d;
-  LAPIS_TRY(upload_csr<I>(pos, crd, val, a, &d, st));
-  DevBuf db, ddinv, dx;
-  LAPIS_TRY(db.alloc((size_t)n * 8));
-  LAPIS_TRY(ddinv.alloc((size_t)n * 8));
-  LAPIS_TRY(dx.alloc((size_t)n * 8));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(db.p, elem_ptr<double>(b), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(ddinv.p, elem_ptr<double>(dinv), (size_t)n * 8, cudaMemcpyHostToDevice, st));
+  Operands ops;
+  CsrOperand A;
+  A.add<I>(ops.up, pos, crd, val, a);
+  const int pb = ops.up.add(elem_ptr<double>(b), (size_t)n * 8), pd = ops.up.add(elem_ptr<double>(dinv), (size_t)n * 8);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts, (size_t)n * 8));
+  LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, false, st));
+  double *dx = ops.extra<double>();
   uint64_t iters = 0;
   double relres = 0.0;
-  LAPIS_TRY(lapis_b200_pcg_f64(d.h, static_cast<const double *>(db.p), static_cast<const double *>(ddinv.p), tol,
-                               (uint64_t)maxiter, static_cast<double *>(dx.p), &iters, &relres, st));
-  // x is a new tensor of the module: owned here until lapis_finalize (LAPISSupport.hpp:93-120).
-  double *hx = static_cast<double *>(std::malloc(n > 0 ? (size_t)n * 8 : 8));
-  if (hx == nullptr) return fail(LAPIS_ECUDA, "pcg: host allocation failed");
-  g_alive_host.push_back(hx);
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(hx, dx.p, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
-  lapis_memref1 out;
-  out.basePtr = hx;
-  out.data = hx;
-  out.offset = 0;
-  out.sizes[0] = n;
-  out.strides[0] = 1;
-  **ret0 = out;
+  LAPIS_TRY(lapis_b200_pcg_f64(&A.h, ops.at<double>(pb), ops.at<double>(pd), tol, (uint64_t)maxiter, dx, &iters, &relres, st));
+  LAPIS_TRY(result_vector(dx, n, *ret0, st));
   if (ret1) *ret1 = (size_t)iters;
   if (ret2) *ret2 = relres;
-  return LAPIS_OK;
-}
-
-// A result vector owned by the module until lapis_finalize (LAPISSupport.hpp:93-120), filled from the device.
-static int result_vector(const void *d_src, int64_t n, lapis_memref1 *out, cudaStream_t st) {
-  double *hx = static_cast<double *>(std::malloc(n > 0 ? (size_t)n * 8 : 8));
-  if (hx == nullptr) return fail(LAPIS_ECUDA, "host allocation failed");
-  g_alive_host.push_back(hx);
-  if (n > 0) LAPIS_CUDA_TRY(cudaMemcpyAsync(hx, d_src, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
-  out->basePtr = hx;
-  out->data = hx;
-  out->offset = 0;
-  out->sizes[0] = n;
-  out->strides[0] = 1;
   return LAPIS_OK;
 }
 
@@ -381,22 +377,17 @@ static int mht_host(lapis_memref1 **ret0, lapis_memref1 **ret1, lapis_memref1 *p
   if (ret0 == nullptr || *ret0 == nullptr || ret1 == nullptr || *ret1 == nullptr)
     return fail(LAPIS_EBADARG, "mht: null result slot");
   cudaStream_t st = nullptr;
-  DeviceCsr d;
-  LAPIS_TRY(upload_csr<I>(pos, crd, val, a, &d, st));
-  DevBuf dmask, dd, dm1, dm2;
-  LAPIS_TRY(dmask.alloc((size_t)n * 8));
-  LAPIS_TRY(dd.alloc((size_t)n * 8));
-  LAPIS_TRY(dm1.alloc((size_t)n * 8));
-  LAPIS_TRY(dm2.alloc((size_t)n * 8));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dmask.p, elem_ptr<double>(mask), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dd.p, elem_ptr<double>(dvec), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_mht_f64(d.h, static_cast<const double *>(dmask.p), static_cast<const double *>(dd.p), alpha, tol,
-                               (uint64_t)maxiter, static_cast<double *>(dm1.p), static_cast<double *>(dm2.p), nullptr,
-                               nullptr, st));
-  LAPIS_TRY(result_vector(dm1.p, n, *ret0, st));
-  LAPIS_TRY(result_vector(dm2.p, n, *ret1, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
-  return LAPIS_OK;
+  Operands ops;
+  CsrOperand A;
+  A.add<I>(ops.up, pos, crd, val, a);
+  const int pm = ops.up.add(elem_ptr<double>(mask), (size_t)n * 8), pd = ops.up.add(elem_ptr<double>(dvec), (size_t)n * 8);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts, 2 * (size_t)n * 8));
+  LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, false, st));
+  double *m1 = ops.extra<double>(), *m2 = m1 + n;
+  LAPIS_TRY(lapis_b200_mht_f64(&A.h, ops.at<double>(pm), ops.at<double>(pd), alpha, tol, (uint64_t)maxiter, m1, m2, nullptr, nullptr, st));
+  LAPIS_TRY(result_vector(m1, n, *ret0, st));
+  return result_vector(m2, n, *ret1, st);
 }
 
 // examples/hitting_times.py:196-218 (@normalize_mom2), call at :218
@@ -409,19 +400,12 @@ static int normalize_mom2_host(lapis_memref1 **ret0, lapis_memref1 *mom1, lapis_
   if (mom2->sizes[0] != n) return fail(LAPIS_EBADSHAPE, "normalize_mom2: lengths differ");
   if (ret0 == nullptr || *ret0 == nullptr) return fail(LAPIS_EBADARG, "normalize_mom2: null result slot");
   cudaStream_t st = nullptr;
-  DevBuf d1, d2, dout;
-  LAPIS_TRY(d1.alloc((size_t)n * 8));
-  LAPIS_TRY(d2.alloc((size_t)n * 8));
-  LAPIS_TRY(dout.alloc((size_t)n * 8));
-  if (n > 0) {
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(d1.p, elem_ptr<double>(mom1), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-    LAPIS_CUDA_TRY(cudaMemcpyAsync(d2.p, elem_ptr<double>(mom2), (size_t)n * 8, cudaMemcpyHostToDevice, st));
-  }
-  LAPIS_TRY(lapis_b200_normalize_mom2_f64(n, static_cast<const double *>(d1.p), static_cast<const double *>(d2.p),
-                                          static_cast<double *>(dout.p), st));
-  LAPIS_TRY(result_vector(dout.p, n, *ret0, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
-  return LAPIS_OK;
+  Operands ops;
+  const int p1 = ops.up.add(elem_ptr<double>(mom1), (size_t)n * 8), p2 = ops.up.add(elem_ptr<double>(mom2), (size_t)n * 8);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts, (size_t)n * 8));
+  LAPIS_TRY(lapis_b200_normalize_mom2_f64(n, ops.at<double>(p1), ops.at<double>(p2), ops.extra<double>(), st));
+  return result_vector(ops.extra<double>(), n, *ret0, st);
 }
 
 // examples/bspmm.py:26-52, call at :103
@@ -444,30 +428,21 @@ static int bspmm_host(lapis_memref3 **ret0, lapis_memref1 *pos, lapis_memref1 *c
     return fail(LAPIS_EBADSHAPE, "crd/val shorter than the specifier says");
   if (B->sizes[0] != n2 || B->sizes[2] != nh) return fail(LAPIS_EBADSHAPE, "bspmm: B must be [n2, dh, nh]");
   const int64_t dh = B->sizes[1];
-  const I *hpos = elem_ptr<I>(pos);
-  LAPIS_TRY(check_pos_host<I>(hpos, n1, nnz));
-  const I *hcrd = elem_ptr<I>(crd);
-  for (int64_t j = 0; j < nnz; ++j)
-    if (hcrd[j] < 0 || (int64_t)hcrd[j] >= n2) return fail(LAPIS_EBADSHAPE, "bspmm: column index out of range at entry %lld", (long long)j);
+  const I *hpos = elem_ptr<I>(pos), *hcrd = elem_ptr<I>(crd);
   cudaStream_t st = nullptr;
-  DevBuf dpos, dcrd, dval, dB, dC;
-  const size_t bB = (size_t)n2 * dh * nh * 4, bC = (size_t)n1 * dh * nh * 4;
-  LAPIS_TRY(dpos.alloc((size_t)npos * sizeof(I)));
-  LAPIS_TRY(dcrd.alloc((size_t)nnz * sizeof(I)));
-  LAPIS_TRY(dval.alloc((size_t)nval * 4));
-  LAPIS_TRY(dB.alloc(bB));
-  LAPIS_TRY(dC.alloc(bC));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dpos.p, hpos, (size_t)npos * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dcrd.p, hcrd, (size_t)nnz * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dval.p, elem_ptr<float>(val), (size_t)nval * 4, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dB.p, elem_ptr<float>(B), bB, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_bspmm_csrv_f32((int)sizeof(I), n1, n2, nh, dh, dpos.p, dcrd.p, static_cast<const float *>(dval.p),
-                                      static_cast<const float *>(dB.p), static_cast<float *>(dC.p), 0, st));
+  Operands ops;
+  const size_t bC = (size_t)n1 * dh * nh * 4;
+  const int ppos = ops.up.add_pos(hpos, npos), pcrd = ops.up.add_crd(hcrd, nnz, n2);
+  const int pval = ops.up.add(elem_ptr<float>(val), (size_t)nval * 4), pB = ops.up.add(elem_ptr<float>(B), (size_t)n2 * dh * nh * 4);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts, bC));
+  LAPIS_TRY(check_facts<I>(facts, hpos, hcrd, n1, nnz, n2, st));
+  LAPIS_TRY(lapis_b200_bspmm_csrv_f32((int)sizeof(I), n1, n2, nh, dh, ops.at<void>(ppos), ops.at<void>(pcrd), ops.at<float>(pval),
+                                      ops.at<float>(pB), ops.extra<float>(), 0, st));
   float *hc = static_cast<float *>(std::malloc(bC > 0 ? bC : 8));
   if (hc == nullptr) return fail(LAPIS_ECUDA, "bspmm: host allocation failed");
   g_alive_host.push_back(hc);
-  if (bC > 0) LAPIS_CUDA_TRY(cudaMemcpyAsync(hc, dC.p, bC, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  LAPIS_TRY(stage_download(hc, ops.extra<float>(), bC, st));
   lapis_memref3 out;
   out.basePtr = hc;
   out.data = hc;
@@ -506,32 +481,21 @@ static int spmm_dcsr_host(lapis_memref2 **ret0, lapis_memref1 *p1, lapis_memref1
   if (B->sizes[0] != ncols || C->sizes[0] != nrows || C->sizes[1] != k) return fail(LAPIS_EBADSHAPE, "spmm_dcsr: B/C shape mismatch");
   const I *hp1 = elem_ptr<I>(p1), *hi1 = elem_ptr<I>(i1), *hp2 = elem_ptr<I>(p2), *hi2 = elem_ptr<I>(i2);
   if (hp1[0] != 0 || (int64_t)hp1[1] != nstored) return fail(LAPIS_EBADSHAPE, "spmm_dcsr: p1 must be {0, stored rows}");
-  LAPIS_TRY(check_pos_host<I>(hp2, nstored, nnz));
   for (int64_t r = 0; r < nstored; ++r)  // ascending row numbers: equal ones are adjacent and one warp takes the run
     if (hi1[r] < 0 || (int64_t)hi1[r] >= nrows || (r > 0 && hi1[r] < hi1[r - 1]))
       return fail(LAPIS_EBADSHAPE, "spmm_dcsr: stored row numbers must ascend within [0, rows)");
-  for (int64_t j = 0; j < nnz; ++j)
-    if (hi2[j] < 0 || (int64_t)hi2[j] >= ncols) return fail(LAPIS_EBADSHAPE, "spmm_dcsr: column index out of range at entry %lld", (long long)j);
   cudaStream_t st = nullptr;
-  DevBuf di1, dp2, di2, dval, dB, dC;
-  const size_t bB = (size_t)ncols * k * 8, bC = (size_t)nrows * k * 8;
-  LAPIS_TRY(di1.alloc((size_t)nstored * sizeof(I)));
-  LAPIS_TRY(dp2.alloc((size_t)(nstored + 1) * sizeof(I)));
-  LAPIS_TRY(di2.alloc((size_t)nnz * sizeof(I)));
-  LAPIS_TRY(dval.alloc((size_t)nnz * 8));
-  LAPIS_TRY(dB.alloc(bB));
-  LAPIS_TRY(dC.alloc(bC));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(di1.p, hi1, (size_t)nstored * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dp2.p, hp2, (size_t)(nstored + 1) * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(di2.p, hi2, (size_t)nnz * sizeof(I), cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dval.p, elem_ptr<double>(val), (size_t)nnz * 8, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dB.p, elem_ptr<double>(B), bB, cudaMemcpyHostToDevice, st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(dC.p, elem_ptr<double>(C), bC, cudaMemcpyHostToDevice, st));
-  LAPIS_TRY(lapis_b200_spmm_dcsr_f64((int)sizeof(I), nrows, ncols, nstored, k, di1.p, dp2.p, di2.p,
-                                     static_cast<const double *>(dval.p), static_cast<const double *>(dB.p),
-                                     static_cast<double *>(dC.p), st));
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(elem_ptr<double>(C), dC.p, bC, cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  Operands ops;
+  const size_t bC = (size_t)nrows * k * 8;
+  const int pi1 = ops.up.add(hi1, (size_t)nstored * sizeof(I)), pp2 = ops.up.add_pos(hp2, nstored + 1);
+  const int pi2 = ops.up.add_crd(hi2, nnz, ncols), pval = ops.up.add(elem_ptr<double>(val), (size_t)nnz * 8);
+  const int pB = ops.up.add(elem_ptr<double>(B), (size_t)ncols * k * 8), pC = ops.up.add(elem_ptr<double>(C), bC);
+  Upload::Facts facts;
+  LAPIS_TRY(ops.send(st, &facts));
+  LAPIS_TRY(check_facts<I>(facts, hp2, hi2, nstored, nnz, ncols, st));
+  LAPIS_TRY(lapis_b200_spmm_dcsr_f64((int)sizeof(I), nrows, ncols, nstored, k, ops.at<void>(pi1), ops.at<void>(pp2), ops.at<void>(pi2),
+                                     ops.at<double>(pval), ops.at<double>(pB), ops.at<double>(pC), st));
+  LAPIS_TRY(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st));
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *C;
   return LAPIS_OK;
 }

@@ -37,22 +37,31 @@ int sm_count();
 // 265 us each where they were measured, an allocation from the pool about 1 us).  Safe with several threads and
 // streams: the driver orders reuse by stream.  The pool keeps at most POOL_KEEP_BYTES of freed memory and gives the
 // rest back at the next synchronisation; pool_trim returns all of it (lapis_finalize).
-constexpr size_t POOL_KEEP_BYTES = size_t(256) << 20;
+constexpr size_t POOL_KEEP_BYTES = size_t(512) << 20;
 int pool_alloc(void **p, size_t bytes, cudaStream_t st);
 void pool_free(void *p, cudaStream_t st);
 void pool_trim();
 
-// Scoped allocation from the pool.
+// Scoped device memory.  Large blocks come from cudaMalloc: mapping memory into the pool and out again costs 25 ms each
+// way for 850 MB, cudaMalloc and cudaFree 1 to 4 ms.
+constexpr size_t POOL_LARGEST = size_t(256) << 20;
 struct PoolBuf {
   void *p = nullptr;
   cudaStream_t st = nullptr;
+  bool pooled = true;
   PoolBuf() = default;
   PoolBuf(const PoolBuf &) = delete;
   PoolBuf &operator=(const PoolBuf &) = delete;
-  ~PoolBuf() { pool_free(p, st); }
+  ~PoolBuf() {
+    if (pooled) pool_free(p, st);
+    else cudaFree(p);
+  }
   int alloc(size_t bytes, cudaStream_t stream) {
     st = stream;
-    return pool_alloc(&p, bytes, stream);
+    pooled = bytes <= POOL_LARGEST;
+    if (pooled) return pool_alloc(&p, bytes, stream);
+    LAPIS_CUDA_TRY(cudaMalloc(&p, bytes));
+    return LAPIS_OK;
   }
 };
 
@@ -111,3 +120,11 @@ struct lapis_b200_csr {
   int64_t walk_nblk;
   int walk_tile;
 };
+
+namespace lapis_b200 {
+// Fills a handle over arrays whose first offset, entry count and longest row are known, allocates its scratch and
+// enqueues the planning kernels.  plan_on_demand: no scratch and no plan when SpMV will run on the kernels for short
+// rows, which need none (for a handle that serves one product).
+int csr_setup(lapis_b200_csr *h, int idx_bytes, int64_t nrows, int64_t ncols, int64_t base, int64_t nnz, int64_t max_row_len,
+              const void *d_pos, const void *d_crd, const double *d_val, bool plan_on_demand, PoolBuf *scratch, cudaStream_t st);
+}  // namespace lapis_b200

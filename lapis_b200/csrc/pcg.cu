@@ -622,8 +622,9 @@ extern "C" int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const d
   }
   // a solve runs the SpMV pass many times: pick the kernel variant for this matrix first
   if (h->tuned_threads == 0 && (maxiter == 0 || maxiter >= 16)) LAPIS_TRY(lapis_b200_csr_tune(h, st));
-  void *work = nullptr;
-  LAPIS_CUDA_TRY(cudaMalloc(&work, (size_t)lapis_b200_pcg_workspace_bytes(n, n)));
+  PoolBuf buf;
+  LAPIS_TRY(buf.alloc((size_t)lapis_b200_pcg_workspace_bytes(n, n), st));
+  void *work = buf.p;
   int status = lapis_b200_pcg_init(work, n, n, 0, d_b, d_dinv, d_x, 1, st);
   int done = 0;
   uint64_t it = 0;
@@ -649,7 +650,6 @@ extern "C" int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const d
   if (status == LAPIS_OK && !done) status = lapis_b200_pcg_status(work, &done, &it, &rel, st);
   // a persistent SpMV block whose bounded wait gave up leaves Ap incomplete: the solve is not valid then
   if (status == LAPIS_OK) status = lapis_b200_spmv_status(st);
-  cudaFree(work);
   if (status != LAPIS_OK) return status;
   if (iters) *iters = it;
   if (relres) *relres = rel;
@@ -1044,8 +1044,9 @@ extern "C" int lapis_b200_mht_f64(lapis_b200_csr_t h, const double *d_mask, cons
   // masked out, not used).
   size_t sval_index = work_doubles + (size_t)n + 4;
   if (((int64_t)sval_index - h->base) & 1) sval_index += 1;
-  double *buf = nullptr;
-  LAPIS_CUDA_TRY(cudaMalloc(&buf, (sval_index + (size_t)h->nnz + 8) * sizeof(double)));
+  PoolBuf mem;
+  LAPIS_TRY(mem.alloc((sval_index + (size_t)h->nnz + 8) * sizeof(double), st));
+  double *buf = static_cast<double *>(mem.p);
   double *work = buf, *bbuf = buf + work_doubles, *sval = buf + sval_index;
   // the emitted code scales the matrix values in place; here the caller's array stays as it is and the
   // solves read a scaled copy through a shallow copy of the handle (same streaming plan)
@@ -1063,7 +1064,6 @@ extern "C" int lapis_b200_mht_f64(lapis_b200_csr_t h, const double *d_mask, cons
     status = mht_solve(&scaled, bbuf, d_d, d_mask, tol, maxiter, d_mom2, work, &it[1], &rel[1], st);
   }
   cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(buf);
   if (status != LAPIS_OK) return status;
   if (e != cudaSuccess) return fail(LAPIS_ECUDA, "mht: %s", cudaGetErrorString(e));
   LAPIS_TRY(lapis_b200_spmv_status(st));  // a persistent SpMV block that gave up leaves its output incomplete

@@ -1677,6 +1677,61 @@ static int launch_spmm(const lapis_b200_csr *h, int64_t k, const double *B, doub
 
 using namespace lapis_b200;
 
+namespace lapis_b200 {
+
+int csr_setup(lapis_b200_csr *h, int idx_bytes, int64_t nrows, int64_t ncols, int64_t base, int64_t nnz, int64_t max_row_len,
+              const void *d_pos, const void *d_crd, const double *d_val, bool plan_on_demand, PoolBuf *scratch, cudaStream_t st) {
+  const int64_t end = base + nnz, abase = base & ~(int64_t)3;
+  int64_t nblk = (end - abase + SPMV_TILE - 1) / SPMV_TILE;
+  if (nblk < 1) nblk = 1;
+  if (nblk > 0x7fffffffLL) return fail(LAPIS_ETOOBIG, "csr_create: more than 2^31 chunks");
+  *h = lapis_b200_csr{};
+  h->idx_bytes = idx_bytes;
+  h->nrows = nrows;
+  h->ncols = ncols;
+  h->nnz = nnz;
+  h->base = base;
+  h->pos = d_pos;
+  h->crd = d_crd;
+  h->val = d_val;
+  h->nblk = nblk;
+  h->max_row_len = max_row_len;
+  LAPIS_CUDA_TRY(cudaGetDevice(&h->device));
+  if (plan_on_demand && uses_rowthread(h)) return LAPIS_OK;
+  // The warp-walk kernel gives one warp a range of entries.  With 2048-entry ranges a matrix needs about eight
+  // times as many ranges as the GPU holds warps (32 per SM) before the last, partly filled round of warps stops
+  // mattering; smaller matrices (a row block of a partitioned one) get a second plan of 512-entry ranges.
+  const int64_t resident_warps = (int64_t)sm_count() * 32;
+  if (nblk > 1 && nblk < 8 * resident_warps) {
+    h->walk_tile = SPMV_WALK_FINE_TILE;
+    h->walk_nblk = (end - abase + h->walk_tile - 1) / h->walk_tile;
+  }
+  // one allocation: plan, partial sums, carries, and the second plan with its carries
+  const size_t words = (size_t)(nblk + 1) + 2 * (size_t)nblk + (h->walk_nblk > 0 ? 2 * (size_t)h->walk_nblk + 1 : 0);
+  scratch->st = st;
+  LAPIS_TRY(pool_alloc(&scratch->p, words * 8, st));  // a handle's destructor frees it as pool memory
+  h->blk_row = static_cast<int64_t *>(scratch->p);
+  h->blk_partial = reinterpret_cast<double *>(h->blk_row + nblk + 1);
+  h->carry = h->blk_partial + nblk;
+  if (h->walk_nblk > 0) {
+    h->walk_plan = reinterpret_cast<int64_t *>(h->carry + nblk);
+    h->walk_carry = reinterpret_cast<double *>(h->walk_plan + h->walk_nblk + 1);
+  }
+  auto plan = [&](int64_t count, int64_t *out, int tile) {
+    const unsigned grid = (unsigned)((count + 1 + 255) / 256);
+    if (idx_bytes == 4)
+      spmv_plan_kernel<int32_t><<<grid, 256, 0, st>>>(static_cast<const int32_t *>(d_pos), nrows, count, out, tile);
+    else
+      spmv_plan_kernel<int64_t><<<grid, 256, 0, st>>>(static_cast<const int64_t *>(d_pos), nrows, count, out, tile);
+  };
+  plan(nblk, h->blk_row, SPMV_TILE);
+  if (h->walk_nblk > 0) plan(h->walk_nblk, h->walk_plan, h->walk_tile);
+  LAPIS_CUDA_TRY(cudaGetLastError());
+  return LAPIS_OK;
+}
+
+}  // namespace lapis_b200
+
 extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64_t nrows, int64_t ncols,
                                      const void *d_pos, const void *d_crd, const double *d_val,
                                      void *stream) {
@@ -1689,8 +1744,6 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
   if ((reinterpret_cast<uintptr_t>(d_val) % 16) || (reinterpret_cast<uintptr_t>(d_crd) % 16))
     return fail(LAPIS_EBADARG, "csr_create: val and crd must be 16-byte aligned");
   cudaStream_t st = as_stream(stream);
-  int dev = 0;
-  LAPIS_CUDA_TRY(cudaGetDevice(&dev));
 
   // pos[0] and pos[nrows] define the nnz range addressed by this matrix; the longest row decides which SpMV kernels
   // serve it
@@ -1713,72 +1766,14 @@ extern "C" int lapis_b200_csr_create(lapis_b200_csr_t *out, int idx_bytes, int64
   if (ends[1] < ends[0] || ends[0] < 0) return fail(LAPIS_EBADSHAPE, "csr_create: pos is not non-decreasing");
   const int64_t nnz = ends[1] - ends[0];
   if (nnz > 0 && (d_crd == nullptr || d_val == nullptr)) return fail(LAPIS_EBADARG, "csr_create: crd/val null");
-  int64_t nblk = (ends[1] - (ends[0] & ~(int64_t)3) + SPMV_TILE - 1) / SPMV_TILE;
-  if (nblk < 1) nblk = 1;
-  if (nblk > 0x7fffffffLL) return fail(LAPIS_ETOOBIG, "csr_create: more than 2^31 chunks");
-
   lapis_b200_csr *h = new lapis_b200_csr();
-  h->idx_bytes = idx_bytes;
-  h->nrows = nrows;
-  h->ncols = ncols;
-  h->nnz = nnz;
-  h->base = ends[0];
-  h->pos = d_pos;
-  h->crd = d_crd;
-  h->val = d_val;
-  h->nblk = nblk;
-  h->blk_row = nullptr;
-  h->blk_partial = nullptr;
-  h->carry = nullptr;
-  h->tuned_threads = h->tuned_minb = h->tuned_hint = 0;
-  h->max_row_len = facts[0];
-  h->device = dev;
-  h->walk_plan = nullptr;
-  h->walk_carry = nullptr;
-  h->walk_nblk = 0;
-  h->walk_tile = 0;
-  // The warp-walk kernel gives one warp a range of entries.  With 2048-entry ranges a matrix needs about eight
-  // times as many ranges as the GPU holds warps (32 per SM) before the last, partly filled round of warps stops
-  // mattering; smaller matrices (a row block of a partitioned one) get a second plan of 512-entry ranges.
-  const int64_t resident_warps = (int64_t)sm_count() * 32;
-  if (nblk > 1 && nblk < 8 * resident_warps) {
-    h->walk_tile = SPMV_WALK_FINE_TILE;
-    h->walk_nblk = (ends[1] - (ends[0] & ~(int64_t)3) + h->walk_tile - 1) / h->walk_tile;
-  }
-  // one allocation: plan, partial sums, carries, and the second plan with its carries
-  const size_t words = (size_t)(nblk + 1) + 2 * (size_t)nblk + (h->walk_nblk > 0 ? 2 * (size_t)h->walk_nblk + 1 : 0);
-  void *scratch = nullptr;
-  if (pool_alloc(&scratch, words * 8, st) != LAPIS_OK) {
+  PoolBuf scratch;
+  const int rc = csr_setup(h, idx_bytes, nrows, ncols, ends[0], nnz, facts[0], d_pos, d_crd, d_val, false, &scratch, st);
+  if (rc != LAPIS_OK) {
     delete h;
-    return lapis_last_error();
+    return rc;
   }
-  h->blk_row = static_cast<int64_t *>(scratch);
-  h->blk_partial = reinterpret_cast<double *>(h->blk_row + nblk + 1);
-  h->carry = h->blk_partial + nblk;
-  if (h->walk_nblk > 0) {
-    h->walk_plan = reinterpret_cast<int64_t *>(h->carry + nblk);
-    h->walk_carry = reinterpret_cast<double *>(h->walk_plan + h->walk_nblk + 1);
-  }
-  const unsigned pgrid = (unsigned)((nblk + 1 + 255) / 256);
-  if (idx_bytes == 4)
-    spmv_plan_kernel<int32_t><<<pgrid, 256, 0, st>>>(static_cast<const int32_t *>(d_pos), nrows, nblk, h->blk_row);
-  else
-    spmv_plan_kernel<int64_t><<<pgrid, 256, 0, st>>>(static_cast<const int64_t *>(d_pos), nrows, nblk, h->blk_row);
-  if (h->walk_nblk > 0) {
-    const unsigned wgrid = (unsigned)((h->walk_nblk + 1 + 255) / 256);
-    if (idx_bytes == 4)
-      spmv_plan_kernel<int32_t><<<wgrid, 256, 0, st>>>(static_cast<const int32_t *>(d_pos), nrows, h->walk_nblk, h->walk_plan,
-                                                       h->walk_tile);
-    else
-      spmv_plan_kernel<int64_t><<<wgrid, 256, 0, st>>>(static_cast<const int64_t *>(d_pos), nrows, h->walk_nblk, h->walk_plan,
-                                                       h->walk_tile);
-  }
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    pool_free(scratch, st);
-    delete h;
-    return fail(LAPIS_ECUDA, "csr_create: plan kernel launch failed: %s", cudaGetErrorString(e));
-  }
+  scratch.p = nullptr;  // the handle's from here on: blk_row is its first word
   *out = h;
   return LAPIS_OK;
 }

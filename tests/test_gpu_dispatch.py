@@ -71,3 +71,37 @@ def test_launches_that_overlap_see_each_others_results():
             ends.append(a)
         assert torch.equal(ends[0], ends[1])
         assert bool(torch.isfinite(ends[0]).all())
+
+
+@pytest.mark.parametrize("rows,mean,pinned", [(1, 1, False), (900, 4, False), (30_000, 9, False), (300_000, 5, False), (300_000, 5, True)])
+def test_host_arrays_travel_in_pieces(rows, mean, pinned):
+    """Calls on host arrays from one piece to more than the staging ring holds, pageable and page-locked: the result of
+    the resident call, bad indices found wherever they are, and y untouched then."""
+    from lapis_b200 import KokkosBackend as KB
+    from lapis_b200 import modules as mm
+    from lapis_b200._lib import LapisError
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(rows)
+    pos, crd, val = _csr(rng, np.full(rows, min(mean, rows)), rows, np.int64)
+    x, y = rng.uniform(-1, 1, rows), rng.uniform(-1, 1, rows)
+    want = CsrMatrix.from_host(pos, crd, val, (rows, rows), dev).spmv(torch.as_tensor(x).to(dev), torch.as_tensor(y).to(dev)).cpu().numpy()
+    module = KB.KokkosBackend(decompose_tensors=True).compile(mm.spmv(mm.CSR64))
+    spec = ((rows, rows), (rows + 1, len(crd), len(crd)))
+    if pinned:
+        pos, crd, val, x, y = (torch.as_tensor(a).pin_memory().numpy() for a in (pos, crd, val, x, y))
+    y0 = y.copy()
+    module.spmv(pos, crd, val, spec, x, y)
+    assert np.array_equal(y, want)
+    y[:] = y0
+    for at, bad in ((0, rows), (len(crd) // 2, -1), (len(crd) - 1, rows)):
+        keep, crd[at] = crd[at], bad
+        with pytest.raises(LapisError, match="column index out of range"):
+            module.spmv(pos, crd, val, spec, x, y)
+        crd[at] = keep
+    for at in {1, rows // 2, rows} - {0}:
+        keep, pos[at] = pos[at], pos[at - 1] - 1
+        with pytest.raises(LapisError, match="pos"):
+            module.spmv(pos, crd, val, spec, x, y)
+        pos[at] = keep
+    assert np.array_equal(y, y0)
