@@ -105,3 +105,40 @@ def test_host_arrays_travel_in_pieces(rows, mean, pinned):
             module.spmv(pos, crd, val, spec, x, y)
         pos[at] = keep
     assert np.array_equal(y, y0)
+
+
+@pytest.mark.parametrize("batch,m,n,k", [
+    (1, 1, 1, 1), (1, 63, 65, 15), (1, 64, 64, 16), (1, 65, 63, 17), (1, 130, 1028, 100), (1, 33, 31, 900), (1, 1000, 1100, 49),  # one product
+    (300, 33, 65, 31), (300, 30, 20, 52), (2000, 4, 5, 6), (150, 64, 40, 33), (65540, 2, 3, 4), (200, 20, 100, 7), (3, 40, 40, 0)])  # batches
+def test_general_shape_matmul_tiles(batch, m, n, k):
+    """Every tile the rule picks, at the edges of tiles and k-slabs, with and without 16-byte accesses: k ascending, the
+    product and the sum rounded separately, C last, bit for bit."""
+    from lapis_b200 import device
+    dev = _dev()
+    g = torch.Generator(device=dev).manual_seed(m * n + k)
+    A, B, C = (torch.rand(s, generator=g, device=dev) * 2 - 1 for s in ((batch, m, k), (batch, k, n), (batch, m, n)))
+    want = torch.zeros_like(C)
+    for i in range(k):  # a product and a sum per k, as torch rounds them
+        want = want + A[:, :, i, None] * B[:, i, None, :]
+    want = want + C
+    shifted = torch.empty(C.numel() + 1, device=dev)[1:].view_as(C)  # C off the 16-byte boundary
+    shifted.copy_(C)
+    assert torch.equal(device.bgemm(A, B, C), want)
+    assert torch.equal(device.bgemm(A, B, shifted), want)
+
+
+def test_general_shape_matmul_special_values():
+    """Signed zeros, infinities and NaN as the sequential loop has them (padding of the last slab adds nothing)."""
+    from lapis_b200 import device
+    dev = _dev()
+    A = torch.tensor([[0.0, -0.0, float("inf")], [-0.0, -1.0, 0.0], [1e-40, 3e38, float("nan")]], device=dev)
+    B = torch.tensor([[-0.0, 1.0], [0.0, 3e38], [1.0, -0.0]], device=dev)
+    C = torch.tensor([[-0.0, 1.0], [-0.0, -0.0], [0.0, -0.0]], device=dev)
+    want = torch.zeros_like(C)
+    for i in range(3):
+        want = want + A[:, i, None] * B[i, None, :]
+    want = want + C
+    got = device.bgemm(A, B, C)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert torch.equal(got[ok].view(torch.int32), want[ok].view(torch.int32))
