@@ -471,7 +471,7 @@ def run_sparse(args, d, hx: Harness):
         xd = torch.as_tensor(d["B"]).to(dev)
         yd = torch.zeros((r1 - r0, 64), dtype=torch.float64, device=dev)
         step = lambda: A.spmm(xd, yd, accumulate=False)
-        kernel, launches_per_step, traffic = "spmm_row_direct_kernel", 1, NCU_TRAFFIC["spmm"]
+        kernel, launches_per_step, traffic = "spmm_kernel", 1, NCU_TRAFFIC["spmm"]
     ms, clocks = hx.timed(step, args.steps, args.warmup)
     ms_step = ms / args.steps
     value = d["work"] / (ms_step * 1e-3) * d["unit_scale"]
@@ -812,7 +812,7 @@ def run_formats(args):
     t0 = time.perf_counter()
     oracle.spmm_dcsr(i1[:rows_cpu], sp["pos"][:rows_cpu + 1], sp["crd"], sp["val"], sp["B"], np.zeros((2 * rows_cpu, 64)))
     cpu_ms = (time.perf_counter() - t0) * 1e3 * n / rows_cpu
-    line("spmm_dcsr_kernel", f"DCSR {2 * n} x {n}, {n} stored rows, 32 per row, k 64, fp64, int64 indices", ms,
+    line("spmm_kernel", f"DCSR {2 * n} x {n}, {n} stored rows, 32 per row, k 64, fp64, int64 indices", ms,
          nnz * 16 + 8 * (2 * n + 1) + 3 * 8 * n * 64, cpu_ms,
          {"gathered_B_bytes": nnz * 64 * 8, "cpu_sample": f"first {rows_cpu} stored rows, scaled by rows"})
     del dB, Cd

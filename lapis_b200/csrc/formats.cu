@@ -8,10 +8,7 @@
 // parallel, so every output element is updated in place once per stored entry, in ascending entry order:
 // out = a*b + out.  One thread owns an output element for the whole row here, which keeps that order.
 //
-// DCSR (examples/spmm_dcsr_opdsl.py:46-101, 137-160): both levels compressed -- p1 = {0, stored rows},
-// i1 = their row numbers, p2 / i2 / val a CSR over the stored rows only.  C[i1[r], :] += sum_j val[j] *
-// B[i2[j], :] in ascending j, updated in place; rows that are not stored are not touched.  i1 ascends (a number
-// may repeat).
+// DCSR (examples/spmm_dcsr_opdsl.py:46-101, 137-160): the entry point is here, the kernel in spmm.cu.
 #include <cstdint>
 
 #include "common.h"
@@ -116,87 +113,6 @@ bspmm_csrv_vec4_kernel(const I *__restrict__ pos, const I *__restrict__ crd, con
   }
 }
 
-// One warp per stored row, 16-byte accesses: a lane owns two adjacent columns of every 64-column tile and
-// keeps four rows of B in flight (k even, B and C 16-byte aligned).
-template <typename I>
-__global__ void __launch_bounds__(256)
-spmm_dcsr_vec2_kernel(const I *__restrict__ i1, const I *__restrict__ p2, const I *__restrict__ i2,
-                      const double *__restrict__ val, int64_t nstored, int64_t k2, const double2 *__restrict__ B2,
-                      double2 *__restrict__ C2) {
-  const int lane = threadIdx.x & 31;
-  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= nstored) return;
-  const I rowid = i1[r];
-  if (r > 0 && i1[r - 1] == rowid) return;  // a repeated row number: the first warp of the run takes all of it
-  int64_t rend = r + 1;
-  while (rend < nstored && i1[rend] == rowid) ++rend;
-  const int64_t lo = (int64_t)p2[r], hi = (int64_t)p2[rend];
-  double2 *crow = C2 + (int64_t)rowid * k2;
-  for (int64_t c = lane; c < k2; c += 32) {
-    double2 acc = crow[c];
-    int64_t j = lo;
-    for (; j + 3 < hi; j += 4) {
-      double a[4];
-      double2 b[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a[u] = __ldg(val + j + u);
-        b[u] = __ldg(B2 + (int64_t)i2[j + u] * k2 + c);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        acc.x = __dadd_rn(acc.x, __dmul_rn(a[u], b[u].x));
-        acc.y = __dadd_rn(acc.y, __dmul_rn(a[u], b[u].y));
-      }
-    }
-    for (; j < hi; ++j) {
-      const double a = __ldg(val + j);
-      const double2 b = __ldg(B2 + (int64_t)i2[j] * k2 + c);
-      acc.x = __dadd_rn(acc.x, __dmul_rn(a, b.x));
-      acc.y = __dadd_rn(acc.y, __dmul_rn(a, b.y));
-    }
-    crow[c] = acc;
-  }
-}
-
-// One warp per stored row; a lane owns the columns lane, lane + 32, ...
-template <typename I>
-__global__ void __launch_bounds__(256)
-spmm_dcsr_kernel(const I *__restrict__ i1, const I *__restrict__ p2, const I *__restrict__ i2,
-                 const double *__restrict__ val, int64_t nstored, int64_t k, const double *__restrict__ B,
-                 double *__restrict__ C) {
-  const int lane = threadIdx.x & 31;
-  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (r >= nstored) return;
-  // A row number may be listed more than once (examples/spmm_dcsr_opdsl.py:140-141 lists one twice, the second
-  // time with no entries): equal numbers are adjacent, the first warp of such a run takes the whole run.
-  const I rowid = i1[r];
-  if (r > 0 && i1[r - 1] == rowid) return;
-  int64_t rend = r + 1;
-  while (rend < nstored && i1[rend] == rowid) ++rend;
-  const int64_t lo = (int64_t)p2[r], hi = (int64_t)p2[rend];
-  double *crow = C + (int64_t)rowid * k;
-  for (int64_t c0 = 0; c0 < k; c0 += 128) {
-    int64_t col[4];
-    double acc[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      col[q] = c0 + lane + 32 * q;
-      acc[q] = col[q] < k ? crow[col[q]] : 0.0;
-    }
-    for (int64_t j = lo; j < hi; ++j) {
-      const double a = val[j];
-      const double *brow = B + (int64_t)i2[j] * k;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (col[q] < k) acc[q] = __dadd_rn(acc[q], __dmul_rn(a, __ldg(brow + col[q])));
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (col[q] < k) crow[col[q]] = acc[q];
-  }
-}
-
 template <typename I>
 static void launch_bspmm(const void *pos, const void *crd, const float *val, int64_t nrows, int64_t nh, int64_t E,
                          const float *B, float *C, int accumulate, cudaStream_t st) {
@@ -254,26 +170,5 @@ extern "C" int lapis_b200_spmm_dcsr_f64(int idx_bytes, int64_t nrows, int64_t nc
     return fail(LAPIS_EBADSHAPE, "spmm_dcsr: bad dimensions");
   if (nstored == 0 || k == 0) return LAPIS_OK;
   if (d_i1 == nullptr || d_p2 == nullptr || d_C == nullptr) return fail(LAPIS_EBADARG, "spmm_dcsr: null operand");
-  cudaStream_t st = as_stream(stream);
-  const unsigned grid = (unsigned)((nstored + 7) / 8);
-  if (k % 2 == 0 && (reinterpret_cast<uintptr_t>(d_B) | reinterpret_cast<uintptr_t>(d_C)) % 16 == 0) {
-    const double2 *B2 = reinterpret_cast<const double2 *>(d_B);
-    double2 *C2 = reinterpret_cast<double2 *>(d_C);
-    if (idx_bytes == 4)
-      spmm_dcsr_vec2_kernel<int32_t><<<grid, 256, 0, st>>>(static_cast<const int32_t *>(d_i1), static_cast<const int32_t *>(d_p2),
-                                                           static_cast<const int32_t *>(d_i2), d_val, nstored, k / 2, B2, C2);
-    else
-      spmm_dcsr_vec2_kernel<int64_t><<<grid, 256, 0, st>>>(static_cast<const int64_t *>(d_i1), static_cast<const int64_t *>(d_p2),
-                                                           static_cast<const int64_t *>(d_i2), d_val, nstored, k / 2, B2, C2);
-    LAPIS_CUDA_TRY(cudaGetLastError());
-    return LAPIS_OK;
-  }
-  if (idx_bytes == 4)
-    spmm_dcsr_kernel<int32_t><<<grid, 256, 0, st>>>(static_cast<const int32_t *>(d_i1), static_cast<const int32_t *>(d_p2),
-                                                    static_cast<const int32_t *>(d_i2), d_val, nstored, k, d_B, d_C);
-  else
-    spmm_dcsr_kernel<int64_t><<<grid, 256, 0, st>>>(static_cast<const int64_t *>(d_i1), static_cast<const int64_t *>(d_p2),
-                                                    static_cast<const int64_t *>(d_i2), d_val, nstored, k, d_B, d_C);
-  LAPIS_CUDA_TRY(cudaGetLastError());
-  return LAPIS_OK;
+  return spmm_launch(idx_bytes, d_i1, d_p2, d_i2, d_val, nstored, k, -1, d_B, d_C, 1, as_stream(stream));
 }

@@ -1,4 +1,4 @@
-// CSR SpMV and SpMM for sm_100a.
+// CSR SpMV for sm_100a (SpMM: spmm.cu).
 //
 // Replaces the loop the LAPIS emitter prints for `linalg.matvec` on a CSR operand
 // (tests/Dialect/Kokkos/loop_mapping_2.mlir.gold:12-37; emitted by
@@ -1216,129 +1216,6 @@ __global__ void csr_facts_kernel(const I *__restrict__ pos, int64_t nrows, unsig
 }
 
 // ---------------------------------------------------------------------------
-// SpMM: C[r, :] = (accumulate ? C[r, :] : 0) + sum_j val[j] * B[crd[j], :].
-// One warp per row; lane l owns columns {2l, 2l+1} of a 64-column panel, so a B
-// row is fetched as one coalesced 512-byte request and every output element is
-// summed in ascending j by a single lane: bit-identical to the sequential row
-// loop (examples/bspmm.py:15-23, spmm_dcsr_opdsl.py:132-135 outer-loop-only
-// parallelism).  Four B rows are in flight per warp.
-// ---------------------------------------------------------------------------
-template <typename I, bool VEC2, int SPMM_WARPS, int SPMM_UNROLL>
-__global__ void __launch_bounds__(SPMM_WARPS * 32)
-spmm_row_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val,
-                int64_t nrows, int64_t k, const double *__restrict__ B, double *__restrict__ C,
-                int accumulate) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * SPMM_WARPS + (threadIdx.x >> 5);
-  if (row >= nrows) return;
-  const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
-  double *crow = C + row * k;
-  for (int64_t c0 = 0; c0 < k; c0 += 64) {
-    const int64_t col = c0 + 2 * lane;
-    const bool in0 = col < k, in1 = col + 1 < k;
-    double acc0 = 0.0, acc1 = 0.0;
-    for (int64_t jb = lo; jb < hi; jb += 32) {
-      // lanes fetch up to 32 (crd, val) pairs of the row at once, then broadcast them
-      const int64_t jm = jb + lane;
-      int64_t cj = 0;
-      double aj = 0.0;
-      if (jm < hi) {
-        cj = (int64_t)__ldcs(crd + jm);
-        aj = __ldcs(val + jm);
-      }
-      const int cnt = (int)((hi - jb) < 32 ? (hi - jb) : 32);
-      for (int t0 = 0; t0 < cnt; t0 += SPMM_UNROLL) {
-        double b0[SPMM_UNROLL], b1[SPMM_UNROLL], a[SPMM_UNROLL];
-#pragma unroll
-        for (int u = 0; u < SPMM_UNROLL; ++u) {
-          const int t = t0 + u;
-          const int src = t < cnt ? t : 0;
-          const int64_t cc = __shfl_sync(0xffffffffu, cj, src);
-          a[u] = __shfl_sync(0xffffffffu, aj, src);
-          b0[u] = 0.0;
-          b1[u] = 0.0;
-          if (t < cnt) {
-            const double *brow = B + cc * k;
-            if (VEC2) {
-              if (in0) {
-                const double2 bb = __ldg(reinterpret_cast<const double2 *>(brow + col));
-                b0[u] = bb.x;
-                b1[u] = bb.y;
-              }
-            } else {
-              if (in0) b0[u] = __ldg(brow + col);
-              if (in1) b1[u] = __ldg(brow + col + 1);
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < SPMM_UNROLL; ++u) {
-          if (t0 + u < cnt) {
-            acc0 = __dadd_rn(acc0, __dmul_rn(a[u], b0[u]));
-            acc1 = __dadd_rn(acc1, __dmul_rn(a[u], b1[u]));
-          }
-        }
-      }
-    }
-    if (VEC2) {
-      if (in0) {
-        double2 cin = make_double2(0.0, 0.0);
-        if (accumulate) cin = *reinterpret_cast<const double2 *>(crow + col);
-        double2 out;
-        out.x = __dadd_rn(acc0, cin.x);
-        out.y = __dadd_rn(acc1, cin.y);
-        *reinterpret_cast<double2 *>(crow + col) = out;
-      }
-    } else {
-      if (in0) crow[col] = __dadd_rn(acc0, accumulate ? crow[col] : 0.0);
-      if (in1) crow[col + 1] = __dadd_rn(acc1, accumulate ? crow[col + 1] : 0.0);
-    }
-  }
-}
-
-// The same row mapping without the shuffle broadcast: every lane reads the row's (crd, val) pairs itself (one
-// address per warp, served as a broadcast) and keeps UNROLL rows of B in flight as 16-byte loads.  k even, B and
-// C 16-byte aligned.  Same sums in the same order as spmm_row_kernel.
-template <typename I, int SPMM_WARPS, int SPMM_UNROLL>
-__global__ void __launch_bounds__(SPMM_WARPS * 32)
-spmm_row_direct_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val,
-                       int64_t nrows, int64_t k2, const double2 *__restrict__ B2, double2 *__restrict__ C2,
-                       int accumulate) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * SPMM_WARPS + (threadIdx.x >> 5);
-  if (row >= nrows) return;
-  const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
-  double2 *crow = C2 + row * k2;
-  for (int64_t c = lane; c < k2; c += 32) {
-    double2 acc = make_double2(0.0, 0.0);
-    int64_t j = lo;
-    for (; j + SPMM_UNROLL <= hi; j += SPMM_UNROLL) {
-      double a[SPMM_UNROLL];
-      double2 b[SPMM_UNROLL];
-#pragma unroll
-      for (int u = 0; u < SPMM_UNROLL; ++u) {
-        a[u] = __ldg(val + j + u);
-        b[u] = __ldg(B2 + (int64_t)crd[j + u] * k2 + c);
-      }
-#pragma unroll
-      for (int u = 0; u < SPMM_UNROLL; ++u) {
-        acc.x = __dadd_rn(acc.x, __dmul_rn(a[u], b[u].x));
-        acc.y = __dadd_rn(acc.y, __dmul_rn(a[u], b[u].y));
-      }
-    }
-    for (; j < hi; ++j) {
-      const double a = __ldg(val + j);
-      const double2 b = __ldg(B2 + (int64_t)crd[j] * k2 + c);
-      acc.x = __dadd_rn(acc.x, __dmul_rn(a, b.x));
-      acc.y = __dadd_rn(acc.y, __dmul_rn(a, b.y));
-    }
-    double2 cin = make_double2(0.0, 0.0);
-    if (accumulate) cin = crow[c];
-    crow[c] = make_double2(__dadd_rn(acc.x, cin.x), __dadd_rn(acc.y, cin.y));
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 // Kernel variant: {threads, blocks per SM, L2 hint}.  threads >= 256: one chunk per block; threads == 2 / 3: the
@@ -1639,40 +1516,6 @@ int spmv_launch_pcg_direction_pass(const lapis_b200_csr *h, int64_t p_off, doubl
   return launch_pcg_direction_pass<int64_t>(h, p_off, pw0, pw1, Ap, blk_partial, st, ex);
 }
 
-template <typename I, int WARPS, int UNROLL>
-static void launch_spmm_variant(const lapis_b200_csr *h, int64_t k, const double *B, double *C, int accumulate,
-                                cudaStream_t st) {
-  const I *pos = static_cast<const I *>(h->pos);
-  const I *crd = static_cast<const I *>(h->crd);
-  const unsigned grid = (unsigned)((h->nrows + WARPS - 1) / WARPS);
-  const bool vec2 = (k % 2 == 0) && ((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) % 16 == 0);
-  if (vec2)
-    spmm_row_kernel<I, true, WARPS, UNROLL><<<grid, WARPS * 32, 0, st>>>(pos, crd, h->val, h->nrows, k, B, C, accumulate);
-  else
-    spmm_row_kernel<I, false, WARPS, UNROLL><<<grid, WARPS * 32, 0, st>>>(pos, crd, h->val, h->nrows, k, B, C, accumulate);
-}
-
-// The direct-load kernel (four rows of B in flight per lane) needs k even and 16-byte aligned B, C; other
-// operands take the shuffle-broadcast kernel.  Measured on the 2^21-row, 32-per-row, k = 64 case: direct 5.10 ms
-// (5.12 ms with eight rows in flight), shuffle-broadcast 6.6 ms.
-template <typename I>
-static int launch_spmm(const lapis_b200_csr *h, int64_t k, const double *B, double *C, int accumulate,
-                       cudaStream_t st) {
-  const bool vec2 = (k % 2 == 0) && ((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) % 16 == 0);
-  if (vec2) {
-    const I *pos = static_cast<const I *>(h->pos);
-    const I *crd = static_cast<const I *>(h->crd);
-    const unsigned grid = (unsigned)((h->nrows + 7) / 8);
-    spmm_row_direct_kernel<I, 8, 4><<<grid, 256, 0, st>>>(pos, crd, h->val, h->nrows, k / 2,
-                                                          reinterpret_cast<const double2 *>(B),
-                                                          reinterpret_cast<double2 *>(C), accumulate);
-  } else {
-    launch_spmm_variant<I, 8, 4>(h, k, B, C, accumulate, st);
-  }
-  LAPIS_CUDA_TRY(cudaGetLastError());
-  return LAPIS_OK;
-}
-
 }  // namespace lapis_b200
 
 using namespace lapis_b200;
@@ -1900,8 +1743,8 @@ extern "C" int lapis_b200_spmm_f64(lapis_b200_csr_t h, int64_t k, const double *
   if (k < 0) return fail(LAPIS_EBADSHAPE, "spmm: negative k");
   if (h->nrows == 0 || k == 0) return LAPIS_OK;
   if (d_C == nullptr || (h->nnz > 0 && d_B == nullptr)) return fail(LAPIS_EBADARG, "spmm: null operand");
-  if (h->idx_bytes == 4) return launch_spmm<int32_t>(h, k, d_B, d_C, accumulate, as_stream(stream));
-  return launch_spmm<int64_t>(h, k, d_B, d_C, accumulate, as_stream(stream));
+  return spmm_launch(h->idx_bytes, nullptr, h->pos, h->crd, h->val, h->nrows, k, h->max_row_len, d_B, d_C, accumulate,
+                     as_stream(stream));
 }
 
 // ---------------------------------------------------------------------------

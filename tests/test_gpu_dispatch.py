@@ -142,3 +142,62 @@ def test_general_shape_matmul_special_values():
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     ok = ~torch.isnan(want)
     assert torch.equal(got[ok].view(torch.int32), want[ok].view(torch.int32))
+
+
+def _lens_with_long_rows(rng, rows):
+    lens = rng.integers(0, 21, rows)
+    for at, n in zip(rng.choice(rows, 7, replace=False), (255, 256, 257, 300, 1025, 2048, 2500)):
+        lens[at] = n
+    lens[-1], lens[rows // 2:rows // 2 + 4] = 400, 500  # the last row, neighbours
+    return lens
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 13, 16, 17, 31, 32, 33, 37, 64, 65, 66, 97, 101, 130, 260])
+def test_spmm_group_sizes_and_long_rows(k):
+    """Every width the rule tells apart, rows on both sides of the limit for long rows, a block of rows that starts inside
+    the arrays, CSR and DCSR (with repeated row numbers), operands on and off 16-byte boundaries: bit for bit."""
+    from lapis_b200.device import CsrMatrix, spmm_dcsr
+    dev = _dev()
+    rng = np.random.default_rng(k)
+    rows, ncols, first = 700, 3000, 5
+    for idx in (np.int32, np.int64):
+        pos, crd, val = _csr(rng, _lens_with_long_rows(rng, rows + first), ncols, idx)
+        B, C = rng.uniform(-1, 1, (ncols, k)), rng.uniform(-1, 1, (rows, k))
+        numbers = np.sort(rng.choice(2 * rows, rows)).astype(idx)  # ascending, some twice
+        C2 = rng.uniform(-1, 1, (2 * rows, k))
+        d = [torch.as_tensor(a).to(dev) for a in (pos, crd, val)]
+        for shift in (0, 1):
+            flat = torch.empty(B.size + shift, dtype=torch.float64, device=dev)
+            Bd = flat[shift:].view(ncols, k)
+            Bd.copy_(torch.as_tensor(B))
+            for lo in (0, first):
+                A = CsrMatrix(d[0][lo:lo + rows + 1], d[1], d[2], (rows, ncols))
+                for acc in (True, False):
+                    # the handle takes the entries that pos names; the oracle reads the same arrays
+                    want = oracle.spmm(pos[lo:lo + rows + 1], crd, val, B, C if acc else np.zeros_like(C))
+                    assert np.array_equal(A.spmm(Bd, torch.as_tensor(C).to(dev), accumulate=acc).cpu().numpy(), want)
+            p2 = pos[first:rows + first + 1]
+            want = oracle.spmm_dcsr(numbers, p2, crd, val, B, C2)
+            got = spmm_dcsr(torch.as_tensor(numbers).to(dev), torch.as_tensor(p2).to(dev), d[1], d[2], Bd, torch.as_tensor(C2).to(dev), ncols)
+            assert np.array_equal(got.cpu().numpy(), want)
+
+
+def test_spmm_with_long_rows_in_a_chain():
+    """The two kernels of a product with long rows overlap; the next product reads what both wrote."""
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(1)
+    n, k = 3000, 20
+    pos, crd, val = _csr(rng, _lens_with_long_rows(rng, n), n, np.int32)
+    A = CsrMatrix.from_host(pos, crd, val / 50, (n, n), dev)
+    start = torch.as_tensor(rng.uniform(-1, 1, (n, k))).to(dev)
+    ends = []
+    for sync in (True, False):
+        a, b = start.clone(), torch.zeros_like(start)
+        for _ in range(30):
+            A.spmm(a, b, accumulate=False)
+            if sync:
+                torch.cuda.synchronize()
+            a, b = b, a
+        ends.append(a)
+    assert torch.equal(ends[0], ends[1])
