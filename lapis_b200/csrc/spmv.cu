@@ -1490,6 +1490,11 @@ int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumul
 // Pass A of a PCG iteration with its head and tail inside the SpMV kernel; only for handles on which
 // spmv_fuses_pcg_pass() is true.
 bool spmv_fuses_pcg_pass(const lapis_b200_csr *h) { return h->nrows > 0 && uses_rowthread(h); }
+// Whether a whole PCG solve runs in one cluster (pcg_small.cu): rows short enough for a thread each, a matrix that the L1
+// caches of eight SMs hold, no SpMV kernel forced.
+bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
+  return h->nrows > 0 && h->nrows <= 16384 && h->nnz <= 131072 && has_short_rows(h) && spmv_override().threads == 0;
+}
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex) {
   if (h->idx_bytes == 4) return launch_spmv<int32_t>(h, x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);

@@ -201,3 +201,50 @@ def test_spmm_with_long_rows_in_a_chain():
             a, b = b, a
         ends.append(a)
     assert torch.equal(ends[0], ends[1])
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 1000, 1024, 1025, 4096, 4097, 8193, 16384])
+def test_small_pcg_against_the_passes(n):
+    """Systems solved in one launch: the iterations and the solution of the launch-per-pass form (taken when an SpMV kernel is
+    forced), which the oracle tests cover; the same bits on a second run."""
+    from lapis_b200._lib import check, load
+    from lapis_b200.device import CsrMatrix
+    dev, lib = _dev(), load()
+    rng = np.random.default_rng(n)
+    import scipy.sparse as sp
+    half = sp.random(n, n, min(1.0, 2.0 / n), random_state=rng, format="csr") if n > 2 else sp.csr_matrix((n, n))
+    sym = (half + half.T).tocsr()
+    for idx in (np.int32, np.int64):
+        a = (sym + sp.diags(np.asarray(abs(sym).sum(1)).ravel() + rng.uniform(0.5, 1, n))).tocsr()
+        a.sort_indices()
+        A = CsrMatrix.from_host(a.indptr.astype(idx), a.indices.astype(idx), a.data, (n, n), dev)
+        b, dinv = torch.as_tensor(rng.uniform(0, 1, n)).to(dev), torch.as_tensor(1 / a.diagonal()).to(dev)
+        for tol, maxiter in ((1e-8, 1000), (0.0, 1), (0.0, 5)):
+            x, it, rel = A.pcg(b, dinv, tol, maxiter)
+            again = A.pcg(b, dinv, tol, maxiter)
+            check(lib.lapis_b200_spmv_select_kernel(1, 0, 1))
+            try:
+                x0, it0, rel0 = A.pcg(b, dinv, tol, maxiter)
+            finally:
+                check(lib.lapis_b200_spmv_select_kernel(0, 0, 0))
+            assert torch.equal(x, again[0]) and again[1] == it and (again[2] == rel or rel != rel)
+            if n <= 2:  # solved exactly after one step or two: what is left is rounding, then 0 / 0
+                continue
+            assert it == it0
+            # a dominant diagonal amplifies the rounding of a dot product little
+            assert float((x - x0).norm()) <= 1e-11 * float(x0.norm()) and abs(rel - rel0) <= 1e-6 * rel0 + 1e-15
+
+
+def test_small_pcg_over_several_launches():
+    """More iterations than one launch makes: the state carried from launch to launch gives the count asked for and the
+    solution (tol 0 goes on past convergence; 4096 iterations a launch)."""
+    from lapis_b200 import workloads
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    d = workloads.pcg_laplacian(128)
+    A = CsrMatrix.from_host(d["pos"], d["crd"], d["val"], (128 * 128,) * 2, dev)
+    b, dinv = torch.as_tensor(d["b"]).to(dev), torch.as_tensor(d["dinv"]).to(dev)
+    x, it, rel = A.pcg(b, dinv, 0.0, 4200)
+    assert it == 4200 and 0 <= rel < 1e-14
+    y, _, _ = A.pcg(b, dinv, 1e-12, 4000)
+    assert float((x - y).norm()) <= 1e-8 * float(y.norm())
