@@ -17,8 +17,8 @@ namespace lapis_b200 {
 
 constexpr int BSPMM_THREADS = 128;
 
-// GROUP threads share one row (GROUP = 32: four rows per block; GROUP = 128: one); each thread owns EPT
-// output elements per pass, GROUP apart, so that B rows and C rows are read and written coalesced.
+// Rows of more than 128 elements that no 16-byte access fits: GROUP threads share one row; each thread owns EPT output
+// elements per pass, GROUP apart, so that B rows and C rows are read and written coalesced.
 template <typename I, int GROUP, int EPT>
 __global__ void __launch_bounds__(BSPMM_THREADS)
 bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float *__restrict__ val, int64_t nrows,
@@ -68,7 +68,8 @@ bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const fl
   }
 }
 
-// The same with 16-byte accesses, for fibers whose length is a multiple of four (and 16-byte aligned arrays): a
+// Rows of up to 256 elements with 16-byte accesses, for fibers whose length is a multiple of four (and 16-byte aligned
+// arrays): a
 // thread owns four consecutive output elements, which lie in one fiber, so one float4 of the entry's values
 // meets one float4 of the B row.  Four stored entries are in flight per thread; the adds stay in entry order.
 template <typename I, int GROUP>
@@ -113,29 +114,136 @@ bspmm_csrv_vec4_kernel(const I *__restrict__ pos, const I *__restrict__ crd, con
   }
 }
 
+__device__ __forceinline__ float madd(float a, float b, float c) { return __fadd_rn(__fmul_rn(a, b), c); }
+
+// The same for short rows and for fibers that are no multiple of four: G threads share one row; a thread owns Q groups of V
+// neighbouring output elements, G groups apart, with U stored entries in flight; the adds stay in entry order.  V = 4:
+// 16-byte accesses to B and C, the values of the elements' fibers one by one, or with FIBER4 (nh a multiple of four) also by
+// 16 bytes: taken for rows of more than 256 elements, where 40 registers and twelve blocks an SM keep more gathers in
+// flight than bspmm_csrv_vec4_kernel's 48 (131,072 rows of 32, 8 x 64: 1217 -> 1056 us; 20,000 of 30, 16 x 128: 558 -> 487).  Bound by the gathers of rows of B; G
+// follows the row's length, so that short rows do not leave most of a warp idle (50,000 rows of 20, 4 elements each: 84 -> 17
+// us; 200,000 rows of 8, 2 x 4: 155 -> 28), and wide accesses halve the requests (50,000 rows of 20, 1 x 64: 85 -> 48; 30,000 of
+// 30, 11 x 40: 269 -> 235; 20,000 of 30, 15 x 128: 718 -> 676).
+template <typename I, int V, bool FIBER4, int G, int Q>
+__global__ void __launch_bounds__(BSPMM_THREADS, FIBER4 ? 12 : 6)
+bspmm_csrv_group_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float *__restrict__ val, int64_t nrows,
+                  int64_t nh, int64_t E, const float *__restrict__ B, float *__restrict__ C, int accumulate) {
+  constexpr int U = V == 4 ? 4 : 8 / Q;
+  const int g = threadIdx.x % G;
+  const int64_t row = (int64_t)blockIdx.x * (BSPMM_THREADS / G) + threadIdx.x / G;
+  if (row >= nrows) return;
+  const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
+  float *crow = C + row * E;
+  for (int64_t e0 = (int64_t)g * V; e0 < E; e0 += G * Q * V) {
+    bool in[Q];
+    int64_t fiber[Q][FIBER4 ? 1 : V];
+    alignas(16) float acc[Q][V];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int64_t e = e0 + q * G * V;
+      in[q] = q == 0 || e < E;
+      fiber[q][0] = e % nh;
+#pragma unroll
+      for (int i = 1; i < (FIBER4 ? 1 : V); ++i) fiber[q][i] = fiber[q][i - 1] + 1 == nh ? 0 : fiber[q][i - 1] + 1;
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[q][i] = 0.0f;
+      if (accumulate && in[q]) {
+        if (V == 4) *reinterpret_cast<float4 *>(acc[q]) = *reinterpret_cast<const float4 *>(crow + e);
+        else acc[q][0] = crow[e];
+      }
+    }
+    auto fetch = [&](int64_t j, int64_t c, float(&a)[Q][V], float(&b)[Q][V]) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const float *v = val + j * nh, *brow = B + c * E + e0 + q * G * V;
+        if (FIBER4) *reinterpret_cast<float4 *>(a[q]) = __ldg(reinterpret_cast<const float4 *>(v + fiber[q][0]));
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+          if (!FIBER4) a[q][i] = Q == 1 || in[q] ? __ldg(v + fiber[q][i]) : 0.0f;
+        if (V == 4) *reinterpret_cast<float4 *>(b[q]) = __ldg(reinterpret_cast<const float4 *>(brow));
+        else b[q][0] = Q == 1 || in[q] ? __ldg(brow) : 0.0f;
+      }
+    };
+    int64_t j = lo;
+    for (; j + U <= hi; j += U) {
+      alignas(16) float a[U][Q][V], b[U][Q][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u) fetch(j + u, (int64_t)crd[j + u], a[u], b[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[q][i] = madd(a[u][q][i], b[u][q][i], acc[q][i]);
+    }
+    for (; j < hi; ++j) {
+      alignas(16) float a[Q][V], b[Q][V];
+      fetch(j, (int64_t)crd[j], a, b);
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[q][i] = madd(a[q][i], b[q][i], acc[q][i]);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (in[q]) {
+        float *c = crow + e0 + q * G * V;
+        if (V == 4) *reinterpret_cast<float4 *>(c) = *reinterpret_cast<const float4 *>(acc[q]);
+        else c[0] = acc[q][0];
+      }
+  }
+}
+
 template <typename I>
-static void launch_bspmm(const void *pos, const void *crd, const float *val, int64_t nrows, int64_t nh, int64_t E,
-                         const float *B, float *C, int accumulate, cudaStream_t st) {
-  const I *p = static_cast<const I *>(pos), *c = static_cast<const I *>(crd);
-  const bool vec4 = nh % 4 == 0 && nh / 4 <= 0x7fffffff &&
-                    ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) % 16 == 0);
-  if (vec4) {
-    const float4 *v4 = reinterpret_cast<const float4 *>(val), *B4 = reinterpret_cast<const float4 *>(B);
-    float4 *C4 = reinterpret_cast<float4 *>(C);
-    if (E / 4 <= 32)
-      bspmm_csrv_vec4_kernel<I, 32><<<(unsigned)((nrows + 3) / 4), BSPMM_THREADS, 0, st>>>(p, c, v4, nrows, (int)(nh / 4), E / 4,
-                                                                                          B4, C4, accumulate);
-    else
-      bspmm_csrv_vec4_kernel<I, 128><<<(unsigned)nrows, BSPMM_THREADS, 0, st>>>(p, c, v4, nrows, (int)(nh / 4), E / 4, B4, C4,
-                                                                                accumulate);
-    return;
-  }
-  if (E <= 128) {
-    const unsigned grid = (unsigned)((nrows + 3) / 4);
-    bspmm_csrv_kernel<I, 32, 4><<<grid, BSPMM_THREADS, 0, st>>>(p, c, val, nrows, nh, E, B, C, accumulate);
-  } else {
-    bspmm_csrv_kernel<I, 128, 4><<<(unsigned)nrows, BSPMM_THREADS, 0, st>>>(p, c, val, nrows, nh, E, B, C, accumulate);
-  }
+struct BspmmArgs {
+  const I *pos, *crd;
+  const float *val;
+  int64_t nrows, nh, E;
+  const float *B;
+  float *C;
+  int accumulate;
+};
+
+template <typename I, int G>
+static void launch_bspmm_vec4(const BspmmArgs<I> &m, cudaStream_t st) {
+  constexpr int ROWS = BSPMM_THREADS / G;
+  bspmm_csrv_vec4_kernel<I, G><<<(unsigned)((m.nrows + ROWS - 1) / ROWS), BSPMM_THREADS, 0, st>>>(
+      m.pos, m.crd, reinterpret_cast<const float4 *>(m.val), m.nrows, (int)(m.nh / 4), m.E / 4, reinterpret_cast<const float4 *>(m.B),
+      reinterpret_cast<float4 *>(m.C), m.accumulate);
+}
+
+template <typename I, int V, bool FIBER4, int G, int Q>
+static void launch_bspmm_group(const BspmmArgs<I> &m, cudaStream_t st) {
+  constexpr int ROWS = BSPMM_THREADS / G;
+  bspmm_csrv_group_kernel<I, V, FIBER4, G, Q><<<(unsigned)((m.nrows + ROWS - 1) / ROWS), BSPMM_THREADS, 0, st>>>(
+      m.pos, m.crd, m.val, m.nrows, m.nh, m.E, m.B, m.C, m.accumulate);
+}
+
+template <typename I>
+static void launch_bspmm(const BspmmArgs<I> &m, cudaStream_t st) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(m.B) | reinterpret_cast<uintptr_t>(m.C)) % 16 == 0;
+  const int64_t E = m.E, E4 = m.E / 4;
+  if (aligned && m.nh % 4 == 0 && m.nh / 4 <= 0x7fffffff && reinterpret_cast<uintptr_t>(m.val) % 16 == 0) {
+    if (E4 <= 4) launch_bspmm_vec4<I, 4>(m, st);
+    else if (E4 <= 8) launch_bspmm_vec4<I, 8>(m, st);
+    else if (E4 <= 16) launch_bspmm_vec4<I, 16>(m, st);
+    else if (E4 <= 32) launch_bspmm_vec4<I, 32>(m, st);
+    else if (E4 <= 64) launch_bspmm_vec4<I, 64>(m, st);
+    else launch_bspmm_group<I, 4, true, 128, 1>(m, st);
+  } else if (aligned && E % 4 == 0) {
+    if (E4 <= 4) launch_bspmm_group<I, 4, false, 4, 1>(m, st);
+    else if (E4 <= 8) launch_bspmm_group<I, 4, false, 8, 1>(m, st);
+    else if (E4 <= 16) launch_bspmm_group<I, 4, false, 16, 1>(m, st);
+    else if (E4 <= 32) launch_bspmm_group<I, 4, false, 32, 1>(m, st);
+    else if (E4 <= 64) launch_bspmm_group<I, 4, false, 64, 1>(m, st);
+    else launch_bspmm_group<I, 4, false, 128, 1>(m, st);
+  } else if (E <= 8) launch_bspmm_group<I, 1, false, 8, 1>(m, st);
+  else if (E <= 16) launch_bspmm_group<I, 1, false, 16, 1>(m, st);
+  else if (E <= 32) launch_bspmm_group<I, 1, false, 32, 1>(m, st);
+  else if (E <= 64) launch_bspmm_group<I, 1, false, 32, 2>(m, st);
+  else if (E <= 128) launch_bspmm_group<I, 1, false, 32, 4>(m, st);
+  else
+    bspmm_csrv_kernel<I, 128, 4><<<(unsigned)m.nrows, BSPMM_THREADS, 0, st>>>(m.pos, m.crd, m.val, m.nrows, m.nh, E, m.B, m.C, m.accumulate);
 }
 
 }  // namespace lapis_b200
@@ -153,10 +261,12 @@ extern "C" int lapis_b200_bspmm_csrv_f32(int idx_bytes, int64_t n1, int64_t n2, 
   if (n1 == 0 || E == 0) return LAPIS_OK;
   if (d_pos == nullptr || d_C == nullptr) return fail(LAPIS_EBADARG, "bspmm: null operand");
   cudaStream_t st = as_stream(stream);
-  if (idx_bytes == 4)
-    launch_bspmm<int32_t>(d_pos, d_crd, d_val, n1, nh, E, d_B, d_C, accumulate, st);
-  else
-    launch_bspmm<int64_t>(d_pos, d_crd, d_val, n1, nh, E, d_B, d_C, accumulate, st);
+  auto run = [&](auto index) {
+    using I = decltype(index);
+    launch_bspmm<I>({static_cast<const I *>(d_pos), static_cast<const I *>(d_crd), d_val, n1, nh, E, d_B, d_C, accumulate}, st);
+  };
+  if (idx_bytes == 4) run(int32_t());
+  else run(int64_t());
   LAPIS_CUDA_TRY(cudaGetLastError());
   return LAPIS_OK;
 }

@@ -248,3 +248,23 @@ def test_small_pcg_over_several_launches():
     assert it == 4200 and 0 <= rel < 1e-14
     y, _, _ = A.pcg(b, dinv, 1e-12, 4000)
     assert float((x - y).norm()) <= 1e-8 * float(y.norm())
+
+
+@pytest.mark.parametrize("nh,dh", [(1, 1), (1, 5), (1, 8), (1, 64), (2, 9), (2, 10), (3, 20), (3, 43), (4, 1), (4, 4), (4, 5), (4, 17), (5, 13), (6, 64),
+                                   (7, 33), (8, 30), (8, 64), (11, 40), (12, 47), (13, 41), (15, 128)])
+def test_bspmm_widths(nh, dh):
+    """Every width the rule tells apart, operands on and off 16-byte boundaries: bit for bit."""
+    from lapis_b200.device import bspmm_csrv
+    dev = _dev()
+    rng = np.random.default_rng(nh * dh)
+    n = 333
+    for idx in (np.int32, np.int64):
+        pos, crd, _ = _csr(rng, rng.integers(0, 23, n), n, idx)
+        val, B = rng.uniform(-1, 1, crd.size * nh).astype(np.float32), rng.uniform(-1, 1, (n, dh, nh)).astype(np.float32)
+        want = oracle.bspmm(pos, crd, val, B)
+        for shift in (0, 1):
+            v, b = (torch.empty(a.size + shift, dtype=torch.float32, device=dev)[shift:].view(a.shape) for a in (val, B))
+            v.copy_(torch.as_tensor(val))
+            b.copy_(torch.as_tensor(B))
+            got = bspmm_csrv(torch.as_tensor(pos).to(dev), torch.as_tensor(crd).to(dev), v, b, n)
+            assert np.array_equal(got.cpu().numpy(), want)
