@@ -794,7 +794,7 @@ def run_formats(args):
     t0 = time.perf_counter()
     oracle.bspmm(sp["pos"][:rows_cpu + 1], sp["crd"][:end], val[:end * nh], B)
     cpu_ms = (time.perf_counter() - t0) * 1e3 * n / rows_cpu
-    line("bspmm_csrv_kernel", f"CSRV {n} x {n}, 32 per row, nh 8, dh 64, fp32, int32 indices", ms,
+    line("bspmm_csrv_group_kernel", f"CSRV {n} x {n}, 32 per row, nh 8, dh 64, fp32, int32 indices", ms,
          nnz * (4 + 4 * nh) + 4 * (n + 1) + 3 * 4 * n * dh * nh, cpu_ms,
          {"gathered_B_bytes": nnz * dh * nh * 4, "cpu_sample": f"first {rows_cpu} rows, scaled by rows"})
     del dB, C, dval
