@@ -9,6 +9,7 @@
 #include <memory>
 #include <mutex>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include <immintrin.h>
@@ -179,15 +180,18 @@ bool page_locked(const void *p) {
   return a.type == cudaMemoryTypeHost;
 }
 
+// Neighbours are compared, never subtracted in the signed type: a corrupt array may hold offsets whose difference does
+// not fit it and wraps to a plausible length.
 template <typename I>
 void check_pos(const I *pos, int64_t from, int64_t to, int64_t *max_len, int64_t *bad_row) {
+  using U = std::make_unsigned_t<I>;
   I longest = 0, bad = 0;
   for (int64_t i = std::max<int64_t>(from, 1); i < to; ++i) {
-    const I len = pos[i] - pos[i - 1];
+    const I len = (I)((U)pos[i] - (U)pos[i - 1]);
     longest = len > longest ? len : longest;
-    bad |= len;
+    bad |= (I)(pos[i] < pos[i - 1]);
   }
-  if (bad < 0)
+  if (bad != 0)
     for (int64_t i = std::max<int64_t>(from, 1); i < to; ++i)
       if (pos[i] < pos[i - 1]) {
         *bad_row = i - 1;

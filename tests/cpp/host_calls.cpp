@@ -1,0 +1,194 @@
+// The calls on host arrays (abi.cu, stage.cu) over a stand-in CUDA runtime in which device memory is host memory, and
+// stand-ins for the kernels: what they do before a launch and after one, on a machine without a GPU.
+//
+//   host_calls <scenario>     prints "ok" and returns 0, or names what did not hold
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <limits>
+#include <mutex>
+#include <set>
+#include <string>
+#include <vector>
+
+#include "../../lapis_b200/csrc/abi.cu"
+#include "../../lapis_b200/csrc/stage.cu"
+
+#define EXPECT(cond)                                                              \
+  do {                                                                            \
+    if (!(cond)) {                                                                \
+      std::printf("%s:%d: %s does not hold (last error: %d %s)\n", __FILE__, __LINE__, #cond, lapis_last_error(), \
+                  lapis_last_error_message());                                    \
+      std::exit(1);                                                               \
+    }                                                                             \
+  } while (0)
+
+// ---- the stand-in runtime ----------------------------------------------------------------------------------------
+static std::mutex g_fake;
+static std::set<void *> g_device, g_locked;  // live device allocations, page-locked host blocks
+static int g_in_place = 0;                   // copies from page-locked memory that no synchronisation has covered
+static int g_launches = 0;                   // calls into the kernels
+static int g_kernel_status = LAPIS_OK;       // what the kernels return
+static std::vector<char *> g_page_locked;    // blocks of a caller, LOCKED_BYTES each
+constexpr size_t LOCKED_BYTES = size_t(4) << 20;
+
+static bool of_caller(const void *p) {
+  for (char *b : g_page_locked)
+    if (p >= b && p < b + LOCKED_BYTES) return true;
+  return false;
+}
+
+extern "C" {
+cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { return *v = 148, cudaSuccess; }
+cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
+cudaError_t cudaMalloc(void **p, size_t n) {
+  std::lock_guard<std::mutex> l(g_fake);
+  *p = std::malloc(n);
+  g_device.insert(*p);
+  return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+  std::lock_guard<std::mutex> l(g_fake);
+  if (p != nullptr) EXPECT(g_device.erase(p) == 1);
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMemPoolCreate(cudaMemPool_t *pool, const cudaMemPoolProps *) { return *pool = (cudaMemPool_t)1, cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) { return cudaMalloc(p, n); }
+cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+  std::lock_guard<std::mutex> l(g_fake);
+  *p = std::aligned_alloc(4096, n);
+  g_locked.insert(*p);
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p) {
+  std::lock_guard<std::mutex> l(g_fake);
+  EXPECT(g_locked.erase(p) == 1);
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return *e = (cudaEvent_t)1, cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
+  a->type = of_caller(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(to, from, n);
+  std::lock_guard<std::mutex> l(g_fake);
+  if (of_caller(from)) ++g_in_place;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+  std::lock_guard<std::mutex> l(g_fake);
+  g_in_place = 0;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize(void) { return cudaStreamSynchronize(nullptr); }
+
+// ---- the stand-in kernels: y = A x and C = A B on the host, the others only count ---------------------------------
+static int launched() { return __atomic_add_fetch(&g_launches, 1, __ATOMIC_SEQ_CST), g_kernel_status; }
+int lapis_b200_spmv_f64(lapis_b200_csr_t h, const double *x, double *y, int, void *) {
+  for (int64_t r = 0; h->idx_bytes == 8 && g_kernel_status == LAPIS_OK && r < h->nrows; ++r) {
+    const int64_t *pos = static_cast<const int64_t *>(h->pos), *crd = static_cast<const int64_t *>(h->crd);
+    for (int64_t j = pos[r]; j < pos[r + 1]; ++j) y[r] += h->val[j] * x[crd[j]];
+  }
+  return launched();
+}
+int lapis_b200_spmm_f64(lapis_b200_csr_t, int64_t, const double *, double *, int, void *) { return launched(); }
+int lapis_b200_bgemm_f32(int64_t, int64_t, int64_t, int64_t, const float *, const float *, float *, void *) { return launched(); }
+int lapis_b200_bgemm_status(void *) { return LAPIS_OK; }
+int lapis_b200_pcg_f64(lapis_b200_csr_t, const double *, const double *, double, uint64_t, double *, uint64_t *, double *, void *) {
+  return launched();
+}
+int lapis_b200_mht_f64(lapis_b200_csr_t, const double *, const double *, double, double, uint64_t, double *, double *, uint64_t *,
+                       double *, void *) {
+  return launched();
+}
+int lapis_b200_normalize_mom2_f64(int64_t, const double *, const double *, double *, void *) { return launched(); }
+int lapis_b200_bspmm_csrv_f32(int, int64_t, int64_t, int64_t, int64_t, const void *, const void *, const float *, const float *, float *,
+                              int, void *) {
+  return launched();
+}
+int lapis_b200_spmm_dcsr_f64(int, int64_t, int64_t, int64_t, int64_t, const void *, const void *, const void *, const double *,
+                             const double *, double *, void *) {
+  return launched();
+}
+}  // extern "C"
+
+namespace lapis_b200 {
+int csr_setup(lapis_b200_csr *h, int idx_bytes, int64_t nrows, int64_t ncols, int64_t base, int64_t nnz, int64_t max_row_len,
+              const void *pos, const void *crd, const double *val, bool, PoolBuf *, cudaStream_t) {
+  *h = lapis_b200_csr{};
+  h->idx_bytes = idx_bytes;
+  h->nrows = nrows;
+  h->ncols = ncols;
+  h->base = base;
+  h->nnz = nnz;
+  h->max_row_len = max_row_len;
+  h->pos = pos;
+  h->crd = crd;
+  h->val = val;
+  return LAPIS_OK;
+}
+}  // namespace lapis_b200
+
+// ---- scenarios ---------------------------------------------------------------------------------------------------
+template <typename T>
+static lapis_memref1 ref(std::vector<T> &v) {
+  return {v.data(), v.data(), 0, {(int64_t)v.size()}, {1}};
+}
+static lapis_memref2 ref2(std::vector<double> &v, int64_t rows, int64_t cols) {
+  return {v.data(), v.data(), 0, {rows, cols}, {cols, 1}};
+}
+
+// Offsets whose differences leave the index type: refused before any kernel, wherever in the array they are.
+template <typename I>
+static void offsets(void (*spmm)(lapis_memref2 **, lapis_memref1 *, lapis_memref1 *, lapis_memref1 *, const lapis_csr_spec *, lapis_memref2 *,
+                                 lapis_memref2 *)) {
+  const I top = std::numeric_limits<I>::max(), low = std::numeric_limits<I>::min();
+  const std::vector<std::vector<I>> middles = {{top, -2}, {top, low, -5}, {low}, {-1}, {top, low + 1, low}, {7, 3}, {top}, {11}};
+  const int64_t nnz = 10, per_block = 65536 / sizeof(I);
+  for (int64_t at : {(int64_t)1, (int64_t)5, per_block - 1, per_block, 9 * per_block - 1, 20 * per_block})
+    for (const auto &m : middles) {
+      std::vector<I> pos(at, 0), crd(nnz, 0);
+      pos.insert(pos.end(), m.begin(), m.end());
+      pos.push_back((I)nnz);
+      const int64_t rows = (int64_t)pos.size() - 1;
+      std::vector<double> val(nnz, 1.0), B(3, 1.0), C(rows, 0.0);
+      lapis_memref1 p = ref(pos), c = ref(crd), v = ref(val);
+      lapis_memref2 b = ref2(B, 3, 1), out = ref2(C, rows, 1);
+      const lapis_csr_spec spec = {{rows, 3}, {rows + 1, nnz, nnz}};
+      spmm(nullptr, &p, &c, &v, &spec, &b, &out);
+      EXPECT(lapis_last_error() == LAPIS_EBADSHAPE && g_launches == 0);
+      for (size_t i = 0; i < m.size(); ++i) pos[at + i] = 4;  // the same array, mended
+      spmm(nullptr, &p, &c, &v, &spec, &b, &out);
+      EXPECT(lapis_last_error() == LAPIS_OK && g_launches == 1);
+      g_launches = 0;
+    }
+}
+
+int main(int argc, char **argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  lapis_initialize();
+  if (what == "offsets") {
+    offsets<int32_t>(py_spmm_f64_i32);
+    offsets<int64_t>(py_spmm_f64_i64);
+  } else {
+    std::printf("unknown scenario '%s'\n", what.c_str());
+    return 1;
+  }
+  lapis_finalize();
+  EXPECT(g_device.empty());
+  std::printf("ok\n");
+  return 0;
+}
