@@ -207,18 +207,27 @@ static int result_vector(const void *d_src, int64_t n, lapis_memref1 *out, cudaS
   return LAPIS_OK;
 }
 
-// Operands of a call: laid out in one device allocation and sent there.  A failure leaves nothing in flight that still
-// reads the caller's arrays.
+// Operands of a call: laid out in one device allocation and sent there.  Page-locked arrays are copied in place, so a call
+// that fails after the upload waits for the stream before the caller has its arrays back; one that succeeds has waited
+// for its result.
 struct Operands {
   Upload up;
   PoolBuf dev;
+  bool in_flight = false;
+  ~Operands() {
+    if (in_flight) cudaStreamSynchronize(dev.st);
+  }
   int send(cudaStream_t st, Upload::Facts *facts, size_t extra = 0) {
     const size_t bytes = up.layout();
     extra_at = bytes;
     LAPIS_TRY(dev.alloc(bytes + extra, st));
-    const int rc = up.run(dev.p, st, facts);
-    if (rc != LAPIS_OK) cudaStreamSynchronize(st);
-    return rc;
+    in_flight = true;
+    return up.run(dev.p, st, facts);
+  }
+  // The last download's status goes through here.
+  int finish(int status) {
+    if (status == LAPIS_OK) in_flight = false;
+    return status;
   }
   template <typename T>
   T *at(int part) const {
@@ -233,18 +242,12 @@ struct Operands {
 
 // What the upload found out about the index arrays, as a status.
 template <typename I>
-static int check_facts(const Upload::Facts &f, const I *pos, const I *crd, int64_t nrows, int64_t nnz, int64_t ncols, cudaStream_t st) {
-  int rc = LAPIS_OK;
-  if (pos[0] != 0)
-    rc = fail(LAPIS_EBADSHAPE, "pos[0] must be 0");
-  else if (f.bad_row >= 0)
-    rc = fail(LAPIS_EBADSHAPE, "pos is not non-decreasing at row %lld", (long long)f.bad_row);
-  else if ((int64_t)pos[nrows] != nnz)
-    rc = fail(LAPIS_EBADSHAPE, "pos[rows] != number of stored entries");
-  else if (!f.crd_in_range)
-    rc = check_crd_host<I>(crd, nnz, ncols);  // finds the values for the message
-  if (rc != LAPIS_OK) cudaStreamSynchronize(st);
-  return rc;
+static int check_facts(const Upload::Facts &f, const I *pos, const I *crd, int64_t nrows, int64_t nnz, int64_t ncols) {
+  if (pos[0] != 0) return fail(LAPIS_EBADSHAPE, "pos[0] must be 0");
+  if (f.bad_row >= 0) return fail(LAPIS_EBADSHAPE, "pos is not non-decreasing at row %lld", (long long)f.bad_row);
+  if ((int64_t)pos[nrows] != nnz) return fail(LAPIS_EBADSHAPE, "pos[rows] != number of stored entries");
+  if (!f.crd_in_range) return check_crd_host<I>(crd, nnz, ncols);  // finds the values for the message
+  return LAPIS_OK;
 }
 
 // A CSR operand of a call: its three arrays among the uploaded parts, and the handle over them.
@@ -261,7 +264,7 @@ struct CsrOperand {
   template <typename I>
   int setup(const Operands &ops, const Upload::Facts &f, const lapis_memref1 *mpos, const lapis_memref1 *mcrd, const CsrArgs &a,
             bool plan_on_demand, cudaStream_t st) {
-    LAPIS_TRY((check_facts<I>(f, elem_ptr<I>(mpos), elem_ptr<I>(mcrd), a.nrows, a.nnz, a.ncols, st)));
+    LAPIS_TRY((check_facts<I>(f, elem_ptr<I>(mpos), elem_ptr<I>(mcrd), a.nrows, a.nnz, a.ncols)));
     return csr_setup(&h, (int)sizeof(I), a.nrows, a.ncols, 0, a.nnz, f.max_row_len, ops.at<void>(pos), ops.at<void>(crd),
                      ops.at<double>(val), plan_on_demand, &scratch, st);
   }
@@ -286,7 +289,7 @@ static int spmv_host(lapis_memref1 **ret0, lapis_memref1 *pos, lapis_memref1 *cr
   LAPIS_TRY(ops.send(st, &facts));
   LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, true, st));
   LAPIS_TRY(lapis_b200_spmv_f64(&A.h, ops.at<double>(px), ops.at<double>(py), 1, st));
-  LAPIS_TRY(stage_download(elem_ptr<double>(y), ops.at<double>(py), (size_t)a.nrows * 8, st));  // emitted fence, :2682
+  LAPIS_TRY(ops.finish(stage_download(elem_ptr<double>(y), ops.at<double>(py), (size_t)a.nrows * 8, st)));  // emitted fence, :2682
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *y;  // the function returns its outs argument
   return LAPIS_OK;
 }
@@ -313,7 +316,7 @@ static int spmm_host(lapis_memref2 **ret0, lapis_memref1 *pos, lapis_memref1 *cr
   LAPIS_TRY(ops.send(st, &facts));
   LAPIS_TRY(A.setup<I>(ops, facts, pos, crd, a, true, st));
   LAPIS_TRY(lapis_b200_spmm_f64(&A.h, k, ops.at<double>(pB), ops.at<double>(pC), 1, st));
-  LAPIS_TRY(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st));
+  LAPIS_TRY(ops.finish(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st)));
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *C;
   return LAPIS_OK;
 }
@@ -327,7 +330,7 @@ static int gemm_host(int64_t batch, int64_t M, int64_t N, int64_t K, const float
   LAPIS_TRY(ops.send(st, &facts));
   LAPIS_TRY(lapis_b200_bgemm_f32(batch, M, N, K, ops.at<float>(pA), ops.at<float>(pB), ops.at<float>(pC), st));
   LAPIS_TRY(lapis_b200_bgemm_status(st));
-  return stage_download(C, ops.at<float>(pC), bC, st);
+  return ops.finish(stage_download(C, ops.at<float>(pC), bC, st));
 }
 
 template <typename I>
@@ -355,7 +358,7 @@ static int pcg_host(lapis_memref1 **ret0, size_t *ret1, double *ret2, lapis_memr
   uint64_t iters = 0;
   double relres = 0.0;
   LAPIS_TRY(lapis_b200_pcg_f64(&A.h, ops.at<double>(pb), ops.at<double>(pd), tol, (uint64_t)maxiter, dx, &iters, &relres, st));
-  LAPIS_TRY(result_vector(dx, n, *ret0, st));
+  LAPIS_TRY(ops.finish(result_vector(dx, n, *ret0, st)));
   if (ret1) *ret1 = (size_t)iters;
   if (ret2) *ret2 = relres;
   return LAPIS_OK;
@@ -387,7 +390,7 @@ static int mht_host(lapis_memref1 **ret0, lapis_memref1 **ret1, lapis_memref1 *p
   double *m1 = ops.extra<double>(), *m2 = m1 + n;
   LAPIS_TRY(lapis_b200_mht_f64(&A.h, ops.at<double>(pm), ops.at<double>(pd), alpha, tol, (uint64_t)maxiter, m1, m2, nullptr, nullptr, st));
   LAPIS_TRY(result_vector(m1, n, *ret0, st));
-  return result_vector(m2, n, *ret1, st);
+  return ops.finish(result_vector(m2, n, *ret1, st));
 }
 
 // examples/hitting_times.py:196-218 (@normalize_mom2), call at :218
@@ -405,7 +408,7 @@ static int normalize_mom2_host(lapis_memref1 **ret0, lapis_memref1 *mom1, lapis_
   Upload::Facts facts;
   LAPIS_TRY(ops.send(st, &facts, (size_t)n * 8));
   LAPIS_TRY(lapis_b200_normalize_mom2_f64(n, ops.at<double>(p1), ops.at<double>(p2), ops.extra<double>(), st));
-  return result_vector(ops.extra<double>(), n, *ret0, st);
+  return ops.finish(result_vector(ops.extra<double>(), n, *ret0, st));
 }
 
 // examples/bspmm.py:26-52, call at :103
@@ -436,13 +439,13 @@ static int bspmm_host(lapis_memref3 **ret0, lapis_memref1 *pos, lapis_memref1 *c
   const int pval = ops.up.add(elem_ptr<float>(val), (size_t)nval * 4), pB = ops.up.add(elem_ptr<float>(B), (size_t)n2 * dh * nh * 4);
   Upload::Facts facts;
   LAPIS_TRY(ops.send(st, &facts, bC));
-  LAPIS_TRY(check_facts<I>(facts, hpos, hcrd, n1, nnz, n2, st));
+  LAPIS_TRY(check_facts<I>(facts, hpos, hcrd, n1, nnz, n2));
   LAPIS_TRY(lapis_b200_bspmm_csrv_f32((int)sizeof(I), n1, n2, nh, dh, ops.at<void>(ppos), ops.at<void>(pcrd), ops.at<float>(pval),
                                       ops.at<float>(pB), ops.extra<float>(), 0, st));
   float *hc = static_cast<float *>(std::malloc(bC > 0 ? bC : 8));
   if (hc == nullptr) return fail(LAPIS_ECUDA, "bspmm: host allocation failed");
   g_alive_host.push_back(hc);
-  LAPIS_TRY(stage_download(hc, ops.extra<float>(), bC, st));
+  LAPIS_TRY(ops.finish(stage_download(hc, ops.extra<float>(), bC, st)));
   lapis_memref3 out;
   out.basePtr = hc;
   out.data = hc;
@@ -492,10 +495,10 @@ static int spmm_dcsr_host(lapis_memref2 **ret0, lapis_memref1 *p1, lapis_memref1
   const int pB = ops.up.add(elem_ptr<double>(B), (size_t)ncols * k * 8), pC = ops.up.add(elem_ptr<double>(C), bC);
   Upload::Facts facts;
   LAPIS_TRY(ops.send(st, &facts));
-  LAPIS_TRY(check_facts<I>(facts, hp2, hi2, nstored, nnz, ncols, st));
+  LAPIS_TRY(check_facts<I>(facts, hp2, hi2, nstored, nnz, ncols));
   LAPIS_TRY(lapis_b200_spmm_dcsr_f64((int)sizeof(I), nrows, ncols, nstored, k, ops.at<void>(pi1), ops.at<void>(pp2), ops.at<void>(pi2),
                                      ops.at<double>(pval), ops.at<double>(pB), ops.at<double>(pC), st));
-  LAPIS_TRY(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st));
+  LAPIS_TRY(ops.finish(stage_download(elem_ptr<double>(C), ops.at<double>(pC), bC, st)));
   if (ret0 != nullptr && *ret0 != nullptr) **ret0 = *C;
   return LAPIS_OK;
 }

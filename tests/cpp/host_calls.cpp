@@ -26,7 +26,7 @@
 // ---- the stand-in runtime ----------------------------------------------------------------------------------------
 static std::mutex g_fake;
 static std::set<void *> g_device, g_locked;  // live device allocations, page-locked host blocks
-static int g_in_place = 0;                   // copies from page-locked memory that no synchronisation has covered
+static int g_copies = 0, g_waited = 0;       // copies from page-locked memory so far; how many of them were waited for
 static int g_launches = 0;                   // calls into the kernels
 static int g_kernel_status = LAPIS_OK;       // what the kernels return
 static std::vector<char *> g_page_locked;    // blocks of a caller, LOCKED_BYTES each
@@ -74,10 +74,24 @@ cudaError_t cudaFreeHost(void *p) {
   std::free(p);
   return cudaSuccess;
 }
-cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return *e = (cudaEvent_t)1, cudaSuccess; }
-cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+  *e = reinterpret_cast<cudaEvent_t>(new int(0));  // an event: the copies in front of it
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  delete reinterpret_cast<int *>(e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+  std::lock_guard<std::mutex> l(g_fake);
+  *reinterpret_cast<int *>(e) = g_copies;
+  return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+  std::lock_guard<std::mutex> l(g_fake);
+  g_waited = std::max(g_waited, *reinterpret_cast<int *>(e));
+  return cudaSuccess;
+}
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
   a->type = of_caller(p) ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
   return cudaSuccess;
@@ -85,18 +99,21 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
 cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t n, cudaMemcpyKind, cudaStream_t) {
   std::memcpy(to, from, n);
   std::lock_guard<std::mutex> l(g_fake);
-  if (of_caller(from)) ++g_in_place;
+  if (of_caller(from)) ++g_copies;
   return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) {
   std::lock_guard<std::mutex> l(g_fake);
-  g_in_place = 0;
+  g_waited = g_copies;
   return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize(void) { return cudaStreamSynchronize(nullptr); }
 
 // ---- the stand-in kernels: y = A x and C = A B on the host, the others only count ---------------------------------
-static int launched() { return __atomic_add_fetch(&g_launches, 1, __ATOMIC_SEQ_CST), g_kernel_status; }
+static int launched() {
+  __atomic_add_fetch(&g_launches, 1, __ATOMIC_SEQ_CST);
+  return g_kernel_status == LAPIS_OK ? LAPIS_OK : lapis_b200::fail(g_kernel_status, "as asked");
+}
 int lapis_b200_spmv_f64(lapis_b200_csr_t h, const double *x, double *y, int, void *) {
   for (int64_t r = 0; h->idx_bytes == 8 && g_kernel_status == LAPIS_OK && r < h->nrows; ++r) {
     const int64_t *pos = static_cast<const int64_t *>(h->pos), *crd = static_cast<const int64_t *>(h->crd);
@@ -177,12 +194,56 @@ static void offsets(void (*spmm)(lapis_memref2 **, lapis_memref1 *, lapis_memref
     }
 }
 
+// A call that fails behind the upload: page-locked operands, which are copied in place, are no longer being read when it
+// returns.
+template <typename T>
+static T *page_locked_block() {
+  g_page_locked.push_back(static_cast<char *>(std::aligned_alloc(4096, LOCKED_BYTES)));
+  std::memset(g_page_locked.back(), 0, LOCKED_BYTES);
+  return reinterpret_cast<T *>(g_page_locked.back());
+}
+static void in_flight() {
+  const int64_t n = 200000;  // 1.6 MB a vector
+  int64_t *pos = page_locked_block<int64_t>(), *crd = page_locked_block<int64_t>();
+  double *val = page_locked_block<double>(), *x = page_locked_block<double>(), *y = page_locked_block<double>();
+  for (int64_t i = 0; i <= n; ++i) pos[i] = i;
+  int64_t two[2] = {0, n};
+  lapis_memref1 p = {pos, pos, 0, {n + 1}, {1}}, c = {crd, crd, 0, {n}, {1}}, v = {val, val, 0, {n}, {1}}, p1 = {two, two, 0, {2}, {1}};
+  lapis_memref1 xv = {x, x, 0, {n}, {1}}, yv = {y, y, 0, {n}, {1}}, i1 = {pos, pos, 0, {n}, {1}};
+  lapis_memref2 xm = {x, x, 0, {n, 1}, {1, 1}}, ym = {y, y, 0, {n, 1}, {1, 1}}, one = {val, val, 0, {1, 1}, {1, 1}};
+  lapis_memref3 xb = {x, x, 0, {n, 1, 1}, {1, 1, 1}}, ob;
+  lapis_memref1 o1, o2, *r1 = &o1, *r2 = &o2;
+  lapis_memref3 *r3 = &ob;
+  const lapis_csr_spec spec = {{n, n}, {n + 1, n, n}};
+  const lapis_csrv_spec vspec = {{n, n, 1}, {n + 1, n, n}};
+  const lapis_dcsr_spec dspec = {{n, n}, {2, n, n + 1, n, n}};
+  for (int status : {LAPIS_ECUDA, LAPIS_OK}) {
+    g_kernel_status = status;
+    auto after = [&](const char *call) {
+      const bool quiet = g_copies > 0 && g_waited == g_copies;
+      if (!quiet || lapis_last_error() != status) std::printf("%s: status %d\n", call, status);
+      EXPECT(quiet && lapis_last_error() == status && g_launches == 1);
+      g_launches = 0;
+    };
+    py_spmv_f64_i64(nullptr, &p, &c, &v, &spec, &xv, &yv), after("spmv");
+    py_spmm_f64_i64(nullptr, &p, &c, &v, &spec, &xm, &ym), after("spmm");
+    py_matmul_f32(nullptr, &xm, &one, &ym), after("matmul");
+    py_pcg_f64_i64(&r1, nullptr, nullptr, &p, &c, &v, &spec, &xv, &yv, 0.0, 1), after("pcg");
+    py_mht_f64_i64(&r1, &r2, &p, &c, &v, &spec, &xv, &yv, 0.5, 0.0, 1), after("mht");
+    py_normalize_mom2_f64(&r1, &xv, &yv), after("normalize_mom2");
+    py_bspmm_f32_i64(&r3, &p, &c, &v, &vspec, &xb), after("bspmm");
+    py_spmm_dcsr_f64_i64(nullptr, &p1, &i1, &p, &c, &v, &dspec, &xm, &ym), after("spmm_dcsr");
+  }
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   lapis_initialize();
   if (what == "offsets") {
     offsets<int32_t>(py_spmm_f64_i32);
     offsets<int64_t>(py_spmm_f64_i64);
+  } else if (what == "in_flight") {
+    in_flight();
   } else {
     std::printf("unknown scenario '%s'\n", what.c_str());
     return 1;

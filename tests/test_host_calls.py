@@ -23,7 +23,8 @@ def program(tmp_path_factory):
 
 
 # offsets: differences that wrap around the index type must not pass as row lengths
-@pytest.mark.parametrize("scenario", ["offsets"])
+# in_flight: a call that fails behind the upload leaves no copy from the caller's page-locked arrays under way
+@pytest.mark.parametrize("scenario", ["offsets", "in_flight"])
 def test_host_calls(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
