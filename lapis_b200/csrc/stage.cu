@@ -40,23 +40,18 @@ struct Job {
 };
 
 // Threads that sleep until there is a job.  A job is complete whether or not they wake up in time for it.
+// They are detached and the pool is never destroyed: a child process forked after the first large call has no such
+// threads to join at its exit.
 class HelperPool {
  public:
-  ~HelperPool() {
-    {
-      std::lock_guard<std::mutex> lock(m_);
-      stop_ = true;
-    }
-    wake_.notify_all();
-    for (std::thread &t : threads_) t.join();
-  }
   void run(const std::shared_ptr<Job> &job, size_t bytes) {
     if (bytes >= HELPED_BYTES) {
       {
         std::lock_guard<std::mutex> lock(m_);
-        if (threads_.empty()) {
+        if (!started_) {
+          started_ = true;
           const int n = std::min<int>(HELPERS, (int)std::thread::hardware_concurrency() - 1);
-          for (int i = 0; i < n; ++i) threads_.emplace_back([this] { loop(); });
+          for (int i = 0; i < n; ++i) std::thread([this] { loop(); }).detach();
         }
         job_ = job;
         ++round_;
@@ -74,8 +69,7 @@ class HelperPool {
       std::shared_ptr<Job> job;
       {
         std::unique_lock<std::mutex> lock(m_);
-        wake_.wait(lock, [&] { return stop_ || round_ != seen; });
-        if (stop_) return;
+        wake_.wait(lock, [&] { return round_ != seen; });
         seen = round_;
         job = job_;
       }
@@ -84,10 +78,9 @@ class HelperPool {
   }
   std::mutex m_;
   std::condition_variable wake_;
-  std::vector<std::thread> threads_;
   std::shared_ptr<Job> job_;
   uint64_t round_ = 0;
-  bool stop_ = false;
+  bool started_ = false;
 };
 
 struct Ring {
@@ -142,8 +135,8 @@ struct Pieces {
 };
 
 HelperPool &helpers() {
-  static HelperPool pool;
-  return pool;
+  static HelperPool *pool = new HelperPool;
+  return *pool;
 }
 
 // Copies into a slot past the caches: the bus then reads memory instead of another core's dirty lines (a 1.9 MB call:

@@ -2,6 +2,7 @@
 // stand-ins for the kernels: what they do before a launch and after one, on a machine without a GPU.
 //
 //   host_calls <scenario>     prints "ok" and returns 0, or names what did not hold
+#include <csignal>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -10,6 +11,9 @@
 #include <set>
 #include <string>
 #include <vector>
+
+#include <sys/wait.h>
+#include <unistd.h>
 
 #include "../../lapis_b200/csrc/abi.cu"
 #include "../../lapis_b200/csrc/stage.cu"
@@ -236,6 +240,51 @@ static void in_flight() {
   }
 }
 
+// y = A x with one entry a row, large enough for the helper threads.
+struct Product {
+  int64_t n;
+  std::vector<int64_t> pos, crd;
+  std::vector<double> val, x, y;
+  explicit Product(int64_t rows) : n(rows), pos(rows + 1), crd(rows), val(rows), x(rows), y(rows) {
+    for (int64_t i = 0; i < n; ++i) pos[i + 1] = i + 1, crd[i] = n - 1 - i, val[i] = 2.0, x[i] = (double)i;
+  }
+  int run() {
+    std::fill(y.begin(), y.end(), 1.0);
+    lapis_memref1 p = ref(pos), c = ref(crd), v = ref(val), xv = ref(x), yv = ref(y);
+    const lapis_csr_spec spec = {{n, n}, {n + 1, n, n}};
+    py_spmv_f64_i64(nullptr, &p, &c, &v, &spec, &xv, &yv);
+    return lapis_last_error();
+  }
+  bool right() const {
+    for (int64_t i = 0; i < n; ++i)
+      if (y[i] != 1.0 + 2.0 * (double)(n - 1 - i)) return false;
+    return true;
+  }
+};
+
+// A child process forked behind a large call exits.
+static void fork_exit() {
+  Product a(300000);
+  EXPECT(a.run() == LAPIS_OK && a.right());
+  const pid_t child = fork();
+  if (child == 0) std::exit(0);
+  int status = -1;
+  for (int i = 0; i < 200 && waitpid(child, &status, WNOHANG) == 0; ++i) usleep(50000);
+  if (status == -1) kill(child, SIGKILL);
+  EXPECT(status == 0);
+}
+
+// Several threads in calls at once share one ring and one set of helpers.
+static void threads() {
+  std::vector<std::thread> pool;
+  for (int t = 0; t < 4; ++t)
+    pool.emplace_back([t] {
+      Product a(1000 + 90000 * t);
+      for (int i = 0; i < 25; ++i) EXPECT(a.run() == LAPIS_OK && a.right());
+    });
+  for (std::thread &t : pool) t.join();
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   lapis_initialize();
@@ -244,6 +293,10 @@ int main(int argc, char **argv) {
     offsets<int64_t>(py_spmm_f64_i64);
   } else if (what == "in_flight") {
     in_flight();
+  } else if (what == "fork_exit") {
+    fork_exit();
+  } else if (what == "threads") {
+    threads();
   } else {
     std::printf("unknown scenario '%s'\n", what.c_str());
     return 1;

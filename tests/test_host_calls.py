@@ -18,13 +18,15 @@ def program(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("host_calls") / "host_calls")
     env = {k: v for k, v in os.environ.items() if k not in ("CC", "CXX")}
     subprocess.run([gxx, "-std=c++17", "-O2", "-pthread", "-rdynamic", "-I", os.path.join(CUDA, "include"),
-                    os.path.join(ROOT, "tests", "cpp", "host_calls.cpp"), "-o", exe], check=True, env=env)
+                    os.path.join(ROOT, "tests", "cpp", "host_calls.cpp"), "-o", exe, "-ldl"], check=True, env=env)
     return exe
 
 
 # offsets: differences that wrap around the index type must not pass as row lengths
 # in_flight: a call that fails behind the upload leaves no copy from the caller's page-locked arrays under way
-@pytest.mark.parametrize("scenario", ["offsets", "in_flight"])
+# fork_exit: a child process forked behind a large call exits
+# threads: four threads in calls at once
+@pytest.mark.parametrize("scenario", ["offsets", "in_flight", "fork_exit", "threads"])
 def test_host_calls(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
