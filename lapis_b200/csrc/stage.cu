@@ -5,6 +5,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <mutex>
@@ -39,7 +40,7 @@ struct Job {
   }
 };
 
-// Threads that sleep until there is a job.  A job is complete whether or not they wake up in time for it.
+// Threads that sleep until there is a job.  A job is complete whether or not they wake up in time for it, or exist.
 // They are detached and the pool is never destroyed: a child process forked after the first large call has no such
 // threads to join at its exit.
 class HelperPool {
@@ -51,7 +52,10 @@ class HelperPool {
         if (!started_) {
           started_ = true;
           const int n = std::min<int>(HELPERS, (int)std::thread::hardware_concurrency() - 1);
-          for (int i = 0; i < n; ++i) std::thread([this] { loop(); }).detach();
+          try {
+            for (int i = 0; i < n; ++i) std::thread([this] { loop(); }).detach();
+          } catch (const std::exception &) {  // no more threads to be had: those that there are, or the caller alone
+          }
         }
         job_ = job;
         ++round_;
@@ -137,6 +141,16 @@ struct Pieces {
 HelperPool &helpers() {
   static HelperPool *pool = new HelperPool;
   return *pool;
+}
+
+// The C entry points let no exception out.  Everything that allocates does so before a helper can have seen the job.
+template <typename F>
+int guarded(const char *what, F &&transfer) {
+  try {
+    return transfer();
+  } catch (const std::exception &e) {
+    return fail(LAPIS_ECUDA, "%s failed: %s", what, e.what());
+  }
 }
 
 // Copies into a slot past the caches: the bus then reads memory instead of another core's dirty lines (a 1.9 MB call:
@@ -242,6 +256,10 @@ void Upload::check_range(const Part &p, size_t from, size_t to, Facts *f) {
 }
 
 int Upload::run(void *device, cudaStream_t st, Facts *facts) {
+  return guarded("upload", [&] { return transfer(device, st, facts); });
+}
+
+int Upload::transfer(void *device, cudaStream_t st, Facts *facts) {
   Ring *ring = nullptr;
   int dev = 0;
   LAPIS_TRY(ring_of_device(&ring, &dev));
@@ -311,7 +329,7 @@ int Upload::run(void *device, cudaStream_t st, Facts *facts) {
   return pieces.status("upload");
 }
 
-int stage_download(void *host, const void *device, size_t bytes, cudaStream_t st) {
+static int download(void *host, const void *device, size_t bytes, cudaStream_t st) {
   if (bytes == 0 || (bytes >= DIRECT_BYTES && page_locked(host))) {
     if (bytes > 0) LAPIS_CUDA_TRY(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, st));
     LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -354,6 +372,10 @@ int stage_download(void *host, const void *device, size_t bytes, cudaStream_t st
   };
   helpers().run(job, bytes);
   return pieces.status("download");
+}
+
+int stage_download(void *host, const void *device, size_t bytes, cudaStream_t st) {
+  return guarded("download", [&] { return download(host, device, bytes, st); });
 }
 
 }  // namespace lapis_b200

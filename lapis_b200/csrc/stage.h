@@ -50,6 +50,7 @@ class Upload {
   int count_ = 0;
   size_t staged_ = 0;  // device bytes [0, staged_) travel through the slots
   int add_part(const void *host, size_t bytes, Check check, int64_t limit);
+  int transfer(void *device, cudaStream_t st, Facts *facts);
   static void check_range(const Part &p, size_t from, size_t to, Facts *f);
 };
 

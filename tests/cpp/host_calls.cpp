@@ -8,10 +8,13 @@
 #include <cstring>
 #include <limits>
 #include <mutex>
+#include <new>
 #include <set>
 #include <string>
 #include <vector>
 
+#include <dlfcn.h>
+#include <pthread.h>
 #include <sys/wait.h>
 #include <unistd.h>
 
@@ -36,6 +39,25 @@ static int g_kernel_status = LAPIS_OK;       // what the kernels return
 static std::vector<char *> g_page_locked;    // blocks of a caller, LOCKED_BYTES each
 constexpr size_t LOCKED_BYTES = size_t(4) << 20;
 
+// The allocation in so many allocations of this thread fails (0: none), and so does every start of a thread.
+static thread_local int g_fail_alloc = 0;
+static bool g_no_threads = false;
+void *operator new(size_t n) {
+  if (g_fail_alloc > 0 && --g_fail_alloc == 0) throw std::bad_alloc();
+  return std::malloc(n);
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
+  if (g_no_threads) return EAGAIN;
+  return reinterpret_cast<decltype(&pthread_create)>(dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, arg);
+}
+struct NoFailure {  // the stand-ins themselves keep their memory
+  int saved = g_fail_alloc;
+  NoFailure() { g_fail_alloc = 0; }
+  ~NoFailure() { g_fail_alloc = saved; }
+};
+
 static bool of_caller(const void *p) {
   for (char *b : g_page_locked)
     if (p >= b && p < b + LOCKED_BYTES) return true;
@@ -50,6 +72,7 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { return *v = 14
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
 cudaError_t cudaMalloc(void **p, size_t n) {
+  NoFailure keep;
   std::lock_guard<std::mutex> l(g_fake);
   *p = std::malloc(n);
   g_device.insert(*p);
@@ -67,6 +90,7 @@ cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+  NoFailure keep;
   std::lock_guard<std::mutex> l(g_fake);
   *p = std::aligned_alloc(4096, n);
   g_locked.insert(*p);
@@ -79,6 +103,7 @@ cudaError_t cudaFreeHost(void *p) {
   return cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+  NoFailure keep;
   *e = reinterpret_cast<cudaEvent_t>(new int(0));  // an event: the copies in front of it
   return cudaSuccess;
 }
@@ -262,6 +287,26 @@ struct Product {
   }
 };
 
+// Memory and threads that cannot be had end a call with a status or slow it down; no exception leaves the C entry point.
+static void exhausted() {
+  Product a(300000);
+  g_no_threads = true;
+  EXPECT(a.run() == LAPIS_OK && a.right());
+  g_no_threads = false;
+  int failures = 0;
+  for (int at = 1;; ++at) {
+    g_fail_alloc = at;
+    const int status = a.run();
+    const bool reached = g_fail_alloc == 0;
+    g_fail_alloc = 0;
+    EXPECT(status == (reached ? LAPIS_ECUDA : LAPIS_OK));
+    if (!reached) break;
+    ++failures;
+  }
+  EXPECT(failures >= 4);
+  EXPECT(a.run() == LAPIS_OK && a.right());
+}
+
 // A child process forked behind a large call exits.
 static void fork_exit() {
   Product a(300000);
@@ -293,6 +338,8 @@ int main(int argc, char **argv) {
     offsets<int64_t>(py_spmm_f64_i64);
   } else if (what == "in_flight") {
     in_flight();
+  } else if (what == "exhausted") {
+    exhausted();
   } else if (what == "fork_exit") {
     fork_exit();
   } else if (what == "threads") {

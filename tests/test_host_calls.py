@@ -24,9 +24,10 @@ def program(tmp_path_factory):
 
 # offsets: differences that wrap around the index type must not pass as row lengths
 # in_flight: a call that fails behind the upload leaves no copy from the caller's page-locked arrays under way
+# exhausted: memory or threads that cannot be had; no exception may leave a C entry point
 # fork_exit: a child process forked behind a large call exits
 # threads: four threads in calls at once
-@pytest.mark.parametrize("scenario", ["offsets", "in_flight", "fork_exit", "threads"])
+@pytest.mark.parametrize("scenario", ["offsets", "in_flight", "exhausted", "fork_exit", "threads"])
 def test_host_calls(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
