@@ -1,0 +1,28 @@
+"""Operands and arguments that the device-resident calls cannot use: a Python exception, without a GPU."""
+import pytest
+import torch
+
+
+def _unbacked(shape, dtype):
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        return torch.empty(shape, dtype=dtype, device="cuda")  # a CUDA tensor without storage
+
+
+def test_operands_that_torch_refuses_raise():
+    """torch refuses the address of a tensor without storage by a C++ exception; it must not end the process."""
+    from lapis_b200 import _calls, device
+    f64, f32, i32 = (_unbacked(s, t) for s, t in (((4, 4), torch.float64), ((4, 4, 4), torch.float32), ((5,), torch.int32)))
+    for call in (lambda: _calls.spmv(0, 16, 16, f64, f64, True), lambda: _calls.spmm(0, 4, 4, f64, f64, True),
+                 lambda: device.bgemm(f32, f32, f32), lambda: device.spmm_dcsr(i32[1:], i32, i32, f64, f64, f64, 4),
+                 lambda: device.bspmm_csrv(i32, i32[1:], f32[0], f32, 4, f32)):
+        with pytest.raises(RuntimeError):
+            call()
+
+
+def test_arguments_of_another_type_raise():
+    from lapis_b200 import _calls
+    x = _unbacked((4, 4), torch.float64)
+    for args in ((None, 4, 4, x, x, True), (0, "4", 4, x, x, True), (0, 4, 4, x, x, torch.ones(2)), (0, 4, 4, x)):
+        with pytest.raises((TypeError, RuntimeError)):
+            _calls.spmm(*args)
