@@ -32,6 +32,15 @@ T *addr_of(const at::Tensor *t) {
 void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 lapis_b200_csr_t handle(PyObject *o) { return static_cast<lapis_b200_csr_t>(PyLong_AsVoidPtr(o)); }
 PyObject *status(int code) { return PyLong_FromLong(code); }
+// Calls the library without the interpreter lock: a launch waits where the stream's queue is full.
+template <typename... P, typename... A>
+PyObject *call(int (*fn)(P...), A... args) {
+  int code;
+  Py_BEGIN_ALLOW_THREADS
+  code = fn(static_cast<P>(args)...);
+  Py_END_ALLOW_THREADS
+  return status(code);
+}
 
 // What Python calls.  torch reports some operands by a C++ exception (a tensor without storage has no address, a sparse
 // one no contiguity), which must not leave a C function; an argument that is no integer leaves a Python one.
@@ -60,7 +69,7 @@ PyObject *py_spmv(PyObject *const *a) {
   const at::Tensor *x = tensor(a[3]), *y = tensor(a[4]);
   if (!is(x, at::kDouble) || !is(y, at::kDouble)) return status(-1);
   if (y->numel() != PyLong_AsLongLong(a[1]) || x->numel() != PyLong_AsLongLong(a[2])) return status(-1);
-  return status(lapis_b200_spmv_f64(handle(a[0]), addr_of<double>(x), addr_of<double>(y), accumulate, stream()));
+  return call(lapis_b200_spmv_f64, handle(a[0]), addr_of<double>(x), addr_of<double>(y), accumulate, stream());
 }
 
 // spmm(handle, nrows, ncols, B, C, accumulate)
@@ -70,7 +79,7 @@ PyObject *py_spmm(PyObject *const *a) {
   const at::Tensor *B = tensor(a[3]), *C = tensor(a[4]);
   if (!is(B, at::kDouble) || !is(C, at::kDouble) || B->dim() != 2 || C->dim() != 2) return status(-1);
   if (C->size(0) != PyLong_AsLongLong(a[1]) || B->size(0) != PyLong_AsLongLong(a[2]) || B->size(1) != C->size(1)) return status(-1);
-  return status(lapis_b200_spmm_f64(handle(a[0]), B->size(1), addr_of<double>(B), addr_of<double>(C), accumulate, stream()));
+  return call(lapis_b200_spmm_f64, handle(a[0]), B->size(1), addr_of<double>(B), addr_of<double>(C), accumulate, stream());
 }
 
 // spmm_dcsr(i1, p2, i2, val, B, C, ncols)
@@ -82,8 +91,8 @@ PyObject *py_spmm_dcsr(PyObject *const *a) {
     return status(-1);
   if (B->dim() != 2 || C->dim() != 2 || B->size(0) != ncols || B->size(1) != C->size(1) || p2->numel() != i1->numel() + 1)
     return status(-1);
-  return status(lapis_b200_spmm_dcsr_f64((int)p2->element_size(), C->size(0), ncols, i1->numel(), B->size(1), addr(i1), addr(p2),
-                                         addr(i2), addr_of<double>(val), addr_of<double>(B), addr_of<double>(C), stream()));
+  return call(lapis_b200_spmm_dcsr_f64, (int)p2->element_size(), C->size(0), ncols, i1->numel(), B->size(1), addr(i1), addr(p2),
+              addr(i2), addr_of<double>(val), addr_of<double>(B), addr_of<double>(C), stream());
 }
 
 // bspmm(pos, crd, val, B, C, n2, accumulate)
@@ -97,8 +106,8 @@ PyObject *py_bspmm(PyObject *const *a) {
     return status(-1);
   const int64_t n1 = pos->numel() - 1, dh = B->size(1), nh = B->size(2);
   if (B->size(0) != n2 || val->numel() != crd->numel() * nh || C->size(0) != n1 || C->size(1) != dh || C->size(2) != nh) return status(-1);
-  return status(lapis_b200_bspmm_csrv_f32((int)pos->element_size(), n1, n2, nh, dh, addr(pos), addr(crd), addr_of<float>(val),
-                                          addr_of<float>(B), addr_of<float>(C), accumulate, stream()));
+  return call(lapis_b200_bspmm_csrv_f32, (int)pos->element_size(), n1, n2, nh, dh, addr(pos), addr(crd), addr_of<float>(val),
+              addr_of<float>(B), addr_of<float>(C), accumulate, stream());
 }
 
 // bgemm(A, B, C): [M,K]x[K,N] or [b,M,K]x[b,K,N]
@@ -110,7 +119,7 @@ PyObject *py_bgemm(PyObject *const *a) {
   const int64_t batch = d == 3 ? A->size(0) : 1, M = A->size(d - 2), K = A->size(d - 1), N = B->size(d - 1);
   if (B->size(d - 2) != K || C->size(d - 2) != M || C->size(d - 1) != N || (d == 3 && (B->size(0) != batch || C->size(0) != batch)))
     return status(-1);
-  return status(lapis_b200_bgemm_f32(batch, M, N, K, addr_of<float>(A), addr_of<float>(B), addr_of<float>(C), stream()));
+  return call(lapis_b200_bgemm_f32, batch, M, N, K, addr_of<float>(A), addr_of<float>(B), addr_of<float>(C), stream());
 }
 
 template <PyObject *(*CALL)(PyObject *const *), Py_ssize_t ARGS>

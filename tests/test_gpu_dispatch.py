@@ -268,3 +268,39 @@ def test_bspmm_widths(nh, dh):
             b.copy_(torch.as_tensor(B))
             got = bspmm_csrv(torch.as_tensor(pos).to(dev), torch.as_tensor(crd).to(dev), v, b, n)
             assert np.array_equal(got.cpu().numpy(), want)
+
+
+def test_calls_that_wait_for_the_queue_leave_python_running():
+    """A launch waits where the stream's queue is full (about a thousand launches); other Python threads go on meanwhile."""
+    import threading
+    import time
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(0)
+    n = 64
+    A = CsrMatrix.from_host(*_csr(rng, np.full(n, 3), n, np.int32), (n, n), dev)
+    x, y = (torch.zeros(n, dtype=torch.float64, device=dev) for _ in range(2))
+    A.spmv(x, y)
+    torch.cuda.synchronize()
+    gaps, stop = [], threading.Event()
+
+    def other():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.0005)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    torch.cuda._sleep(int(1e9))  # half a second of GPU time
+    start = time.perf_counter()
+    for _ in range(4000):
+        A.spmv(x, y)
+    waited = time.perf_counter() - start
+    stop.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.2, "the queue never filled up"
+    assert max(gaps) < 0.5 * waited
