@@ -96,7 +96,7 @@ class CsrMatrix:
         h = getattr(self, "_h", None)
         if h:
             self._lib.lapis_b200_csr_destroy(h)
-            self._h = None
+            self._h, self._addr = None, 0  # a call on it is refused as one on a null handle
 
     def spmv(self, x: torch.Tensor, y: torch.Tensor, accumulate: bool = True) -> torch.Tensor:
         """y = (y if accumulate else 0) + A x, in place."""

@@ -26,3 +26,21 @@ def test_arguments_of_another_type_raise():
     for args in ((None, 4, 4, x, x, True), (0, "4", 4, x, x, True), (0, 4, 4, x, x, torch.ones(2)), (0, 4, 4, x)):
         with pytest.raises((TypeError, RuntimeError)):
             _calls.spmm(*args)
+
+
+def test_a_released_matrix_refuses_products():
+    """After its release a matrix must not pass the old handle on."""
+    from lapis_b200.device import CsrMatrix
+
+    class Library:
+        released = 0
+
+        def lapis_b200_csr_destroy(self, h):
+            self.released += 1
+
+    A = object.__new__(CsrMatrix)
+    A._lib, A._h, A._addr, A.nrows, A.ncols = Library(), 4096, 4096, 0, 0
+    A.__del__()
+    assert (A._lib.released, A._h, A._addr) == (1, None, 0)
+    A.__del__()
+    assert A._lib.released == 1
