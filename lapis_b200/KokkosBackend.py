@@ -238,21 +238,22 @@ _MEMREF = {rank: struct.Struct("PPq%dq" % (2 * rank)) for rank in (1, 2, 3)}
 _CSR_SPEC = struct.Struct("5q")
 
 
-def _desc(arr):
+def _desc(arr, rank):
     """The memref descriptor of a C-contiguous array as bytes (passed by address; ``arr`` must stay alive)."""
     address, shape = arr.__array_interface__["data"][0], arr.shape
-    if len(shape) == 1:
+    if rank == 1:
         return _MEMREF[1].pack(address, address, 0, shape[0], 1)
-    if len(shape) == 2:
+    if rank == 2:
         return _MEMREF[2].pack(address, address, 0, shape[0], shape[1], shape[1], 1)
-    return _MEMREF[3].pack(address, address, 0, *shape, shape[1] * shape[2], shape[2], 1)
+    return _MEMREF[3].pack(address, address, 0, *shape[:3], shape[1] * shape[2], shape[2], 1)
 
 
 def _c_array(a, dtype, rank):
-    """``a`` as a C-contiguous numpy array of ``dtype`` and the rank the function was compiled for."""
+    """``a`` as a C-contiguous numpy array of ``dtype`` and the rank the function was compiled for, or of a higher one
+    when every extent after the first is 1 (a column for a vector): its elements lie the same way."""
     if type(a) is not np.ndarray or a.dtype != dtype or not a.flags.c_contiguous:
         a = np.require(a, dtype=dtype, requirements=["C"])
-    if a.ndim != rank:
+    if a.ndim != rank and (a.ndim < rank or any(extent != 1 for extent in a.shape[1:])):
         raise ValueError(f"expected an array of rank {rank}, got rank {a.ndim}")
     return a
 
@@ -463,7 +464,7 @@ class LAPISModule:
         def csr_args(pos, crd, val, spec):
             pos, crd, val = _c_array(pos, idx_dtype, 1), _c_array(crd, idx_dtype, 1), _c_array(val, np.float64, 1)
             (rows, cols), (npos, ncrd, nval) = spec
-            return (pos, crd, val), (_desc(pos), _desc(crd), _desc(val), _CSR_SPEC.pack(rows, cols, npos, ncrd, nval))
+            return (pos, crd, val), (_desc(pos, 1), _desc(crd, 1), _desc(val, 1), _CSR_SPEC.pack(rows, cols, npos, ncrd, nval))
 
         if kind == "spmv":
             fn = getattr(lib, symbol)
@@ -488,7 +489,7 @@ class LAPISModule:
                     return y
                 keep, cargs = csr_args(pos, crd, val, spec)
                 x, y = _c_array(x, np.float64, 1), _c_array(y, np.float64, 1)
-                fn(None, *cargs, _desc(x), _desc(y))  # no result slot: the result is the caller's y
+                fn(None, *cargs, _desc(x, 1), _desc(y, 1))  # no result slot: the result is the caller's y
                 check_last()
                 del keep
                 return y  # the function returns its outs argument
@@ -512,7 +513,7 @@ class LAPISModule:
                     return C
                 keep, cargs = csr_args(pos, crd, val, spec)
                 B, C = _c_array(B, np.float64, 2), _c_array(C, np.float64, 2)
-                fn(None, *cargs, _desc(B), _desc(C))
+                fn(None, *cargs, _desc(B, 2), _desc(C, 2))
                 check_last()
                 del keep
                 return C
@@ -530,7 +531,7 @@ class LAPISModule:
                     C.modifyDevice()
                     return C
                 A, B, C = (_c_array(t, np.float32, rank) for t in (A, B, C))
-                fn(None, _desc(A), _desc(B), _desc(C))
+                fn(None, _desc(A, rank), _desc(B, rank), _desc(C, rank))
                 check_last()
                 return C
 
@@ -550,7 +551,7 @@ class LAPISModule:
                 ret0 = _ret_slot(1)
                 ret1 = ctypes.c_size_t(0)
                 ret2 = ctypes.c_double(0.0)
-                fn(ret0, ctypes.byref(ret1), ctypes.byref(ret2), *cargs, _desc(b), _desc(dinv),
+                fn(ret0, ctypes.byref(ret1), ctypes.byref(ret2), *cargs, _desc(b, 1), _desc(dinv, 1),
                    ctypes.c_double(tol), ctypes.c_size_t(maxiter))
                 check_last()
                 del keep
@@ -602,7 +603,7 @@ class LAPISModule:
                 pos, crd, val = _c_array(pos, idx_dtype, 1), _c_array(crd, idx_dtype, 1), _c_array(val, np.float32, 1)
                 B = _c_array(B, np.float32, 3)
                 ret0 = _ret_slot(3)
-                fn(ret0, _desc(pos), _desc(crd), _desc(val), flat.ctypes.data_as(ctypes.c_void_p), _desc(B))
+                fn(ret0, _desc(pos, 1), _desc(crd, 1), _desc(val, 1), flat.ctypes.data_as(ctypes.c_void_p), _desc(B, 3))
                 check_last()
                 return rt.ranked_memref_to_numpy(ret0[0], np.float32)
 
@@ -626,7 +627,7 @@ class LAPISModule:
                     return C
                 arrs = [_c_array(t, idx_dtype, 1) for t in (p1, i1, p2, i2)]
                 val, B, C = _c_array(val, np.float64, 1), _c_array(B, np.float64, 2), _c_array(C, np.float64, 2)
-                fn(None, *[_desc(t) for t in arrs], _desc(val), flat.ctypes.data_as(ctypes.c_void_p), _desc(B), _desc(C))
+                fn(None, *[_desc(t, 1) for t in arrs], _desc(val, 1), flat.ctypes.data_as(ctypes.c_void_p), _desc(B, 2), _desc(C, 2))
                 check_last()
                 return C
 
@@ -644,7 +645,7 @@ class LAPISModule:
                 keep, cargs = csr_args(pos, crd, val, spec)
                 mask, d = _c_array(mask, np.float64, 1), _c_array(d, np.float64, 1)
                 ret0, ret1 = _ret_slot(1), _ret_slot(1)
-                fn(ret0, ret1, *cargs, _desc(mask), _desc(d), ctypes.c_double(alpha), ctypes.c_double(tol),
+                fn(ret0, ret1, *cargs, _desc(mask, 1), _desc(d, 1), ctypes.c_double(alpha), ctypes.c_double(tol),
                    ctypes.c_size_t(maxiter))
                 check_last()
                 del keep
@@ -662,7 +663,7 @@ class LAPISModule:
                     return DualView.from_device(D.normalize_mom2(mom1.device_view(), mom2.device_view()))
                 mom1, mom2 = _c_array(mom1, np.float64, 1), _c_array(mom2, np.float64, 1)
                 ret0 = _ret_slot(1)
-                fn(ret0, _desc(mom1), _desc(mom2))
+                fn(ret0, _desc(mom1, 1), _desc(mom2, 1))
                 check_last()
                 return rt.ranked_memref_to_numpy(ret0[0], np.float64)
 
