@@ -49,3 +49,12 @@ def test_matrices_of_one_column_may_come_with_more_extents():
     for bad in (np.ones(2), np.ones((2, 3, 1))):
         with pytest.raises(ValueError):
             spmm(pos, crd, val, ((2, 2), (3, 2, 2)), bad, C)
+
+
+@pytest.mark.parametrize("spec", [((2, 2), (3, 2, 2)), ((2.0, 2.0), (3.0, 2, 2)), [np.array([2, 2]), np.array([3.0, 2.0, 2.0])],
+                                  ((2, 2, 7), (3, 2, 2, 9))])
+def test_specifiers_of_every_number_type(spec):
+    spmv, calls = _bound("spmv")
+    pos, crd, val = np.array([0, 1, 2], np.int32), np.array([0, 1], np.int32), np.ones(2)
+    spmv(pos, crd, val, spec, np.ones(2), np.zeros(2))
+    assert struct.unpack("5q", calls[0][4]) == (2, 2, 3, 2, 2)
