@@ -21,6 +21,12 @@ const at::Tensor *tensor(PyObject *o) { return THPVariable_Check(o) ? &THPVariab
 bool is(const at::Tensor *t, at::ScalarType st) {
   return t != nullptr && t->is_cuda() && t->scalar_type() == st && t->is_contiguous();
 }
+// Two extents, further ones being 1: a row-major matrix.
+bool is_matrix(const at::Tensor *t) {
+  for (int64_t d = 2; d < t->dim(); ++d)
+    if (t->size(d) != 1) return false;
+  return t->dim() >= 2;
+}
 bool is_index(const at::Tensor *t) {
   return t != nullptr && t->is_cuda() && (t->scalar_type() == at::kInt || t->scalar_type() == at::kLong) && t->is_contiguous();
 }
@@ -77,7 +83,7 @@ PyObject *py_spmm(PyObject *const *a) {
   const int accumulate = PyObject_IsTrue(a[5]);
   if (accumulate < 0) return nullptr;
   const at::Tensor *B = tensor(a[3]), *C = tensor(a[4]);
-  if (!is(B, at::kDouble) || !is(C, at::kDouble) || B->dim() != 2 || C->dim() != 2) return status(-1);
+  if (!is(B, at::kDouble) || !is(C, at::kDouble) || !is_matrix(B) || !is_matrix(C)) return status(-1);
   if (C->size(0) != PyLong_AsLongLong(a[1]) || B->size(0) != PyLong_AsLongLong(a[2]) || B->size(1) != C->size(1)) return status(-1);
   return call(lapis_b200_spmm_f64, handle(a[0]), B->size(1), addr_of<double>(B), addr_of<double>(C), accumulate, stream());
 }

@@ -44,3 +44,13 @@ def test_a_released_matrix_refuses_products():
     assert (A._lib.released, A._h, A._addr) == (1, None, 0)
     A.__del__()
     assert A._lib.released == 1
+
+
+def test_matrices_may_have_further_extents_of_one():
+    """Row-major all the same: the call gets as far as the address, which a tensor without storage does not have."""
+    from lapis_b200 import _calls
+    for shape in ((4, 4), (4, 4, 1), (4, 4, 1, 1)):
+        with pytest.raises(RuntimeError):
+            _calls.spmm(0, 4, 4, _unbacked(shape, torch.float64), _unbacked((4, 4), torch.float64), True)
+    for shape in ((4,), (16,), (4, 4, 2), (4, 1, 4)):
+        assert _calls.spmm(0, 4, 4, _unbacked(shape, torch.float64), _unbacked((4, 4), torch.float64), True) == -1
