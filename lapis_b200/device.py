@@ -205,7 +205,7 @@ def bgemm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor) -> torch.Tensor:
             for t in (A, B, C):
                 if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
                     raise TypeError("bgemm operands must be contiguous float32 CUDA tensors")
-            if A.dim() != B.dim() or A.shape[-1] != B.shape[-2] or A.shape[:-2] != B.shape[:-2]:
+            if A.dim() not in (2, 3) or A.dim() != B.dim() or A.shape[-1] != B.shape[-2] or A.shape[:-2] != B.shape[:-2]:
                 raise ValueError("mismatching contracting dimension")
             raise ValueError("bgemm: output shape mismatch")
         check(status)

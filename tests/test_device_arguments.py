@@ -54,3 +54,11 @@ def test_matrices_may_have_further_extents_of_one():
             _calls.spmm(0, 4, 4, _unbacked(shape, torch.float64), _unbacked((4, 4), torch.float64), True)
     for shape in ((4,), (16,), (4, 4, 2), (4, 1, 4)):
         assert _calls.spmm(0, 4, 4, _unbacked(shape, torch.float64), _unbacked((4, 4), torch.float64), True) == -1
+
+
+@pytest.mark.parametrize("dims", [1, 4])
+def test_matmul_of_other_ranks_is_a_value_error(dims):
+    from lapis_b200 import device
+    x = _unbacked((4,) * dims, torch.float32)
+    with pytest.raises(ValueError):
+        device.bgemm(x, x, x)
