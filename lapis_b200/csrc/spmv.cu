@@ -1336,6 +1336,8 @@ static SpmvVariant spmv_variant(const lapis_b200_csr *h) {
   if (v.threads == 0 && h->tuned_threads != 0) v = SpmvVariant{h->tuned_threads, h->tuned_minb, h->tuned_hint};
   else if (v.threads == 0) v = has_short_rows(h) ? SpmvVariant{1, 0, 1} : SPMV_DEFAULT;
   if (v.threads == 1 && !has_short_rows(h)) v = SPMV_DEFAULT;
+  // a handle without a plan (csr_setup) was meant for the kernels for short rows; the override may have changed since
+  if (v.threads != 1 && h->blk_row == nullptr && has_short_rows(h)) v = SpmvVariant{1, 0, 1};
   return v;
 }
 
@@ -1367,10 +1369,9 @@ static int pcg_pass_grid(const lapis_b200_csr *h, unsigned *grid) {
 }
 
 template <typename I>
-static int launch_spmv(const lapis_b200_csr *h, const double *x, double *y, int accumulate,
+static int launch_spmv(const lapis_b200_csr *h, SpmvVariant v, const double *x, double *y, int accumulate,
                        const double *dotvec, double *blk_partial, const int *skip_flag,
                        cudaStream_t st, const PcgExchange *ex) {
-  SpmvVariant v = spmv_variant(h);
   if (v.threads == 1) {
     const I *pos = static_cast<const I *>(h->pos);
     const I *crd = static_cast<const I *>(h->crd);
@@ -1479,12 +1480,16 @@ static int launch_spmv(const lapis_b200_csr *h, const double *x, double *y, int 
   return launch_fixup<I>(h, h->blk_row, h->carry, h->nblk, SPMV_TILE, y, skip_flag, st);
 }
 
-int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumulate,
-                const double *dotvec, double *blk_partial, const int *skip_flag, cudaStream_t st) {
+static int spmv_launch_as(const lapis_b200_csr *h, const SpmvVariant &v, const double *x, double *y, int accumulate,
+                          const double *dotvec, double *blk_partial, const int *skip_flag, cudaStream_t st) {
   if (h->nrows == 0) return LAPIS_OK;
   if (h->idx_bytes == 4)
-    return launch_spmv<int32_t>(h, x, y, accumulate, dotvec, blk_partial, skip_flag, st, nullptr);
-  return launch_spmv<int64_t>(h, x, y, accumulate, dotvec, blk_partial, skip_flag, st, nullptr);
+    return launch_spmv<int32_t>(h, v, x, y, accumulate, dotvec, blk_partial, skip_flag, st, nullptr);
+  return launch_spmv<int64_t>(h, v, x, y, accumulate, dotvec, blk_partial, skip_flag, st, nullptr);
+}
+int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumulate,
+                const double *dotvec, double *blk_partial, const int *skip_flag, cudaStream_t st) {
+  return spmv_launch_as(h, spmv_variant(h), x, y, accumulate, dotvec, blk_partial, skip_flag, st);
 }
 
 // Pass A of a PCG iteration with its head and tail inside the SpMV kernel; only for handles on which
@@ -1497,8 +1502,8 @@ bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
 }
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex) {
-  if (h->idx_bytes == 4) return launch_spmv<int32_t>(h, x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
-  return launch_spmv<int64_t>(h, x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
+  if (h->idx_bytes == 4) return launch_spmv<int32_t>(h, spmv_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
+  return launch_spmv<int64_t>(h, spmv_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
 }
 
 // Pass A with the direction update folded in (two-pass PCG); only where spmv_fuses_pcg_pass() is true.
@@ -1656,7 +1661,6 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
   const SpmvVariant cand[] = {{256, 4, 1}, {256, 6, 1}, {512, 3, 1}, {-256, pipe_blocks, 1},
                               {1, 0, SHORT_ROW_PER_THREAD}, {1, 0, SHORT_64_ROWS}, {1, 0, SHORT_32_ROWS},
                               {2, 5, 1}, {2, 5, 0}, {3, 4, 1}, {3, 4, 0}, {4, 0, 0}};
-  const SpmvVariant saved = spmv_override();
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1667,11 +1671,10 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
     if ((c.threads == 2 || c.threads == 3 || c.threads == 4) && !relaxed) continue;
     if (c.threads == 4 && ((reinterpret_cast<uintptr_t>(h->val) | reinterpret_cast<uintptr_t>(h->crd)) & 31) != 0) continue;
     if (!spmv_variant_known(c.threads, c.minb)) continue;
-    spmv_override() = c;
-    status = spmv_launch(h, x, y, 0, nullptr, nullptr, nullptr, st);  // warm-up
+    status = spmv_launch_as(h, c, x, y, 0, nullptr, nullptr, nullptr, st);  // warm-up
     if (status != LAPIS_OK) break;
     cudaEventRecord(e0, st);
-    for (int r = 0; r < 3 && status == LAPIS_OK; ++r) status = spmv_launch(h, x, y, 0, nullptr, nullptr, nullptr, st);
+    for (int r = 0; r < 3 && status == LAPIS_OK; ++r) status = spmv_launch_as(h, c, x, y, 0, nullptr, nullptr, nullptr, st);
     cudaEventRecord(e1, st);
     if (status != LAPIS_OK || cudaEventSynchronize(e1) != cudaSuccess) {
       if (status == LAPIS_OK) status = fail(LAPIS_ECUDA, "csr_tune: timing run failed");
@@ -1686,7 +1689,6 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
       h->tuned_hint = c.hint;
     }
   }
-  spmv_override() = saved;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   return status;

@@ -304,3 +304,38 @@ def test_calls_that_wait_for_the_queue_leave_python_running():
     torch.cuda.synchronize()
     assert waited > 0.2, "the queue never filled up"
     assert max(gaps) < 0.5 * waited
+
+
+def test_tuning_beside_calls_on_host_arrays():
+    """A thread that tunes a matrix leaves the kernel choice of other threads' calls alone: a call on host arrays of short
+    rows makes no plan for the kernels that need one."""
+    import threading
+    from lapis_b200 import KokkosBackend as KB
+    from lapis_b200 import modules as mm
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(5)
+    n = 5000
+    pos, crd, val = _csr(rng, np.full(n, 9), n, np.int64)
+    x, y = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    A = CsrMatrix.from_host(pos, crd, val, (n, n), dev)
+    want = A.spmv(torch.as_tensor(x).to(dev), torch.as_tensor(y).to(dev)).cpu().numpy()  # every kind of kernel has these bits
+    module = KB.KokkosBackend(decompose_tensors=True).compile(mm.spmv(mm.CSR64))
+    stop = threading.Event()
+
+    def tune():
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            while not stop.is_set():
+                A.tune()
+
+    thread = threading.Thread(target=tune)
+    thread.start()
+    try:
+        for _ in range(300):
+            got = y.copy()
+            module.spmv(pos, crd, val, ((n, n), (n + 1, len(crd), len(crd))), x, got)
+            assert np.array_equal(got, want)
+    finally:
+        stop.set()
+        thread.join()
