@@ -585,14 +585,15 @@ def run_pcg(args, d, hx: Harness, iterations: int, with_e2e: bool):
     ms, clocks = hx.timed(lambda: solve(iterations), 1, 0)
     it = state["out"][1]
     tuned = solver.matrix.tuned_kernel()
+    row_thread = bool(solver._lib.lapis_b200_pcg_folds_direction(solver.matrix.handle))  # no carry fix-up launch
     if solver.comm == "nccl":
-        launches_per_it = 8 - (1 if tuned[0] == 1 else 0)
+        launches_per_it = 8 - (1 if row_thread else 0)
     elif solver.fused and solver._two_pass():
         launches_per_it = 2
     elif solver.fused:
-        launches_per_it = 3 if tuned[0] == 1 else (5 if tuned[0] in (-256, -512) else 6)
+        launches_per_it = 3 if row_thread else (5 if tuned[0] in (-256, -512) else 6)
     else:
-        launches_per_it = (6 if world == 1 and solver.comm == "none" else 12) - (1 if tuned[0] == 1 else 0)
+        launches_per_it = (6 if world == 1 and solver.comm == "none" else 12) - (1 if row_thread else 0)
     ms_it = ms / max(1, it)
     roof = hx.hbm_roofline(d["bytes_per_step"] / world, ms_it,
                            "pcg_spmv_direction_kernel + pcg_update_fused_kernel" if solver.fused and solver._two_pass() else

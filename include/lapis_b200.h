@@ -184,7 +184,10 @@ int lapis_b200_spmv_f64(lapis_b200_csr_t h, const double *d_x, double *d_y, int 
  * per 32 or 64 rows that stages their products); the tuner considers it (and the launch honours it) only for
  * matrices whose longest row has at most 32 entries -- up to there it returns the same bits as the others.  Such
  * matrices (stencils, bounded-degree graphs) are where it wins, and handles that were never tuned use it for them;
- * on other matrices a request for it runs (256,4).  l2_hint 2, 3 or 4 names one of its three kernels.
+ * on other matrices a request for it runs (256,4).  l2_hint 2, 3 or 4 names one of its three kernels.  The passes of a
+ * solver (pcg, mht), which fuse a dot product, have only the one-thread-per-row form of this kind: a tuned handle keeps
+ * the fastest kernel among those that have the form beside the winner, an untuned one uses (256,4) for them, and matrices
+ * of short rows with fewer than 2^19 entries always one thread per row.
  * A fourth kind, threads = 2 (256 threads, blocks_per_sm in {4, 5}) or threads = 3 (512 threads,
  * blocks_per_sm in {2, 3, 4}), is the chunk kernel with the row sums done by a
  * segmented scan in registers instead of one lane per row over shared memory (less shared-memory traffic

@@ -110,6 +110,9 @@ struct lapis_b200_csr {
   double *blk_partial;
   // Kernel variant chosen by lapis_b200_csr_tune (tuned_threads == 0: not tuned).
   int tuned_threads, tuned_minb, tuned_hint;
+  // The fastest of the candidates that the passes of a solver run as they are timed (with a dot product fused, rows one
+  // thread each are spmv_rowthread_kernel whatever short-row kernel wins a plain product).
+  int fused_threads, fused_minb, fused_hint;
   // Longest row (-1: not known).  The kernels for short rows are only used when no row has more than 32 entries: up
   // to there they return the same bits as the chunk kernels.
   int64_t max_row_len;

@@ -1341,9 +1341,21 @@ static SpmvVariant spmv_variant(const lapis_b200_csr *h) {
   return v;
 }
 
-// Whether spmv_launch will run the kernels for short rows on this handle (one thread per row: the variant that can
-// carry the head and tail of a PCG iteration's first pass).
-static bool uses_rowthread(const lapis_b200_csr *h) { return spmv_variant(h).threads == 1; }
+// The same for the passes of a solver, which fuse a dot product.  The block-per-rows kernels have no such form, and where
+// they win a plain product one thread per row may still lose to a chunk kernel, so a tuned handle remembers its fastest
+// kernel among the others, and an untuned one runs the chunk kernel.  us per PCG iteration, random symmetric matrices, one
+// thread per row and the chunk kernel: 1e6 rows of 11 entries 134 and 108 (64-bit indices 147 and 107), of 7 93 and 81.
+// Small systems are bound by their launches, of which one thread per row needs two an iteration and a chunk kernel three:
+// 16,000 rows of 7 22.5 and 23.7, 30,000 of 9 21.7 and 23.7; 100,000 of 11 take 30 and 28 to 30.
+constexpr int64_t FUSED_LAUNCH_BOUND = 1 << 19;  // stored entries
+static SpmvVariant spmv_fused_variant(const lapis_b200_csr *h) {
+  SpmvVariant v = spmv_override();
+  if (v.threads == 0 && has_short_rows(h) && h->nnz < FUSED_LAUNCH_BOUND) v = SpmvVariant{1, 0, SHORT_ROW_PER_THREAD};
+  else if (v.threads == 0 && h->fused_threads != 0) v = SpmvVariant{h->fused_threads, h->fused_minb, h->fused_hint};
+  else if (v.threads == 0) v = SPMV_DEFAULT;
+  if (v.threads == 1 && !has_short_rows(h)) v = SPMV_DEFAULT;
+  return v;
+}
 
 // Grid of the SpMV pass of a PCG iteration in both of its forms (spmv_rowthread_kernel with head and tail,
 // pcg_spmv_direction_kernel): the blocks that are resident at once for either kernel, looping over the row
@@ -1489,12 +1501,13 @@ static int spmv_launch_as(const lapis_b200_csr *h, const SpmvVariant &v, const d
 }
 int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumulate,
                 const double *dotvec, double *blk_partial, const int *skip_flag, cudaStream_t st) {
-  return spmv_launch_as(h, spmv_variant(h), x, y, accumulate, dotvec, blk_partial, skip_flag, st);
+  const SpmvVariant v = dotvec != nullptr ? spmv_fused_variant(h) : spmv_variant(h);
+  return spmv_launch_as(h, v, x, y, accumulate, dotvec, blk_partial, skip_flag, st);
 }
 
 // Pass A of a PCG iteration with its head and tail inside the SpMV kernel; only for handles on which
 // spmv_fuses_pcg_pass() is true.
-bool spmv_fuses_pcg_pass(const lapis_b200_csr *h) { return h->nrows > 0 && uses_rowthread(h); }
+bool spmv_fuses_pcg_pass(const lapis_b200_csr *h) { return h->nrows > 0 && spmv_fused_variant(h).threads == 1; }
 // Whether a whole PCG solve runs in one cluster (pcg_small.cu): rows short enough for a thread each, a matrix that the L1
 // caches of eight SMs hold, no SpMV kernel forced.
 bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
@@ -1502,8 +1515,8 @@ bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
 }
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex) {
-  if (h->idx_bytes == 4) return launch_spmv<int32_t>(h, spmv_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
-  return launch_spmv<int64_t>(h, spmv_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
+  if (h->idx_bytes == 4) return launch_spmv<int32_t>(h, spmv_fused_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
+  return launch_spmv<int64_t>(h, spmv_fused_variant(h), x, y, 0, dotvec, blk_partial, skip_flag, st, &ex);
 }
 
 // Pass A with the direction update folded in (two-pass PCG); only where spmv_fuses_pcg_pass() is true.
@@ -1550,7 +1563,7 @@ int csr_setup(lapis_b200_csr *h, int idx_bytes, int64_t nrows, int64_t ncols, in
   h->nblk = nblk;
   h->max_row_len = max_row_len;
   LAPIS_CUDA_TRY(cudaGetDevice(&h->device));
-  if (plan_on_demand && uses_rowthread(h)) return LAPIS_OK;
+  if (plan_on_demand && spmv_variant(h).threads == 1) return LAPIS_OK;
   // The warp-walk kernel gives one warp a range of entries.  With 2048-entry ranges a matrix needs about eight
   // times as many ranges as the GPU holds warps (32 per SM) before the last, partly filled round of warps stops
   // mattering; smaller matrices (a row block of a partitioned one) get a second plan of 512-entry ranges.
@@ -1664,7 +1677,7 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  float best = 0.f;
+  float best = 0.f, best_fused = 0.f;
   int status = LAPIS_OK;
   for (const SpmvVariant &c : cand) {
     if (c.threads == 1 && !short_rows) continue;
@@ -1687,6 +1700,13 @@ static int csr_tune_impl(lapis_b200_csr_t h, void *stream, bool relaxed) {
       h->tuned_threads = c.threads;
       h->tuned_minb = c.minb;
       h->tuned_hint = c.hint;
+    }
+    if (c.threads == 1 && c.hint != SHORT_ROW_PER_THREAD) continue;
+    if (h->fused_threads == 0 || ms < best_fused) {
+      best_fused = ms;
+      h->fused_threads = c.threads;
+      h->fused_minb = c.minb;
+      h->fused_hint = c.hint;
     }
   }
   cudaEventDestroy(e0);
@@ -1850,6 +1870,7 @@ extern "C" int lapis_b200_spmv_f64_noalloc(int idx_bytes, int64_t nrows, int64_t
   h.blk_partial = nullptr;
   h.carry = reinterpret_cast<double *>(plan + NOALLOC_MAX_TILES + 1);
   h.tuned_threads = h.tuned_minb = h.tuned_hint = 0;
+  h.fused_threads = h.fused_minb = h.fused_hint = 0;
   h.max_row_len = -1;
   h.device = dev;
   h.walk_plan = nullptr;

@@ -339,3 +339,32 @@ def test_tuning_beside_calls_on_host_arrays():
     finally:
         stop.set()
         thread.join()
+
+
+@pytest.mark.parametrize("n,idx", [(30_000, np.int32), (60_000, np.int64)])
+def test_solver_passes_have_their_own_kernel(n, idx):
+    """Rows of 10 to 32 scattered entries on both sides of the limit for launch-bound systems: an untuned matrix above it
+    runs the chunk kernel, which needs the direction pass; tuned or not, PCG makes the oracle's iterations."""
+    import scipy.sparse as sp
+    from lapis_b200._lib import load
+    from lapis_b200.device import CsrMatrix
+    dev, lib = _dev(), load()
+    rng = np.random.default_rng(n)
+    half = sp.coo_matrix((rng.uniform(-1, 0, 5 * n), (np.repeat(np.arange(n), 5), rng.integers(0, n, 5 * n))), shape=(n, n)).tocsr()
+    sym = (half + half.T).tocsr()
+    sym -= sp.diags(sym.diagonal())
+    a = (sym + sp.diags(np.asarray(abs(sym).sum(1)).ravel() + 1.0)).tocsr()
+    a.sort_indices()
+    assert 10 <= np.diff(a.indptr).max() <= 32
+    A = CsrMatrix.from_host(a.indptr.astype(idx), a.indices.astype(idx), a.data, (n, n), dev)
+    assert bool(lib.lapis_b200_pcg_folds_direction(A.handle)) == (a.nnz < 1 << 19)
+    b, dinv = rng.uniform(0, 1, n), 1 / a.diagonal()
+    x0, it0, rel0 = oracle.pcg(a.indptr.astype(idx), a.indices.astype(idx), a.data, b, dinv, 1e-10, 500)
+    for tune in (False, True):
+        if tune:
+            A.tune()
+        for maxiter in (500, 8):  # a short solve does not tune
+            x, it, rel = A.pcg(torch.as_tensor(b).to(dev), torch.as_tensor(dinv).to(dev), 1e-10, maxiter)
+            assert it == min(it0, maxiter)
+            if maxiter == 500:
+                assert abs(rel - rel0) <= 1e-6 * rel0 and np.linalg.norm(x.cpu().numpy() - x0) <= 1e-11 * np.linalg.norm(x0)
