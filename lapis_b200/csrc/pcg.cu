@@ -34,7 +34,7 @@ int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumul
 bool spmv_fuses_pcg_pass(const lapis_b200_csr *h);
 bool spmv_fits_small_pcg(const lapis_b200_csr *h);
 int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
-              uint64_t *iters, double *relres, cudaStream_t st);
+              uint64_t *iters, double *relres, bool *solved, cudaStream_t st);
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex);
 int spmv_launch_pcg_direction_pass(const lapis_b200_csr *h, int64_t p_off, double *pw0, double *pw1, double *Ap,
@@ -623,7 +623,11 @@ extern "C" int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const d
     if (relres) *relres = NAN;
     return LAPIS_OK;
   }
-  if (spmv_fits_small_pcg(h)) return pcg_small(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, st);
+  if (spmv_fits_small_pcg(h)) {
+    bool solved = false;
+    LAPIS_TRY(pcg_small(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
+    if (solved) return LAPIS_OK;
+  }
   // a solve runs the SpMV pass many times: pick the kernel variant for this matrix first
   if (h->tuned_threads == 0 && (maxiter == 0 || maxiter >= 16)) LAPIS_TRY(lapis_b200_csr_tune(h, st));
   PoolBuf buf;

@@ -5,7 +5,14 @@
 // dinv in registers, p lives in the shared memory of the CTAs, a slice each, and the SpMV gathers it from there; the
 // partial sums of a dot product are stored into every CTA's shared memory by the warps that made them and added in one
 // fixed order by the first warp of every CTA after the cluster's barrier, so that all CTAs derive the same alpha, beta and
-// stop test (one warp, not all: the divisions of 32 warps take longer than the barrier they save).  Three barriers of the cluster an iteration, no global memory but the matrix, which stays in L1.
+// stop test (one warp, not all: the divisions of 32 warps take longer than the barrier they save).  Three barriers of the
+// cluster an iteration, no global memory but the matrix, which the L1 caches of the SMs in use hold up to about 200 KB each
+// and L2 beyond (1000 rows of 29, 64-bit indices, 460 KB on one SM: 17 us an iteration, 12.5 with 32-bit ones).
+//
+// Bound by the barriers (5-point stencils: 3.0 us an iteration at 1024 rows, 6.2 at 16,384; the passes of pcg.cu take 17 to
+// 19) and, with scattered columns, by the gathers from the other CTAs' memory: 8000 rows of 11, 70,000 such
+// gathers, 20.9 us, passes 21.5; 8000 of 15, 98,000 gathers, 29.2 and 22.5, where a band of the same size takes 8.1.  The
+// solve therefore counts them first where there may be too many, and leaves the system to the passes.
 //
 // The recurrences are those of pcg.cu (examples/pcg_solve.py:65-98 in the LAPIS project), element by element; a row of A p
 // is added in entry order.  Results are identical from run to run; against the other passes they differ by the order of the
@@ -17,6 +24,8 @@
 
 namespace lapis_b200 {
 
+constexpr int SMALL_FAR = 75000;  // gathers from other CTAs' memory in an iteration, beyond which the passes are faster
+constexpr int SMALL_LEFT = 2;     // FL_DONE of a system that was left to the passes
 constexpr int SMALL_BUDGET = 4096;  // iterations per launch (a few milliseconds): the host looks at the outcome in between
 
 struct SmallSolve {
@@ -27,7 +36,7 @@ struct SmallSolve {
   double tol;
   unsigned long long maxiter;
   int n;
-  bool first;
+  bool first, count_far;
 };
 
 template <int CTAS>
@@ -106,6 +115,21 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     x[i] = in && !s.first ? s.x[row] : 0.0;
     z[i] = __dmul_rn(r[i], d[i]);
     s_p[tid + i * THREADS] = in ? (s.first ? z[i] : s.p[row]) : 0.0;
+  }
+  if (CTAS > 1 && s.count_far) {
+    int far = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      for (int j = 0; j < len[i]; ++j) far += (uint32_t)__ldg(crd + lo[i] + j) / SLICE != rank;
+    small_barrier<CTAS>();  // every CTA of the cluster runs before its shared memory is written
+    send(0, (double)far);
+    small_barrier<CTAS>();
+    if (warp == 0) s_done = total(0) > SMALL_FAR ? 1 : 0;
+    __syncthreads();
+    if (s_done != 0) {  // in all CTAs alike; nothing of theirs is read or written any more
+      if (rank == 0 && tid == 0) s.fl[FL_DONE] = SMALL_LEFT;
+      return;
+    }
   }
   double initres = 0.0, rz = 0.0, relres = 0.0;  // of warp 0, as the sums are
   unsigned long long iters = 0;
@@ -240,9 +264,10 @@ static cudaError_t launch_small_size(const lapis_b200_csr *h, const SmallSolve &
   return launch_small<I, 8, 1024, 2>(h, s, st);
 }
 
-// Only for handles on which spmv_fits_small_pcg() is true (at most 16384 rows).
+// Only for handles on which spmv_fits_small_pcg() is true (at most 16384 rows).  *solved: false where the system is left
+// to the passes.
 int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
-              uint64_t *iters, double *relres, cudaStream_t st) {
+              uint64_t *iters, double *relres, bool *solved, cudaStream_t st) {
   const int64_t n = h->nrows;
   PoolBuf buf;
   LAPIS_TRY(buf.alloc((size_t)(16 + 2 * n) * sizeof(double), st));
@@ -258,13 +283,16 @@ int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, 
   s.maxiter = maxiter;
   s.n = (int)n;
   s.first = true;
+  s.count_far = h->nnz > SMALL_FAR;
   const uint64_t limit = maxiter == 0 ? (1ull << 31) : maxiter;
   int done = 0;
   uint64_t it = 0;
   do {
     LAPIS_CUDA_TRY(h->idx_bytes == 4 ? launch_small_size<int32_t>(h, s, st) : launch_small_size<int64_t>(h, s, st));
-    s.first = false;
+    s.first = s.count_far = false;
     LAPIS_TRY(lapis_b200_pcg_status(s.sc, &done, &it, relres, st));
+    *solved = done != SMALL_LEFT;
+    if (!*solved) return LAPIS_OK;
   } while (!done && it < limit);
   if (iters) *iters = it;
   return LAPIS_OK;

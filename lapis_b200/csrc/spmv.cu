@@ -1508,8 +1508,8 @@ int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumul
 // Pass A of a PCG iteration with its head and tail inside the SpMV kernel; only for handles on which
 // spmv_fuses_pcg_pass() is true.
 bool spmv_fuses_pcg_pass(const lapis_b200_csr *h) { return h->nrows > 0 && spmv_fused_variant(h).threads == 1; }
-// Whether a whole PCG solve runs in one cluster (pcg_small.cu): rows short enough for a thread each, a matrix that the L1
-// caches of eight SMs hold, no SpMV kernel forced.
+// Whether a whole PCG solve may run in one cluster (pcg_small.cu): rows short enough for a thread each, entries that eight
+// SMs get through (a band of 127,000 takes 10 us an iteration, the passes 22), no SpMV kernel forced.
 bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
   return h->nrows > 0 && h->nrows <= 16384 && h->nnz <= 131072 && has_short_rows(h) && spmv_override().threads == 0;
 }

@@ -368,3 +368,58 @@ def test_solver_passes_have_their_own_kernel(n, idx):
             assert it == min(it0, maxiter)
             if maxiter == 500:
                 assert abs(rel - rel0) <= 1e-6 * rel0 and np.linalg.norm(x.cpu().numpy() - x0) <= 1e-11 * np.linalg.norm(x0)
+
+
+def _passes(A, *args):
+    """PCG in a launch per pass, whatever the size."""
+    from lapis_b200._lib import check, load
+    check(load().lapis_b200_spmv_select_kernel(1, 0, 1))
+    try:
+        return A.pcg(*args)
+    finally:
+        check(load().lapis_b200_spmv_select_kernel(0, 0, 0))
+
+
+@pytest.mark.parametrize("idx", [np.int32, np.int64])
+@pytest.mark.parametrize("n,half,scattered", [(8000, 7, True), (16000, 3, True), (8000, 7, False), (4096, 15, False)])
+def test_small_pcg_leaves_scattered_systems_to_the_passes(n, half, scattered, idx):
+    """More than 75,000 entries: solved in one launch where most columns are near the diagonal, by the passes (their bits)
+    where they are not."""
+    import scipy.sparse as sp
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(n + half)
+    if scattered:
+        a = sp.coo_matrix((rng.uniform(-1, 0, half * n), (np.repeat(np.arange(n), half), rng.integers(0, n, half * n))), shape=(n, n)).tocsr()
+    else:
+        a = sp.diags([rng.uniform(-1, 0, n - d) for d in range(1, half + 1)], list(range(1, half + 1))).tocsr()
+    a = (a + a.T).tocsr()
+    a -= sp.diags(a.diagonal())
+    a = (a + sp.diags(np.asarray(abs(a).sum(1)).ravel() + 1.0)).tocsr()
+    a.sort_indices()
+    assert 75_000 < a.nnz <= 131_072 and np.diff(a.indptr).max() <= 32
+    A = CsrMatrix.from_host(a.indptr.astype(idx), a.indices.astype(idx), a.data, (n, n), dev)
+    b, dinv = torch.as_tensor(rng.uniform(0, 1, n)).to(dev), torch.as_tensor(1 / a.diagonal()).to(dev)
+    for tol, maxiter in ((1e-9, 500), (0.0, 3)):
+        (x, it, rel), (x0, it0, rel0) = A.pcg(b, dinv, tol, maxiter), _passes(A, b, dinv, tol, maxiter)
+        assert it == it0 and abs(rel - rel0) <= 1e-6 * rel0
+        assert float((x - x0).norm()) <= 1e-11 * float(x0.norm())
+        assert bool(torch.equal(x, x0)) or not scattered
+
+
+@pytest.mark.parametrize("n", [5, 1024, 5000, 16384])
+def test_small_pcg_special_right_hand_sides(n):
+    """A zero right-hand side, infinities and NaN stop after the iterations that the passes make, with the same values."""
+    import scipy.sparse as sp
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    a = sp.diags([-np.ones(n - 1), np.full(n, 2.5), -np.ones(n - 1)], [-1, 0, 1]).tocsr()
+    A = CsrMatrix.from_host(a.indptr.astype(np.int32), a.indices.astype(np.int32), a.data, (n, n), dev)
+    dinv = torch.full((n,), 0.4, dtype=torch.float64, device=dev)
+    for at, value in ((None, 0.0), (n - 1, float("nan")), (n // 2, float("inf")), (0, float("-inf"))):
+        b = torch.full((n,), 0.0 if at is None else 1.0, dtype=torch.float64, device=dev)
+        if at is not None:
+            b[at] = value
+        (x, it, rel), (x0, it0, rel0) = A.pcg(b, dinv, 1e-8, 50), _passes(A, b, dinv, 1e-8, 50)
+        assert it == it0 == 1 and np.isnan(rel) and np.isnan(rel0)
+        assert torch.equal(torch.isnan(x), torch.isnan(x0)) and torch.equal(torch.nan_to_num(x), torch.nan_to_num(x0))
