@@ -103,12 +103,28 @@ __device__ __forceinline__ double block_sum(double v, double *s_red) {
   return t;  // valid in thread 0
 }
 
+// Ordinary loads, for what the launch in front may still have been writing when this kernel became resident (launch_pdl):
+// the y of a product may be the next one's x, values or dot operand, and its carries are the fix-up kernel's.  The
+// read-only path (ld.global.nc, which __ldg and reads through const __restrict__ compile to) asks that data stays as it is
+// for the kernel's whole lifetime, which begins in front of pdl_wait().
+__device__ __forceinline__ double load_now(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ bool skipped(const int *flag) {
+  if (flag == nullptr) return false;
+  int v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(flag));
+  return v != 0;
+}
+
 // x is re-read by every block: ask L2 to keep it (evict_last) while the streamed
 // val/crd entries, read once, are marked evict_first by ld.global.cs.
 __device__ __forceinline__ double load_x(const double *p, uint64_t policy, bool hint) {
-  if (!hint) return __ldg(p);
+  if (!hint) return load_now(p);
   double v;
-  asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(policy));
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(policy));
   return v;
 }
 
@@ -164,7 +180,7 @@ __device__ __forceinline__ void reduce_short_rows(const ChunkCtx &c, const int *
       e = rel_at<I>(c, s_rel, pos, i + 1);
       is_long = (e - s) > SPMV_LONG_ROW;
       if (accumulate && lane == 0 && !is_long && !(c.has_tail && i == c.nr - 1)) yin = y[c.row0 + i];
-      if (FUSE_DOT && lane == 0 && !is_long) dv = dotvec[c.row0 + i];  // in flight while the row is summed
+      if (FUSE_DOT && lane == 0 && !is_long) dv = load_now(dotvec + c.row0 + i);  // in flight while the row is summed
       if (!is_long)
         for (int j = s + lane; j < e; j += L) acc = __dadd_rn(acc, s_prod[j]);
     }
@@ -199,7 +215,7 @@ spmv_chunk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const do
 
   pdl_release();  // only the small fix-up kernel follows at once
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
 
   const int tid = threadIdx.x;
   ChunkCtx c;
@@ -268,7 +284,7 @@ spmv_chunk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const do
     const int s = rel_at<I>(c, s_rel, pos, i), e = rel_at<I>(c, s_rel, pos, i + 1);
     double yin = 0.0, dv = 0.0;
     if (accumulate && lane == 0 && !(c.has_tail && i == c.nr - 1)) yin = y[c.row0 + i];
-    if (FUSE_DOT && lane == 0) dv = dotvec[c.row0 + i];
+    if (FUSE_DOT && lane == 0) dv = load_now(dotvec + c.row0 + i);
     double acc = 0.0;
     for (int j = s + lane; j < e; j += 32) acc = __dadd_rn(acc, s_prod[j]);
 #pragma unroll
@@ -322,7 +338,7 @@ spmv_scan_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
 
   pdl_release();  // only the small fix-up kernel follows at once
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int chunk = (int)blockIdx.x;
@@ -414,7 +430,7 @@ spmv_scan_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     const bool is_tail = c.has_tail && i == c.nr - 1;
     double yin = 0.0, dv = 0.0;
     if (accumulate && !is_tail) yin = y[c.row0 + i];
-    if (FUSE_DOT) dv = dotvec[c.row0 + i];
+    if (FUSE_DOT) dv = load_now(dotvec + c.row0 + i);
     double acc = 0.0;
     if (e > s) {
       const int g = (e - 1) >> 6;
@@ -489,7 +505,7 @@ spmv_pipe_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
 
   pdl_release();  // only the small fix-up kernel follows at once
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
   const int tid = threadIdx.x;
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&full[0])));
@@ -577,7 +593,7 @@ spmv_pipe_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
       if (j < len4)
         prod[j] = __dmul_rn(prod[j], xv[k]);
       else if (j < c.len)
-        prod[j] = __dmul_rn(val[c.c0 + j], xv[k]);
+        prod[j] = __dmul_rn(load_now(val + c.c0 + j), xv[k]);
     }
     __syncthreads();
 
@@ -592,7 +608,7 @@ spmv_pipe_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
       const int s0 = rel_at<I>(c, s_rel, pos, i), e0 = rel_at<I>(c, s_rel, pos, i + 1);
       double yin = 0.0, dv = 0.0;
       if (accumulate && lane == 0 && !(c.has_tail && i == c.nr - 1)) yin = y[c.row0 + i];
-      if (FUSE_DOT && lane == 0) dv = dotvec[c.row0 + i];
+      if (FUSE_DOT && lane == 0) dv = load_now(dotvec + c.row0 + i);
       double acc = 0.0;
       for (int j = s0 + lane; j < e0; j += 32) acc = __dadd_rn(acc, prod[j]);
 #pragma unroll
@@ -639,7 +655,7 @@ spmv_pipe_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
 // sum, not the bits of the chunk kernels (relaxed tuner only).  val and crd must be 32-byte aligned.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void load_stream_256(const void *p, uint64_t &a, uint64_t &b, uint64_t &c, uint64_t &d) {
-  asm volatile("ld.global.nc.L1::evict_first.L2::evict_first.v4.b64 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::evict_first.L2::evict_first.v4.b64 {%0,%1,%2,%3}, [%4];"
                : "=l"(a), "=l"(b), "=l"(c), "=l"(d)
                : "l"(p));
 }
@@ -659,12 +675,6 @@ __device__ __forceinline__ void load_entries4(const int32_t *crd, const double *
   a[0] = __longlong_as_double((long long)v0); a[1] = __longlong_as_double((long long)v1);
   a[2] = __longlong_as_double((long long)v2); a[3] = __longlong_as_double((long long)v3);
 }
-__device__ __forceinline__ double load_x_ordered(const double *p) {  // volatile: stays behind the loads issued before it
-  double v;
-  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
 constexpr int SPMV_WALK_THREADS = 128;
 constexpr int SPMV_WALK_FINE_TILE = 512;  // entries per warp on matrices too small to fill the SMs with 2048-entry ranges
 constexpr int SPMV_WALK_STEP = 128;  // entries per step: four per lane
@@ -680,7 +690,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   constexpr int S = SPMV_WALK_STEP;
   pdl_release();  // only the small fix-up kernel follows at once
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * (SPMV_WALK_THREADS / 32) + (threadIdx.x >> 5);
   if (w >= nblk) return;
@@ -702,7 +712,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
         aa[k] = 0.0;
         if (j0 + k < c_end) {
           cc[k] = (int64_t)crd[j0 + k];
-          aa[k] = val[j0 + k];
+          aa[k] = load_now(val + j0 + k);
         }
       }
     }
@@ -741,7 +751,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     const int e = end_offset(r_cur + lane, c);
     double xv[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) xv[k] = load_x_ordered(x + ci[k]);
+    for (int k = 0; k < 4; ++k) xv[k] = load_now(x + ci[k]);  // volatile: behind the loads issued before
     if (c + S < c_end) fetch(c + S, cn, an);
 
     // ---- rows that end in this step; bit e of the mask for every end offset e < S ------------------
@@ -787,7 +797,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
         if (h5 & (2u << k)) {
           const int64_t row = r_cur + below + __popc(h & (((2u << k) - 1u) & ~1u));
           if (accumulate) yin[k] = y[row];
-          if (FUSE_DOT) dv[k] = dotvec[row];
+          if (FUSE_DOT) dv[k] = load_now(dotvec + row);
         }
     }
 
@@ -853,7 +863,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
           const int64_t row = rbase + lane;
           const double yi = accumulate ? y[row] : 0.0;
           y[row] = __dadd_rn(sum, yi);
-          if (FUSE_DOT) dot_local = __dadd_rn(dot_local, __dmul_rn(sum, dotvec[row]));
+          if (FUSE_DOT) dot_local = __dadd_rn(dot_local, __dmul_rn(sum, load_now(dotvec + row)));
         }
         prev_e = __shfl_sync(FULL, re, 31);
       }
@@ -863,7 +873,7 @@ spmv_walk_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   if (lane == 0) {
     const bool has_tail = r_cur < nrows && c_end < nnz_end;  // row r_cur runs past this chunk (or starts at its end: open == 0)
     carry[w] = has_tail ? open : 0.0;
-    if (FUSE_DOT && has_tail) dot_local = __dadd_rn(dot_local, __dmul_rn(open, dotvec[r_cur]));
+    if (FUSE_DOT && has_tail) dot_local = __dadd_rn(dot_local, __dmul_rn(open, load_now(dotvec + r_cur)));
   }
   if (FUSE_DOT) {
 #pragma unroll
@@ -889,7 +899,7 @@ __global__ void spmv_fixup_kernel(const I *__restrict__ pos, const int64_t *__re
   // kernel drains; nothing is read before that kernel has completed and its writes are visible.
   pdl_wait();
   pdl_release();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk - 1) return;
   const int64_t q = plan[b + 1];
@@ -898,8 +908,8 @@ __global__ void spmv_fixup_kernel(const I *__restrict__ pos, const int64_t *__re
   const int64_t c0 = abase + b * (int64_t)tile;
   if (start >= c0 + tile) return;                   // row q starts in a later chunk: nothing carried
   if (b > 0 && plan[b] == q && start < c0) return;  // chunk b-1 carried into q too: not the head of the run
-  double acc = carry[b];
-  for (int64_t b2 = b + 1; b2 < nblk - 1 && plan[b2 + 1] == q; ++b2) acc = __dadd_rn(acc, carry[b2]);
+  double acc = load_now(carry + b);
+  for (int64_t b2 = b + 1; b2 < nblk - 1 && plan[b2 + 1] == q; ++b2) acc = __dadd_rn(acc, load_now(carry + b2));
   y[q] = __dadd_rn(y[q], acc);
 }
 
@@ -919,15 +929,18 @@ __device__ __forceinline__ double row_piece_sum(const I *__restrict__ crd, const
   int64_t j = lo;
   for (; j + 3 < hi; j += 4) {
     double a[4], xv[4];
+    I ci[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      a[u] = __ldg(val + j + u);
-      xv[u] = __ldg(x + (int64_t)__ldg(crd + j + u));
+      ci[u] = __ldg(crd + j + u);
+      a[u] = load_now(val + j + u);
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) xv[u] = load_now(x + (int64_t)ci[u]);
 #pragma unroll
     for (int u = 0; u < 4; ++u) acc = __dadd_rn(acc, __dmul_rn(a[u], xv[u]));
   }
-  for (; j < hi; ++j) acc = __dadd_rn(acc, __dmul_rn(__ldg(val + j), __ldg(x + (int64_t)__ldg(crd + j))));
+  for (; j < hi; ++j) acc = __dadd_rn(acc, __dmul_rn(load_now(val + j), load_now(x + (int64_t)__ldg(crd + j))));
   return acc;
 }
 
@@ -943,7 +956,7 @@ spmv_rowthread_kernel(const I *__restrict__ pos, const I *__restrict__ crd, cons
   __shared__ double s_red[8];
   __shared__ int s_flag;
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
   if (PCG_FUSED && ex.mbox != nullptr && !pcg_wait_halo(ex, &s_flag)) return;
   double dot_local = 0.0;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -952,7 +965,7 @@ spmv_rowthread_kernel(const I *__restrict__ pos, const I *__restrict__ crd, cons
     const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
     const double yin = accumulate ? y[row] : 0.0;
     double dv = 0.0;
-    if (FUSE_DOT) dv = dotvec[row];
+    if (FUSE_DOT) dv = load_now(dotvec + row);
     const int64_t bnd = abase + ((lo - abase) / SPMV_TILE + 1) * (int64_t)SPMV_TILE;  // first chunk boundary after lo
     if (bnd >= hi) {
       const double s = row_piece_sum<I>(crd, val, x, lo, hi);
@@ -998,7 +1011,7 @@ spmv_rowblock_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const
   static_assert(ROWS <= THREADS, "one thread per row");
   extern __shared__ double s_rowprod[];
   pdl_wait();
-  if (skip_flag != nullptr && *skip_flag != 0) return;
+  if (skipped(skip_flag)) return;
   const int64_t r0 = (int64_t)blockIdx.x * ROWS;
   const int nr = (int)(nrows - r0 < ROWS ? nrows - r0 : ROWS);
   const int64_t e0 = (int64_t)pos[r0];
@@ -1022,7 +1035,7 @@ spmv_rowblock_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const
       a[u] = __ldcs(v + j + u * THREADS);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) xv[u] = __ldg(x + (int64_t)ci[u]);
+    for (int u = 0; u < 4; ++u) xv[u] = load_now(x + (int64_t)ci[u]);
 #pragma unroll
     for (int u = 0; u < 4; ++u) s_rowprod[j + u * THREADS] = __dmul_rn(a[u], xv[u]);
   }
@@ -1036,7 +1049,7 @@ spmv_rowblock_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const
       a[u] = in ? __ldcs(v + j + u * THREADS) : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 3; ++u) xv[u] = j + u * THREADS < n ? __ldg(x + (int64_t)ci[u]) : 0.0;
+    for (int u = 0; u < 3; ++u) xv[u] = j + u * THREADS < n ? load_now(x + (int64_t)ci[u]) : 0.0;
 #pragma unroll
     for (int u = 0; u < 3; ++u)
       if (j + u * THREADS < n) s_rowprod[j + u * THREADS] = __dmul_rn(a[u], xv[u]);

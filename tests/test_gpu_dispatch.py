@@ -423,3 +423,34 @@ def test_small_pcg_special_right_hand_sides(n):
         (x, it, rel), (x0, it0, rel0) = A.pcg(b, dinv, 1e-8, 50), _passes(A, b, dinv, 1e-8, 50)
         assert it == it0 == 1 and np.isnan(rel) and np.isnan(rel0)
         assert torch.equal(torch.isnan(x), torch.isnan(x0)) and torch.equal(torch.nan_to_num(x), torch.nan_to_num(x0))
+
+
+@pytest.mark.parametrize("kernel", [(1, 0, 2), (1, 0, 3), (1, 0, 4), (256, 4, 1), (512, 3, 0), (-256, 3, 1), (2, 5, 1), (3, 4, 0), (4, 0, 0)], ids=str)
+def test_products_read_the_values_that_the_one_before_wrote(kernel):
+    """Overlapped launches of every kernel: the result of a product is the next one's vector and then its matrix values."""
+    from lapis_b200._lib import check, load
+    from lapis_b200.device import CsrMatrix
+    dev, lib = _dev(), load()
+    rng = np.random.default_rng(7)
+    n, mean = 4000, 9
+    pos, crd, val = (torch.as_tensor(a).to(dev) for a in _csr(rng, np.full(n, mean), n, np.int64))
+    wide = CsrMatrix.from_host(*_csr(rng, np.full(n * mean, 3), n, np.int64), (n * mean, n), dev)  # y of this: the values of that
+    ends = []
+    check(lib.lapis_b200_spmv_select_kernel(*kernel))
+    try:
+        for sync in (True, False):
+            v = val.clone()
+            A = CsrMatrix(pos, crd, v, (n, n))
+            a, b = torch.ones(n, dtype=torch.float64, device=dev), torch.zeros(n, dtype=torch.float64, device=dev)
+            for _ in range(30):
+                for call in (lambda: A.spmv(a, b, accumulate=False), lambda: wide.spmv(b, v, accumulate=False)):
+                    call()
+                    if sync:
+                        torch.cuda.synchronize()
+                v.clamp_(-1, 1)
+                a, b = b, a
+            ends.append((a, v))
+    finally:
+        check(lib.lapis_b200_spmv_select_kernel(0, 0, 0))
+    assert torch.equal(ends[0][0], ends[1][0]) and torch.equal(ends[0][1], ends[1][1])
+    assert bool(torch.isfinite(ends[0][0]).all())
