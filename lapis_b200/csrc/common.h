@@ -126,9 +126,9 @@ struct lapis_b200_csr {
 
 namespace lapis_b200 {
 // SpMM over a CSR matrix (rowno null) or the stored rows of a DCSR matrix (their numbers in rowno), spmm.cu.
-// max_row_len: an upper bound, -1 if not known.
+// nnz, max_row_len (-1: not known): of a CSR matrix only.
 int spmm_launch(int idx_bytes, const void *rowno, const void *pos, const void *crd, const double *val, int64_t nrows, int64_t k,
-                int64_t max_row_len, const double *B, double *C, int accumulate, cudaStream_t st);
+                int64_t nnz, int64_t max_row_len, const double *B, double *C, int accumulate, cudaStream_t st);
 // Fills a handle over arrays whose first offset, entry count and longest row are known, allocates its scratch and
 // enqueues the planning kernels.  plan_on_demand: no scratch and no plan when SpMV will run on the kernels for short
 // rows, which need none (for a handle that serves one product).

@@ -280,5 +280,5 @@ extern "C" int lapis_b200_spmm_dcsr_f64(int idx_bytes, int64_t nrows, int64_t nc
     return fail(LAPIS_EBADSHAPE, "spmm_dcsr: bad dimensions");
   if (nstored == 0 || k == 0) return LAPIS_OK;
   if (d_i1 == nullptr || d_p2 == nullptr || d_C == nullptr) return fail(LAPIS_EBADARG, "spmm_dcsr: null operand");
-  return spmm_launch(idx_bytes, d_i1, d_p2, d_i2, d_val, nstored, k, -1, d_B, d_C, 1, as_stream(stream));
+  return spmm_launch(idx_bytes, d_i1, d_p2, d_i2, d_val, nstored, k, 0, -1, d_B, d_C, 1, as_stream(stream));
 }

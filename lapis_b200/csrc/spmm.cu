@@ -55,12 +55,14 @@ __device__ __forceinline__ double cols_mul(double a, double b) { return __dmul_r
 __device__ __forceinline__ double2 cols_mul(double a, double2 b) { return make_double2(__dmul_rn(a, b.x), __dmul_rn(a, b.y)); }
 
 // Whether a row of len entries is left to spmm_long_kernel.  A group of lanes walks it in a chain of trips to memory, about
-// 0.15 us an entry and 64 columns; it may last half as long as the whole product does (8 (k + 8) bytes an entry at
-// 5 TB/s), and is then hidden by it.
+// 0.15 us an entry and 64 columns; it may last half as long as the whole product of nnz entries does (8 (k + 8) bytes an
+// entry at 5 TB/s), and is then hidden by it.
+__host__ __device__ __forceinline__ bool spmm_is_long(int64_t len, int64_t nnz, int64_t k) {
+  return len > SPMM_LONG && len > nnz * (k + 8) / ((k + 63) / 64) >> 17;
+}
 template <typename I>
 __device__ __forceinline__ bool spmm_is_long(int64_t len, const I *__restrict__ pos, int64_t nrows, int64_t k) {
-  if (len <= SPMM_LONG) return false;
-  return len > ((int64_t)pos[nrows] - (int64_t)pos[0]) * (k + 8) / ((k + 63) / 64) >> 17;
+  return len > SPMM_LONG && spmm_is_long(len, (int64_t)pos[nrows] - (int64_t)pos[0], k);
 }
 
 // The stored entries [lo, hi) of row r and the row of C it belongs to; false: nothing to do for r.
@@ -256,12 +258,14 @@ static cudaError_t launch_spmm_as(const SpmmArgs<I> &m, cudaStream_t st) {
   const unsigned grid = (unsigned)((m.nrows + ROWS - 1) / ROWS);
   const T *B = reinterpret_cast<const T *>(m.B);
   T *C = reinterpret_cast<T *>(m.C);
-  if (m.long_rows)
-    return launch_pdl(spmm_kernel<I, DCSR, true, V, G, Q>, grid + 1, SPMM_THREADS, 0, st, m.rowno, m.pos, m.crd, m.val, m.nrows, m.k / V,
-                      B, C, m.accumulate);
-  spmm_kernel<I, DCSR, false, V, G, Q><<<grid, SPMM_THREADS, 0, st>>>(m.rowno, m.pos, m.crd, m.val, m.nrows, m.k / V, B, C,
-                                                                      m.accumulate);
-  return cudaGetLastError();
+  if constexpr (!DCSR)
+    if (!m.long_rows) {
+      spmm_kernel<I, false, false, V, G, Q><<<grid, SPMM_THREADS, 0, st>>>(m.rowno, m.pos, m.crd, m.val, m.nrows, m.k / V, B, C,
+                                                                           m.accumulate);
+      return cudaGetLastError();
+    }
+  return launch_pdl(spmm_kernel<I, DCSR, true, V, G, Q>, grid + 1, SPMM_THREADS, 0, st, m.rowno, m.pos, m.crd, m.val, m.nrows, m.k / V, B,
+                    C, m.accumulate);
 }
 
 // Pairs keep one pair per lane and pass (Q = 2 and 3 measured 10 to 17 % slower at k = 66 and 96); single columns, which move
@@ -294,8 +298,9 @@ static cudaError_t launch_spmm(const SpmmArgs<I> &m, cudaStream_t st) {
 }
 
 int spmm_launch(int idx_bytes, const void *rowno, const void *pos, const void *crd, const double *val, int64_t nrows, int64_t k,
-                int64_t max_row_len, const double *B, double *C, int accumulate, cudaStream_t st) {
-  const bool long_rows = max_row_len < 0 || max_row_len > SPMM_LONG;
+                int64_t nnz, int64_t max_row_len, const double *B, double *C, int accumulate, cudaStream_t st) {
+  // nothing is known of the stored rows of a DCSR matrix
+  const bool long_rows = rowno != nullptr || max_row_len < 0 || spmm_is_long(max_row_len, nnz, k);
   auto run = [&](auto index) {
     using I = decltype(index);
     const SpmmArgs<I> m = {static_cast<const I *>(rowno), static_cast<const I *>(pos), static_cast<const I *>(crd), val, nrows, k, B, C,

@@ -1783,8 +1783,8 @@ extern "C" int lapis_b200_spmm_f64(lapis_b200_csr_t h, int64_t k, const double *
   if (k < 0) return fail(LAPIS_EBADSHAPE, "spmm: negative k");
   if (h->nrows == 0 || k == 0) return LAPIS_OK;
   if (d_C == nullptr || (h->nnz > 0 && d_B == nullptr)) return fail(LAPIS_EBADARG, "spmm: null operand");
-  return spmm_launch(h->idx_bytes, nullptr, h->pos, h->crd, h->val, h->nrows, k, h->max_row_len, d_B, d_C, accumulate,
-                     as_stream(stream));
+  return spmm_launch(h->idx_bytes, nullptr, h->pos, h->crd, h->val, h->nrows, k, h->nnz, h->max_row_len, d_B, d_C,
+                     accumulate, as_stream(stream));
 }
 
 // ---------------------------------------------------------------------------

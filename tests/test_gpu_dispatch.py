@@ -454,3 +454,52 @@ def test_products_read_the_values_that_the_one_before_wrote(kernel):
         check(lib.lapis_b200_spmv_select_kernel(0, 0, 0))
     assert torch.equal(ends[0][0], ends[1][0]) and torch.equal(ends[0][1], ends[1][1])
     assert bool(torch.isfinite(ends[0][0]).all())
+
+
+@pytest.mark.parametrize("over", [0, 1])
+@pytest.mark.parametrize("k,rows", [(16, 110_000), (65, 30_000)])
+def test_spmm_at_the_limit_for_long_rows(k, rows, over):
+    """The longest row at and just above what the kernel beside the main one takes: the host's rule and the kernels' agree."""
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    rng = np.random.default_rng(k)
+    lens = np.full(rows, 16)
+    rule = lambda nnz: max(256, (nnz * (k + 8) // ((k + 63) // 64)) >> 17)
+    longest = 256
+    while longest < rule(16 * (rows - 3) + 3 * longest) + over:
+        longest += 1
+    lens[[0, rows // 2, rows - 1]] = longest
+    assert (longest > rule(int(lens.sum()))) == bool(over)
+    pos, crd, val = _csr(rng, lens, rows, np.int32)
+    B, C = rng.uniform(-1, 1, (rows, k)), rng.uniform(-1, 1, (rows, k))
+    A = CsrMatrix.from_host(pos, crd, val, (rows, rows), dev)
+    got = A.spmm(torch.as_tensor(B).to(dev), torch.as_tensor(C).to(dev))
+    assert np.array_equal(got.cpu().numpy(), oracle.spmm(pos, crd, val, B, C))
+
+
+@pytest.mark.parametrize("k", [1, 3, 8, 64, 101])
+def test_spmm_special_values(k):
+    """Infinities and NaN in values and operands, short and long rows, empty rows and an all-zero product: what the
+    sequential loop makes of them, and nothing of them in the rows beside."""
+    from lapis_b200.device import CsrMatrix, spmm_dcsr
+    dev = _dev()
+    rng = np.random.default_rng(k)
+    rows, ncols = 300, 900
+    lens = rng.integers(0, 12, rows)
+    lens[[3, 150, 299]] = (700, 301, 513)
+    for idx in (np.int32, np.int64):
+        pos, crd, val = _csr(rng, lens, ncols, idx)
+        for v in (np.inf, -np.inf, np.nan, -0.0):
+            val[rng.integers(0, val.size, 6)] = v
+        B, C = rng.uniform(-1, 1, (ncols, k)), rng.uniform(-1, 1, (rows, k))
+        for v in (np.inf, np.nan, 0.0):
+            B[rng.integers(0, ncols, 9), rng.integers(0, k, 9)] = v
+        d = [torch.as_tensor(a).to(dev) for a in (pos, crd, val)]
+        with np.errstate(all="ignore"):
+            want = oracle.spmm(pos, crd, val, B, C)
+        assert 0 < np.isnan(want).sum() < want.size
+        got = [CsrMatrix(*d, (rows, ncols)).spmm(torch.as_tensor(B).to(dev), torch.as_tensor(C).to(dev)),
+               spmm_dcsr(torch.arange(rows, device=dev, dtype=d[0].dtype), *d, torch.as_tensor(B).to(dev), torch.as_tensor(C).to(dev), ncols)]
+        wants = [want, oracle.spmm_dcsr(np.arange(rows).astype(idx), pos, crd, val, B, C)]
+        for g, w_ in zip(got, wants):
+            assert np.array_equal(g.cpu().numpy(), w_, equal_nan=True)
