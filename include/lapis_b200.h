@@ -79,7 +79,9 @@ typedef struct { int64_t dims[2]; int64_t mem_sizes[5]; } lapis_dcsr_spec;
 /* ---- layer 1: emitted-module ABI ------------------------------------------ */
 
 /* TranslateToKokkosCpp.cpp:4281-4378.  initialize is idempotent; finalize frees
- * every result buffer handed out since initialize (LAPISSupport.hpp:93-120). */
+ * every result buffer handed out since initialize (LAPISSupport.hpp:93-120), and gives
+ * the device memory back that the library holds idle (at most 256 MB per device); without
+ * an initialize it does the latter only. */
 void lapis_initialize(void);
 void lapis_finalize(void);
 

@@ -75,15 +75,33 @@ static int pool_of_device(cudaMemPool_t *out) {
   return LAPIS_OK;
 }
 
+// Where the device is full, the memory that the pools hold idle goes back to it and the allocation is tried again.
+template <typename F>
+static cudaError_t alloc_or_trim(F &&alloc) {
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaDeviceSynchronize();  // what was freed behind work still running
+    pool_trim();
+    e = alloc();
+  }
+  return e;
+}
+
+static int alloc_status(cudaError_t e, void **p, size_t bytes) {
+  if (e == cudaSuccess) return LAPIS_OK;
+  *p = nullptr;
+  return fail(LAPIS_ECUDA, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+}
+
 int pool_alloc(void **p, size_t bytes, cudaStream_t st) {
   cudaMemPool_t pool = nullptr;
   LAPIS_TRY(pool_of_device(&pool));
-  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 16, pool, st);
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return fail(LAPIS_ECUDA, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-  }
-  return LAPIS_OK;
+  return alloc_status(alloc_or_trim([&] { return cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 16, pool, st); }), p, bytes);
+}
+
+int large_alloc(void **p, size_t bytes) {
+  return alloc_status(alloc_or_trim([&] { return cudaMalloc(p, bytes); }), p, bytes);
 }
 
 void pool_free(void *p, cudaStream_t st) {
@@ -529,7 +547,10 @@ extern "C" void lapis_initialize(void) {
 
 extern "C" void lapis_finalize(void) {
   clear_error();
-  if (g_init_count <= 0) return;
+  if (g_init_count <= 0) {
+    pool_trim();  // a program that holds matrix handles only gives idle memory back this way
+    return;
+  }
   if (--g_init_count == 0) {
     for (void *p : g_alive_host) std::free(p);
     g_alive_host.clear();

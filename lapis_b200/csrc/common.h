@@ -35,16 +35,18 @@ int sm_count();
 
 // Stream-ordered device memory from a pool of this library, one per device (cudaMalloc and cudaFree cost 330 and
 // 265 us each where they were measured, an allocation from the pool about 1 us).  Safe with several threads and
-// streams: the driver orders reuse by stream.  The pool keeps at most POOL_KEEP_BYTES of freed memory and gives the
-// rest back at the next synchronisation; pool_trim returns all of it (lapis_finalize).
-constexpr size_t POOL_KEEP_BYTES = size_t(512) << 20;
+// streams: the driver orders reuse by stream.  The pool keeps at most POOL_KEEP_BYTES of freed memory, which is the
+// largest block that it serves, and gives the rest back at the next synchronisation; pool_trim returns all of it
+// (lapis_finalize, and an allocation that fails).
+constexpr size_t POOL_LARGEST = size_t(256) << 20;
+constexpr size_t POOL_KEEP_BYTES = POOL_LARGEST;
 int pool_alloc(void **p, size_t bytes, cudaStream_t st);
 void pool_free(void *p, cudaStream_t st);
 void pool_trim();
+int large_alloc(void **p, size_t bytes);  // cudaMalloc
 
 // Scoped device memory.  Large blocks come from cudaMalloc: mapping memory into the pool and out again costs 25 ms each
 // way for 850 MB, cudaMalloc and cudaFree 1 to 4 ms.
-constexpr size_t POOL_LARGEST = size_t(256) << 20;
 struct PoolBuf {
   void *p = nullptr;
   cudaStream_t st = nullptr;
@@ -59,9 +61,7 @@ struct PoolBuf {
   int alloc(size_t bytes, cudaStream_t stream) {
     st = stream;
     pooled = bytes <= POOL_LARGEST;
-    if (pooled) return pool_alloc(&p, bytes, stream);
-    LAPIS_CUDA_TRY(cudaMalloc(&p, bytes));
-    return LAPIS_OK;
+    return pooled ? pool_alloc(&p, bytes, stream) : large_alloc(&p, bytes);
   }
 };
 

@@ -36,6 +36,8 @@ static std::set<void *> g_device, g_locked;  // live device allocations, page-lo
 static int g_copies = 0, g_waited = 0;       // copies from page-locked memory so far; how many of them were waited for
 static int g_launches = 0;                   // calls into the kernels
 static int g_kernel_status = LAPIS_OK;       // what the kernels return
+static size_t g_idle = 0, g_keep = 0;        // what the pool holds freed, what it may hold
+static bool g_full = false;                  // the device has no room but what the pool holds idle
 static std::vector<char *> g_page_locked;    // blocks of a caller, LOCKED_BYTES each
 constexpr size_t LOCKED_BYTES = size_t(4) << 20;
 
@@ -74,6 +76,7 @@ const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
 cudaError_t cudaMalloc(void **p, size_t n) {
   NoFailure keep;
   std::lock_guard<std::mutex> l(g_fake);
+  if (g_full && g_idle > 0) return cudaErrorMemoryAllocation;
   *p = std::malloc(n);
   g_device.insert(*p);
   return cudaSuccess;
@@ -85,8 +88,8 @@ cudaError_t cudaFree(void *p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t *pool, const cudaMemPoolProps *) { return *pool = (cudaMemPool_t)1, cudaSuccess; }
-cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
-cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *v) { return g_keep = *static_cast<uint64_t *>(v), cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return g_idle = 0, cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
@@ -330,6 +333,26 @@ static void threads() {
   for (std::thread &t : pool) t.join();
 }
 
+// A device that is full but for what the pool holds idle: the call gets that memory, from the pool and beside it.
+static void full_device() {
+  Product small(1000), large(9000000);  // 300 MB of operands
+  EXPECT(small.run() == LAPIS_OK && small.right());
+  EXPECT(0 < g_keep && g_keep <= POOL_LARGEST);
+  g_full = true;
+  for (Product *a : {&small, &large}) {
+    g_idle = g_keep;
+    EXPECT(a->run() == LAPIS_OK && a->right() && g_idle == 0);
+  }
+  g_full = false;
+  g_idle = g_keep;
+  lapis_finalize();
+  EXPECT(g_idle == 0);
+  g_idle = g_keep;
+  lapis_finalize();  // no module is alive: idle memory is given back all the same
+  EXPECT(g_idle == 0);
+  lapis_initialize();
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   lapis_initialize();
@@ -342,6 +365,8 @@ int main(int argc, char **argv) {
     exhausted();
   } else if (what == "fork_exit") {
     fork_exit();
+  } else if (what == "full_device") {
+    full_device();
   } else if (what == "threads") {
     threads();
   } else {

@@ -26,8 +26,9 @@ def program(tmp_path_factory):
 # in_flight: a call that fails behind the upload leaves no copy from the caller's page-locked arrays under way
 # exhausted: memory or threads that cannot be had; no exception may leave a C entry point
 # fork_exit: a child process forked behind a large call exits
+# full_device: idle memory of the pool goes to an allocation that fails without it, and back to the device
 # threads: four threads in calls at once
-@pytest.mark.parametrize("scenario", ["offsets", "in_flight", "exhausted", "fork_exit", "threads"])
+@pytest.mark.parametrize("scenario", ["offsets", "in_flight", "exhausted", "fork_exit", "full_device", "threads"])
 def test_host_calls(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
