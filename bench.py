@@ -345,7 +345,7 @@ NCU_TRAFFIC = {
     "spmv_chunk_kernel": 3.325e9,   # profiles/spmv_chunk_kernel_config2.md
     "spmv_scan_kernel": 3.290e9,    # profiles/spmv_walk_kernel_config2.md (launch list of the tuner's candidates)
     "spmv_pipe_kernel": 3.160e9,    # same list
-    "spmm": 3.387e10,               # profiles/spmm_row_kernel_config3.md
+    "spmm": 3.386e10,               # profiles/general_kernels.md (spmm_kernel, 2^21 rows, k = 64)
     "bgemm": 1.036e9,               # profiles/bgemm_tcgen05_kernel.md (4096 x 128^3)
     "gemm": 8.15e9,                 # profiles/bgemm_tcgen05_kernel.md (8192^3, K in segments of 1024)
     "pcg": 2.715e9,                 # profiles/pcg_iteration_config5.md (the three kernels of one iteration)
