@@ -66,8 +66,10 @@ struct PoolBuf {
 };
 
 // Launch that may start while the kernel in front of it drains (programmatic stream serialization): the blocks become
-// resident early and stop at pdl_wait().  Only for kernels that call pdl_wait() before their first access to global
-// memory.  Back-to-back small launches then follow each other without the gap of about 1.5 us.
+// resident early and stop at pdl_wait().  Only for kernels that call pdl_wait() before their first access to memory that
+// the kernel in front writes (the main SpMM kernel shares nothing but inputs with the one for long rows in front of it);
+// what that kernel may still be writing is read by ordinary loads, not by the read-only path.  Back-to-back small launches
+// then follow each other without the gap of about 1.5 us.
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};

@@ -120,10 +120,10 @@ __device__ __forceinline__ float madd(float a, float b, float c) { return __fadd
 // neighbouring output elements, G groups apart, with U stored entries in flight; the adds stay in entry order.  V = 4:
 // 16-byte accesses to B and C, the values of the elements' fibers one by one, or with FIBER4 (nh a multiple of four) also by
 // 16 bytes: taken for rows of more than 256 elements, where 40 registers and twelve blocks an SM keep more gathers in
-// flight than bspmm_csrv_vec4_kernel's 48 (131,072 rows of 32, 8 x 64: 1217 -> 1056 us; 20,000 of 30, 16 x 128: 558 -> 487).  Bound by the gathers of rows of B; G
-// follows the row's length, so that short rows do not leave most of a warp idle (50,000 rows of 20, 4 elements each: 84 -> 17
-// us; 200,000 rows of 8, 2 x 4: 155 -> 28), and wide accesses halve the requests (50,000 rows of 20, 1 x 64: 85 -> 48; 30,000 of
-// 30, 11 x 40: 269 -> 235; 20,000 of 30, 15 x 128: 718 -> 676).
+// flight than bspmm_csrv_vec4_kernel's 48 (131,072 rows of 32, 8 x 64: 1.29 -> 1.15 ms; 20,000 of 30, 16 x 128: 558 -> 487 us).  Bound by the gathers of
+// rows of B; G follows the row's length, so that short rows do not leave most of a warp idle (50,000 rows of 20, 4 elements
+// each: 84 -> 17 us; 200,000 rows of 8, 2 x 4: 155 -> 28), and wide accesses halve the requests (50,000 rows of 20, 1 x 64:
+// 85 -> 48; 30,000 of 30, 11 x 40: 269 -> 235; 20,000 of 30, 15 x 128: 718 -> 676).
 template <typename I, int V, bool FIBER4, int G, int Q>
 __global__ void __launch_bounds__(BSPMM_THREADS, FIBER4 ? 12 : 6)
 bspmm_csrv_group_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float *__restrict__ val, int64_t nrows,

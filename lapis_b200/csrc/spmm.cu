@@ -9,11 +9,12 @@
 // most of a warp idle, and Q follows an odd k so that the entries of a row are read once for up to 128 columns.  With a
 // whole warp per row and one entry in flight per lane at odd k, before: 142,060 rows of 21, k = 3, 172 us (DCSR 136),
 // now 25; k = 6, 104 -> 32; 63,642 rows of 24, k = 33, 87 -> 63.  2^21 rows of 32, k = 64, is at DRAM bandwidth as it
-// was: 5.06 ms.
+// was: 5.1 to 5.3 ms before and now (33.9 GB).
 //
 // A row of 4096 entries walked U at a time is a chain of 4096 / U trips to memory, which outlasts everything else in a
 // skewed matrix.  Such rows go to a kernel of their own that runs beside this one (spmm_long_kernel): 50,021 rows with
-// a mean of 16 and a longest of 3845, k = 37: 466 -> 265 us (DCSR 773 -> 264); 10,000 rows, mean 30, k = 128: 839 -> 235.
+// a mean of 16 and rows up to 4096, k = 37, DCSR: 884 -> 218 to 283 us with the matrix drawn; 10,000 rows, mean 30,
+// k = 128: 839 -> 235.
 #include <algorithm>
 #include <cstdint>
 
@@ -87,7 +88,7 @@ __device__ __forceinline__ bool spmm_row(const I *__restrict__ rowno, const I *_
 // rowno: null for CSR; the stored rows' numbers for DCSR.  kv: columns in units of V.  With LONG_ROWS the long rows are
 // left to spmm_long_kernel, which this kernel overlaps: an extra block at its end waits for that kernel.
 // Blocks per SM: 32-bit indices fit 40 registers without the compiler pulling the gathers of a batch apart (six blocks:
-// 2^20 rows of 32, k = 64, 2.50 ms, without the bound 2.67); 64-bit ones need 48 (2^21 rows 5.27 ms, with six 5.36).
+// 2^20 rows of 32, k = 64, 2.50 ms, without the bound 2.67); 64-bit ones need 48 (2^21 rows: 2 % slower with six).
 template <typename I, bool DCSR, bool LONG_ROWS, int V, int G, int Q>
 __global__ void __launch_bounds__(SPMM_THREADS, sizeof(I) == 8 ? 1 : 6)
 spmm_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val,

@@ -10,7 +10,7 @@
 //   * The entry range is cut into chunks of a fixed size T (2048 by default); thread
 //     block b processes exactly chunk b, so every block streams T consecutive
 //     (val, crd) pairs with aligned 16-byte loads that are fully coalesced whatever
-//     the row lengths are, gathers x through the read-only path, and parks the
+//     the row lengths are, gathers x, and parks the
 //     products in shared memory.  All in-chunk indexing is 32-bit.
 //   * A per-matrix plan (8 bytes per chunk, one binary search each) gives the first
 //     row that ends inside each chunk.  Rows that end in the chunk are reduced out
