@@ -503,3 +503,35 @@ def test_spmm_special_values(k):
         wants = [want, oracle.spmm_dcsr(np.arange(rows).astype(idx), pos, crd, val, B, C)]
         for g, w_ in zip(got, wants):
             assert np.array_equal(g.cpu().numpy(), w_, equal_nan=True)
+
+
+def test_calls_on_host_arrays_from_two_threads():
+    """Two threads in calls at once, operands of one piece and of more than the staging ring holds: each gets its own result."""
+    import threading
+    from lapis_b200 import KokkosBackend as KB
+    from lapis_b200 import modules as mm
+    from lapis_b200.device import CsrMatrix
+    dev = _dev()
+    module = KB.KokkosBackend(decompose_tensors=True).compile(mm.spmv(mm.CSR64))
+    jobs, wrong = [], []
+    for n in (900, 250_000):
+        rng = np.random.default_rng(n)
+        pos, crd, val = _csr(rng, np.full(n, 5), n, np.int64)
+        x, y = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+        A = CsrMatrix.from_host(pos, crd, val, (n, n), dev)
+        want = A.spmv(torch.as_tensor(x).to(dev), torch.as_tensor(y).to(dev)).cpu().numpy()
+        jobs.append((pos, crd, val, ((n, n), (n + 1, len(crd), len(crd))), x, y, want))
+
+    def work(pos, crd, val, spec, x, y, want):
+        for _ in range(40):
+            got = y.copy()
+            module.spmv(pos, crd, val, spec, x, got)
+            if not np.array_equal(got, want):
+                wrong.append(len(x))
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
