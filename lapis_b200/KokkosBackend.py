@@ -464,7 +464,10 @@ class LAPISModule:
         def csr_args(pos, crd, val, spec):
             pos, crd, val = _c_array(pos, idx_dtype, 1), _c_array(crd, idx_dtype, 1), _c_array(val, np.float64, 1)
             dims, sizes = spec[0], spec[1]
-            packed = _CSR_SPEC.pack(int(dims[0]), int(dims[1]), int(sizes[0]), int(sizes[1]), int(sizes[2]))
+            try:
+                packed = _CSR_SPEC.pack(dims[0], dims[1], sizes[0], sizes[1], sizes[2])
+            except struct.error:  # extents that are no integers
+                packed = _CSR_SPEC.pack(*(int(v) for v in (dims[0], dims[1], sizes[0], sizes[1], sizes[2])))
             return (pos, crd, val), (_desc(pos, 1), _desc(crd, 1), _desc(val, 1), packed)
 
         if kind == "spmv":

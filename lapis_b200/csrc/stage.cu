@@ -187,8 +187,9 @@ bool page_locked(const void *p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// Neighbours are compared, never subtracted in the signed type: a corrupt array may hold offsets whose difference does
-// not fit it and wraps to a plausible length.
+// A corrupt array may hold offsets whose difference does not fit the type and wraps to a plausible length; between offsets
+// that are not negative none does, so a negative offset is looked for beside a negative length.  (Where the offsets of a
+// range are negative but ascend, the descent to them lies in a range in front, or pos[0] is not 0.)
 template <typename I>
 void check_pos(const I *pos, int64_t from, int64_t to, int64_t *max_len, int64_t *bad_row) {
   using U = std::make_unsigned_t<I>;
@@ -196,9 +197,9 @@ void check_pos(const I *pos, int64_t from, int64_t to, int64_t *max_len, int64_t
   for (int64_t i = std::max<int64_t>(from, 1); i < to; ++i) {
     const I len = (I)((U)pos[i] - (U)pos[i - 1]);
     longest = len > longest ? len : longest;
-    bad |= (I)(pos[i] < pos[i - 1]);
+    bad |= len | pos[i];
   }
-  if (bad != 0)
+  if (bad < 0)
     for (int64_t i = std::max<int64_t>(from, 1); i < to; ++i)
       if (pos[i] < pos[i - 1]) {
         *bad_row = i - 1;

@@ -205,7 +205,7 @@ template <typename I>
 static void offsets(void (*spmm)(lapis_memref2 **, lapis_memref1 *, lapis_memref1 *, lapis_memref1 *, const lapis_csr_spec *, lapis_memref2 *,
                                  lapis_memref2 *)) {
   const I top = std::numeric_limits<I>::max(), low = std::numeric_limits<I>::min();
-  const std::vector<std::vector<I>> middles = {{top, -2}, {top, low, -5}, {low}, {-1}, {top, low + 1, low}, {7, 3}, {top}, {11}};
+  const std::vector<std::vector<I>> middles = {{top, -2}, {top, low, -5}, {low}, {-1}, {top, low + 1, low}, {7, 3}, {top}, {11}, {top, low, low + 1, -1}};
   const int64_t nnz = 10, per_block = 65536 / sizeof(I);
   for (int64_t at : {(int64_t)1, (int64_t)5, per_block - 1, per_block, 9 * per_block - 1, 20 * per_block})
     for (const auto &m : middles) {
