@@ -1,0 +1,726 @@
+// fp32 matmul on the 5th-generation tensor cores from operands that are split once:  C[b] = C_in[b] + A[b] B[b]  for any M,
+// N, K and any alignment.
+//
+// x 2^e = hi + 2^-11 lo with hi and lo in fp16 (11 bits each, lo rounded), e one exponent for each row of A and each column
+// of B; the product is hi hi + 2^-11 (hi lo + lo hi), three fp16 products at twice the rate of the three TF32 products of
+// gemm_tcgen05.cu.  What is left out (lo lo, the rounding of lo) is at most 2^-21 of a product, where the TF32 split, whose
+// parts the tensor core truncates, leaves up to 2^-19.
+//
+//   split_kernel       reads A and B once, writes hi and lo as fp16 matrices with 16-byte rows (so that TMA can load shapes
+//                      and pointers of any alignment), and the scales.  K is cut into stretches of at most 1024, each with
+//                      scales of its own.
+//   gemm_split_kernel  a persistent GEMM over the parts: TMA -> tcgen05.mma.kind::f16 -> two accumulators in tensor memory
+//                      (hi hi, and the two mixed products, which are 2^-11 as large) -> scaled, joined, added to C.
+//
+// 8192^3: 5.05 -> 2.70 ms where the clock holds (407 TFLOP/s, three products at 75 % of cuBLAS's bf16 rate), 5.91 -> 3.33 where
+// power caps it; 5000 x 3000 x 1999 2.05 ms -> 0.21; 1000 x 1501 x 777 142 us -> 30 (a pass over the operands of 5, the
+// product 20, the look at the marks 3: latencies).  Against 64 bits: 8192^3 1.25e-6 (TF32 split 8.0e-6), 1000 x 1501 x 777
+// 3.9e-7 (sequential sum 5.0e-7), 100 x 100 x 130 1.9e-7 (2.1e-7).
+//
+// fp16 has 5 bits of exponent: an element below 2^-16 of the scaled range (2^-31 of the largest of its row or column) would
+// lose bits, and an infinity or NaN has no scale.  split_kernel marks the 128-row and 128-column panels that hold such an
+// element; the products of those panels are left to the kernels on unsplit operands (PanelFlags), which run behind
+// this one and return at once where there are none.  In 8192 x 8192 normally distributed numbers one is expected in every
+// eighth matrix, in uniformly distributed ones none.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cuda_fp16.h>
+
+#include "tcgen05.h"
+
+namespace lapis_b200 {
+
+namespace split {
+
+constexpr int KC = 1024;  // longest stretch of K: one scale for each row or column and stretch, one chain in tensor memory
+constexpr int GROUP_ROWS = 16, GROUP_COLS = 16;  // rows of A, columns of B that a block of split_kernel takes
+constexpr int SPLIT_THREADS = 512;
+constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f;
+
+struct Shape {
+  int M, N, Np, K;          // Np: columns of the split B, a multiple of GROUP_COLS
+  int chain;                 // k blocks of 64 that are added in tensor memory
+  int kc, first, stretches;  // stretches first .. first + stretches - 1, of kc (a multiple of 64) each, the last one shorter
+  int panels_a, panels_b;
+  __host__ __device__ int length(int s) const { return K - (first + s) * kc < kc ? K - (first + s) * kc : kc; }
+};
+
+struct Scratch {
+  __half *a, *b;             // [batch][stretch][hi, lo][M][kc], [batch][stretch][hi, lo][kc][Np]
+  float *scale_a, *scale_b;  // [batch][stretch][M], [batch][stretch][Np]: 2^-e
+  unsigned char *flag_a, *flag_b;  // [batch][stretch][panels][8]: a byte for every 16 rows or columns
+};
+
+// Exponent of the scale for a row or column whose largest magnitude has these bits: the largest power of two that keeps it
+// below 65504.  False: it has none (infinity, NaN) or one so far out that two scales might leave fp32's range together.
+__device__ __forceinline__ bool scale_exponent(uint32_t max_bits, int &e) {
+  const int ex = (int)(max_bits >> 23) - 127;
+  e = max_bits == 0 ? 0 : (max_bits & 0x7fffffu) < 0x7fe000u ? 15 - ex : 14 - ex;
+  return max_bits == 0 || (ex >= -48 && ex <= 48);
+}
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// hi and lo of four scaled elements; true if one of them is too small to be split without loss.
+__device__ __forceinline__ bool split4(const float (&x)[4], float s, uint2 &hi, uint2 &lo) {
+  __half h[4], l[4];
+  bool small = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float v = __fmul_rn(x[i], s);
+    small |= x[i] != 0.0f && fabsf(v) < 1.0f / 65536.0f;
+    h[i] = __float2half_rn(v);
+    l[i] = __float2half_rn(__fmul_rn(__fsub_rn(v, __half2float(h[i])), LO_SCALE));
+  }
+  hi = make_uint2(__half_as_ushort(h[0]) | (uint32_t)__half_as_ushort(h[1]) << 16, __half_as_ushort(h[2]) | (uint32_t)__half_as_ushort(h[3]) << 16);
+  lo = make_uint2(__half_as_ushort(l[0]) | (uint32_t)__half_as_ushort(l[1]) << 16, __half_as_ushort(l[2]) | (uint32_t)__half_as_ushort(l[3]) << 16);
+  return small;
+}
+__device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+
+// Bound by memory: reads an element once, writes two halves.  Blocks 0 .. 8 panels_a - 1 take 16 rows of A, a warp each;
+// the others 16 columns of B: four threads a row, 128 rows at a time.  A thread keeps its elements in registers between
+// the search for the largest and the split.
+template <bool VEC_A, bool VEC_B>
+__global__ void __launch_bounds__(SPLIT_THREADS, 2)
+split_kernel(const float *__restrict__ A, const float *__restrict__ B, Shape sh, Scratch w) {
+  __shared__ uint32_t s_max[SPLIT_THREADS / 32][4][4];
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int s = blockIdx.y, kc = sh.length(s);
+  const int64_t batch = blockIdx.z, at = batch * sh.stretches + s, k0 = (int64_t)(sh.first + s) * sh.kc;
+  const int kpad = (kc + 63) & ~63;
+  constexpr int STEPS = KC / 128;
+  if ((int)blockIdx.x < 8 * sh.panels_a) {
+    const int row = blockIdx.x * GROUP_ROWS + warp;
+    bool bad = false;
+    if (row < sh.M) {
+      const float *src = A + (batch * sh.M + row) * sh.K + k0;
+      float v[STEPS][4];
+      uint32_t m = 0;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k = 128 * i + 4 * lane;
+        if (VEC_A) {
+          const float4 q = k < kc ? *reinterpret_cast<const float4 *>(src + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[i][j] = k + j < kc ? src[k + j] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) m = max(m, magnitude(v[i][j]));
+      m = __reduce_max_sync(0xffffffffu, m);
+      int e;
+      bad = !scale_exponent(m, e);
+      const float sc = pow2(bad ? 0 : e);
+      __half *hi = w.a + ((2 * at) * sh.M + row) * sh.kc, *lo = hi + (int64_t)sh.M * sh.kc;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k = 128 * i + 4 * lane;
+        uint2 h, l;
+        bad |= split4(v[i], sc, h, l);
+        if (k < kpad) {
+          *reinterpret_cast<uint2 *>(hi + k) = h;
+          *reinterpret_cast<uint2 *>(lo + k) = l;
+        }
+      }
+      if (lane == 0) w.scale_a[at * sh.M + row] = pow2(bad ? 0 : -e);
+    }
+    pdl_release();
+    const int any = __syncthreads_or(bad);
+    if (tid == 0) w.flag_a[at * 8 * sh.panels_a + blockIdx.x] = any ? 1 : 0;
+  } else {
+    const int group = blockIdx.x - 8 * sh.panels_a, col = group * GROUP_COLS + 4 * (tid & 3), r0 = tid >> 2;
+    bool bad = false;
+    if (group * GROUP_COLS < sh.Np) {
+      const float *src = B + (batch * sh.K + k0) * sh.N + col;
+      float v[STEPS][4];
+      uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k = r0 + 128 * i;
+        if (VEC_B) {
+          const float4 q = k < kc && col < sh.N ? *reinterpret_cast<const float4 *>(src + (int64_t)k * sh.N) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[i][j] = k < kc && col + j < sh.N ? src[(int64_t)k * sh.N + j] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) m[j] = max(m[j], magnitude(v[i][j]));
+        m[j] = max(m[j], __shfl_xor_sync(0xffffffffu, m[j], 4));
+        m[j] = max(m[j], __shfl_xor_sync(0xffffffffu, m[j], 8));
+        m[j] = max(m[j], __shfl_xor_sync(0xffffffffu, m[j], 16));
+      }
+      if (lane < 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s_max[warp][lane][j] = m[j];
+      }
+      __syncthreads();
+      float sc[4];
+      int e[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int q = 0; q < SPLIT_THREADS / 32; ++q) m[j] = max(m[j], s_max[q][tid & 3][j]);
+        const bool no = !scale_exponent(m[j], e[j]);
+        bad |= no;
+        e[j] = no ? 0 : e[j];
+        sc[j] = pow2(e[j]);
+      }
+      if (tid < 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w.scale_b[at * sh.Np + col + j] = pow2(-e[j]);
+      }
+      __half *hi = w.b + (2 * at) * sh.kc * sh.Np + col, *lo = hi + (int64_t)sh.kc * sh.Np;
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int k = r0 + 128 * i;
+        float x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          x[j] = __fmul_rn(v[i][j], sc[j]);
+          bad |= v[i][j] != 0.0f && x[j] == 0.0f;
+        }
+        uint2 h, l;
+        bad |= split4(x, 1.0f, h, l);
+        if (k < kpad) {
+          *reinterpret_cast<uint2 *>(hi + (int64_t)k * sh.Np) = h;
+          *reinterpret_cast<uint2 *>(lo + (int64_t)k * sh.Np) = l;
+        }
+      }
+    }
+    pdl_release();
+    const int any = __syncthreads_or(bad);
+    if (tid == 0) w.flag_b[at * 8 * sh.panels_b + group] = any ? 1 : 0;
+  }
+}
+
+// ---- the product of the parts ------------------------------------------------------------------------------------
+constexpr int BK = 64;                       // k block: rows of 128 B, 128-byte swizzle
+constexpr int BOX_BYTES = 64 * BK * 2;       // one TMA box of B: 64 k-rows x 64 columns
+constexpr int THREADS = 384;                 // producer, MMA issuer, two idle warps, eight epilogue warps
+constexpr int TILE_BYTES = 32 * 32 * 4;      // an epilogue warp's staging tile
+
+// CTAS CTAs own a tile of 128 CTAS x BN: each loads its 128 rows of A and its share of B's columns, the first one issues the
+// MMAs for all.  In tensor memory: hi hi and mixed products of a tile, 2 BN columns, once or twice.
+template <int CTAS_, int BN_>
+struct Config {
+  static constexpr int CTAS = CTAS_, BN = BN_, BUFS = 256 / BN, NB = BN / CTAS;
+  static constexpr int A_BYTES = tc::BM * BK * 2, B_BYTES = NB * BK * 2;  // of hi or lo
+  static constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES), STAGES = 196608 / STAGE_BYTES;
+  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 8 * TILE_BYTES + 256;
+  // D = f32, A and B = f16, A K-major, B MN-major
+  static constexpr uint32_t IDESC = (1u << 4) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(tc::BM * CTAS >> 4) << 24);
+  static_assert(NB % 64 == 0 && 4 * BN * BUFS == 1024 && SMEM_BYTES <= 232448, "tile");
+};
+
+template <int CTAS>
+__device__ __forceinline__ uint32_t leader_addr(const void *p) {  // the same place in the shared memory of the pair's first CTA
+  uint32_t a = tc::smem_u32(p);
+  if (CTAS == 2) asm("mapa.shared::cluster.u32 %0, %0, 0;" : "+r"(a));
+  return a;
+}
+// Load into this CTA's shared memory; the bytes are counted by the barrier at `bar`, the leader's.
+template <int CTAS>
+__device__ __forceinline__ void load(void *dst, const CUtensorMap *map, uint32_t bar, int x, int y, int z) {
+  if (CTAS == 2)
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(tc::smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(tc::smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+template <int CTAS>
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+  if (CTAS == 2)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                 "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+                 "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+                 : "memory");
+}
+// Arrives at `bar` of every CTA of the pair once the MMAs issued so far have finished.
+template <int CTAS>
+__device__ __forceinline__ void commit(uint64_t *bar) {
+  if (CTAS == 2)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     tc::smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+template <int CTAS>
+__device__ __forceinline__ void arrive_leader(uint64_t *bar) {
+  if (CTAS == 2)
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr<2>(bar)) : "memory");
+  else
+    tc::mbar_arrive(bar);
+}
+template <int CTAS>
+__device__ __forceinline__ void all_ctas_barrier() {
+  if (CTAS == 2) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+}
+// K-major rows of 128 B (A): 8-row groups 1024 B apart.  MN-major (B): 64-column boxes BOX_BYTES apart, groups of 8 k-rows
+// 1024 B apart.  Both with the 128-byte swizzle (layout type 2).
+__device__ __forceinline__ uint64_t desc_a(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t desc_b(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(BOX_BYTES >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// What the kernel in front wrote is read by ordinary loads (it may still run when this one starts), at this place.
+__device__ __forceinline__ unsigned long long load_flag(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_scale(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+}
+// Waits for this thread's loads from tensor memory; r is not touched before.
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                 "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+
+// In shared memory, of 128 bytes a cycle: <2, 256> 43 written by TMA and 64 read by the tensor core, <2, 128> 64 and 96,
+// <1, 128> 85 and 128.  The first is for many tiles; its accumulators fill tensor memory, so the sums are drained to registers
+// (eight warps, 128 columns a thread) before the epilogue touches C, the mixed products first, because the next chain
+// starts with those.  The others hold two tiles and give a small product more of them.
+//
+// The tensor core truncates when it adds to its accumulator, an error that grows with the length of the chain (chain / 16
+// additions, 2^-25 of the partial sum each on average); sh.chain k blocks are added there, the rest in registers, rounded.
+template <typename C_>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, float *__restrict__ C, Shape sh,
+                  Scratch w, PanelFlags flags, int tiles, bool vec, int *__restrict__ error_flag) {
+  constexpr int CTAS = C_::CTAS, BN = C_::BN, BUFS = C_::BUFS, NB = C_::NB, A_BYTES = C_::A_BYTES, B_BYTES = C_::B_BYTES,
+                STAGE_BYTES = C_::STAGE_BYTES, STAGES = C_::STAGES, COLS = BN / 2;  // COLS: of an epilogue thread
+  constexpr uint32_t IDESC = C_::IDESC;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES + 8 * TILE_BYTES);
+  uint64_t *full = bars, *empty = bars + STAGES, *acc_full = bars + 2 * STAGES, *mixed_empty = acc_full + BUFS, *main_empty = mixed_empty + BUFS;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(main_empty + BUFS);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t rank = 0;
+  if (CTAS == 2) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int tm = (sh.M + tc::BM * CTAS - 1) / (tc::BM * CTAS), tn = (sh.N + BN - 1) / BN;
+  const int unit0 = blockIdx.x / CTAS, units = gridDim.x / CTAS;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < BUFS; ++i) {
+      tc::mbar_init(&acc_full[i], 1);
+      tc::mbar_init(&mixed_empty[i], 8 * CTAS);
+      tc::mbar_init(&main_empty[i], 8 * CTAS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    if (CTAS == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc::smem_u32(tmem_slot)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tc::smem_u32(tmem_slot)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  all_ctas_barrier<CTAS>();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+  pdl_release();  // the kernel for the marked panels needs only the flags, unless there are several stretches
+
+  // Nothing of the tile is computed here: every row panel or every column panel of it is left to the other kernel.
+  auto skipped = [&](const tc::TileCoord &t, int s) {
+    bool row_in = false, col_in = false;
+#pragma unroll
+    for (int i = 0; i < CTAS; ++i) {
+      const int pa = t.m0 / 128 + i;
+      if (pa < sh.panels_a) row_in |= load_flag(flags.row(t.batch, s) + pa) == 0;
+    }
+#pragma unroll
+    for (int i = 0; i < BN / 128; ++i) {
+      const int pb = t.n0 / 128 + i;
+      if (pb < sh.panels_b) col_in |= load_flag(flags.col(t.batch, s) + pb) == 0;
+    }
+    return !(row_in && col_in);
+  };
+  auto coord = [&](int t) { return tc::tile_coord(t, tm, tn, tc::BM * CTAS, BN); };
+  bool ok = true;
+
+  if (warp == 0) {
+    // ---------------- TMA producer ----------------
+    if (lane == 0) {
+      uint32_t g = 0;
+      for (int t = unit0; t < tiles && ok; t += units) {
+        const tc::TileCoord c = coord(t);
+        for (int s = 0; s < sh.stretches && ok; ++s) {
+          if (skipped(c, s)) continue;
+          const int z = 2 * (c.batch * sh.stretches + s), nk = (sh.length(s) + BK - 1) / BK;
+          for (int kb = 0; kb < nk; ++kb, ++g) {
+            const int st = g % STAGES;
+            ok = tc::mbar_wait(&empty[st], ((g / STAGES) & 1) ^ 1);
+            if (!ok) break;
+            if (rank == 0) tc::mbar_expect_tx(&full[st], CTAS * STAGE_BYTES);
+            const uint32_t bar = leader_addr<CTAS>(&full[st]);
+            uint8_t *p = smem + st * STAGE_BYTES;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+              load<CTAS>(p + part * A_BYTES, &map_a, bar, kb * BK, c.m0 + 128 * rank, z + part);
+#pragma unroll
+              for (int j = 0; j < NB / 64; ++j)
+                load<CTAS>(p + 2 * A_BYTES + part * B_BYTES + j * BOX_BYTES, &map_b, bar, c.n0 + NB * rank + 64 * j, kb * BK, z + part);
+            }
+          }
+        }
+      }
+      if (!ok) atomicExch(error_flag, 5);
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer: one thread of the pair ----------------
+    if (lane == 0 && rank == 0) {
+      uint32_t g = 0, it = 0;
+      for (int t = unit0; t < tiles && ok; t += units) {
+        const tc::TileCoord c = coord(t);
+        for (int s = 0; s < sh.stretches && ok; ++s) {
+          if (skipped(c, s)) continue;
+          const int nk = (sh.length(s) + BK - 1) / BK;
+          for (int kb = 0; kb < nk && ok; ++it) {  // chains
+            const int end = nk - kb < sh.chain ? nk : kb + sh.chain;
+            const uint32_t buf = it % BUFS, phase = (it / BUFS) & 1;
+            const uint32_t d_main = tmem + buf * 2 * BN, d_mixed = d_main + BN;
+            ok = tc::mbar_wait_cluster(&mixed_empty[buf], phase ^ 1);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (bool first = true; kb < end; ++kb, ++g, first = false) {
+              const int st = g % STAGES;
+              ok = tc::mbar_wait_cluster(&full[st], (g / STAGES) & 1);
+              if (!ok) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t p = tc::smem_u32(smem + st * STAGE_BYTES);
+              const uint64_t a_hi = desc_a(p), a_lo = desc_a(p + A_BYTES), b_hi = desc_b(p + 2 * A_BYTES), b_lo = desc_b(p + 2 * A_BYTES + B_BYTES);
+#pragma unroll
+              for (int ks = 0; ks < BK / 16; ++ks) {  // 32 bytes of a row of A, two groups of 8 k-rows of B
+                mma<CTAS>(d_mixed, a_hi + 2 * ks, b_lo + 128 * ks, IDESC, !first || ks > 0);
+                mma<CTAS>(d_mixed, a_lo + 2 * ks, b_hi + 128 * ks, IDESC, true);
+              }
+              if (first) {
+                ok = tc::mbar_wait_cluster(&main_empty[buf], phase ^ 1);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              }
+#pragma unroll
+              for (int ks = 0; ks < BK / 16; ++ks) mma<CTAS>(d_main, a_hi + 2 * ks, b_hi + 128 * ks, IDESC, !first || ks > 0);
+              commit<CTAS>(&empty[st]);
+            }
+            if (ok) commit<CTAS>(&acc_full[buf]);
+          }
+        }
+      }
+      if (!ok) atomicExch(error_flag, 6);
+    }
+  } else if (warp >= 4) {
+    // ---------------- epilogue ----------------
+    constexpr int DEPTH = COLS == 128 ? 4 : 8;  // requests for C in flight: what the registers beside the sums allow
+    const int q = warp & 3, half = (warp - 4) >> 2;  // lanes 32 q .. of tensor memory, columns COLS * half ..
+    float *stile = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES) + (warp - 4) * 32 * 32;
+    uint32_t it = 0;
+    for (int t = unit0; t < tiles && ok; t += units) {
+      const tc::TileCoord c = coord(t);
+      const int m0 = c.m0 + 128 * rank, row0 = m0 + 32 * q, col0 = c.n0 + COLS * half;
+      for (int s = 0; s < sh.stretches; ++s) {
+        // every load of this stretch at once: the marks, then the scales of this thread's row and columns
+        const bool row_in = m0 / 128 < sh.panels_a, col_in = col0 / 128 < sh.panels_b;
+        const int64_t at = (int64_t)c.batch * sh.stretches + s;
+        const float *scale_a = w.scale_a + at * sh.M, *scale_b = w.scale_b + at * sh.Np;
+        const unsigned long long mark_a = row_in ? load_flag(flags.row(c.batch, s) + m0 / 128) : 1;
+        const unsigned long long mark_b = col_in ? load_flag(flags.col(c.batch, s) + col0 / 128) : 1;
+        const float fa = row0 + lane < sh.M ? load_scale(scale_a + row0 + lane) : 0.0f;
+        float fb[COLS / 32];  // of the columns 32 ch + lane
+#pragma unroll
+        for (int ch = 0; ch < COLS / 32; ++ch) fb[ch] = col0 + 32 * ch + lane < sh.N ? load_scale(scale_b + col0 + 32 * ch + lane) : 0.0f;
+        if (skipped(c, s)) continue;
+        const bool mine = (mark_a | mark_b) == 0;
+        if (s == 0 && mine && row0 + lane < sh.M) {  // C into L2 while the product is computed
+          const float *p = C + ((int64_t)c.batch * sh.M + row0 + lane) * sh.N + col0;
+          const int cols = sh.N - col0 < COLS ? sh.N - col0 : COLS;
+          for (int i = 0; i < cols; i += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+          if (cols > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + cols - 1));
+        }
+        uint32_t acc[COLS / 16][16];
+        for (int kb = 0, nk = (sh.length(s) + BK - 1) / BK; kb < nk; kb += sh.chain, ++it) {
+          const uint32_t buf = it % BUFS;
+          ok = tc::mbar_wait(&acc_full[buf], (it / BUFS) & 1);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t addr = tmem + buf * 2 * BN + ((uint32_t)(32 * q) << 16) + COLS * half;
+          if (kb == 0) {
+#pragma unroll
+            for (int i = 0; i < COLS / 16; ++i) tmem_load16(addr + BN + 16 * i, acc[i]);
+#pragma unroll
+            for (int i = 0; i < COLS / 16; ++i) {
+              tmem_wait(acc[i]);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) acc[i][j] = __float_as_uint(__fmul_rn(__uint_as_float(acc[i][j]), LO_UNSCALE));
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < COLS / 16; ++i) {
+              uint32_t r[16];
+              tmem_load16(addr + BN + 16 * i, r);
+              tmem_wait(r);
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                acc[i][j] = __float_as_uint(__fmaf_rn(__uint_as_float(r[j]), LO_UNSCALE, __uint_as_float(acc[i][j])));
+            }
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive_leader<CTAS>(&mixed_empty[buf]);
+#pragma unroll
+          for (int i = 0; i < COLS / 16; ++i) {
+            uint32_t r[16];
+            tmem_load16(addr + 16 * i, r);
+            tmem_wait(r);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[i][j] = __float_as_uint(__fadd_rn(__uint_as_float(acc[i][j]), __uint_as_float(r[j])));
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive_leader<CTAS>(&main_empty[buf]);
+        }
+        if (!ok) break;
+        if (!mine) continue;
+        const int rows = sh.M - row0 < 32 ? sh.M - row0 : 32;
+        const int64_t row4 = 4 * (int64_t)sh.N;
+        // 32 columns at a time through shared memory (float4 slots rotated by the row: no bank conflicts), so that C is
+        // accessed by rows
+#pragma unroll
+        for (int ch = 0; ch < COLS / 32; ++ch) {
+          const int c0 = col0 + 32 * ch;
+          float *cp = C + ((int64_t)c.batch * sh.M + row0) * sh.N + c0;
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t *a = &acc[2 * ch + i / 4][4 * (i & 3)];
+            *reinterpret_cast<float4 *>(stile + lane * 32 + 4 * (i ^ (lane & 7))) =
+                make_float4(__fmul_rn(__uint_as_float(a[0]), fa), __fmul_rn(__uint_as_float(a[1]), fa), __fmul_rn(__uint_as_float(a[2]), fa),
+                            __fmul_rn(__uint_as_float(a[3]), fa));
+          }
+          __syncwarp();
+          if (vec) {
+            const int qc = lane & 7, col = c0 + 4 * qc;
+            const float4 f = make_float4(__shfl_sync(0xffffffffu, fb[ch], 4 * qc), __shfl_sync(0xffffffffu, fb[ch], 4 * qc + 1),
+                                         __shfl_sync(0xffffffffu, fb[ch], 4 * qc + 2), __shfl_sync(0xffffffffu, fb[ch], 4 * qc + 3));
+            if (col < sh.N) {
+              int row = lane >> 3;
+              float *p = cp + (int64_t)row * sh.N + 4 * qc;
+#pragma unroll 1
+              for (int pass = 0; pass < 8; pass += DEPTH) {
+                float4 cin[DEPTH];
+#pragma unroll
+                for (int i = 0; i < DEPTH; ++i)
+                  if (row + 4 * i < rows) cin[i] = *reinterpret_cast<const float4 *>(p + i * row4);
+#pragma unroll
+                for (int i = 0; i < DEPTH; ++i) {
+                  const float4 a = *reinterpret_cast<const float4 *>(stile + (row + 4 * i) * 32 + 4 * (qc ^ ((row + 4 * i) & 7)));
+                  if (row + 4 * i < rows)
+                    *reinterpret_cast<float4 *>(p + i * row4) =
+                        make_float4(__fadd_rn(__fmul_rn(a.x, f.x), cin[i].x), __fadd_rn(__fmul_rn(a.y, f.y), cin[i].y),
+                                    __fadd_rn(__fmul_rn(a.z, f.z), cin[i].z), __fadd_rn(__fmul_rn(a.w, f.w), cin[i].w));
+                }
+                row += 4 * DEPTH;
+                p += DEPTH * row4;
+              }
+            }
+          } else if (c0 + lane < sh.N) {
+            const float f = fb[ch];
+            float *p = cp + lane;
+#pragma unroll 1
+            for (int row = 0; row < rows; row += 2 * DEPTH) {
+              float cin[2 * DEPTH];
+#pragma unroll
+              for (int i = 0; i < 2 * DEPTH; ++i)
+                if (row + i < rows) cin[i] = p[(int64_t)i * sh.N];
+#pragma unroll
+              for (int i = 0; i < 2 * DEPTH; ++i) {
+                const float a = stile[(row + i) * 32 + 4 * ((lane >> 2) ^ (i & 7)) + (lane & 3)];  // row is a multiple of 8
+                if (row + i < rows) p[(int64_t)i * sh.N] = __fadd_rn(__fmul_rn(a, f), cin[i]);
+              }
+              p += 2 * DEPTH * (int64_t)sh.N;
+            }
+          }
+        }
+      }
+    }
+    if (!ok) atomicExch(error_flag, 7);
+  }
+
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  all_ctas_barrier<CTAS>();  // neither CTA frees or leaves what the other still uses
+  if (warp == 1) {
+    if (CTAS == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+template <typename C_>
+static int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float *C, const Shape &sh, const Scratch &w, const PanelFlags &flags,
+                       int64_t tiles, bool vec, int *error_flag, int dev, cudaStream_t st) {
+  static std::atomic<uint64_t> allowed{0};  // devices on which this kernel may use its shared memory
+  if ((allowed.load(std::memory_order_relaxed) >> dev & 1) == 0) {
+    LAPIS_CUDA_TRY(cudaFuncSetAttribute(gemm_split_kernel<C_>, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM_BYTES));
+    allowed.fetch_or(uint64_t(1) << dev, std::memory_order_relaxed);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(C_::CTAS * std::min<int64_t>(tiles, sm_count() / C_::CTAS)));
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = C_::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = C_::CTAS;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C_::CTAS == 2 ? 2 : 1;
+  LAPIS_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_split_kernel<C_>, map_a, map_b, C, sh, w, flags, (int)tiles, vec, error_flag));
+  return LAPIS_OK;
+}
+
+using Wide = Config<2, 256>;
+using Pair = Config<2, 128>;
+using Single = Config<1, 128>;
+
+}  // namespace split
+
+int bgemm_unsplit_panels(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
+                         int first, cudaStream_t st);
+
+constexpr size_t SPLIT_BYTES = size_t(160) << 20;
+
+// *done: false where the caller has to use another kernel (no memory for the split operands).
+int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, bool exact_order,
+                       bool *done, cudaStream_t st) {
+  using namespace split;
+  *done = false;
+  int dev = 0;
+  LAPIS_CUDA_TRY(cudaGetDevice(&dev));
+  int *error_flag = bgemm_error_flag(dev);
+  if (error_flag == nullptr) return LAPIS_ECUDA;
+
+  Shape sh = {};
+  sh.M = (int)M;
+  sh.N = (int)N;
+  sh.K = (int)K;
+  sh.Np = (int)((N + GROUP_COLS - 1) / GROUP_COLS * GROUP_COLS);
+  sh.panels_a = (int)((M + 127) / 128);
+  sh.panels_b = (int)((N + 127) / 128);
+  sh.chain = exact_order ? std::min(KC / BK, std::max(2, (int)(std::sqrt((double)K) / 5))) : KC / BK;
+  int64_t all = 0;  // stretches of K
+  size_t per = 0;   // bytes of a stretch: parts, scales, flags, each from a 256-byte boundary
+  size_t bytes_a = 0, bytes_b = 0;
+  for (int longest = KC; longest >= 64; longest /= 2) {
+    all = (K + longest - 1) / longest;
+    sh.kc = (int)(((K + all - 1) / all + 63) / 64 * 64);
+    all = (K + sh.kc - 1) / sh.kc;
+    bytes_a = (size_t)4 * M * sh.kc;
+    bytes_b = (size_t)4 * sh.kc * sh.Np;
+    per = bytes_a + bytes_b + 4 * (size_t)(M + sh.Np) + 8 * (size_t)(sh.panels_a + sh.panels_b);
+    if (per <= SPLIT_BYTES) break;
+  }
+  if (per > SPLIT_BYTES) return LAPIS_OK;
+  const int64_t group_s = std::min<int64_t>({all, (int64_t)(SPLIT_BYTES / per), 65535});
+  const int64_t group_b = std::min<int64_t>({batch, std::max<int64_t>(1, SPLIT_BYTES / (per * group_s)), 65535});
+  auto round = [](size_t x) { return (x + 255) & ~size_t(255); };
+  const size_t n = (size_t)(group_s * group_b);
+  const size_t off_b = round(n * bytes_a), off_sa = off_b + round(n * bytes_b), off_sb = off_sa + round(n * M * 4),
+               off_fa = off_sb + round(n * sh.Np * 4), off_fb = off_fa + round(n * 8 * sh.panels_a), total = off_fb + round(n * 8 * sh.panels_b);
+  PoolBuf buf;
+  if (buf.alloc(total, st) != LAPIS_OK) {
+    clear_error();
+    return LAPIS_OK;
+  }
+  uint8_t *p = static_cast<uint8_t *>(buf.p);
+  Scratch w = {reinterpret_cast<__half *>(p), reinterpret_cast<__half *>(p + off_b), reinterpret_cast<float *>(p + off_sa),
+               reinterpret_cast<float *>(p + off_sb), p + off_fa, p + off_fb};
+  const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, vec_b = N % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  const bool vec_c = N % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
+  auto count = [&](int64_t rows, int64_t cols) { return ((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
+  // rounds of tiles that the busiest SM works through, by what one takes
+  const int64_t sms = sm_count();
+  auto cost = [&](int64_t n, int64_t at_once, int64_t each) { return (n * group_b + at_once - 1) / at_once * each; };
+  const int64_t wide = cost(count(256, 256), sms / 2, 128), pair = cost(count(256, 128), sms / 2, 80), single = cost(count(128, 128), sms, 107);
+  for (int64_t b0 = 0; b0 < batch; b0 += group_b) {
+    const int64_t nb = std::min(group_b, batch - b0);
+    const float *Ab = A + b0 * M * K, *Bb = B + b0 * K * N;
+    float *Cb = C + b0 * M * N;
+    for (int64_t s0 = 0; s0 < all; s0 += group_s) {
+      sh.first = (int)s0;
+      sh.stretches = (int)std::min(group_s, all - s0);
+      const dim3 grid((unsigned)(8 * (sh.panels_a + sh.panels_b)), (unsigned)sh.stretches, (unsigned)nb);
+      auto kernel = vec_a ? (vec_b ? split_kernel<true, true> : split_kernel<true, false>)
+                          : (vec_b ? split_kernel<false, true> : split_kernel<false, false>);
+      LAPIS_CUDA_TRY(launch_pdl(kernel, grid, SPLIT_THREADS, 0, st, Ab, Bb, sh, w));
+      CUtensorMap map_a, map_b;
+      const int64_t parts = 2 * nb * sh.stretches;
+      LAPIS_TRY(tc::make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.a, parts, M, sh.kc, 2 * (int64_t)sh.kc, tc::BM, BK, CU_TENSOR_MAP_SWIZZLE_128B));
+      LAPIS_TRY(tc::make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.b, parts, sh.kc, sh.Np, 2 * (int64_t)sh.Np, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+      const PanelFlags flags = {reinterpret_cast<const unsigned long long *>(w.flag_a), reinterpret_cast<const unsigned long long *>(w.flag_b),
+                                sh.panels_a, sh.panels_b, sh.stretches, sh.kc};
+      if (wide < pair && wide < single)
+        LAPIS_TRY(launch_gemm<Wide>(map_a, map_b, Cb, sh, w, flags, nb * count(256, 256), vec_c, error_flag, dev, st));
+      else if (pair < single)
+        LAPIS_TRY(launch_gemm<Pair>(map_a, map_b, Cb, sh, w, flags, nb * count(256, 128), vec_c, error_flag, dev, st));
+      else
+        LAPIS_TRY(launch_gemm<Single>(map_a, map_b, Cb, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st));
+      LAPIS_TRY(bgemm_unsplit_panels(nb, M, N, K, Ab, Bb, Cb, flags, (int)s0, st));
+    }
+  }
+  *done = true;
+  return LAPIS_OK;
+}
+
+}  // namespace lapis_b200

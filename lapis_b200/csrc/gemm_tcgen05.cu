@@ -30,19 +30,15 @@
 // Every mbarrier wait is bounded: after WAIT_LIMIT polls the thread records an error code
 // in a global flag and stops waiting, the block still frees its tensor memory and exits,
 // and the host turns the flag into LAPIS_ECUDA.
-#include <cuda.h>
-
 #include <cstdlib>
 
-#include "common.h"
+#include "tcgen05.h"
 
 namespace lapis_b200 {
 
 namespace tc {
 
-constexpr int BM = 128;
 constexpr int THREADS = 320;  // producer, MMA issuer, 4 split warps, 4 epilogue warps
-constexpr uint32_t WAIT_LIMIT = 1u << 22;
 // k extent accumulated in tensor memory before the epilogue adds it to C.  Measured on 8192^3 with entries in
 // [-1, 1): max error / max |C| = 6.3e-5 unsegmented, 1.5e-5 / 8.2e-6 / 4.4e-6 / 2.3e-6 with segments of
 // 2048 / 1024 / 512 / 256 (it grows linearly with the segment: the tensor core truncates when it adds to the
@@ -75,41 +71,6 @@ struct Cfg {
   static_assert(BK == 32 || BK == 16, "A tile rows must be 128 or 64 bytes");
   static_assert(TMEM_COLS <= 512 && SMEM_BYTES <= 232448, "tile configuration does not fit");
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Bounded wait: false when the phase did not complete within WAIT_LIMIT polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
 
 // K-major operand, swizzled rows: 8-row groups `sbo` (16-byte units) apart.
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint64_t sbo, uint64_t layout) {
@@ -147,31 +108,23 @@ __device__ __forceinline__ void split_tf32(float4 &hi_lo_in_out, float4 &lo) {
   lo.w = split_lo(x.w);
 }
 
-// Tile t of the persistent schedule -> (batch, m block, n block).  Within a batch entry the tiles
-// are walked in groups of 8 m-blocks so that the blocks running at the same time share A and B
-// panels in L2.
-struct TileCoord {
-  int batch, m0, n0;
-};
-__device__ __forceinline__ TileCoord tile_coord(int t, int tm, int tn, int bn) {
-  constexpr int GROUP = 8;
-  const int per = tm * tn;
-  const int batch = t / per, r = t - batch * per;
-  const int g = r / (GROUP * tn), first_m = g * GROUP;
-  const int gsize = tm - first_m < GROUP ? tm - first_m : GROUP;
-  const int q = r - g * GROUP * tn;
-  return TileCoord{batch, (first_m + q % gsize) * BM, (q / gsize) * bn};
-}
-
 template <typename C_>
 __global__ void __launch_bounds__(THREADS, 1)
 bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     float *__restrict__ C, int M, int N, int K, int total_tiles, int kseg,
+                     float *__restrict__ C, int M, int N, int K, int total_tiles, int kseg, PanelFlags flags, int first,
                      int *__restrict__ error_flag) {
   constexpr int BN = C_::BN, BK = C_::BK, STAGES = C_::STAGES, A_BYTES = C_::A_BYTES, B_BYTES = C_::B_BYTES,
                 BOX_BYTES = C_::BOX_BYTES, STAGE_BYTES = C_::STAGE_BYTES, TMEM_COLS = C_::TMEM_COLS;
   constexpr uint32_t IDESC = C_::IDESC;
   constexpr uint64_t A_SBO = C_::A_SBO, A_LAYOUT = C_::A_LAYOUT;
+  pdl_wait();
+  if (flags.a != nullptr) {  // usually nothing is marked
+    const int na = total_tiles / ((M / BM) * (N / BN)) * flags.stretches * flags.panels_a, nb = na / flags.panels_a * flags.panels_b;
+    bool any = false;
+    for (int i = threadIdx.x; i < na; i += THREADS) any |= flags.a[i] != 0;
+    for (int i = threadIdx.x; i < nb; i += THREADS) any |= flags.b[i] != 0;
+    if (!__syncthreads_or(any)) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
@@ -186,7 +139,14 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   // its accumulator, an error that grows with the number of additions onto a large partial sum, and the
   // epilogue's adds round to nearest.  The segments of a tile are walked by the same block in order, and an
   // epilogue thread reads back exactly the elements of C it stored for the previous segment.
-  const int nseg = (nk + kseg - 1) / kseg;
+  // With flags: the segments are stretches first .. of the split operands, and only the blocks of 128 x 128 elements whose
+  // row or column panel is marked are computed.
+  const int nseg = flags.a != nullptr ? flags.stretches : (nk + kseg - 1) / kseg;
+  auto coord = [&](int t) { return tile_coord(t, tm, tn, BM, BN); };
+  auto marked = [&](const TileCoord &tc, int sg, int n0) {
+    return flags.a == nullptr || (flags.row(tc.batch, sg)[tc.m0 / 128] | flags.col(tc.batch, sg)[n0 / 128]) != 0;
+  };
+  auto left_out = [&](const TileCoord &tc, int sg) { return !marked(tc, sg, tc.n0) && (BN == 128 || !marked(tc, sg, tc.n0 + 128)); };
 
   auto stage_a = [&](int s) { return smem + s * STAGE_BYTES; };
   auto stage_alo = [&](int s) { return smem + s * STAGE_BYTES + A_BYTES; };
@@ -221,17 +181,21 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     if (lane == 0) {
       uint32_t g = 0;  // k blocks issued so far by this CTA
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        const TileCoord tc = tile_coord(t, tm, tn, BN);
+        const TileCoord tc = coord(t);
         bool ok = true;
-        for (int kb = 0; kb < nk; ++kb, ++g) {  // the segments of a tile are consecutive k blocks
-          const int s = g % STAGES;
-          ok = mbar_wait(&empty[s], ((g / STAGES) & 1) ^ 1);
-          if (!ok) break;
-          mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
-          tma_load_3d(stage_a(s), &map_a, &full[s], kb * BK, tc.m0, tc.batch);
+        for (int sg = 0; sg < nseg && ok; ++sg) {
+          if (left_out(tc, sg)) continue;
+          const int kb0 = (first + sg) * kseg, kb1 = kb0 + kseg < nk ? kb0 + kseg : nk;
+          for (int kb = kb0; kb < kb1; ++kb, ++g) {
+            const int s = g % STAGES;
+            ok = mbar_wait(&empty[s], ((g / STAGES) & 1) ^ 1);
+            if (!ok) break;
+            mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
+            tma_load_3d(stage_a(s), &map_a, &full[s], kb * BK, tc.m0, tc.batch);
 #pragma unroll
-          for (int j = 0; j < BN / 32; ++j)
-            tma_load_3d(stage_b(s) + j * BOX_BYTES, &map_b, &full[s], tc.n0 + 32 * j, kb * BK, tc.batch);
+            for (int j = 0; j < BN / 32; ++j)
+              tma_load_3d(stage_b(s) + j * BOX_BYTES, &map_b, &full[s], tc.n0 + 32 * j, kb * BK, tc.batch);
+          }
         }
         if (!ok) {
           atomicExch(error_flag, 1);
@@ -245,13 +209,14 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       uint32_t g = 0, it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        for (int sg = 0; sg < nseg && ok; ++sg, ++it) {
+        for (int sg = 0; sg < nseg && ok; ++sg) {
+          if (left_out(coord(t), sg)) continue;
           const uint32_t buf = it & 1;
           ok = mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1);  // the epilogue has drained this accumulator
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t d_tmem = tmem_base + buf * BN;
-          const int kb0 = sg * kseg, kb1 = kb0 + kseg < nk ? kb0 + kseg : nk;
+          const int kb0 = (first + sg) * kseg, kb1 = kb0 + kseg < nk ? kb0 + kseg : nk;
           for (int kb = kb0; kb < kb1; ++kb, ++g) {
             const int s = g % STAGES;
             // hi*hi needs only what TMA wrote: issue it as soon as the stage has landed, while the split
@@ -284,6 +249,7 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            smem_u32(&acc_full[buf]))
                        : "memory");
+          ++it;
         }
       }
       if (!ok) atomicExch(error_flag, 2);
@@ -294,7 +260,10 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint32_t g = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-      for (int kb = 0; kb < nk; ++kb, ++g) {
+      for (int sg = 0; sg < nseg && ok; ++sg) {
+        if (left_out(coord(t), sg)) continue;
+        const int kb0 = (first + sg) * kseg, kb1 = kb0 + kseg < nk ? kb0 + kseg : nk;
+        for (int kb = kb0; kb < kb1; ++kb, ++g) {
         const int s = g % STAGES;
         ok = mbar_wait(&full[s], (g / STAGES) & 1);
         if (!ok) break;
@@ -316,6 +285,7 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> tensor-core reads
         mbar_arrive(&conv[s]);
+        }
       }
     }
     if (!ok) atomicExch(error_flag, 3);
@@ -327,17 +297,17 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     constexpr int NC = BN / 32;  // 32-column chunks of a tile
     static_assert(NC % 2 == 0 && NC >= 2, "the epilogue walks the chunks in pairs");
     auto warp_rows = [&](int t) {  // this warp's 32 rows of tile t in C
-      const TileCoord tc = tile_coord(t, tm, tn, BN);
+      const TileCoord tc = coord(t);
       return C + ((size_t)tc.batch * M + tc.m0 + 32 * q) * (size_t)N + tc.n0;
     };
     // C_in chunk (32 rows x 32 columns), coalesced: 8 lanes cover the 128 bytes of one row.  Two chunks are
     // requested together, so that the latency of these loads is paid once per pair.
-    auto load_cin = [&](float4(&cin)[8], const float *cwarp, int c) {
+    auto load_cin = [&](float4(&cin)[8], const float *cwarp, int c, bool store) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        cin[i] = *reinterpret_cast<const float4 *>(cwarp + (size_t)(4 * i + (lane >> 3)) * N + 32 * c + 4 * (lane & 7));
+        if (store) cin[i] = *reinterpret_cast<const float4 *>(cwarp + (size_t)(4 * i + (lane >> 3)) * N + 32 * c + 4 * (lane & 7));
     };
-    auto drain = [&](const float4(&cin)[8], float *cwarp, int c, uint32_t buf, bool last) {
+    auto drain = [&](const float4(&cin)[8], float *cwarp, int c, uint32_t buf, bool last, bool store) {
       // thread = row in tensor memory; transpose through shared memory so that stores are coalesced.  The 32
       // columns come in two halves of 16 (the registers of a half are free before the next is read).
       const uint32_t taddr = tmem_base + buf * BN + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * c);
@@ -363,6 +333,7 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                           __uint_as_float(r[4 * i + 3]));
       }
       __syncwarp();
+      if (!store) return;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int row = 4 * i + (lane >> 3);
@@ -377,32 +348,38 @@ bgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     };
     uint32_t it = 0;
     bool ok = true;
-    for (int u = 0, t = blockIdx.x; t < total_tiles && ok; ++it) {
+    for (int u = 0, t = blockIdx.x; t < total_tiles && ok;) {
       // unit of work: one K segment of one tile; u counts the segments of tile t
       float *cwarp = warp_rows(t);
+      const TileCoord tc = coord(t);
+      const int sg = u;
       if (++u == nseg) {
         u = 0;
         t += gridDim.x;
       }
+      if (left_out(tc, sg)) continue;
+      const bool store0 = marked(tc, sg, tc.n0), store1 = BN == 128 ? store0 : marked(tc, sg, tc.n0 + 128);
       const uint32_t buf = it & 1;
-      ok = mbar_wait(&acc_full[buf], (it >> 1) & 1);
+      const uint32_t parity = (it++ >> 1) & 1;
+      ok = mbar_wait(&acc_full[buf], parity);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (BN == 128) {
 #pragma unroll 1
         for (int c = 0; c < NC; c += 2) {
           float4 cin_a[8], cin_b[8];
-          load_cin(cin_a, cwarp, c);
-          load_cin(cin_b, cwarp, c + 1);
-          drain(cin_a, cwarp, c, buf, false);
-          drain(cin_b, cwarp, c + 1, buf, c + 2 == NC);
+          load_cin(cin_a, cwarp, c, store0);
+          load_cin(cin_b, cwarp, c + 1, store0);
+          drain(cin_a, cwarp, c, buf, false, store0);
+          drain(cin_b, cwarp, c + 1, buf, c + 2 == NC, store0);
         }
       } else {
 #pragma unroll 1
         for (int c = 0; c < NC; ++c) {
           float4 cin_a[8];
-          load_cin(cin_a, cwarp, c);
-          drain(cin_a, cwarp, c, buf, c + 1 == NC);
+          const bool store = c < NC / 2 ? store0 : store1;
+          load_cin(cin_a, cwarp, c, store);
+          drain(cin_a, cwarp, c, buf, c + 1 == NC, store);
         }
       }
     }
@@ -436,18 +413,16 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Row-major [batch][rows][cols] fp32 tensor, box = box_rows x box_cols, swizzled.
-static int make_map(CUtensorMap *map, const float *base, int64_t batch, int64_t rows, int64_t cols, int box_rows,
-                    int box_cols, CUtensorMapSwizzle swizzle) {
+int make_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64_t batch, int64_t rows, int64_t cols,
+             int64_t row_bytes, int box_rows, int box_cols, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return fail(LAPIS_ECUDA, "bgemm: cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
-  cuuint64_t strides[2] = {(cuuint64_t)cols * 4, (cuuint64_t)cols * rows * 4};
+  cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)row_bytes * rows};
   cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, type, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(LAPIS_ECUDA, "bgemm: cuTensorMapEncodeTiled failed with code %d", (int)r);
   return LAPIS_OK;
 }
@@ -455,15 +430,32 @@ static int make_map(CUtensorMap *map, const float *base, int64_t batch, int64_t 
 }  // namespace tc
 
 static int *error_flag[64] = {nullptr};
+int *bgemm_error_flag(int dev) {
+  if (dev < 0 || dev >= 64) {
+    fail(LAPIS_EBADARG, "bgemm: device index %d not supported", dev);
+    return nullptr;
+  }
+  if (error_flag[dev] == nullptr) {
+    int *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(p, 0, sizeof(int));
+    if (e != cudaSuccess) {
+      fail(LAPIS_ECUDA, "bgemm: %s", cudaGetErrorString(e));
+      return nullptr;
+    }
+    error_flag[dev] = p;
+  }
+  return error_flag[dev];
+}
 
 template <typename C_>
 static int launch_cfg(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C,
-                      int dev, cudaStream_t st) {
+                      const PanelFlags &flags, int first, int dev, cudaStream_t st) {
   static bool attr_set[64] = {false};
   CUtensorMap map_a, map_b;
-  LAPIS_TRY(tc::make_map(&map_a, A, batch, M, K, tc::BM, C_::BK,
+  LAPIS_TRY(tc::make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, A, batch, M, K, 4 * K, tc::BM, C_::BK,
                          C_::BK == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B));
-  LAPIS_TRY(tc::make_map(&map_b, B, batch, K, N, C_::BK, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B));
+  LAPIS_TRY(tc::make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, B, batch, K, N, 4 * N, C_::BK, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B));
   if (!attr_set[dev]) {
     LAPIS_CUDA_TRY(cudaFuncSetAttribute(tc::bgemm_tcgen05_kernel<C_>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         C_::SMEM_BYTES));
@@ -471,10 +463,9 @@ static int launch_cfg(int64_t batch, int64_t M, int64_t N, int64_t K, const floa
   }
   const int64_t total = batch * (M / tc::BM) * (N / C_::BN);
   const int64_t grid = total < sm_count() ? total : sm_count();  // persistent: one block per SM
-  const int kseg = tc::K_SEGMENT / C_::BK;
-  tc::bgemm_tcgen05_kernel<C_><<<(unsigned)grid, tc::THREADS, C_::SMEM_BYTES, st>>>(map_a, map_b, C, (int)M, (int)N,
-                                                                                  (int)K, (int)total, kseg, error_flag[dev]);
-  LAPIS_CUDA_TRY(cudaGetLastError());
+  const int kseg = (flags.a != nullptr ? flags.kc : tc::K_SEGMENT) / C_::BK;
+  LAPIS_CUDA_TRY(launch_pdl(tc::bgemm_tcgen05_kernel<C_>, (unsigned)grid, tc::THREADS, C_::SMEM_BYTES, st, map_a, map_b, C, (int)M,
+                            (int)N, (int)K, (int)total, kseg, flags, first, error_flag[dev]));
   return LAPIS_OK;
 }
 
@@ -488,16 +479,12 @@ int bgemm_tcgen05_supported(int64_t batch, int64_t M, int64_t N, int64_t K) {
 }
 
 int bgemm_tcgen05_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C,
-                         cudaStream_t st) {
+                         const PanelFlags &flags, int first, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) % 16)
     return fail(LAPIS_EBADARG, "bgemm: operands must be 16-byte aligned");
   int dev = 0;
   LAPIS_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return fail(LAPIS_EBADARG, "bgemm: device index %d not supported", dev);
-  if (error_flag[dev] == nullptr) {
-    LAPIS_CUDA_TRY(cudaMalloc(&error_flag[dev], sizeof(int)));
-    LAPIS_CUDA_TRY(cudaMemset(error_flag[dev], 0, sizeof(int)));
-  }
+  if (bgemm_error_flag(dev) == nullptr) return LAPIS_ECUDA;
   // 128 x 256 tiles when N allows and there are enough of them to fill the SMs; LAPIS_B200_GEMM_TILE=128 forces
   // the 128 x 128 configuration.
   static const int forced = [] {
@@ -506,8 +493,8 @@ int bgemm_tcgen05_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const f
   }();
   const bool wide = forced != 128 && N % CfgWide::BN == 0 && K >= 8 * CfgWide::BK &&
                     batch * (M / tc::BM) * (N / CfgWide::BN) >= sm_count();
-  if (wide) return launch_cfg<CfgWide>(batch, M, N, K, A, B, C, dev, st);
-  return launch_cfg<CfgSmall>(batch, M, N, K, A, B, C, dev, st);
+  if (wide) return launch_cfg<CfgWide>(batch, M, N, K, A, B, C, flags, first, dev, st);
+  return launch_cfg<CfgSmall>(batch, M, N, K, A, B, C, flags, first, dev, st);
 }
 
 }  // namespace lapis_b200
