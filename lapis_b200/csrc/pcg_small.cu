@@ -4,15 +4,16 @@
 // last-block tail in each, and by the tuner that picks the SpMV kernel first.  Here every thread keeps its rows of x, r and
 // dinv in registers, p lives in the shared memory of the CTAs, a slice each, and the SpMV gathers it from there; the
 // partial sums of a dot product are stored into every CTA's shared memory by the warps that made them and added in one
-// fixed order by the first warp of every CTA after the cluster's barrier, so that all CTAs derive the same alpha, beta and
-// stop test (one warp, not all: the divisions of 32 warps take longer than the barrier they save).  Three barriers of the
-// cluster an iteration, no global memory but the matrix, which the L1 caches of the SMs in use hold up to about 200 KB each
-// and L2 beyond (1000 rows of 29, 64-bit indices, 460 KB on one SM: 17 us an iteration, 12.5 with 32-bit ones).
+// fixed order by every warp after the cluster's barrier, so that all derive the same alpha, beta and stop test.  Three
+// barriers of the cluster an iteration, no global memory but the matrix, which the L1 caches of the SMs in use hold up to
+// about 200 KB each and L2 beyond.
 //
-// Bound by the barriers (5-point stencils: 3.0 us an iteration at 1024 rows, 6.2 at 16,384; the passes of pcg.cu take 17 to
-// 19) and, with scattered columns, by the gathers from the other CTAs' memory: 8000 rows of 11, 70,000 such
-// gathers, 20.9 us, passes 21.5; 8000 of 15, 98,000 gathers, 29.2 and 22.5, where a band of the same size takes 8.1.  The
-// solve therefore counts them first where there may be too many, and leaves the system to the passes.
+// Bound by the chains of dependent additions and shuffles between the barriers.  5-point stencils, us an iteration, with
+// 512 to 1024 threads a CTA and the totals left to one warp, and now: 1024 rows 2.9 and 2.1, 4096 rows 3.5 and 3.3, 6400
+// rows 4.7 and 3.7, 16,384 rows 6.1 and 5.4 (the passes of pcg.cu 18); 2000 scattered rows of 10, 9.3 and 8.7.  With
+// scattered columns by the gathers from the other CTAs' memory: 8000 rows of 11, 70,000 such gathers, 23.3 us,
+// passes 20 to 21.5.  The solve therefore counts them first where there may be too many, and leaves the system to the
+// passes.
 //
 // The recurrences are those of pcg.cu (examples/pcg_solve.py:65-98 in the LAPIS project), element by element; a row of A p
 // is added in entry order.  Results are identical from run to run; against the other passes they differ by the order of the
@@ -24,7 +25,7 @@
 
 namespace lapis_b200 {
 
-constexpr int SMALL_FAR = 75000;  // gathers from other CTAs' memory in an iteration, beyond which the passes are faster
+constexpr int SMALL_FAR = 60000;  // gathers from other CTAs' memory in an iteration, beyond which the passes are faster
 constexpr int SMALL_LEFT = 2;     // FL_DONE of a system that was left to the passes
 constexpr int SMALL_BUDGET = 4096;  // iterations per launch (a few milliseconds): the host looks at the outcome in between
 
@@ -64,20 +65,21 @@ __device__ __forceinline__ double warp_total(double v) {
   return v;
 }
 
-// CTAS x THREADS threads, R rows each.
+// CTAS x THREADS threads, R rows each.  Eight warps a CTA: with 32 the shuffles of the partial sums took longer than the work
+// between them, and a total had to be formed by one warp and handed out behind another barrier, where eight can each form it
+// (the same additions, so the same bits) together with alpha, beta and the stop test.
 template <typename I, int CTAS, int THREADS, int R>
 __global__ void __launch_bounds__(THREADS)
 pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, SmallSolve s) {
   constexpr int SLICE = THREADS * R, WARPS = THREADS / 32, PARTS = CTAS * WARPS;
-  static_assert(PARTS % 32 == 0, "a warp adds whole rounds of parts");
+  constexpr int STEP = R >= 4 ? 2 : 4;  // entries of each row requested together
+  static_assert(PARTS % 32 == 0 || 32 % PARTS == 0, "a warp adds whole rounds of parts, or has each of them in several lanes");
   __shared__ double s_p[SLICE];
   __shared__ double s_part[3][PARTS];
-  __shared__ double s_alpha, s_beta;
-  __shared__ int s_done;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = CTAS == 1 ? 0 : small_rank();
 
-  // this warp's part of a sum goes to every CTA; total() adds the parts after the barrier
+  // this warp's part of a sum goes to every CTA; total() adds the parts after the barrier, in every warp alike
   auto send = [&](int which, double v) {
     const double t = warp_total(v);
     double *slot = &s_part[which][rank * WARPS + warp];
@@ -89,9 +91,15 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   };
   auto total = [&](int which) {
     double t = 0.0;
+    if (PARTS >= 32) {
 #pragma unroll
-    for (int q = 0; q < PARTS / 32; ++q) t = __dadd_rn(t, s_part[which][lane + 32 * q]);
-    return warp_total(t);
+      for (int q = 0; q < PARTS / 32; ++q) t = __dadd_rn(t, s_part[which][lane + 32 * q]);
+    } else {
+      t = s_part[which][lane % PARTS];
+    }
+#pragma unroll
+    for (int off = (PARTS < 32 ? PARTS : 32) / 2; off > 0; off >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+    return t;
   };
   auto gather = [&](I col) {
     const uint32_t c = min((uint32_t)col, (uint32_t)s.n - 1);  // a bad index stays inside the cluster's memory
@@ -101,15 +109,19 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     return v;
   };
 
-  int64_t lo[R];
-  int len[R];
+  const I *c[R];
+  const double *v[R];
+  int len[R], longest = 0;
   double x[R], r[R], z[R], d[R];
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int row = (int)rank * SLICE + tid + i * THREADS;
     const bool in = row < s.n;
-    lo[i] = in ? (int64_t)pos[row] : 0;
-    len[i] = in ? (int)((int64_t)pos[row + 1] - lo[i]) : 0;
+    const int64_t lo = in ? (int64_t)pos[row] : 0;
+    c[i] = crd + lo;
+    v[i] = val + lo;
+    len[i] = in ? (int)((int64_t)pos[row + 1] - lo) : 0;
+    longest = max(longest, len[i]);
     d[i] = in ? s.dinv[row] : 0.0;
     r[i] = in ? (s.first ? s.b[row] : s.r[row]) : 0.0;
     x[i] = in && !s.first ? s.x[row] : 0.0;
@@ -120,18 +132,16 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     int far = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i)
-      for (int j = 0; j < len[i]; ++j) far += (uint32_t)__ldg(crd + lo[i] + j) / SLICE != rank;
+      for (int j = 0; j < len[i]; ++j) far += (uint32_t)__ldg(c[i] + j) / SLICE != rank;
     small_barrier<CTAS>();  // every CTA of the cluster runs before its shared memory is written
     send(0, (double)far);
     small_barrier<CTAS>();
-    if (warp == 0) s_done = total(0) > SMALL_FAR ? 1 : 0;
-    __syncthreads();
-    if (s_done != 0) {  // in all CTAs alike; nothing of theirs is read or written any more
+    if (total(0) > SMALL_FAR) {  // in all CTAs alike; nothing of theirs is read or written any more
       if (rank == 0 && tid == 0) s.fl[FL_DONE] = SMALL_LEFT;
       return;
     }
   }
-  double initres = 0.0, rz = 0.0, relres = 0.0;  // of warp 0, as the sums are
+  double initres = 0.0, rz = 0.0, relres = 0.0;
   unsigned long long iters = 0;
   bool done = false;
   if (s.first) {
@@ -145,10 +155,8 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     send(1, rr);
     send(2, rzp);
     small_barrier<CTAS>();
-    if (warp == 0) {
-      initres = sqrt(total(1));
-      rz = total(2);
-    }
+    initres = sqrt(total(1));
+    rz = total(2);
   } else {
     initres = s.sc[SC_INITRES];
     rz = s.sc[SC_RZ];
@@ -159,30 +167,29 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
   for (int left = SMALL_BUDGET; left > 0 && !done; --left) {
     double ap[R], pap = 0.0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const I *c = crd + lo[i];
-      const double *v = val + lo[i];
-      double sum = 0.0;
-      for (int j = 0; j < len[i]; j += 4) {
-        double a[4], g[4];
+    for (int i = 0; i < R; ++i) ap[i] = 0.0;
+    for (int j = 0; j < longest; j += STEP) {  // the rows side by side, each in entry order
+      double a[R][STEP], g[R][STEP];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) {
           const bool in = j + u < len[i];
-          a[u] = in ? __ldg(v + j + u) : 0.0;
-          g[u] = in ? gather(__ldg(c + j + u)) : 0.0;
+          a[i][u] = in ? __ldg(v[i] + j + u) : 0.0;
+          g[i][u] = in ? gather(__ldg(c[i] + j + u)) : 0.0;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (j + u < len[i]) sum = __dadd_rn(sum, __dmul_rn(a[u], g[u]));
-      }
-      ap[i] = sum;
-      if ((int)rank * SLICE + tid + i * THREADS < s.n) pap = __dadd_rn(pap, __dmul_rn(sum, s_p[tid + i * THREADS]));
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int u = 0; u < STEP; ++u)
+          if (j + u < len[i]) ap[i] = __dadd_rn(ap[i], __dmul_rn(a[i][u], g[i][u]));
     }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if ((int)rank * SLICE + tid + i * THREADS < s.n) pap = __dadd_rn(pap, __dmul_rn(ap[i], s_p[tid + i * THREADS]));
     send(0, pap);
     small_barrier<CTAS>();
-    if (warp == 0) s_alpha = rz / total(0);
-    __syncthreads();
-    const double alpha = s_alpha, malpha = -alpha;
+    const double alpha = rz / total(0), malpha = -alpha;
     double rr = 0.0, rzp = 0.0;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -198,20 +205,12 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     send(2, rzp);
     small_barrier<CTAS>();
     ++iters;
-    if (warp == 0) {
-      relres = sqrt(total(1)) / initres;
-      const double rznew = total(2);
-      const bool stop = !(relres > s.tol && iters != s.maxiter);  // ordered compare: NaN stops the loop
-      if (!stop) {
-        s_beta = rznew / rz;
-        rz = rznew;
-      }
-      s_done = stop ? 1 : 0;
-    }
-    __syncthreads();
-    done = s_done != 0;
+    const double rznew = total(2);
+    const double beta = rznew / rz;
+    relres = sqrt(total(1)) / initres;
+    done = !(relres > s.tol && iters != s.maxiter);  // ordered compare: NaN stops the loop
     if (!done) {
-      const double beta = s_beta;
+      rz = rznew;
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         double *p = s_p + tid + i * THREADS;
@@ -220,6 +219,7 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
       small_barrier<CTAS>();
     }
   }
+  if (CTAS > 1) small_barrier<CTAS>();  // no CTA leaves while its parts may still be read or written
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int row = (int)rank * SLICE + tid + i * THREADS;
@@ -258,10 +258,10 @@ static cudaError_t launch_small(const lapis_b200_csr *h, const SmallSolve &s, cu
 
 template <typename I>
 static cudaError_t launch_small_size(const lapis_b200_csr *h, const SmallSolve &s, cudaStream_t st) {
-  if (s.n <= 1024) return launch_small<I, 1, 1024, 1>(h, s, st);
-  if (s.n <= 4096) return launch_small<I, 8, 512, 1>(h, s, st);
-  if (s.n <= 8192) return launch_small<I, 8, 512, 2>(h, s, st);
-  return launch_small<I, 8, 1024, 2>(h, s, st);
+  if (s.n <= 1024) return launch_small<I, 1, 256, 4>(h, s, st);
+  if (s.n <= 4096) return launch_small<I, 8, 256, 2>(h, s, st);
+  if (s.n <= 8192) return launch_small<I, 8, 256, 4>(h, s, st);
+  return launch_small<I, 8, 512, 4>(h, s, st);  // 256 x 8: 6.9 us an iteration where this takes 5.3
 }
 
 // Only for handles on which spmv_fits_small_pcg() is true (at most 16384 rows).  *solved: false where the system is left
