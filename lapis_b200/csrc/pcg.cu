@@ -22,6 +22,7 @@
 //
 // Arithmetic follows the emitted element-wise bodies: axpby is (x*a) + (y*b) with
 // separate roundings (examples/pcg_solve.py:30-39), mult is x*y (:41-48).
+#include <algorithm>
 #include <cmath>
 
 #include "common.h"
@@ -874,11 +875,11 @@ extern "C" int lapis_b200_pcg_p2p_halo_wait(void *d_work, void *d_mbox, const vo
 // ---------------------------------------------------------------------------------------------
 // Hitting-time moments (examples/hitting_times.py:151-194 in the LAPIS project): two Jacobi-PCG solves
 // with the masked graph Laplacian y = M (D - alpha A) M x as the operator (@plpt, :73-92) and z = r / d
-// as the preconditioner (:113, :140).  Same three passes per iteration as the plain solver:
-//   A  t = (alpha A) mp with the fused partial sums of mp.t        (mp = mask * p, kept beside p)
-//   B  Ap = (d*mp - t)*mask on the fly; x, r, z updates; partial sums of r.r and r.z
-//   C  p = z + beta p; mp = mask*p; partial sums of d*mp*mp
-// so p.Ap = sum d mp^2 - mp.t needs no pass of its own.
+// as the preconditioner (:113, :140).  Two passes per iteration where the one-thread-per-row SpMV serves the matrix:
+//   A  p = z + beta p, at the own row and at every column of it; t = (alpha A)(mask p); Ap = (d mask p - t) mask;
+//      partial sums of (mask p).t and d (mask p)^2, whose difference is p.Ap; tail: alpha
+//   B  x, r, z updates; partial sums of r.r and r.z; tail: stop test, beta
+// and four launches otherwise, around the SpMV kernel that suits the matrix (t, mask p and p stored).
 // ---------------------------------------------------------------------------------------------
 namespace lapis_b200 {
 
@@ -890,19 +891,20 @@ scale_copy_kernel(int64_t n, const double *__restrict__ src, double a, double *_
 
 // r = b; z = r/d; p = z; mp = mask*p; x = 0; partial sums of r.r, r.z and d*mp*mp  (hitting_times.py:111-117)
 __global__ void __launch_bounds__(VEC_THREADS)
-mht_init_kernel(int64_t n, const double *__restrict__ b, const double *__restrict__ d, const double *__restrict__ mask,
-                double *__restrict__ r, double *__restrict__ z, double *__restrict__ p, double *__restrict__ mp,
-                double *__restrict__ x, double *__restrict__ partials) {
+mht_init_kernel(int64_t n, const double *b, const double *__restrict__ d, const double *__restrict__ mask, double *r,
+                double *__restrict__ z, double *__restrict__ p, double *__restrict__ mp,
+                double *__restrict__ x, double *__restrict__ partials, double *sc, long long *fl) {
   __shared__ double s_red[VEC_THREADS / 32];
+  __shared__ int s_flag;
   double rr = 0.0, rz = 0.0, dm = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * VEC_THREADS) {
     const double ri = b[i], di = d[i];
     const double zi = __ddiv_rn(ri, di);
     const double mpi = __dmul_rn(zi, mask[i]);
-    r[i] = ri;
+    if (r != b) r[i] = ri;
     z[i] = zi;
     p[i] = zi;
-    mp[i] = mpi;
+    if (mp != nullptr) mp[i] = mpi;
     x[i] = 0.0;
     rr = __dadd_rn(rr, __dmul_rn(ri, ri));
     rz = __dadd_rn(rz, __dmul_rn(ri, zi));
@@ -916,15 +918,208 @@ mht_init_kernel(int64_t n, const double *__restrict__ b, const double *__restric
     partials[gridDim.x + blockIdx.x] = t1;
     partials[2 * gridDim.x + blockIdx.x] = t2;
   }
+  if (!pcg_last_block(pcg_tickets(sc) + 0, gridDim.x, &s_flag)) return;
+  const double srr = pcg_block_total(partials, gridDim.x, s_red);
+  const double srz = pcg_block_total(partials + gridDim.x, gridDim.x, s_red);
+  const double sdm = pcg_block_total(partials + 2 * gridDim.x, gridDim.x, s_red);
+  if (threadIdx.x == 0) {
+    sc[SC_RR] = srr;
+    sc[SC_RZNEW] = srz;
+    sc[SC_DMP2] = sdm;
+    pcg_derive(DERIVE_INIT, sc, fl, 0.0, 0);
+  }
 }
 
+// The tail of a pass that updates the residual, in the block that finishes last: sums in a fixed order, stop test, beta.
+__device__ __forceinline__ void mht_tail_update(double rr, double rz, double *partials, double *sc, long long *fl, double tol,
+                                                unsigned long long maxiter, double *s_red, int *s_flag) {
+  const double t0 = block_sum_vec(rr, s_red);
+  const double t1 = block_sum_vec(rz, s_red);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = t0;
+    partials[gridDim.x + blockIdx.x] = t1;
+  }
+  if (!pcg_last_block(pcg_tickets(sc) + 1, gridDim.x, s_flag)) return;
+  const double srr = pcg_block_total(partials, gridDim.x, s_red);
+  const double srz = pcg_block_total(partials + gridDim.x, gridDim.x, s_red);
+  if (threadIdx.x == 0) {
+    sc[SC_RR] = srr;
+    sc[SC_RZNEW] = srz;
+    pcg_derive(DERIVE_DECIDE, sc, fl, tol, maxiter);
+  }
+}
+
+// ---- two passes an iteration -----------------------------------------------------------------------------------
+// Sum of the entries [lo, hi) of a row times mask * (z + beta p) at their columns, in entry order; DIR false: times mask * p; not
+// MASKED: times p.
+template <typename I, bool DIR, bool MASKED>
+__device__ __forceinline__ double mht_piece(const I *__restrict__ crd, const double *__restrict__ val, double alpha,
+                                            const double *__restrict__ mask, const double *__restrict__ z,
+                                            const double *__restrict__ p, double beta, int64_t lo, int64_t hi) {
+  double acc = 0.0;
+  for (int64_t j = lo; j < hi; j += 4) {
+    double a[4], m[4], zv[4], pv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = j + u < hi;
+      const int64_t c = in ? (int64_t)crd[j + u] : 0;
+      a[u] = in ? val[j + u] : 0.0;
+      m[u] = in && MASKED ? mask[c] : 0.0;
+      pv[u] = in ? p[c] : 0.0;
+      zv[u] = in && DIR ? z[c] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double pc = DIR ? __dadd_rn(__dmul_rn(zv[u], 1.0), __dmul_rn(pv[u], beta)) : pv[u];
+      if (j + u < hi) acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(a[u], alpha), MASKED ? __dmul_rn(pc, m[u]) : pc));
+    }
+  }
+  return acc;
+}
+// Row sum in the pieces and the order of spmv_rowthread_kernel (spmv.cu): rows cut at multiples of SPMV_CHUNK entries.
+constexpr int64_t SPMV_CHUNK = 2048;
+template <typename I, bool DIR, bool MASKED>
+__device__ __forceinline__ double mht_row(const I *__restrict__ crd, const double *__restrict__ val, double alpha, int64_t abase,
+                                          const double *__restrict__ mask, const double *__restrict__ z, const double *__restrict__ p,
+                                          double beta, int64_t lo, int64_t hi, double &stored) {
+  const int64_t bnd = abase + ((lo - abase) / SPMV_CHUNK + 1) * SPMV_CHUNK;
+  const double s = mht_piece<I, DIR, MASKED>(crd, val, alpha, mask, z, p, beta, lo, hi < bnd ? hi : bnd);
+  stored = __dadd_rn(s, 0.0);
+  if (hi <= bnd) return s;
+  const double last = mht_piece<I, DIR, MASKED>(crd, val, alpha, mask, z, p, beta, bnd, hi);  // rows of at most 32 entries: one boundary
+  stored = __dadd_rn(__dadd_rn(last, 0.0), s);
+  return __dadd_rn(s, last);
+}
+
+// Pass A.  Bound by memory: the matrix, d, mask, z, p once, p and Ap written; the columns of a row come from cache.
+// Before, SpMV, update and direction pass with a single-block sum behind each, over a scaled copy of the values: 2048 x
+// 2048 grid, 185 us an iteration.
+template <typename I, bool DIR>
+__device__ __forceinline__ void mht_rows(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, double alpha,
+                                         int64_t abase, int64_t n, const double *__restrict__ d, const double *__restrict__ mask,
+                                         const double *__restrict__ z, const double *__restrict__ p, double *__restrict__ pnew, double beta,
+                                         double *__restrict__ Ap, double &mpt, double &dm) {
+  const int64_t stride = (int64_t)gridDim.x * VEC_THREADS;
+  int64_t i = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x;
+  I next_lo = i < n ? pos[i] : (I)0, next_hi = i < n ? pos[i + 1] : (I)0;  // of the next row, one trip to memory less in the chain
+  for (; i < n; i += stride) {
+    const int64_t lo = (int64_t)next_lo, hi = (int64_t)next_hi;
+    if (i + stride < n) {
+      next_lo = pos[i + stride];
+      next_hi = pos[i + stride + 1];
+    }
+    const double di = d[i], mi = mask[i];
+    double pi = p[i];
+    if (DIR) {
+      pi = __dadd_rn(__dmul_rn(z[i], 1.0), __dmul_rn(pi, beta));
+      pnew[i] = pi;
+    }
+    const double mp = __dmul_rn(pi, mi);
+    double t;
+    const double s = mht_row<I, DIR, true>(crd, val, alpha, abase, mask, z, p, beta, lo, hi, t);
+    Ap[i] = __dmul_rn(__dsub_rn(__dmul_rn(di, mp), t), mi);
+    mpt = __dadd_rn(mpt, __dmul_rn(s, mp));
+    dm = __dadd_rn(dm, __dmul_rn(__dmul_rn(di, mp), mp));
+  }
+}
+template <typename I>
+__global__ void __launch_bounds__(VEC_THREADS, 4)
+mht_operator_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, double alpha, int64_t abase, int64_t n,
+                    const double *__restrict__ d, const double *__restrict__ mask, const double *__restrict__ z, double *p0, double *p1,
+                    double *__restrict__ Ap, double *__restrict__ partials, double *sc, long long *fl) {
+  __shared__ double s_red[VEC_THREADS / 32];
+  __shared__ int s_flag;
+  pdl_wait();
+  if (fl[FL_DONE] != 0) return;
+  long long *hdr = reinterpret_cast<long long *>(sc);
+  const long long stage = hdr[SC_STAGE], cur = hdr[SC_PCUR];
+  double mpt = 0.0, dm = 0.0;
+  if (stage == 0) mht_rows<I, false>(pos, crd, val, alpha, abase, n, d, mask, z, p0, p1, 0.0, Ap, mpt, dm);
+  else mht_rows<I, true>(pos, crd, val, alpha, abase, n, d, mask, z, cur != 0 ? p1 : p0, cur != 0 ? p0 : p1, sc[SC_BETA], Ap, mpt, dm);
+  pdl_release();
+  const double t0 = block_sum_vec(mpt, s_red);
+  const double t1 = block_sum_vec(dm, s_red);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = t0;
+    partials[gridDim.x + blockIdx.x] = t1;
+  }
+  if (!pcg_last_block(pcg_tickets(sc) + 0, gridDim.x, &s_flag)) return;
+  const double smpt = pcg_block_total(partials, gridDim.x, s_red);
+  const double sdm = pcg_block_total(partials + gridDim.x, gridDim.x, s_red);
+  if (threadIdx.x == 0) {
+    sc[SC_PAP] = smpt;
+    sc[SC_DMP2] = sdm;
+    if (stage == 0) hdr[SC_STAGE] = 1;
+    else hdr[SC_PCUR] = cur ^ 1;
+    pcg_derive(DERIVE_ALPHA_MASKED, sc, fl, 0.0, 0);
+  }
+}
+
+// Pass B: x += alpha p; r -= alpha Ap; z = r/d; partial sums of r.r, r.z.  Two elements a round, all loads first;
+// exactly the blocks that are resident (with four elements and 85 registers, three blocks an SM, 57 us at 2048 x 2048).
+constexpr int MHT_RESIDENT = 5;
+__global__ void __launch_bounds__(VEC_THREADS, MHT_RESIDENT)
+mht_residual_kernel(int64_t n, double *sc, long long *fl, double tol, unsigned long long maxiter, const double *p0, const double *p1,
+                    const double *__restrict__ Ap, const double *__restrict__ d, double *__restrict__ x, double *__restrict__ r,
+                    double *__restrict__ z, double *__restrict__ partials) {
+  __shared__ double s_red[VEC_THREADS / 32];
+  __shared__ int s_flag;
+  pdl_wait();
+  if (fl[FL_DONE] != 0) return;
+  const double *__restrict__ p = reinterpret_cast<const long long *>(sc)[SC_PCUR] != 0 ? p1 : p0;
+  const double alpha = sc[SC_ALPHA], malpha = -alpha;
+  double rr = 0.0, rz = 0.0;
+  const int64_t stride = (int64_t)gridDim.x * VEC_THREADS;
+  for (int64_t i0 = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x; i0 < n; i0 += 2 * stride) {
+    double xv[2], pv[2], rv[2], av[2], dv[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t i = i0 + k * stride;
+      const bool in = i < n;
+      xv[k] = in ? x[i] : 0.0;
+      pv[k] = in ? p[i] : 0.0;
+      rv[k] = in ? r[i] : 0.0;
+      av[k] = in ? Ap[i] : 0.0;
+      dv[k] = in ? d[i] : 1.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t i = i0 + k * stride;
+      if (i >= n) break;
+      const double ri = __dadd_rn(__dmul_rn(rv[k], 1.0), __dmul_rn(av[k], malpha));
+      const double zi = __ddiv_rn(ri, dv[k]);
+      x[i] = __dadd_rn(__dmul_rn(xv[k], 1.0), __dmul_rn(pv[k], alpha));
+      r[i] = ri;
+      z[i] = zi;
+      rr = __dadd_rn(rr, __dmul_rn(ri, ri));
+      rz = __dadd_rn(rz, __dmul_rn(ri, zi));
+    }
+  }
+  pdl_release();
+  mht_tail_update(rr, rz, partials, sc, fl, tol, maxiter, s_red, &s_flag);
+}
+
+// b2 = mask * (d*mom1 + (alpha A) mom1)  (hitting_times.py:163-176)
+template <typename I>
+__global__ void __launch_bounds__(VEC_THREADS)
+mht_rhs2_rows_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, double alpha, int64_t abase, int64_t n,
+                     const double *__restrict__ d, const double *__restrict__ mask, const double *__restrict__ mom1, double *__restrict__ b2) {
+  for (int64_t i = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * VEC_THREADS) {
+    double t;
+    mht_row<I, false, false>(crd, val, alpha, abase, nullptr, nullptr, mom1, 0.0, (int64_t)pos[i], (int64_t)pos[i + 1], t);
+    b2[i] = __dmul_rn(__dadd_rn(__dmul_rn(d[i], mom1[i]), t), mask[i]);
+  }
+}
+
+// ---- any SpMV kernel ---------------------------------------------------------------------------------------------
 // Ap = (d*mp - t)*mask (hitting_times.py:84-88); x += alpha p; r -= alpha Ap; z = r/d; partial sums of r.r, r.z
 __global__ void __launch_bounds__(VEC_THREADS)
-mht_update_kernel(int64_t n, const double *__restrict__ sc, const long long *__restrict__ fl,
-                  const double *__restrict__ p, const double *__restrict__ mp, const double *__restrict__ t,
-                  const double *__restrict__ d, const double *__restrict__ mask, double *__restrict__ x,
-                  double *__restrict__ r, double *__restrict__ z, double *__restrict__ partials) {
+mht_update_kernel(int64_t n, double *sc, long long *fl, double tol, unsigned long long maxiter, const double *__restrict__ p,
+                  const double *__restrict__ mp, const double *__restrict__ t, const double *__restrict__ d,
+                  const double *__restrict__ mask, double *__restrict__ x, double *__restrict__ r, double *__restrict__ z,
+                  double *__restrict__ partials) {
   __shared__ double s_red[VEC_THREADS / 32];
+  __shared__ int s_flag;
   if (fl[FL_DONE] != 0) return;
   const double alpha = sc[SC_ALPHA];
   const double malpha = -alpha;
@@ -941,20 +1136,15 @@ mht_update_kernel(int64_t n, const double *__restrict__ sc, const long long *__r
     rr = __dadd_rn(rr, __dmul_rn(ri, ri));
     rz = __dadd_rn(rz, __dmul_rn(ri, zi));
   }
-  const double t0 = block_sum_vec(rr, s_red);
-  const double t1 = block_sum_vec(rz, s_red);
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x] = t0;
-    partials[gridDim.x + blockIdx.x] = t1;
-  }
+  mht_tail_update(rr, rz, partials, sc, fl, tol, maxiter, s_red, &s_flag);
 }
 
 // p = z + beta p (hitting_times.py:143); mp = mask*p; partial sums of d*mp*mp
 __global__ void __launch_bounds__(VEC_THREADS)
-mht_direction_kernel(int64_t n, const double *__restrict__ sc, const long long *__restrict__ fl,
-                     const double *__restrict__ z, const double *__restrict__ d, const double *__restrict__ mask,
-                     double *__restrict__ p, double *__restrict__ mp, double *__restrict__ partials) {
+mht_direction_kernel(int64_t n, double *sc, const long long *__restrict__ fl, const double *__restrict__ z, const double *__restrict__ d,
+                     const double *__restrict__ mask, double *__restrict__ p, double *__restrict__ mp, double *__restrict__ partials) {
   __shared__ double s_red[VEC_THREADS / 32];
+  __shared__ int s_flag;
   if (fl[FL_DONE] != 0) return;
   const double beta = sc[SC_BETA];
   double dm = 0.0;
@@ -966,7 +1156,10 @@ mht_direction_kernel(int64_t n, const double *__restrict__ sc, const long long *
     dm = __dadd_rn(dm, __dmul_rn(__dmul_rn(d[i], mpi), mpi));
   }
   const double t0 = block_sum_vec(dm, s_red);
-  if (threadIdx.x == 0) partials[2 * gridDim.x + blockIdx.x] = t0;
+  if (threadIdx.x == 0) partials[blockIdx.x] = t0;
+  if (!pcg_last_block(pcg_tickets(sc) + 2, gridDim.x, &s_flag)) return;
+  const double sdm = pcg_block_total(partials, gridDim.x, s_red);
+  if (threadIdx.x == 0) sc[SC_DMP2] = sdm;
 }
 
 // b2 = mask * (d*mom1 + t) with t = (alpha A) mom1  (hitting_times.py:163-176)
@@ -984,46 +1177,66 @@ normalize_mom2_kernel(int64_t n, const double *__restrict__ mom1, const double *
     out[i] = sqrt(__dsub_rn(mom2[i], __dmul_rn(mom1[i], mom1[i])));
 }
 
-// One masked solve.  work: [16 header][3*G partials][r][z][p][mp][t], G = vec_grid(n).
-static int mht_solve(const lapis_b200_csr *A, const double *d_b, const double *d_d, const double *d_mask, double tol,
-                     uint64_t maxiter, double *d_x, double *work, uint64_t *iters, double *relres, cudaStream_t st) {
+// What a masked solve works on.  r holds the right-hand side at its start; p1: the second p buffer of the two-pass form, mp
+// of the other; t: Ap or t.
+struct MhtWork {
+  double *sc, *partials, *r, *z, *p, *p1, *t;
+};
+
+template <typename I>
+static int mht_operator_launch(const lapis_b200_csr *A, double alpha, const double *d_d, const double *d_mask, const MhtWork &w, cudaStream_t st) {
+  static int per_sm[64] = {0};  // resident blocks, for 4-byte or for 8-byte indices
+  const int dev = A->device >= 0 && A->device < 64 ? A->device : 0;
+  if (per_sm[dev] == 0) {
+    int m = 0;
+    LAPIS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, mht_operator_kernel<I>, VEC_THREADS, 0));
+    per_sm[dev] = m > 0 && m <= 8 ? m : 4;
+  }
+  const int64_t tiles = (A->nrows + VEC_THREADS - 1) / VEC_THREADS, resident = (int64_t)sm_count() * per_sm[dev];
+  LAPIS_CUDA_TRY(launch_pdl(mht_operator_kernel<I>, (unsigned)(tiles < resident ? tiles : resident), VEC_THREADS, 0, st,
+                            static_cast<const I *>(A->pos), static_cast<const I *>(A->crd), A->val, alpha, A->base & ~(int64_t)3, A->nrows, d_d,
+                            d_mask, w.z, w.p, w.p1, w.t, w.partials, w.sc, reinterpret_cast<long long *>(w.sc + SC_COUNT)));
+  return LAPIS_OK;
+}
+
+// One masked solve.  two_pass: A is the caller's matrix, otherwise its values have been scaled by alpha.
+static int mht_solve(const lapis_b200_csr *A, bool two_pass, double alpha, const double *d_d, const double *d_mask, double tol,
+                     uint64_t maxiter, double *d_x, const MhtWork &w, uint64_t *iters, double *relres, cudaStream_t st) {
   const int64_t n = A->nrows;
   const unsigned G = vec_grid(n);
-  double *sc = work;
-  long long *fl = reinterpret_cast<long long *>(work + SC_COUNT);
-  double *partials = work + 16;
-  double *r = partials + 3 * (int64_t)G, *z = r + n, *p = z + n, *mp = p + n, *t = mp + n;
+  double *sc = w.sc;
+  long long *fl = reinterpret_cast<long long *>(sc + SC_COUNT);
   const int *skip = reinterpret_cast<const int *>(fl);
-  LAPIS_CUDA_TRY(cudaMemsetAsync(work, 0, 16 * sizeof(double), st));
-  mht_init_kernel<<<G, VEC_THREADS, 0, st>>>(n, d_b, d_d, d_mask, r, z, p, mp, d_x, partials);
-  sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(partials + 2 * (int64_t)G, G, 1, sc + SC_DMP2, nullptr, DERIVE_NONE, sc, fl,
-                                                 0.0, 0, nullptr);
-  sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(partials, G, 2, sc + SC_RR, sc + SC_RZNEW, DERIVE_INIT, sc, fl, 0.0, 0,
-                                                 nullptr);
+  LAPIS_CUDA_TRY(cudaMemsetAsync(sc, 0, 16 * sizeof(double), st));
+  mht_init_kernel<<<G, VEC_THREADS, 0, st>>>(n, w.r, d_d, d_mask, w.r, w.z, w.p, two_pass ? nullptr : w.p1, d_x, w.partials, sc, fl);
   LAPIS_CUDA_TRY(cudaGetLastError());
   const uint64_t limit = maxiter == 0 ? (1ull << 31) : maxiter;
   const uint64_t check_every = 16;
   int done = 0;
   double host[16];
   for (uint64_t i = 1; !done && i <= limit; ++i) {
-    LAPIS_TRY(spmv_launch(A, mp, t, 0, mp, A->blk_partial, skip, st));
-    sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(A->blk_partial, A->nblk, 1, sc + SC_PAP, nullptr, DERIVE_ALPHA_MASKED, sc,
-                                                   fl, 0.0, 0, fl);
-    mht_update_kernel<<<G, VEC_THREADS, 0, st>>>(n, sc, fl, p, mp, t, d_d, d_mask, d_x, r, z, partials);
-    sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(partials, G, 2, sc + SC_RR, sc + SC_RZNEW, DERIVE_DECIDE, sc, fl, tol,
-                                                   maxiter, fl);
-    mht_direction_kernel<<<G, VEC_THREADS, 0, st>>>(n, sc, fl, z, d_d, d_mask, p, mp, partials);
-    sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(partials + 2 * (int64_t)G, G, 1, sc + SC_DMP2, nullptr, DERIVE_NONE, sc,
-                                                   fl, 0.0, 0, fl);
+    if (two_pass) {
+      LAPIS_TRY(A->idx_bytes == 4 ? mht_operator_launch<int32_t>(A, alpha, d_d, d_mask, w, st)
+                                  : mht_operator_launch<int64_t>(A, alpha, d_d, d_mask, w, st));
+      LAPIS_CUDA_TRY(launch_pdl(mht_residual_kernel, std::min<unsigned>(G, MHT_RESIDENT * sm_count()), VEC_THREADS, 0, st, n, sc, fl, tol,
+                                (unsigned long long)maxiter, w.p, w.p1, w.t, d_d, d_x, w.r, w.z, w.partials));
+    } else {
+      LAPIS_TRY(spmv_launch(A, w.p1, w.t, 0, w.p1, A->blk_partial, skip, st));
+      sum_partials_kernel<<<1, SUM_THREADS, 0, st>>>(A->blk_partial, A->nblk, 1, sc + SC_PAP, nullptr, DERIVE_ALPHA_MASKED, sc, fl, 0.0, 0, fl);
+      mht_update_kernel<<<G, VEC_THREADS, 0, st>>>(n, sc, fl, tol, maxiter, w.p, w.p1, w.t, d_d, d_mask, d_x, w.r, w.z, w.partials);
+      mht_direction_kernel<<<G, VEC_THREADS, 0, st>>>(n, sc, fl, w.z, d_d, d_mask, w.p, w.p1, w.partials);
+    }
     LAPIS_CUDA_TRY(cudaGetLastError());
     if (i % check_every == 0 || i == limit) {
-      LAPIS_CUDA_TRY(cudaMemcpyAsync(host, work, sizeof(host), cudaMemcpyDeviceToHost, st));
+      LAPIS_CUDA_TRY(cudaMemcpyAsync(host, sc, sizeof(host), cudaMemcpyDeviceToHost, st));
       LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
       done = (int)reinterpret_cast<const long long *>(host + SC_COUNT)[FL_DONE];
     }
   }
-  LAPIS_CUDA_TRY(cudaMemcpyAsync(host, work, sizeof(host), cudaMemcpyDeviceToHost, st));
-  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  if (!done) {
+    LAPIS_CUDA_TRY(cudaMemcpyAsync(host, sc, sizeof(host), cudaMemcpyDeviceToHost, st));
+    LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   if (iters) *iters = (uint64_t) reinterpret_cast<const long long *>(host + SC_COUNT)[FL_ITERS];
   if (relres) *relres = host[SC_RELRES];
   return LAPIS_OK;
@@ -1044,33 +1257,52 @@ extern "C" int lapis_b200_mht_f64(lapis_b200_csr_t h, const double *d_mask, cons
   cudaStream_t st = as_stream(stream);
   // two solves run the SpMV pass many times: pick the kernel variant for this matrix first
   if (h->tuned_threads == 0 && (maxiter == 0 || maxiter >= 16)) LAPIS_TRY(lapis_b200_csr_tune(h, st));
+  const bool two_pass = spmv_fuses_pcg_pass(h);  // one thread per row, which multiplies by alpha as it goes
   const unsigned G = vec_grid(n);
-  const size_t work_doubles = 16 + 3 * (size_t)G + 5 * (size_t)n;
-  // [work][b][pad][scaled values][pad]: the SpMV kernels stream the values with 16-byte accesses starting at
+  // partials: three sums of G blocks, or two of at most eight blocks per SM
+  const size_t partials = std::max<size_t>(3 * (size_t)G, 2 * 8 * (size_t)sm_count());
+  const size_t work_doubles = 16 + partials + 5 * (size_t)n;
+  // [work][pad][scaled values][pad]: the SpMV kernels stream the values with 16-byte accesses starting at
   // entry (base & ~3) of the array the handle points to, so "scaled copy - base" must be 16-byte aligned
   // like the caller's array is, and the few entries in front of the copy must be readable (they are
   // masked out, not used).
-  size_t sval_index = work_doubles + (size_t)n + 4;
+  size_t sval_index = work_doubles + 4;
   if (((int64_t)sval_index - h->base) & 1) sval_index += 1;
   PoolBuf mem;
-  LAPIS_TRY(mem.alloc((sval_index + (size_t)h->nnz + 8) * sizeof(double), st));
+  LAPIS_TRY(mem.alloc((two_pass ? work_doubles : sval_index + (size_t)h->nnz + 8) * sizeof(double), st));
   double *buf = static_cast<double *>(mem.p);
-  double *work = buf, *bbuf = buf + work_doubles, *sval = buf + sval_index;
+  MhtWork w = {buf, buf + 16, buf + 16 + partials};
+  w.z = w.r + n;
+  w.p = w.z + n;
+  w.p1 = w.p + n;
+  w.t = w.p1 + n;
   // the emitted code scales the matrix values in place; here the caller's array stays as it is and the
   // solves read a scaled copy through a shallow copy of the handle (same streaming plan)
   lapis_b200_csr scaled = *h;
-  const double *val0 = h->val + h->base;  // the handle's arrays are indexed by absolute offsets
-  if (h->nnz > 0) scale_copy_kernel<<<vec_grid(h->nnz), VEC_THREADS, 0, st>>>(h->nnz, val0, alpha, sval);
-  scaled.val = sval - h->base;
+  if (!two_pass) {
+    const double *val0 = h->val + h->base;  // the handle's arrays are indexed by absolute offsets
+    if (h->nnz > 0) scale_copy_kernel<<<vec_grid(h->nnz), VEC_THREADS, 0, st>>>(h->nnz, val0, alpha, buf + sval_index);
+    scaled.val = buf + sval_index - h->base;
+  }
   uint64_t it[2] = {0, 0};
   double rel[2] = {0.0, 0.0};
-  mult_kernel<<<G, VEC_THREADS, 0, st>>>(n, d_d, d_mask, bbuf);  // hitting_times.py:158
-  int status = mht_solve(&scaled, bbuf, d_d, d_mask, tol, maxiter, d_mom1, work, &it[0], &rel[0], st);
-  if (status == LAPIS_OK) status = spmv_launch(&scaled, d_mom1, work + 16, 0, nullptr, nullptr, nullptr, st);
+  mult_kernel<<<G, VEC_THREADS, 0, st>>>(n, d_d, d_mask, w.r);  // hitting_times.py:158
+  int status = mht_solve(&scaled, two_pass, alpha, d_d, d_mask, tol, maxiter, d_mom1, w, &it[0], &rel[0], st);
   if (status == LAPIS_OK) {
-    mht_rhs2_kernel<<<G, VEC_THREADS, 0, st>>>(n, work + 16, d_mask, d_mom1, d_d, bbuf);
-    status = mht_solve(&scaled, bbuf, d_d, d_mask, tol, maxiter, d_mom2, work, &it[1], &rel[1], st);
+    if (!two_pass) {
+      status = spmv_launch(&scaled, d_mom1, w.t, 0, nullptr, nullptr, nullptr, st);
+      mht_rhs2_kernel<<<G, VEC_THREADS, 0, st>>>(n, w.t, d_mask, d_mom1, d_d, w.r);
+    } else {
+      auto rhs2 = [&](auto index) {
+        using I = decltype(index);
+        mht_rhs2_rows_kernel<I><<<G, VEC_THREADS, 0, st>>>(static_cast<const I *>(h->pos), static_cast<const I *>(h->crd), h->val, alpha,
+                                                          h->base & ~(int64_t)3, n, d_d, d_mask, d_mom1, w.r);
+      };
+      if (h->idx_bytes == 4) rhs2(int32_t());
+      else rhs2(int64_t());
+    }
   }
+  if (status == LAPIS_OK) status = mht_solve(&scaled, two_pass, alpha, d_d, d_mask, tol, maxiter, d_mom2, w, &it[1], &rel[1], st);
   cudaError_t e = cudaStreamSynchronize(st);
   if (status != LAPIS_OK) return status;
   if (e != cudaSuccess) return fail(LAPIS_ECUDA, "mht: %s", cudaGetErrorString(e));
