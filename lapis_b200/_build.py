@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblapis_b200.so")
 CALLS = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
-SOURCES = ["abi.cu", "stage.cu", "spmv.cu", "spmm.cu", "pcg.cu", "pcg_small.cu", "gemm.cu", "gemm_tcgen05.cu", "gemm_split.cu", "mmio.cu", "formats.cu"]
+SOURCES = ["abi.cu", "stage.cu", "spmv.cu", "spmm.cu", "pcg.cu", "pcg_small.cu", "pcg_grid.cu", "gemm.cu", "gemm_tcgen05.cu", "gemm_split.cu", "mmio.cu", "formats.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--fmad=false",

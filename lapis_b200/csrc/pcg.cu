@@ -36,6 +36,9 @@ bool spmv_fuses_pcg_pass(const lapis_b200_csr *h);
 bool spmv_fits_small_pcg(const lapis_b200_csr *h);
 int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
               uint64_t *iters, double *relres, bool *solved, cudaStream_t st);
+bool spmv_fits_grid_pcg(const lapis_b200_csr *h);
+int pcg_grid(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
+             uint64_t *iters, double *relres, bool *solved, cudaStream_t st);
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex);
 int spmv_launch_pcg_direction_pass(const lapis_b200_csr *h, int64_t p_off, double *pw0, double *pw1, double *Ap,
@@ -627,6 +630,10 @@ extern "C" int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const d
   if (spmv_fits_small_pcg(h)) {
     bool solved = false;
     LAPIS_TRY(pcg_small(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
+    if (solved) return LAPIS_OK;
+  } else if (spmv_fits_grid_pcg(h)) {
+    bool solved = false;
+    LAPIS_TRY(pcg_grid(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
     if (solved) return LAPIS_OK;
   }
   // a solve runs the SpMV pass many times: pick the kernel variant for this matrix first

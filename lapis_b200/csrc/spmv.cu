@@ -40,6 +40,8 @@
 
 namespace lapis_b200 {
 
+bool pcg_grid_fits(int64_t nrows, int64_t nnz);
+
 #ifndef LAPIS_SPMV_TILE
 #define LAPIS_SPMV_TILE 2048
 #endif
@@ -1525,6 +1527,10 @@ bool spmv_fuses_pcg_pass(const lapis_b200_csr *h) { return h->nrows > 0 && spmv_
 // SMs get through (a band of 127,000 takes 10 us an iteration, the passes 22), no SpMV kernel forced.
 bool spmv_fits_small_pcg(const lapis_b200_csr *h) {
   return h->nrows > 0 && h->nrows <= 16384 && h->nnz <= 131072 && has_short_rows(h) && spmv_override().threads == 0;
+}
+// The same for one cooperative launch (pcg_grid.cu).
+bool spmv_fits_grid_pcg(const lapis_b200_csr *h) {
+  return h->nrows > 0 && has_short_rows(h) && spmv_override().threads == 0 && pcg_grid_fits(h->nrows, h->nnz);
 }
 int spmv_launch_pcg_pass(const lapis_b200_csr *h, const double *x, double *y, const double *dotvec, double *blk_partial,
                          const int *skip_flag, cudaStream_t st, const PcgExchange &ex) {
