@@ -22,13 +22,14 @@ constexpr int BSPMM_THREADS = 128;
 template <typename I, int GROUP, int EPT>
 __global__ void __launch_bounds__(BSPMM_THREADS)
 bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float *__restrict__ val, int64_t nrows,
-                  int64_t nh, int64_t E, const float *__restrict__ B, float *__restrict__ C, int accumulate) {
+                  int64_t nh, int64_t E, int64_t width, const float *__restrict__ B, float *__restrict__ C, int accumulate) {
   const int g = threadIdx.x % GROUP;
   const int64_t row = (int64_t)blockIdx.x * (BSPMM_THREADS / GROUP) + threadIdx.x / GROUP;
   if (row >= nrows) return;
   const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
   float *crow = C + row * E;
-  for (int64_t e0 = 0; e0 < E; e0 += (int64_t)GROUP * EPT) {
+  const int64_t first = (int64_t)blockIdx.y * width, last = first + width < E ? first + width : E;
+  for (int64_t e0 = first; e0 < last; e0 += (int64_t)GROUP * EPT) {
     int64_t e[EPT];
     int fiber[EPT];
     float acc[EPT];
@@ -36,7 +37,7 @@ bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const fl
     for (int q = 0; q < EPT; ++q) {
       e[q] = e0 + g + (int64_t)q * GROUP;
       fiber[q] = (int)(e[q] % nh);
-      acc[q] = (accumulate && e[q] < E) ? crow[e[q]] : 0.0f;
+      acc[q] = (accumulate && e[q] < last) ? crow[e[q]] : 0.0f;
     }
     int64_t j = lo;
     for (; j + 1 < hi; j += 2) {  // two stored entries in flight; the adds stay in entry order
@@ -44,7 +45,7 @@ bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const fl
       float a0[EPT], b0[EPT], a1[EPT], b1[EPT];
 #pragma unroll
       for (int q = 0; q < EPT; ++q) {
-        const bool in = e[q] < E;
+        const bool in = e[q] < last;
         a0[q] = in ? val[j * nh + fiber[q]] : 0.0f;
         b0[q] = in ? __ldg(B + c0 * E + e[q]) : 0.0f;
         a1[q] = in ? val[(j + 1) * nh + fiber[q]] : 0.0f;
@@ -60,91 +61,112 @@ bspmm_csrv_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const fl
       const int64_t c0 = (int64_t)crd[j];
 #pragma unroll
       for (int q = 0; q < EPT; ++q)
-        if (e[q] < E) acc[q] = __fadd_rn(__fmul_rn(val[j * nh + fiber[q]], __ldg(B + c0 * E + e[q])), acc[q]);
+        if (e[q] < last) acc[q] = __fadd_rn(__fmul_rn(val[j * nh + fiber[q]], __ldg(B + c0 * E + e[q])), acc[q]);
     }
 #pragma unroll
     for (int q = 0; q < EPT; ++q)
-      if (e[q] < E) crow[e[q]] = acc[q];
+      if (e[q] < last) crow[e[q]] = acc[q];
   }
 }
 
 // Rows of up to 256 elements with 16-byte accesses, for fibers whose length is a multiple of four (and 16-byte aligned
-// arrays): a
-// thread owns four consecutive output elements, which lie in one fiber, so one float4 of the entry's values
-// meets one float4 of the B row.  Four stored entries are in flight per thread; the adds stay in entry order.
-template <typename I, int GROUP>
-__global__ void __launch_bounds__(BSPMM_THREADS)
+// arrays): a thread owns Q times four consecutive output elements, which lie in one fiber, so one float4 of the entry's values
+// meets one float4 of the B row; with SAME the Q fours stand at the same place of their fibers and share the values.  Four
+// stored entries are in flight per thread; the adds stay in entry order.  Where the rows of B come from L2 (bspmm_slice) the
+// trips to L2 and the instructions bound it, about 25 for each entry and Q = 1, which is what Q = 2 is for.  131,072 rows of
+// 32, 8 x 64: 1.05 ms with B whole and Q = 1 (DRAM: 6.5 GB), 1.01 in slices (1.9 GB), 0.69 in slices with Q = 2, 0.95 with
+// Q = 4; 20,000 of 30, 16 x 128: 493 -> 385 us; 262,144 of 10, 4 x 64: 466 -> 324; 50,000 of 20, 8 x 32 (B in L2): 122 -> 82.
+// Passing the columns of 32 entries round by shuffles, one trip to memory for them all, took 1.52 ms.
+template <typename I, int GROUP, int Q, bool SAME>
+__global__ void __launch_bounds__(BSPMM_THREADS, Q == 1 ? 10 : 8)
 bspmm_csrv_vec4_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float4 *__restrict__ val4,
-                       int64_t nrows, int nh4, int64_t E4, const float4 *__restrict__ B4, float4 *__restrict__ C4,
+                       int64_t nrows, int nh4, int64_t E4, int64_t width4, const float4 *__restrict__ B4, float4 *__restrict__ C4,
                        int accumulate) {
+  constexpr int QA = SAME ? 1 : Q;
   const int g = threadIdx.x % GROUP;
   const int64_t row = (int64_t)blockIdx.x * (BSPMM_THREADS / GROUP) + threadIdx.x / GROUP;
   if (row >= nrows) return;
   const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
   float4 *crow = C4 + row * E4;
-  for (int64_t f = g; f < E4; f += GROUP) {  // f: index of this thread's float4 inside the row
-    const float4 *vcol = val4 + (f % nh4);   // + j * nh4 selects the entry
-    const float4 *bcol = B4 + f;             // + crd[j] * E4 selects the row of B
-    float4 acc = accumulate ? crow[f] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int64_t first = (int64_t)blockIdx.y * width4, last = first + width4 < E4 ? first + width4 : E4;
+  for (int64_t f = first + g; f < last; f += GROUP * Q) {  // f: index of this thread's first float4 inside the row
+    const float4 *vcol[QA];                // + j * nh4 selects the entry
+    const float4 *bcol = B4 + f;           // + crd[j] * E4 selects the row of B
+    bool in[Q];
+    float4 acc[Q];
+#pragma unroll
+    for (int q = 0; q < QA; ++q) vcol[q] = val4 + ((f + q * GROUP) % nh4);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      in[q] = q == 0 || f + q * GROUP < last;
+      acc[q] = accumulate && in[q] ? crow[f + q * GROUP] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    auto add = [&](const float4(&a)[QA], const float4(&b)[Q]) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const float4 &v = a[SAME ? 0 : q];
+        acc[q].x = __fadd_rn(__fmul_rn(v.x, b[q].x), acc[q].x);
+        acc[q].y = __fadd_rn(__fmul_rn(v.y, b[q].y), acc[q].y);
+        acc[q].z = __fadd_rn(__fmul_rn(v.z, b[q].z), acc[q].z);
+        acc[q].w = __fadd_rn(__fmul_rn(v.w, b[q].w), acc[q].w);
+      }
+    };
+    auto fetch = [&](int64_t j, float4(&a)[QA], float4(&b)[Q]) {
+      const float4 *brow = bcol + (int64_t)crd[j] * E4;
+#pragma unroll
+      for (int q = 0; q < QA; ++q) a[q] = __ldg(vcol[q] + j * nh4);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) b[q] = in[q] ? __ldg(brow + q * GROUP) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
     int64_t j = lo;
     for (; j + 3 < hi; j += 4) {
-      float4 a[4], b[4];
+      float4 a[4][QA], b[4][Q];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t c = (int64_t)crd[j + u];
-        a[u] = __ldg(vcol + (j + u) * nh4);
-        b[u] = __ldg(bcol + c * E4);
-      }
+      for (int u = 0; u < 4; ++u) fetch(j + u, a[u], b[u]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        acc.x = __fadd_rn(__fmul_rn(a[u].x, b[u].x), acc.x);
-        acc.y = __fadd_rn(__fmul_rn(a[u].y, b[u].y), acc.y);
-        acc.z = __fadd_rn(__fmul_rn(a[u].z, b[u].z), acc.z);
-        acc.w = __fadd_rn(__fmul_rn(a[u].w, b[u].w), acc.w);
-      }
+      for (int u = 0; u < 4; ++u) add(a[u], b[u]);
     }
     for (; j < hi; ++j) {
-      const float4 a = __ldg(vcol + j * nh4), b = __ldg(bcol + (int64_t)crd[j] * E4);
-      acc.x = __fadd_rn(__fmul_rn(a.x, b.x), acc.x);
-      acc.y = __fadd_rn(__fmul_rn(a.y, b.y), acc.y);
-      acc.z = __fadd_rn(__fmul_rn(a.z, b.z), acc.z);
-      acc.w = __fadd_rn(__fmul_rn(a.w, b.w), acc.w);
+      float4 a[QA], b[Q];
+      fetch(j, a, b);
+      add(a, b);
     }
-    crow[f] = acc;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (in[q]) crow[f + q * GROUP] = acc[q];
   }
 }
 
 __device__ __forceinline__ float madd(float a, float b, float c) { return __fadd_rn(__fmul_rn(a, b), c); }
 
-// The same for short rows and for fibers that are no multiple of four: G threads share one row; a thread owns Q groups of V
-// neighbouring output elements, G groups apart, with U stored entries in flight; the adds stay in entry order.  V = 4:
-// 16-byte accesses to B and C, the values of the elements' fibers one by one, or with FIBER4 (nh a multiple of four) also by
-// 16 bytes: taken for rows of more than 256 elements, where 40 registers and twelve blocks an SM keep more gathers in
-// flight than bspmm_csrv_vec4_kernel's 48 (131,072 rows of 32, 8 x 64: 1.29 -> 1.15 ms; 20,000 of 30, 16 x 128: 558 -> 487 us).  Bound by the gathers of
-// rows of B; G follows the row's length, so that short rows do not leave most of a warp idle (50,000 rows of 20, 4 elements
-// each: 84 -> 17 us; 200,000 rows of 8, 2 x 4: 155 -> 28), and wide accesses halve the requests (50,000 rows of 20, 1 x 64:
-// 85 -> 48; 30,000 of 30, 11 x 40: 269 -> 235; 20,000 of 30, 15 x 128: 718 -> 676).
-template <typename I, int V, bool FIBER4, int G, int Q>
-__global__ void __launch_bounds__(BSPMM_THREADS, FIBER4 ? 12 : 6)
+// The same for fibers that are no multiple of four: G threads share one row; a thread owns Q groups of V neighbouring output
+// elements, G groups apart, with U stored entries in flight; the adds stay in entry order.  V = 4: 16-byte accesses to B and
+// C, the values of the elements' fibers one by one.  Bound by the gathers of rows of B; G follows the row's length, so that
+// short rows do not leave most of a warp idle (50,000 rows of 20, 4 elements each: 84 -> 17 us; 200,000 rows of 8, 2 x 4:
+// 155 -> 28), and wide accesses halve the requests (50,000 rows of 20, 1 x 64: 85 -> 48; 30,000 of 30, 11 x 40: 269 -> 235;
+// 20,000 of 30, 15 x 128: 718 -> 676).
+template <typename I, int V, int G, int Q>
+__global__ void __launch_bounds__(BSPMM_THREADS, 6)
 bspmm_csrv_group_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const float *__restrict__ val, int64_t nrows,
-                  int64_t nh, int64_t E, const float *__restrict__ B, float *__restrict__ C, int accumulate) {
+                  int64_t nh, int64_t E, int64_t width, const float *__restrict__ B, float *__restrict__ C, int accumulate) {
   constexpr int U = V == 4 ? 4 : 8 / Q;
   const int g = threadIdx.x % G;
   const int64_t row = (int64_t)blockIdx.x * (BSPMM_THREADS / G) + threadIdx.x / G;
   if (row >= nrows) return;
   const int64_t lo = (int64_t)pos[row], hi = (int64_t)pos[row + 1];
   float *crow = C + row * E;
-  for (int64_t e0 = (int64_t)g * V; e0 < E; e0 += G * Q * V) {
+  const int64_t first = (int64_t)blockIdx.y * width, last = first + width < E ? first + width : E;
+  for (int64_t e0 = first + (int64_t)g * V; e0 < last; e0 += G * Q * V) {
     bool in[Q];
-    int64_t fiber[Q][FIBER4 ? 1 : V];
+    int64_t fiber[Q][V];
     alignas(16) float acc[Q][V];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const int64_t e = e0 + q * G * V;
-      in[q] = q == 0 || e < E;
+      in[q] = q == 0 || e < last;
       fiber[q][0] = e % nh;
 #pragma unroll
-      for (int i = 1; i < (FIBER4 ? 1 : V); ++i) fiber[q][i] = fiber[q][i - 1] + 1 == nh ? 0 : fiber[q][i - 1] + 1;
+      for (int i = 1; i < (V); ++i) fiber[q][i] = fiber[q][i - 1] + 1 == nh ? 0 : fiber[q][i - 1] + 1;
 #pragma unroll
       for (int i = 0; i < V; ++i) acc[q][i] = 0.0f;
       if (accumulate && in[q]) {
@@ -156,10 +178,9 @@ bspmm_csrv_group_kernel(const I *__restrict__ pos, const I *__restrict__ crd, co
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const float *v = val + j * nh, *brow = B + c * E + e0 + q * G * V;
-        if (FIBER4) *reinterpret_cast<float4 *>(a[q]) = __ldg(reinterpret_cast<const float4 *>(v + fiber[q][0]));
 #pragma unroll
         for (int i = 0; i < V; ++i)
-          if (!FIBER4) a[q][i] = Q == 1 || in[q] ? __ldg(v + fiber[q][i]) : 0.0f;
+          a[q][i] = Q == 1 || in[q] ? __ldg(v + fiber[q][i]) : 0.0f;
         if (V == 4) *reinterpret_cast<float4 *>(b[q]) = __ldg(reinterpret_cast<const float4 *>(brow));
         else b[q][0] = Q == 1 || in[q] ? __ldg(brow) : 0.0f;
       }
@@ -198,52 +219,89 @@ template <typename I>
 struct BspmmArgs {
   const I *pos, *crd;
   const float *val;
-  int64_t nrows, nh, E;
+  int64_t nrows, nh, E, width;  // width: elements of a row that one pass over the matrix takes
   const float *B;
   float *C;
   int accumulate;
 };
 
-template <typename I, int G>
-static void launch_bspmm_vec4(const BspmmArgs<I> &m, cudaStream_t st) {
-  constexpr int ROWS = BSPMM_THREADS / G;
-  bspmm_csrv_vec4_kernel<I, G><<<(unsigned)((m.nrows + ROWS - 1) / ROWS), BSPMM_THREADS, 0, st>>>(
-      m.pos, m.crd, reinterpret_cast<const float4 *>(m.val), m.nrows, (int)(m.nh / 4), m.E / 4, reinterpret_cast<const float4 *>(m.B),
-      reinterpret_cast<float4 *>(m.C), m.accumulate);
-}
-
-template <typename I, int V, bool FIBER4, int G, int Q>
-static void launch_bspmm_group(const BspmmArgs<I> &m, cudaStream_t st) {
-  constexpr int ROWS = BSPMM_THREADS / G;
-  bspmm_csrv_group_kernel<I, V, FIBER4, G, Q><<<(unsigned)((m.nrows + ROWS - 1) / ROWS), BSPMM_THREADS, 0, st>>>(
-      m.pos, m.crd, m.val, m.nrows, m.nh, m.E, m.B, m.C, m.accumulate);
+// Elements of a row of B (E floats, n2 rows) that one pass over the matrix gathers.  A gather from L2 runs at 20 TB/s as long
+// as what is gathered from stays under about 70 MB, from DRAM at 7 (measured with random rows of 256 and 512 bytes), so a
+// larger B is taken in slices of at most 72 MB, the slice slowest: every slice is read from DRAM once, and only the entries
+// of the matrix, a few bytes beside 128 to 1024 gathered ones, are read once a slice.  Slices are as wide as a group of
+// lanes takes at once.  Where the values come one by one, rows of at most 256 elements only: that kernel is bound by its
+// instructions, which slices of unequal width make more (60,000 rows of 20, 11 x 80: 0.89 ms whole, 1.04 in four slices).
+static int64_t bspmm_slice(int64_t n2, int64_t E) {
+  if (4.0 * (double)n2 * (double)E <= 96e6) return E;
+  int64_t width = 256;
+  while (width > 32 && 4.0 * (double)n2 * (double)width > 72e6) width /= 2;
+  return width < E ? width : E;
 }
 
 template <typename I>
-static void launch_bspmm(const BspmmArgs<I> &m, cudaStream_t st) {
+static dim3 bspmm_grid(const BspmmArgs<I> &m, int rows) {
+  return dim3((unsigned)((m.nrows + rows - 1) / rows), (unsigned)((m.E + m.width - 1) / m.width));
+}
+
+template <typename I, int G, int Q, bool SAME>
+static void launch_bspmm_vec4_as(const BspmmArgs<I> &m, cudaStream_t st) {
+  constexpr int ROWS = BSPMM_THREADS / G;
+  bspmm_csrv_vec4_kernel<I, G, Q, SAME><<<bspmm_grid(m, ROWS), BSPMM_THREADS, 0, st>>>(
+      m.pos, m.crd, reinterpret_cast<const float4 *>(m.val), m.nrows, (int)(m.nh / 4), m.E / 4, m.width / 4, reinterpret_cast<const float4 *>(m.B),
+      reinterpret_cast<float4 *>(m.C), m.accumulate);
+}
+template <typename I, int G>
+static void launch_bspmm_vec4(const BspmmArgs<I> &m, cudaStream_t st) {
+  launch_bspmm_vec4_as<I, G, 1, true>(m, st);
+}
+// Two fours a thread, for rows that fill the group twice.
+template <typename I, int G>
+static void launch_bspmm_vec4_twice(const BspmmArgs<I> &m, cudaStream_t st) {
+  if (G % (m.nh / 4) == 0) launch_bspmm_vec4_as<I, G, 2, true>(m, st);
+  else launch_bspmm_vec4_as<I, G, 2, false>(m, st);
+}
+
+template <typename I, int V, int G, int Q>
+static void launch_bspmm_group(const BspmmArgs<I> &m, cudaStream_t st) {
+  constexpr int ROWS = BSPMM_THREADS / G;
+  bspmm_csrv_group_kernel<I, V, G, Q><<<bspmm_grid(m, ROWS), BSPMM_THREADS, 0, st>>>(
+      m.pos, m.crd, m.val, m.nrows, m.nh, m.E, m.width, m.B, m.C, m.accumulate);
+}
+
+template <typename I>
+static void launch_bspmm(const BspmmArgs<I> &m, int64_t n2, cudaStream_t st) {
   const bool aligned = (reinterpret_cast<uintptr_t>(m.B) | reinterpret_cast<uintptr_t>(m.C)) % 16 == 0;
-  const int64_t E = m.E, E4 = m.E / 4;
-  if (aligned && m.nh % 4 == 0 && m.nh / 4 <= 0x7fffffff && reinterpret_cast<uintptr_t>(m.val) % 16 == 0) {
-    if (E4 <= 4) launch_bspmm_vec4<I, 4>(m, st);
-    else if (E4 <= 8) launch_bspmm_vec4<I, 8>(m, st);
-    else if (E4 <= 16) launch_bspmm_vec4<I, 16>(m, st);
-    else if (E4 <= 32) launch_bspmm_vec4<I, 32>(m, st);
-    else if (E4 <= 64) launch_bspmm_vec4<I, 64>(m, st);
-    else launch_bspmm_group<I, 4, true, 128, 1>(m, st);
-  } else if (aligned && E % 4 == 0) {
-    if (E4 <= 4) launch_bspmm_group<I, 4, false, 4, 1>(m, st);
-    else if (E4 <= 8) launch_bspmm_group<I, 4, false, 8, 1>(m, st);
-    else if (E4 <= 16) launch_bspmm_group<I, 4, false, 16, 1>(m, st);
-    else if (E4 <= 32) launch_bspmm_group<I, 4, false, 32, 1>(m, st);
-    else if (E4 <= 64) launch_bspmm_group<I, 4, false, 64, 1>(m, st);
-    else launch_bspmm_group<I, 4, false, 128, 1>(m, st);
-  } else if (E <= 8) launch_bspmm_group<I, 1, false, 8, 1>(m, st);
-  else if (E <= 16) launch_bspmm_group<I, 1, false, 16, 1>(m, st);
-  else if (E <= 32) launch_bspmm_group<I, 1, false, 32, 1>(m, st);
-  else if (E <= 64) launch_bspmm_group<I, 1, false, 32, 2>(m, st);
-  else if (E <= 128) launch_bspmm_group<I, 1, false, 32, 4>(m, st);
+  if (aligned && m.E % 4 == 0 && m.nh % 4 == 0 && m.nh / 4 <= 0x7fffffff && reinterpret_cast<uintptr_t>(m.val) % 16 == 0) {
+    BspmmArgs<I> s = m;
+    s.width = bspmm_slice(n2, m.E);
+    const int64_t E4 = s.width / 4;
+    if (E4 <= 4) launch_bspmm_vec4<I, 4>(s, st);
+    else if (E4 <= 8) launch_bspmm_vec4<I, 8>(s, st);
+    else if (E4 <= 12) launch_bspmm_vec4<I, 16>(s, st);
+    else if (E4 <= 16) launch_bspmm_vec4_twice<I, 8>(s, st);
+    else if (E4 <= 32) launch_bspmm_vec4_twice<I, 16>(s, st);
+    else if (E4 <= 64) launch_bspmm_vec4_twice<I, 32>(s, st);
+    else launch_bspmm_vec4_twice<I, 64>(s, st);
+    return;
+  }
+  const int64_t E = m.E;
+  if (aligned && E % 4 == 0) {
+    BspmmArgs<I> s = m;
+    if (E <= 256) s.width = bspmm_slice(n2, E);
+    const int64_t E4 = s.width / 4;
+    if (E4 <= 4) launch_bspmm_group<I, 4, 4, 1>(s, st);
+    else if (E4 <= 8) launch_bspmm_group<I, 4, 8, 1>(s, st);
+    else if (E4 <= 16) launch_bspmm_group<I, 4, 16, 1>(s, st);
+    else if (E4 <= 32) launch_bspmm_group<I, 4, 32, 1>(s, st);
+    else if (E4 <= 64) launch_bspmm_group<I, 4, 64, 1>(s, st);
+    else launch_bspmm_group<I, 4, 128, 1>(s, st);
+  } else if (E <= 8) launch_bspmm_group<I, 1, 8, 1>(m, st);
+  else if (E <= 16) launch_bspmm_group<I, 1, 16, 1>(m, st);
+  else if (E <= 32) launch_bspmm_group<I, 1, 32, 1>(m, st);
+  else if (E <= 64) launch_bspmm_group<I, 1, 32, 2>(m, st);
+  else if (E <= 128) launch_bspmm_group<I, 1, 32, 4>(m, st);
   else
-    bspmm_csrv_kernel<I, 128, 4><<<(unsigned)m.nrows, BSPMM_THREADS, 0, st>>>(m.pos, m.crd, m.val, m.nrows, m.nh, E, m.B, m.C, m.accumulate);
+    bspmm_csrv_kernel<I, 128, 4><<<bspmm_grid(m, 1), BSPMM_THREADS, 0, st>>>(m.pos, m.crd, m.val, m.nrows, m.nh, m.E, m.width, m.B, m.C, m.accumulate);
 }
 
 }  // namespace lapis_b200
@@ -263,7 +321,7 @@ extern "C" int lapis_b200_bspmm_csrv_f32(int idx_bytes, int64_t n1, int64_t n2, 
   cudaStream_t st = as_stream(stream);
   auto run = [&](auto index) {
     using I = decltype(index);
-    launch_bspmm<I>({static_cast<const I *>(d_pos), static_cast<const I *>(d_crd), d_val, n1, nh, E, d_B, d_C, accumulate}, st);
+    launch_bspmm<I>({static_cast<const I *>(d_pos), static_cast<const I *>(d_crd), d_val, n1, nh, E, E, d_B, d_C, accumulate}, n2, st);
   };
   if (idx_bytes == 4) run(int32_t());
   else run(int64_t());
