@@ -15,6 +15,8 @@
 // skewed matrix.  Such rows go to a kernel of their own that runs beside this one (spmm_long_kernel): 50,021 rows with
 // a mean of 16 and rows up to 4096, k = 37, DCSR: 884 -> 218 to 283 us with the matrix drawn; 10,000 rows, mean 30,
 // k = 128: 839 -> 235.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdint>
 
@@ -24,8 +26,13 @@ namespace lapis_b200 {
 
 constexpr int SPMM_THREADS = 256;
 constexpr int SPMM_LONG = 256;  // shorter rows never leave their group (a few dozen trips to memory)
-constexpr int SPMM_LONG_THREADS = 512;
-constexpr int SPMM_TILE = 2048;  // products per tile of a long row
+constexpr int SPMM_PANEL = 64;                     // columns of a row that a block takes at once
+constexpr int SPMM_ADDERS = 2, SPMM_FEEDERS = 10;  // warps that add and warps that gather and multiply
+constexpr int SPMM_LONG_THREADS = 32 * (SPMM_ADDERS + SPMM_FEEDERS);
+constexpr int SPMM_PER = 4, SPMM_TILE = 32 * SPMM_FEEDERS * SPMM_PER;  // products of a feeder, of a tile
+constexpr int SPMM_CLUSTER = 4;                       // blocks that share their long rows
+constexpr int SPMM_LIST = SPMM_LONG_THREADS + 64;     // long rows that a block notes before it works on them
+constexpr int SPMM_SHARED = 768;                      // pieces that a cluster divides among its blocks
 
 template <int V>
 struct Columns;
@@ -56,10 +63,10 @@ __device__ __forceinline__ double cols_mul(double a, double b) { return __dmul_r
 __device__ __forceinline__ double2 cols_mul(double a, double2 b) { return make_double2(__dmul_rn(a, b.x), __dmul_rn(a, b.y)); }
 
 // Whether a row of len entries is left to spmm_long_kernel.  A group of lanes walks it in a chain of trips to memory, about
-// 0.15 us an entry and 64 columns; it may last half as long as the whole product of nnz entries does (8 (k + 8) bytes an
-// entry at 5 TB/s), and is then hidden by it.
+// 0.15 us an entry and 64 columns; it may last a quarter as long as the whole product of nnz entries does (8 (k + 8) bytes an
+// entry at 5 TB/s), and is then hidden by it, also where it comes late.
 __host__ __device__ __forceinline__ bool spmm_is_long(int64_t len, int64_t nnz, int64_t k) {
-  return len > SPMM_LONG && len > nnz * (k + 8) / ((k + 63) / 64) >> 17;
+  return len > SPMM_LONG && len < (1 << 30) && k < (1 << 30) && len > nnz * (k + 8) / ((k + 63) / 64) >> 18;
 }
 template <typename I>
 __device__ __forceinline__ bool spmm_is_long(int64_t len, const I *__restrict__ pos, int64_t nrows, int64_t k) {
@@ -155,87 +162,202 @@ spmm_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__r
   }
 }
 
-// The long rows.  A block looks for them among its rows (eight neighbours, then the eight gridDim.x * 8 further on, so
-// that neighbouring long rows meet different blocks) and walks each in tiles of SPMM_TILE products: all threads gather and
-// multiply the next tile while the first `width` add the current one, a column each, in entry order out of shared
-// memory.  Bound by one trip to memory per tile; at most one block per SM, so that half of the registers and most of L1
-// stay with the kernel beside it.  blockIdx.y: panel of `width` <= 32 columns.
+// The long rows.  A block notes those among its rows (eight neighbours, then the eight gridDim.x * 8 further on, so that
+// neighbouring long rows meet different blocks); at the end the blocks of a cluster divide what they noted, a piece being a row
+// and up to 64 columns: by length, the longest first, 0 1 2 3 3 2 1 0 0 1 .. (too many pieces: each block keeps its own).
+// A block works through its pieces in tiles of SPMM_TILE products: ten warps gather and multiply, two tiles ahead of the one
+// they store, across the ends of pieces, and two warps add, a lane one column, in entry order out of shared memory.
+// One tile ahead, one row on an SM, a barrier for both, and now: 50,021 rows, k = 37 264 -> 104 us; 40,000, k = 130 374 -> 252;
+// 30,000 of 39, k = 100 476 -> 363; 200,000 of 30, k = 16 566 -> 274.
 template <typename I, bool DCSR>
-__global__ void __launch_bounds__(SPMM_LONG_THREADS, 2)
+__global__ void __launch_bounds__(SPMM_LONG_THREADS, 2)  // registers: the kernel beside this one needs half of them
 spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val,
-                 int64_t nrows, int64_t k, int width, const double *__restrict__ B, double *__restrict__ C, int accumulate) {
-  constexpr int PER = SPMM_TILE / SPMM_LONG_THREADS;
+                 int64_t nrows, int64_t k, const double *__restrict__ B, double *__restrict__ C, int accumulate) {
+  namespace cg = cooperative_groups;
   __shared__ double s_prod[2][SPMM_TILE];
-  __shared__ int64_t s_lo[SPMM_LONG_THREADS], s_hi[SPMM_LONG_THREADS], s_out[SPMM_LONG_THREADS];
-  __shared__ int s_n;
+  __shared__ int64_t s_lo[SPMM_LIST], s_out[SPMM_LIST];  // noted rows
+  __shared__ int s_len[SPMM_LIST];
+  __shared__ int64_t w_lo[SPMM_LIST], w_out[SPMM_LIST];  // pieces of work
+  __shared__ int w_len[SPMM_LIST], w_c0[SPMM_LIST], w_c1[SPMM_LIST];
+  __shared__ int s_all[SPMM_SHARED];
+  __shared__ int s_n, s_count;
   pdl_release();  // the kernel for the other rows shares nothing with this one but inputs
-  const int tid = threadIdx.x;
-  const int entries = SPMM_TILE / width;  // per tile
-  int je[PER], ce[PER];  // this thread's products in a tile: entry and column
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, feeder = tid - 32 * SPMM_ADDERS;  // negative: an adder
+  const int64_t panels = (k + SPMM_PANEL - 1) / SPMM_PANEL;
+  const int width = (int)((k + panels - 1) / panels), entries = SPMM_TILE / width;  // of a tile
+  int je[SPMM_PER], ce[SPMM_PER];  // this feeder's products in a tile: entry (beyond any row: none) and column
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    je[i] = (tid + i * SPMM_LONG_THREADS) / width;
-    ce[i] = (tid + i * SPMM_LONG_THREADS) % width;
+  for (int i = 0; i < SPMM_PER; ++i) {
+    const int at = feeder + 32 * SPMM_FEEDERS * i;
+    je[i] = feeder >= 0 && at < entries * width ? at / width : 0x40000000;
+    ce[i] = at - at / width * width;
   }
   if (tid == 0) s_n = 0;
   __syncthreads();
   const int64_t turn = (int64_t)gridDim.x * SPMM_LONG_THREADS;
-  for (int64_t r0 = 0; r0 < nrows; r0 += turn) {
-    int64_t lo = 0, hi = 0, out = 0;
-    const int64_t r = r0 + ((int64_t)(tid / 8) * gridDim.x + blockIdx.x) * 8 + tid % 8;
-    const bool found = spmm_row<I, DCSR>(rowno, pos, nrows, r, lo, hi, out) && spmm_is_long(hi - lo, pos, nrows, k);
-    if (found) {
-      const int at = atomicAdd(&s_n, 1);  // the order of the list does not matter: rows are independent
-      s_lo[at] = lo;
-      s_hi[at] = hi;
-      s_out[at] = out;
+  for (int64_t r0 = 0;;) {
+    int noted = 0;
+    for (; r0 < nrows && noted <= SPMM_LIST - SPMM_LONG_THREADS; r0 += turn) {
+      int64_t lo = 0, hi = 0, out = 0;
+      const int64_t r = r0 + ((int64_t)(tid / 8) * gridDim.x + blockIdx.x) * 8 + tid % 8;
+      const bool found = spmm_row<I, DCSR>(rowno, pos, nrows, r, lo, hi, out) && spmm_is_long(hi - lo, pos, nrows, k);
+      if (found) {
+        const int at = atomicAdd(&s_n, 1);  // the order of the list does not matter: rows are independent
+        s_lo[at] = lo;
+        s_len[at] = (int)(hi - lo);
+        s_out[at] = out;
+      }
+      noted += __syncthreads_count(found);
     }
-    if (!__syncthreads_or(found)) continue;
-    const int n = s_n;
-    for (int q = 0; q < n; ++q) {
-      const int64_t first = s_lo[q], last = s_hi[q];
-      for (int64_t c0 = (int64_t)blockIdx.y * width; c0 < k; c0 += (int64_t)gridDim.y * width) {
-        const int cols = k - c0 < width ? (int)(k - c0) : width;
-        double *c = C + s_out[q] * k + c0 + tid;
-        double acc = DCSR && tid < cols ? *c : 0.0;
-        I ci[PER];
-        double b[PER], a[PER];
-        auto columns = [&](int64_t j0) {
+    const bool end = r0 >= nrows;
+    int n = 0;  // pieces
+    bool shared = false;
+    if (end) {
+      if (tid == 0) s_count = 0;
+      cluster.sync();
+      int all = 0, begin[SPMM_CLUSTER + 1];
 #pragma unroll
-          for (int i = 0; i < PER; ++i) ci[i] = je[i] < entries && ce[i] < cols && j0 + je[i] < last ? crd[j0 + je[i]] : (I)-1;
-        };
-        auto gather = [&](int64_t j0) {
+      for (int c = 0; c < SPMM_CLUSTER; ++c) {
+        begin[c] = all;
+        all += *cluster.map_shared_rank(&s_n, c);
+      }
+      begin[SPMM_CLUSTER] = all;
+      shared = all * panels <= SPMM_SHARED;
+      if (shared) {
+        const int np = (int)panels, pieces = all * np;
+        for (int u = tid; u < pieces; u += SPMM_LONG_THREADS) {
+          const int row = u / np;
+          int c = 0;
+          while (row >= begin[c + 1]) ++c;
+          s_all[u] = cluster.map_shared_rank(s_len, c)[row - begin[c]];
+        }
+        __syncthreads();
+        for (int u = tid; u < pieces; u += SPMM_LONG_THREADS) {
+          const int mine = s_all[u];
+          int rank = 0;  // longer ones, and equal ones in front
+          for (int v = 0; v < pieces; ++v) rank += s_all[v] > mine || (s_all[v] == mine && v < u);
+          const int place = rank % (2 * SPMM_CLUSTER);
+          if ((place < SPMM_CLUSTER ? place : 2 * SPMM_CLUSTER - 1 - place) != (int)cluster.block_rank()) continue;
+          const int row = u / np, at = rank / SPMM_CLUSTER;  // its turn in this block
+          int c = 0;
+          while (row >= begin[c + 1]) ++c;
+          w_lo[at] = cluster.map_shared_rank(s_lo, c)[row - begin[c]];
+          w_out[at] = cluster.map_shared_rank(s_out, c)[row - begin[c]];
+          w_len[at] = mine;
+          w_c0[at] = (u - row * np) * width;
+          w_c1[at] = min(w_c0[at] + width, (int)k);
+          atomicAdd(&s_count, 1);
+        }
+      }
+      cluster.sync();  // nobody reads another block's list any more
+      n = shared ? s_count : 0;
+    }
+    if (!shared) {
+      n = noted;
+      for (int u = tid; u < n; u += SPMM_LONG_THREADS) {
+        w_lo[u] = s_lo[u];
+        w_out[u] = s_out[u];
+        w_len[u] = s_len[u];
+        w_c0[u] = 0;
+        w_c1[u] = (int)k;
+      }
+      __syncthreads();
+    }
+    // a place in the sequence of tiles: piece, first column of the panel, first entry of the tile
+    struct Place {
+      int q, c0, j;
+    };
+    auto start = [&](int q) { return Place{q, q < n ? w_c0[q] : 0, 0}; };
+    auto step = [&](Place &p) {  // true: the next tile belongs to another piece or panel
+      p.j += entries;
+      if (p.j < w_len[p.q]) return false;
+      p.j = 0;
+      p.c0 += width;
+      if (p.c0 >= w_c1[p.q]) p = start(p.q + 1);
+      return true;
+    };
+    if (feeder >= 0) {
+      I ci[SPMM_PER];                                                 // columns of the tile that is gathered next
+      double b0[SPMM_PER], a0[SPMM_PER], b1[SPMM_PER], a1[SPMM_PER];  // operands of the next two tiles
+      Place cols = start(0), rows = start(0);
+      auto columns = [&] {
+        if (cols.q < n) {
+          const int left = w_len[cols.q] - cols.j, wide = w_c1[cols.q] - cols.c0;
+          const I *c = crd + w_lo[cols.q] + cols.j;
 #pragma unroll
-          for (int i = 0; i < PER; ++i) {
-            const bool there = ci[i] >= 0;
-            a[i] = there ? __ldg(val + j0 + je[i]) : 0.0;
-            b[i] = there ? __ldg(B + (int64_t)ci[i] * k + c0 + ce[i]) : 0.0;
-          }
-        };
-        columns(first);
-        gather(first);
-        columns(first + entries);
-        int buf = 0;
-        for (int64_t j0 = first; j0 < last; j0 += entries, buf ^= 1) {
+          for (int i = 0; i < SPMM_PER; ++i) ci[i] = je[i] < left && ce[i] < wide ? c[je[i]] : (I)-1;
+          step(cols);
+        } else {
 #pragma unroll
-          for (int i = 0; i < PER; ++i) s_prod[buf][tid + i * SPMM_LONG_THREADS] = __dmul_rn(a[i], b[i]);
+          for (int i = 0; i < SPMM_PER; ++i) ci[i] = (I)-1;
+        }
+      };
+      auto gather = [&](double(&b)[SPMM_PER], double(&a)[SPMM_PER]) {
+        const bool more = rows.q < n;
+        const double *v = val + (more ? w_lo[rows.q] + rows.j : 0), *Bc = B + rows.c0;
+#pragma unroll
+        for (int i = 0; i < SPMM_PER; ++i) {
+          const bool there = ci[i] >= 0;
+          a[i] = there ? __ldg(v + je[i]) : 0.0;
+          b[i] = there ? cols_load(Bc + (int64_t)ci[i] * k + ce[i]) : 0.0;
+        }
+        if (more) step(rows);
+      };
+      auto store = [&](int buf, const double(&b)[SPMM_PER], const double(&a)[SPMM_PER]) {
+#pragma unroll
+        for (int i = 0; i < SPMM_PER; ++i) s_prod[buf][feeder + 32 * SPMM_FEEDERS * i] = __dmul_rn(a[i], b[i]);
+      };
+      columns();
+      gather(b0, a0);
+      columns();
+      gather(b1, a1);
+      columns();
+      // a tile is stored while the one before is added; its buffer was left at the barrier behind that one's store
+      for (Place p = start(0); p.q < n;) {
+        store(0, b0, a0);
+        gather(b0, a0);
+        columns();
+        __syncthreads();
+        step(p);
+        if (p.q >= n) break;
+        store(1, b1, a1);
+        gather(b1, a1);
+        columns();
+        __syncthreads();
+        step(p);
+      }
+    } else {
+      auto element = [&](const Place &p) { return C + w_out[p.q] * k + p.c0 + tid; };
+      auto mine = [&](const Place &p) { return p.q < n && tid < width && p.c0 + tid < w_c1[p.q]; };
+      const bool read = DCSR || accumulate;
+      Place p = start(0);
+      double next = mine(p) && read ? *element(p) : 0.0;  // of C, fetched a piece or panel ahead
+      int buf = 0;
+      while (p.q < n) {
+        const bool in = mine(p);
+        const double cin = next;
+        double *c = in ? element(p) : nullptr;
+        Place after = p;
+        after.j = w_len[p.q];
+        step(after);
+        next = mine(after) && read ? *element(after) : 0.0;
+        double acc = DCSR ? cin : 0.0;
+        bool ended = false;
+        while (!ended) {
           __syncthreads();
-          gather(j0 + entries);
-          columns(j0 + 2 * entries);
-          if (tid < cols) {
-            const double *p = s_prod[buf] + tid;
-            const int m = last - j0 < entries ? (int)(last - j0) : entries;
-#pragma unroll 8
-            for (int t = 0; t < m; ++t) acc = __dadd_rn(acc, p[t * width]);
-          }
+          const double *s = s_prod[buf] + (in ? tid : 0);
+          const int left = w_len[p.q] - p.j, m = left < entries ? left : entries;
+#pragma unroll 16
+          for (int e = 0; e < m; ++e) acc = __dadd_rn(acc, s[e * width]);
+          buf ^= 1;
+          ended = step(p);
         }
-        if (tid < cols) {
-          if (!DCSR) acc = __dadd_rn(acc, accumulate ? *c : 0.0);
-          *c = acc;
-        }
-        __syncthreads();  // the buffers are free
+        if (in) *c = DCSR ? acc : __dadd_rn(acc, cin);
       }
     }
+    if (end) break;
+    __syncthreads();
     if (tid == 0) s_n = 0;
     __syncthreads();
   }
@@ -286,11 +408,18 @@ static cudaError_t launch_spmm_width(const SpmmArgs<I> &m, cudaStream_t st) {
 template <typename I, bool DCSR>
 static cudaError_t launch_spmm(const SpmmArgs<I> &m, cudaStream_t st) {
   if (m.long_rows) {
-    const int64_t panels = (m.k + 31) / 32, chunks = (m.nrows + 7) / 8, py = std::min<int64_t>(panels, 8);
-    const dim3 grid((unsigned)std::min<int64_t>(chunks, sm_count() / py), (unsigned)py);
-    spmm_long_kernel<I, DCSR><<<grid, SPMM_LONG_THREADS, 0, st>>>(m.rowno, m.pos, m.crd, m.val, m.nrows, m.k,
-                                                                  (int)((m.k + panels - 1) / panels), m.B, m.C, m.accumulate);
-    const cudaError_t e = cudaGetLastError();
+    const int64_t clusters = std::min<int64_t>((m.nrows + 8 * SPMM_CLUSTER - 1) / (8 * SPMM_CLUSTER), sm_count() / SPMM_CLUSTER);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * SPMM_CLUSTER));
+    cfg.blockDim = dim3(SPMM_LONG_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SPMM_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, spmm_long_kernel<I, DCSR>, m.rowno, m.pos, m.crd, m.val, m.nrows, m.k, m.B, m.C, m.accumulate);
     if (e != cudaSuccess) return e;
   }
   // pairs of columns travel as 16-byte accesses when k is even and B and C are aligned for it
