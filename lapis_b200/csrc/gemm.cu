@@ -15,7 +15,7 @@
 //     TF32 products.
 //   * products of either kind that are large enough to pay for a pass over their operands first (split_pays): gemm_split.cu,
 //     fp32 from three fp16 products, with a smaller error than the other two.  What that split does not cover (infinities,
-//     NaN, elements 2^31 times smaller than the largest of their row or column) is left to them, panel by panel.
+//     NaN, elements 2^29 times smaller than the largest of their row or column) is left to them, panel by panel.
 #include <algorithm>
 #include <cmath>
 

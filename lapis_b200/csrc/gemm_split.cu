@@ -3,8 +3,8 @@
 //
 // x 2^e = hi + 2^-11 lo with hi and lo in fp16 (11 bits each, lo rounded), e one exponent for each row of A and each column
 // of B; the product is hi hi + 2^-11 (hi lo + lo hi), three fp16 products at twice the rate of the three TF32 products of
-// gemm_tcgen05.cu.  What is left out (lo lo, the rounding of lo) is at most 2^-21 of a product, where the TF32 split, whose
-// parts the tensor core truncates, leaves up to 2^-19.
+// gemm_tcgen05.cu.  What is left out (lo lo, the rounding of lo) is at most 2^-21 of a product as long as hi is a normal fp16
+// number, where the TF32 split, whose parts the tensor core truncates, leaves up to 2^-19.
 //
 //   split_kernel       reads A and B once, writes hi and lo as fp16 matrices with 16-byte rows (so that TMA can load shapes
 //                      and pointers of any alignment), and the scales.  K is cut into stretches of at most 1024, each with
@@ -17,11 +17,11 @@
 // product 20, the look at the marks 3: latencies).  Against 64 bits: 8192^3 1.25e-6 (TF32 split 8.0e-6), 1000 x 1501 x 777
 // 3.9e-7 (sequential sum 5.0e-7), 100 x 100 x 130 1.9e-7 (2.1e-7).
 //
-// fp16 has 5 bits of exponent: an element below 2^-16 of the scaled range (2^-31 of the largest of its row or column) would
-// lose bits, and an infinity or NaN has no scale.  split_kernel marks the 128-row and 128-column panels that hold such an
-// element; the products of those panels are left to the kernels on unsplit operands (PanelFlags), which run behind
-// this one and return at once where there are none.  In 8192 x 8192 normally distributed numbers one is expected in every
-// eighth matrix, in uniformly distributed ones none.
+// fp16 has 5 bits of exponent: the hi of an element below 2^-14 after scaling (2^-29 of the largest of its row or column)
+// would be subnormal and lo lo up to 2^-17 of a product of two such, and an infinity or NaN has no scale.  split_kernel marks
+// the 128-row and 128-column panels that hold such an element; the products of those panels are left to the kernels on unsplit
+// operands (PanelFlags), which run behind this one and return at once where there are none.  In 8192 x 8192 normally
+// distributed numbers one is expected in every second matrix, in uniformly distributed ones (multiples of 2^-24) none.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -61,14 +61,14 @@ __device__ __forceinline__ bool scale_exponent(uint32_t max_bits, int &e) {
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
-// hi and lo of four scaled elements; true if one of them is too small to be split without loss.
+// hi and lo of four scaled elements; true if one of them is so small that its hi would be subnormal.
 __device__ __forceinline__ bool split4(const float (&x)[4], float s, uint2 &hi, uint2 &lo) {
   __half h[4], l[4];
   bool small = false;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float v = __fmul_rn(x[i], s);
-    small |= x[i] != 0.0f && fabsf(v) < 1.0f / 65536.0f;
+    small |= x[i] != 0.0f && fabsf(v) < 1.0f / 16384.0f;
     h[i] = __float2half_rn(v);
     l[i] = __float2half_rn(__fmul_rn(__fsub_rn(v, __half2float(h[i])), LO_SCALE));
   }
