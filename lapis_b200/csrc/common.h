@@ -91,6 +91,14 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // kernel still fills some SMs are placed on the others, and a grid that does not fill the GPU ends up unevenly spread
 // (measured: 1e6 entries, 11 -> 16 us with the call at the top).
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
+// Ordinary load, for what the launch in front may still have been writing when this kernel became resident (launch_pdl).
+// The read-only path (ld.global.nc, which __ldg and reads through const __restrict__ compile to) asks that data stays as it
+// is for the kernel's whole lifetime, which begins in front of pdl_wait().
+__device__ __forceinline__ double load_now(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
 #endif
 
 }  // namespace lapis_b200

@@ -961,8 +961,8 @@ __device__ __forceinline__ void mht_tail_update(double rr, double rz, double *pa
 // MASKED: times p.
 template <typename I, bool DIR, bool MASKED>
 __device__ __forceinline__ double mht_piece(const I *__restrict__ crd, const double *__restrict__ val, double alpha,
-                                            const double *__restrict__ mask, const double *__restrict__ z,
-                                            const double *__restrict__ p, double beta, int64_t lo, int64_t hi) {
+                                            const double *__restrict__ mask, const double *z, const double *p, double beta,
+                                            int64_t lo, int64_t hi) {
   double acc = 0.0;
   for (int64_t j = lo; j < hi; j += 4) {
     double a[4], m[4], zv[4], pv[4];
@@ -972,8 +972,8 @@ __device__ __forceinline__ double mht_piece(const I *__restrict__ crd, const dou
       const int64_t c = in ? (int64_t)crd[j + u] : 0;
       a[u] = in ? val[j + u] : 0.0;
       m[u] = in && MASKED ? mask[c] : 0.0;
-      pv[u] = in ? p[c] : 0.0;
-      zv[u] = in && DIR ? z[c] : 0.0;
+      pv[u] = in ? load_now(p + c) : 0.0;  // the pass in front may still have been writing z and p
+      zv[u] = in && DIR ? load_now(z + c) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -987,8 +987,8 @@ __device__ __forceinline__ double mht_piece(const I *__restrict__ crd, const dou
 constexpr int64_t SPMV_CHUNK = 2048;
 template <typename I, bool DIR, bool MASKED>
 __device__ __forceinline__ double mht_row(const I *__restrict__ crd, const double *__restrict__ val, double alpha, int64_t abase,
-                                          const double *__restrict__ mask, const double *__restrict__ z, const double *__restrict__ p,
-                                          double beta, int64_t lo, int64_t hi, double &stored) {
+                                          const double *__restrict__ mask, const double *z, const double *p, double beta, int64_t lo,
+                                          int64_t hi, double &stored) {
   const int64_t bnd = abase + ((lo - abase) / SPMV_CHUNK + 1) * SPMV_CHUNK;
   const double s = mht_piece<I, DIR, MASKED>(crd, val, alpha, mask, z, p, beta, lo, hi < bnd ? hi : bnd);
   stored = __dadd_rn(s, 0.0);
@@ -1004,8 +1004,8 @@ __device__ __forceinline__ double mht_row(const I *__restrict__ crd, const doubl
 template <typename I, bool DIR>
 __device__ __forceinline__ void mht_rows(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, double alpha,
                                          int64_t abase, int64_t n, const double *__restrict__ d, const double *__restrict__ mask,
-                                         const double *__restrict__ z, const double *__restrict__ p, double *__restrict__ pnew, double beta,
-                                         double *__restrict__ Ap, double &mpt, double &dm) {
+                                         const double *z, const double *p, double *__restrict__ pnew, double beta, double *__restrict__ Ap,
+                                         double &mpt, double &dm) {
   const int64_t stride = (int64_t)gridDim.x * VEC_THREADS;
   int64_t i = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x;
   I next_lo = i < n ? pos[i] : (I)0, next_hi = i < n ? pos[i + 1] : (I)0;  // of the next row, one trip to memory less in the chain
@@ -1016,9 +1016,9 @@ __device__ __forceinline__ void mht_rows(const I *__restrict__ pos, const I *__r
       next_hi = pos[i + stride + 1];
     }
     const double di = d[i], mi = mask[i];
-    double pi = p[i];
+    double pi = load_now(p + i);
     if (DIR) {
-      pi = __dadd_rn(__dmul_rn(z[i], 1.0), __dmul_rn(pi, beta));
+      pi = __dadd_rn(__dmul_rn(load_now(z + i), 1.0), __dmul_rn(pi, beta));
       pnew[i] = pi;
     }
     const double mp = __dmul_rn(pi, mi);
@@ -1032,7 +1032,7 @@ __device__ __forceinline__ void mht_rows(const I *__restrict__ pos, const I *__r
 template <typename I>
 __global__ void __launch_bounds__(VEC_THREADS, 4)
 mht_operator_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, double alpha, int64_t abase, int64_t n,
-                    const double *__restrict__ d, const double *__restrict__ mask, const double *__restrict__ z, double *p0, double *p1,
+                    const double *__restrict__ d, const double *__restrict__ mask, const double *z, double *p0, double *p1,
                     double *__restrict__ Ap, double *__restrict__ partials, double *sc, long long *fl) {
   __shared__ double s_red[VEC_THREADS / 32];
   __shared__ int s_flag;
@@ -1067,13 +1067,13 @@ mht_operator_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const 
 constexpr int MHT_RESIDENT = 5;
 __global__ void __launch_bounds__(VEC_THREADS, MHT_RESIDENT)
 mht_residual_kernel(int64_t n, double *sc, long long *fl, double tol, unsigned long long maxiter, const double *p0, const double *p1,
-                    const double *__restrict__ Ap, const double *__restrict__ d, double *__restrict__ x, double *__restrict__ r,
+                    const double *Ap, const double *__restrict__ d, double *__restrict__ x, double *__restrict__ r,
                     double *__restrict__ z, double *__restrict__ partials) {
   __shared__ double s_red[VEC_THREADS / 32];
   __shared__ int s_flag;
   pdl_wait();
   if (fl[FL_DONE] != 0) return;
-  const double *__restrict__ p = reinterpret_cast<const long long *>(sc)[SC_PCUR] != 0 ? p1 : p0;
+  const double *p = reinterpret_cast<const long long *>(sc)[SC_PCUR] != 0 ? p1 : p0;
   const double alpha = sc[SC_ALPHA], malpha = -alpha;
   double rr = 0.0, rz = 0.0;
   const int64_t stride = (int64_t)gridDim.x * VEC_THREADS;
@@ -1084,9 +1084,9 @@ mht_residual_kernel(int64_t n, double *sc, long long *fl, double tol, unsigned l
       const int64_t i = i0 + k * stride;
       const bool in = i < n;
       xv[k] = in ? x[i] : 0.0;
-      pv[k] = in ? p[i] : 0.0;
+      pv[k] = in ? load_now(p + i) : 0.0;  // p and Ap: the operator's pass may still have been writing them
       rv[k] = in ? r[i] : 0.0;
-      av[k] = in ? Ap[i] : 0.0;
+      av[k] = in ? load_now(Ap + i) : 0.0;
       dv[k] = in ? d[i] : 1.0;
     }
 #pragma unroll

@@ -105,15 +105,7 @@ __device__ __forceinline__ double block_sum(double v, double *s_red) {
   return t;  // valid in thread 0
 }
 
-// Ordinary loads, for what the launch in front may still have been writing when this kernel became resident (launch_pdl):
-// the y of a product may be the next one's x, values or dot operand, and its carries are the fix-up kernel's.  The
-// read-only path (ld.global.nc, which __ldg and reads through const __restrict__ compile to) asks that data stays as it is
-// for the kernel's whole lifetime, which begins in front of pdl_wait().
-__device__ __forceinline__ double load_now(const double *p) {
-  double v;
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
+// By load_now: the y of a product may be the next one's x, values or dot operand, and its carries are the fix-up kernel's.
 __device__ __forceinline__ bool skipped(const int *flag) {
   if (flag == nullptr) return false;
   int v;
