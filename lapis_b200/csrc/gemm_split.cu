@@ -76,6 +76,17 @@ __device__ __forceinline__ bool split4(const float (&x)[4], float s, uint2 &hi, 
   lo = make_uint2(__half_as_ushort(l[0]) | (uint32_t)__half_as_ushort(l[1]) << 16, __half_as_ushort(l[2]) | (uint32_t)__half_as_ushort(l[3]) << 16);
   return small;
 }
+// A or B may be what the launch in front has written.
+__device__ __forceinline__ float load_now(const float *p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 load_now4(const float *p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
 // Bound by memory: reads an element once, writes two halves.  Blocks 0 .. 8 panels_a - 1 take 16 rows of A, a warp each;
@@ -83,7 +94,7 @@ __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(
 // the search for the largest and the split.
 template <bool VEC_A, bool VEC_B>
 __global__ void __launch_bounds__(SPLIT_THREADS, 2)
-split_kernel(const float *__restrict__ A, const float *__restrict__ B, Shape sh, Scratch w) {
+split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
   __shared__ uint32_t s_max[SPLIT_THREADS / 32][4][4];
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -102,11 +113,11 @@ split_kernel(const float *__restrict__ A, const float *__restrict__ B, Shape sh,
       for (int i = 0; i < STEPS; ++i) {
         const int k = 128 * i + 4 * lane;
         if (VEC_A) {
-          const float4 q = k < kc ? *reinterpret_cast<const float4 *>(src + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float4 q = k < kc ? load_now4(src + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[i][j] = k + j < kc ? src[k + j] : 0.0f;
+          for (int j = 0; j < 4; ++j) v[i][j] = k + j < kc ? load_now(src + k + j) : 0.0f;
         }
       }
 #pragma unroll
@@ -144,11 +155,11 @@ split_kernel(const float *__restrict__ A, const float *__restrict__ B, Shape sh,
       for (int i = 0; i < STEPS; ++i) {
         const int k = r0 + 128 * i;
         if (VEC_B) {
-          const float4 q = k < kc && col < sh.N ? *reinterpret_cast<const float4 *>(src + (int64_t)k * sh.N) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float4 q = k < kc && col < sh.N ? load_now4(src + (int64_t)k * sh.N) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[i][j] = k < kc && col + j < sh.N ? src[(int64_t)k * sh.N + j] : 0.0f;
+          for (int j = 0; j < 4; ++j) v[i][j] = k < kc && col + j < sh.N ? load_now(src + (int64_t)k * sh.N + j) : 0.0f;
         }
       }
 #pragma unroll

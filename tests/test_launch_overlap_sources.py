@@ -15,6 +15,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
     ("pcg.cu", "mht_rows", {"pos", "crd", "val", "d", "mask"}),
     ("pcg.cu", "mht_operator_kernel", {"pos", "crd", "val", "d", "mask"}),
     ("pcg.cu", "mht_residual_kernel", {"d"}),
+    ("gemm_split.cu", "split_kernel", set()),
 ])
 def test_read_only_path_is_for_what_stays(source, function, constant):
     """`constant`: what no kernel of the solve writes."""
