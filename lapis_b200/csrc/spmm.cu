@@ -162,6 +162,10 @@ spmm_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__r
   }
 }
 
+// Between the warps that feed and those that add, which meet at different places of the code, once a tile each: barrier 1 with a
+// count, because __syncthreads() in one branch of an if is undefined even where the other branch has as many.
+__device__ __forceinline__ void tile_barrier() { asm volatile("barrier.sync 1, %0;" ::"n"(SPMM_LONG_THREADS) : "memory"); }
+
 // The long rows.  A block notes those among its rows (eight neighbours, then the eight gridDim.x * 8 further on, so that
 // neighbouring long rows meet different blocks); at the end the blocks of a cluster divide what they noted, a piece being a row
 // and up to 64 columns: by length, the longest first, 0 1 2 3 3 2 1 0 0 1 .. (too many pieces: each block keeps its own).
@@ -318,13 +322,13 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
         store(0, b0, a0);
         gather(b0, a0);
         columns();
-        __syncthreads();
+        tile_barrier();
         step(p);
         if (p.q >= n) break;
         store(1, b1, a1);
         gather(b1, a1);
         columns();
-        __syncthreads();
+        tile_barrier();
         step(p);
       }
     } else {
@@ -345,7 +349,7 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
         double acc = DCSR ? cin : 0.0;
         bool ended = false;
         while (!ended) {
-          __syncthreads();
+          tile_barrier();
           const double *s = s_prod[buf] + (in ? tid : 0);
           const int left = w_len[p.q] - p.j, m = left < entries ? left : entries;
 #pragma unroll 16
