@@ -13,7 +13,8 @@
 // A slot is written again only behind a meeting that needed every block's reading of it.
 //
 // The launch is cooperative: all blocks are resident, so every wait ends; each is bounded all the same, and a block whose
-// wait runs out sets a flag that ends the others' waits, and the host leaves the system to the passes of pcg.cu.
+// wait runs out sets a flag that ends the others' waits, and the host leaves the system to the passes of pcg.cu.  So it does
+// where the driver refuses the launch, because the context has fewer SMs than the device.
 //
 // us an iteration, in passes and now: 25,600 rows of a 5-point stencil 18.4 and 9.5, 62,500 20 and 11, 160,000 25 and 13.4,
 // 291,600 30 and 15.5; scattered columns, 30,000 rows of 12 21.4 and 16.5, 100,000 of 12 31 and 26, 300,000 of 10 56 and
@@ -285,7 +286,7 @@ bool pcg_grid_fits(int64_t nrows, int64_t nnz) {
   return nrows <= (int64_t)GRID_ROWS * GRID_THREADS * sm_count() && nnz <= 16 * nrows;
 }
 
-// *solved: false where a wait ran out and the system is left to the passes.
+// *solved: false where the launch was refused or a wait ran out and the system is left to the passes.
 int pcg_grid(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x, uint64_t *iters,
              double *relres, bool *solved, cudaStream_t st) {
   const int64_t n = h->nrows, slots = 3 * (int64_t)sm_count();
@@ -313,7 +314,13 @@ int pcg_grid(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, d
   int done = 0;
   uint64_t it = 0;
   do {
-    LAPIS_CUDA_TRY(h->idx_bytes == 4 ? launch_grid<int32_t>(h, s, st) : launch_grid<int64_t>(h, s, st));
+    const cudaError_t e = h->idx_bytes == 4 ? launch_grid<int32_t>(h, s, st) : launch_grid<int64_t>(h, s, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+      cudaGetLastError();
+      *solved = false;
+      return LAPIS_OK;
+    }
+    LAPIS_CUDA_TRY(e);
     s.first = false;
     LAPIS_TRY(lapis_b200_pcg_status(s.sc, &done, &it, relres, st));
     *solved = done != GRID_GAVE_UP;
