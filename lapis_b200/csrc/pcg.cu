@@ -23,6 +23,7 @@
 // Arithmetic follows the emitted element-wise bodies: axpby is (x*a) + (y*b) with
 // separate roundings (examples/pcg_solve.py:30-39), mult is x*y (:41-48).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "common.h"
@@ -1192,14 +1193,15 @@ struct MhtWork {
 
 template <typename I>
 static int mht_operator_launch(const lapis_b200_csr *A, double alpha, const double *d_d, const double *d_mask, const MhtWork &w, cudaStream_t st) {
-  static int per_sm[64] = {0};  // resident blocks, for 4-byte or for 8-byte indices
+  static std::atomic<int> per_sm[64];  // resident blocks, for 4-byte or for 8-byte indices
   const int dev = A->device >= 0 && A->device < 64 ? A->device : 0;
-  if (per_sm[dev] == 0) {
-    int m = 0;
+  int m = per_sm[dev].load(std::memory_order_relaxed);
+  if (m == 0) {
     LAPIS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, mht_operator_kernel<I>, VEC_THREADS, 0));
-    per_sm[dev] = m > 0 && m <= 8 ? m : 4;
+    if (m <= 0 || m > 8) m = 4;
+    per_sm[dev].store(m, std::memory_order_relaxed);
   }
-  const int64_t tiles = (A->nrows + VEC_THREADS - 1) / VEC_THREADS, resident = (int64_t)sm_count() * per_sm[dev];
+  const int64_t tiles = (A->nrows + VEC_THREADS - 1) / VEC_THREADS, resident = (int64_t)sm_count() * m;
   LAPIS_CUDA_TRY(launch_pdl(mht_operator_kernel<I>, (unsigned)(tiles < resident ? tiles : resident), VEC_THREADS, 0, st,
                             static_cast<const I *>(A->pos), static_cast<const I *>(A->crd), A->val, alpha, A->base & ~(int64_t)3, A->nrows, d_d,
                             d_mask, w.z, w.p, w.p1, w.t, w.partials, w.sc, reinterpret_cast<long long *>(w.sc + SC_COUNT)));
