@@ -14,8 +14,8 @@
 //   * tile-aligned shapes (M, N multiples of 128, K of 32): the tcgen05 kernel in gemm_tcgen05.cu, fp32 emulated with three
 //     TF32 products.
 //   * products of either kind that are large enough to pay for a pass over their operands first (split_pays): gemm_split.cu,
-//     fp32 from three fp16 products, with a smaller error than the other two.  What that split does not cover (infinities,
-//     NaN, elements 2^29 times smaller than the largest of their row or column) is left to them, panel by panel.
+//     fp32 from three fp16 or six bf16 products.  What that split does not cover (infinities, NaN, elements 2^29 times smaller
+//     than the largest of their row or column) is left to the other two, panel by panel.
 #include <algorithm>
 #include <cmath>
 

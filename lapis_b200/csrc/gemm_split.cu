@@ -1,30 +1,39 @@
 // fp32 matmul on the 5th-generation tensor cores from operands that are split once:  C[b] = C_in[b] + A[b] B[b]  for any M,
 // N, K and any alignment.
 //
-// x 2^e = hi + 2^-11 lo with hi and lo in fp16 (11 bits each, lo rounded), e one exponent for each row of A and each column
-// of B; the product is hi hi + 2^-11 (hi lo + lo hi), three fp16 products at twice the rate of the three TF32 products of
+// Whole tiles, two parts in fp16:  x 2^e = hi + 2^-11 lo (11 bits each, lo rounded), e one exponent for each row of A and each
+// column of B; the product is hi hi + 2^-11 (hi lo + lo hi), three fp16 products at twice the rate of the three TF32 products of
 // gemm_tcgen05.cu.  What is left out (lo lo, the rounding of lo) is at most 2^-21 of a product as long as hi is a normal fp16
 // number, where the TF32 split, whose parts the tensor core truncates, leaves up to 2^-19.
 //
-//   split_kernel       reads A and B once, writes hi and lo as fp16 matrices with 16-byte rows (so that TMA can load shapes
+// Other shapes, three parts in bf16:  x = b1 + b2 + b3, 8 bits each and signed, which is all 24 bits of x; six products, b1 b1 in
+// one accumulator, the others down to 2^-16 of it (b2 b2, b1 b3) in the second.  What is left out is at most 2^-24 of a product,
+// less than its rounding in the kernel for such shapes, and nothing where one factor has 8 bits: products with a permutation or
+// a selection are exact, as they are there.  With two parts they were not (a quarter of the elements off by a bit).
+//
+//   split_kernel       reads A and B once, writes the parts as 16-bit matrices with 16-byte rows (so that TMA can load shapes
 //                      and pointers of any alignment), and the scales.  K is cut into stretches of at most 1024, each with
 //                      scales of its own.
 //   gemm_split_kernel  a persistent GEMM over the parts: TMA -> tcgen05.mma.kind::f16 -> two accumulators in tensor memory
-//                      (hi hi, and the two mixed products, which are 2^-11 as large) -> scaled, joined, added to C.
+//                      (the large product, and the mixed ones) -> scaled, joined, added to C.
 //
 // 8192^3: 5.05 -> 2.70 ms where the clock holds (407 TFLOP/s, three products at 75 % of cuBLAS's bf16 rate), 5.91 -> 3.33 where
-// power caps it; 5000 x 3000 x 1999 2.05 ms -> 0.21; 1000 x 1501 x 777 142 us -> 30 (a pass over the operands of 5, the
-// product 20, the look at the marks 3: latencies).  Against 64 bits: 8192^3 1.25e-6 (TF32 split 8.0e-6), 1000 x 1501 x 777
-// 3.9e-7 (sequential sum 5.0e-7), 100 x 100 x 130 1.9e-7 (2.1e-7).
+// power caps it, with an error of 1.25e-6 against 64 bits (2-norm; TF32 split 8.0e-6).  Three parts cost 5 to 65 % more time
+// than two: 1000 x 1501 x 777 142 us in the kernel for general shapes, 30.6 with two parts, 35.7 with three; 5000 x 3000 x 1999
+// 2270, 260 and 361; 8191^3 46, 4.3 and 6.1 ms.  Their errors, that kernel's first: 1000 x 1501 x 777 uniform in [-1, 1) 5.0e-7,
+// 3.9e-7 and 1.6e-7, in [0, 1) 4.2e-7, 1.4e-6 and 2.4e-7, A with 1 % nonzeros 6.3e-8, 7.5e-8 and 4.7e-8, 100 x 200^3 2.6e-7,
+// 1.8e-7 and 9.8e-8.
 //
 // fp16 has 5 bits of exponent: the hi of an element below 2^-14 after scaling (2^-29 of the largest of its row or column)
 // would be subnormal and lo lo up to 2^-17 of a product of two such, and an infinity or NaN has no scale.  split_kernel marks
-// the 128-row and 128-column panels that hold such an element; the products of those panels are left to the kernels on unsplit
-// operands (PanelFlags), which run behind this one and return at once where there are none.  In 8192 x 8192 normally
-// distributed numbers one is expected in every second matrix, in uniformly distributed ones (multiples of 2^-24) none.
+// the 128-row and 128-column panels that hold such an element (three parts: below 2^-31); the products of those panels are left to
+// the kernels on unsplit operands (PanelFlags), which run behind this one and return at once where there are none.  In 8192 x
+// 8192 normally distributed numbers one is expected in every second matrix, in uniformly distributed ones (multiples of 2^-24)
+// none.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "tcgen05.h"
@@ -40,14 +49,14 @@ constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f;
 
 struct Shape {
   int M, N, Np, K;          // Np: columns of the split B, a multiple of GROUP_COLS
-  int chain;                 // k blocks of 64 that are added in tensor memory
+  int chain;                 // elements of K that are added in tensor memory, a multiple of 64
   int kc, first, stretches;  // stretches first .. first + stretches - 1, of kc (a multiple of 64) each, the last one shorter
   int panels_a, panels_b;
   __host__ __device__ int length(int s) const { return K - (first + s) * kc < kc ? K - (first + s) * kc : kc; }
 };
 
 struct Scratch {
-  __half *a, *b;             // [batch][stretch][hi, lo][M][kc], [batch][stretch][hi, lo][kc][Np]
+  uint16_t *a, *b;           // [batch][stretch][part][M][kc], [batch][stretch][part][kc][Np]: fp16 or bf16
   float *scale_a, *scale_b;  // [batch][stretch][M], [batch][stretch][Np]: 2^-e
   unsigned char *flag_a, *flag_b;  // [batch][stretch][panels][8]: a byte for every 16 rows or columns
 };
@@ -61,19 +70,33 @@ __device__ __forceinline__ bool scale_exponent(uint32_t max_bits, int &e) {
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
-// hi and lo of four scaled elements; true if one of them is so small that its hi would be subnormal.
-__device__ __forceinline__ bool split4(const float (&x)[4], float s, uint2 &hi, uint2 &lo) {
-  __half h[4], l[4];
+// The parts of four elements, scaled by s where there are two; true if one of them is too small beside the largest of its row
+// or column.  Two parts: its hi would be subnormal.  Three parts hold it, but rows graded like that keep the loop's order.
+template <int PARTS>
+__device__ __forceinline__ bool split4(const float (&x)[4], float s, uint2 (&part)[PARTS]) {
+  uint16_t h[PARTS][4];
   bool small = false;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float v = __fmul_rn(x[i], s);
-    small |= x[i] != 0.0f && fabsf(v) < 1.0f / 16384.0f;
-    h[i] = __float2half_rn(v);
-    l[i] = __float2half_rn(__fmul_rn(__fsub_rn(v, __half2float(h[i])), LO_SCALE));
+    if (PARTS == 2) {
+      small |= x[i] != 0.0f && fabsf(v) < 1.0f / 16384.0f;
+      const __half hi = __float2half_rn(v);
+      h[0][i] = __half_as_ushort(hi);
+      h[1][i] = __half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(v, __half2float(hi)), LO_SCALE)));
+    } else {
+      small |= x[i] != 0.0f && fabsf(v) < 1.0f / 65536.0f;
+      float rest = x[i];
+#pragma unroll
+      for (int q = 0; q < PARTS; ++q) {
+        const __nv_bfloat16 b = __float2bfloat16_rn(rest);
+        h[q][i] = __bfloat16_as_ushort(b);
+        rest = __fsub_rn(rest, __bfloat162float(b));
+      }
+    }
   }
-  hi = make_uint2(__half_as_ushort(h[0]) | (uint32_t)__half_as_ushort(h[1]) << 16, __half_as_ushort(h[2]) | (uint32_t)__half_as_ushort(h[3]) << 16);
-  lo = make_uint2(__half_as_ushort(l[0]) | (uint32_t)__half_as_ushort(l[1]) << 16, __half_as_ushort(l[2]) | (uint32_t)__half_as_ushort(l[3]) << 16);
+#pragma unroll
+  for (int q = 0; q < PARTS; ++q) part[q] = make_uint2(h[q][0] | (uint32_t)h[q][1] << 16, h[q][2] | (uint32_t)h[q][3] << 16);
   return small;
 }
 // A or B may be what the launch in front has written.
@@ -92,7 +115,7 @@ __device__ __forceinline__ uint32_t magnitude(float x) { return __float_as_uint(
 // Bound by memory: reads an element once, writes two halves.  Blocks 0 .. 8 panels_a - 1 take 16 rows of A, a warp each;
 // the others 16 columns of B: four threads a row, 128 rows at a time.  A thread keeps its elements in registers between
 // the search for the largest and the split.
-template <bool VEC_A, bool VEC_B>
+template <int PARTS, bool VEC_A, bool VEC_B>
 __global__ void __launch_bounds__(SPLIT_THREADS, 2)
 split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
   __shared__ uint32_t s_max[SPLIT_THREADS / 32][4][4];
@@ -128,18 +151,18 @@ split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
       int e;
       bad = !scale_exponent(m, e);
       const float sc = pow2(bad ? 0 : e);
-      __half *hi = w.a + ((2 * at) * sh.M + row) * sh.kc, *lo = hi + (int64_t)sh.M * sh.kc;
+      uint16_t *dst = w.a + ((PARTS * at) * sh.M + row) * sh.kc;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
         const int k = 128 * i + 4 * lane;
-        uint2 h, l;
-        bad |= split4(v[i], sc, h, l);
+        uint2 part[PARTS];
+        bad |= split4<PARTS>(v[i], sc, part);
         if (k < kpad) {
-          *reinterpret_cast<uint2 *>(hi + k) = h;
-          *reinterpret_cast<uint2 *>(lo + k) = l;
+#pragma unroll
+          for (int q = 0; q < PARTS; ++q) *reinterpret_cast<uint2 *>(dst + (int64_t)q * sh.M * sh.kc + k) = part[q];
         }
       }
-      if (lane == 0) w.scale_a[at * sh.M + row] = pow2(bad ? 0 : -e);
+      if (PARTS == 2 && lane == 0) w.scale_a[at * sh.M + row] = pow2(bad ? 0 : -e);
     }
     pdl_release();
     const int any = __syncthreads_or(bad);
@@ -186,25 +209,26 @@ split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
         e[j] = no ? 0 : e[j];
         sc[j] = pow2(e[j]);
       }
-      if (tid < 4) {
+      if (PARTS == 2 && tid < 4) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) w.scale_b[at * sh.Np + col + j] = pow2(-e[j]);
       }
-      __half *hi = w.b + (2 * at) * sh.kc * sh.Np + col, *lo = hi + (int64_t)sh.kc * sh.Np;
+      uint16_t *dst = w.b + (PARTS * at) * sh.kc * sh.Np + col;
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
         const int k = r0 + 128 * i;
         float x[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          x[j] = __fmul_rn(v[i][j], sc[j]);
-          bad |= v[i][j] != 0.0f && x[j] == 0.0f;
+          x[j] = PARTS == 2 ? __fmul_rn(v[i][j], sc[j]) : v[i][j];
+          bad |= v[i][j] != 0.0f && (PARTS == 2 ? x[j] == 0.0f : fabsf(__fmul_rn(v[i][j], sc[j])) < 1.0f / 65536.0f);
         }
-        uint2 h, l;
-        bad |= split4(x, 1.0f, h, l);
+        uint2 part[PARTS];
+        const bool small = split4<PARTS>(x, 1.0f, part);  // three parts: seen above
+        bad |= PARTS == 2 && small;
         if (k < kpad) {
-          *reinterpret_cast<uint2 *>(hi + (int64_t)k * sh.Np) = h;
-          *reinterpret_cast<uint2 *>(lo + (int64_t)k * sh.Np) = l;
+#pragma unroll
+          for (int q = 0; q < PARTS; ++q) *reinterpret_cast<uint2 *>(dst + ((int64_t)q * sh.kc + k) * sh.Np) = part[q];
         }
       }
     }
@@ -222,14 +246,15 @@ constexpr int TILE_BYTES = 32 * 32 * 4;      // an epilogue warp's staging tile
 
 // CTAS CTAs own a tile of 128 CTAS x BN: each loads its 128 rows of A and its share of B's columns, the first one issues the
 // MMAs for all.  In tensor memory: hi hi and mixed products of a tile, 2 BN columns, once or twice.
-template <int CTAS_, int BN_>
+template <int PARTS_, int CTAS_, int BN_>
 struct Config {
-  static constexpr int CTAS = CTAS_, BN = BN_, BUFS = 256 / BN, NB = BN / CTAS;
-  static constexpr int A_BYTES = tc::BM * BK * 2, B_BYTES = NB * BK * 2;  // of hi or lo
-  static constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES), STAGES = 196608 / STAGE_BYTES;
+  static constexpr int PARTS = PARTS_, CTAS = CTAS_, BN = BN_, BUFS = 256 / BN, NB = BN / CTAS;
+  static constexpr int A_BYTES = tc::BM * BK * 2, B_BYTES = NB * BK * 2;  // of a part
+  static constexpr int STAGE_BYTES = PARTS * (A_BYTES + B_BYTES), STAGES = 196608 / STAGE_BYTES;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 8 * TILE_BYTES + 256;
-  // D = f32, A and B = f16, A K-major, B MN-major
-  static constexpr uint32_t IDESC = (1u << 4) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(tc::BM * CTAS >> 4) << 24);
+  static constexpr uint32_t TYPE = PARTS == 2 ? 0 : 1;  // f16, bf16
+  // D = f32, A and B of TYPE, A K-major, B MN-major
+  static constexpr uint32_t IDESC = (1u << 4) | (TYPE << 7) | (TYPE << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(tc::BM * CTAS >> 4) << 24);
   static_assert(NB % 64 == 0 && 4 * BN * BUFS == 1024 && SMEM_BYTES <= 232448, "tile");
 };
 
@@ -325,20 +350,24 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
                  "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
 
-// In shared memory, of 128 bytes a cycle: <2, 256> 43 written by TMA and 64 read by the tensor core, <2, 128> 64 and 96,
+// Two parts, in shared memory, of 128 bytes a cycle: <2, 256> 43 written by TMA and 64 read by the tensor core, <2, 128> 64 and 96,
 // <1, 128> 85 and 128.  The first is for many tiles; its accumulators fill tensor memory, so the sums are drained to registers
 // (eight warps, 128 columns a thread) before the epilogue touches C, the mixed products first, because the next chain
-// starts with those.  The others hold two tiles and give a small product more of them.
+// starts with those.  The others hold two tiles and give a small product more of them.  Three parts: <1, 128>, whose 24 MMAs a
+// k block (32 cycles each) wait for 96 KB from L2.
 //
 // The tensor core truncates when it adds to its accumulator, an error that grows with the length of the chain (chain / 16
-// additions, 2^-25 of the partial sum each on average); sh.chain k blocks are added there, the rest in registers, rounded.
+// additions, 2^-25 of the partial sum each on average); sh.chain of K are added there, the rest in registers, rounded.  For
+// operands of one sign that is the largest error: chains of 9 sqrt(K) keep it below the sequential sum's (K = 8189 1.08e-6 and
+// 1.19e-6, K = 777 2.4e-7 and 4.2e-7; with 13 sqrt(K) 1.70e-6 and 4.1e-7).
 template <typename C_>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, float *__restrict__ C, Shape sh,
                   Scratch w, PanelFlags flags, int tiles, bool vec, int *__restrict__ error_flag) {
-  constexpr int CTAS = C_::CTAS, BN = C_::BN, BUFS = C_::BUFS, NB = C_::NB, A_BYTES = C_::A_BYTES, B_BYTES = C_::B_BYTES,
+  constexpr int PARTS = C_::PARTS, CTAS = C_::CTAS, BN = C_::BN, BUFS = C_::BUFS, NB = C_::NB, A_BYTES = C_::A_BYTES, B_BYTES = C_::B_BYTES,
                 STAGE_BYTES = C_::STAGE_BYTES, STAGES = C_::STAGES, COLS = BN / 2;  // COLS: of an epilogue thread
   constexpr uint32_t IDESC = C_::IDESC;
+  const int chain = sh.chain / BK;  // k blocks
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES + 8 * TILE_BYTES);
@@ -406,7 +435,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const tc::TileCoord c = coord(t);
         for (int s = 0; s < sh.stretches && ok; ++s) {
           if (skipped(c, s)) continue;
-          const int z = 2 * (c.batch * sh.stretches + s), nk = (sh.length(s) + BK - 1) / BK;
+          const int z = PARTS * (c.batch * sh.stretches + s), nk = (sh.length(s) + BK - 1) / BK;
           for (int kb = 0; kb < nk; ++kb, ++g) {
             const int st = g % STAGES;
             ok = tc::mbar_wait(&empty[st], ((g / STAGES) & 1) ^ 1);
@@ -415,11 +444,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const uint32_t bar = leader_addr<CTAS>(&full[st]);
             uint8_t *p = smem + st * STAGE_BYTES;
 #pragma unroll
-            for (int part = 0; part < 2; ++part) {
+            for (int part = 0; part < PARTS; ++part) {
               load<CTAS>(p + part * A_BYTES, &map_a, bar, kb * BK, c.m0 + 128 * rank, z + part);
 #pragma unroll
               for (int j = 0; j < NB / 64; ++j)
-                load<CTAS>(p + 2 * A_BYTES + part * B_BYTES + j * BOX_BYTES, &map_b, bar, c.n0 + NB * rank + 64 * j, kb * BK, z + part);
+                load<CTAS>(p + PARTS * A_BYTES + part * B_BYTES + j * BOX_BYTES, &map_b, bar, c.n0 + NB * rank + 64 * j, kb * BK, z + part);
             }
           }
         }
@@ -436,7 +465,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (skipped(c, s)) continue;
           const int nk = (sh.length(s) + BK - 1) / BK;
           for (int kb = 0; kb < nk && ok; ++it) {  // chains
-            const int end = nk - kb < sh.chain ? nk : kb + sh.chain;
+            const int end = nk - kb < chain ? nk : kb + chain;
             const uint32_t buf = it % BUFS, phase = (it / BUFS) & 1;
             const uint32_t d_main = tmem + buf * 2 * BN, d_mixed = d_main + BN;
             ok = tc::mbar_wait_cluster(&mixed_empty[buf], phase ^ 1);
@@ -448,11 +477,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               if (!ok) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
               const uint32_t p = tc::smem_u32(smem + st * STAGE_BYTES);
-              const uint64_t a_hi = desc_a(p), a_lo = desc_a(p + A_BYTES), b_hi = desc_b(p + 2 * A_BYTES), b_lo = desc_b(p + 2 * A_BYTES + B_BYTES);
+              uint64_t a[PARTS], b[PARTS];
+#pragma unroll
+              for (int q = 0; q < PARTS; ++q) {
+                a[q] = desc_a(p + q * A_BYTES);
+                b[q] = desc_b(p + PARTS * A_BYTES + q * B_BYTES);
+              }
 #pragma unroll
               for (int ks = 0; ks < BK / 16; ++ks) {  // 32 bytes of a row of A, two groups of 8 k-rows of B
-                mma<CTAS>(d_mixed, a_hi + 2 * ks, b_lo + 128 * ks, IDESC, !first || ks > 0);
-                mma<CTAS>(d_mixed, a_lo + 2 * ks, b_hi + 128 * ks, IDESC, true);
+                if (PARTS == 3) {
+                  mma<CTAS>(d_mixed, a[0] + 2 * ks, b[PARTS - 1] + 128 * ks, IDESC, !first || ks > 0);
+                  mma<CTAS>(d_mixed, a[PARTS - 1] + 2 * ks, b[0] + 128 * ks, IDESC, true);
+                  mma<CTAS>(d_mixed, a[1] + 2 * ks, b[1] + 128 * ks, IDESC, true);
+                }
+                mma<CTAS>(d_mixed, a[0] + 2 * ks, b[1] + 128 * ks, IDESC, PARTS == 3 || !first || ks > 0);
+                mma<CTAS>(d_mixed, a[1] + 2 * ks, b[0] + 128 * ks, IDESC, true);
               }
               if (first) {
                 ok = tc::mbar_wait_cluster(&main_empty[buf], phase ^ 1);
@@ -460,7 +499,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
               }
 #pragma unroll
-              for (int ks = 0; ks < BK / 16; ++ks) mma<CTAS>(d_main, a_hi + 2 * ks, b_hi + 128 * ks, IDESC, !first || ks > 0);
+              for (int ks = 0; ks < BK / 16; ++ks) mma<CTAS>(d_main, a[0] + 2 * ks, b[0] + 128 * ks, IDESC, !first || ks > 0);
               commit<CTAS>(&empty[st]);
             }
             if (ok) commit<CTAS>(&acc_full[buf]);
@@ -471,6 +510,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
+    constexpr float MIXED = PARTS == 2 ? LO_UNSCALE : 1.0f;  // weight of the mixed products
     constexpr int DEPTH = COLS == 128 ? 4 : 8;  // requests for C in flight: what the registers beside the sums allow
     const int q = warp & 3, half = (warp - 4) >> 2;  // lanes 32 q .. of tensor memory, columns COLS * half ..
     float *stile = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES) + (warp - 4) * 32 * 32;
@@ -485,10 +525,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const float *scale_a = w.scale_a + at * sh.M, *scale_b = w.scale_b + at * sh.Np;
         const unsigned long long mark_a = row_in ? load_flag(flags.row(c.batch, s) + m0 / 128) : 1;
         const unsigned long long mark_b = col_in ? load_flag(flags.col(c.batch, s) + col0 / 128) : 1;
-        const float fa = row0 + lane < sh.M ? load_scale(scale_a + row0 + lane) : 0.0f;
+        const float fa = PARTS == 3 ? 1.0f : row0 + lane < sh.M ? load_scale(scale_a + row0 + lane) : 0.0f;
         float fb[COLS / 32];  // of the columns 32 ch + lane
 #pragma unroll
-        for (int ch = 0; ch < COLS / 32; ++ch) fb[ch] = col0 + 32 * ch + lane < sh.N ? load_scale(scale_b + col0 + 32 * ch + lane) : 0.0f;
+        for (int ch = 0; ch < COLS / 32; ++ch)
+          fb[ch] = PARTS == 3 ? 1.0f : col0 + 32 * ch + lane < sh.N ? load_scale(scale_b + col0 + 32 * ch + lane) : 0.0f;
         if (skipped(c, s)) continue;
         const bool mine = (mark_a | mark_b) == 0;
         if (s == 0 && mine && row0 + lane < sh.M) {  // C into L2 while the product is computed
@@ -498,7 +539,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (cols > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + cols - 1));
         }
         uint32_t acc[COLS / 16][16];
-        for (int kb = 0, nk = (sh.length(s) + BK - 1) / BK; kb < nk; kb += sh.chain, ++it) {
+        for (int kb = 0, nk = (sh.length(s) + BK - 1) / BK; kb < nk; kb += chain, ++it) {
           const uint32_t buf = it % BUFS;
           ok = tc::mbar_wait(&acc_full[buf], (it / BUFS) & 1);
           if (!ok) break;
@@ -511,7 +552,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (int i = 0; i < COLS / 16; ++i) {
               tmem_wait(acc[i]);
 #pragma unroll
-              for (int j = 0; j < 16; ++j) acc[i][j] = __float_as_uint(__fmul_rn(__uint_as_float(acc[i][j]), LO_UNSCALE));
+              for (int j = 0; j < 16; ++j) acc[i][j] = __float_as_uint(__fmul_rn(__uint_as_float(acc[i][j]), MIXED));
             }
           } else {
 #pragma unroll
@@ -521,7 +562,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               tmem_wait(r);
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                acc[i][j] = __float_as_uint(__fmaf_rn(__uint_as_float(r[j]), LO_UNSCALE, __uint_as_float(acc[i][j])));
+                acc[i][j] = __float_as_uint(__fmaf_rn(__uint_as_float(r[j]), MIXED, __uint_as_float(acc[i][j])));
             }
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -641,9 +682,34 @@ static int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float
   return LAPIS_OK;
 }
 
-using Wide = Config<2, 256>;
-using Pair = Config<2, 128>;
-using Single = Config<1, 128>;
+// With PARTS = 2 or 3.
+template <int PARTS>
+static int launch_tiles(int64_t M, int64_t N, int64_t group_b, int64_t nb, const float *A, const float *B, float *C, const Shape &sh,
+                        const Scratch &w, const PanelFlags &flags, int *error_flag, int dev, cudaStream_t st) {
+  const int64_t K = sh.K;
+  const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, vec_b = N % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  const bool vec_c = N % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
+  const dim3 grid((unsigned)(8 * (sh.panels_a + sh.panels_b)), (unsigned)sh.stretches, (unsigned)nb);
+  auto kernel = vec_a ? (vec_b ? split_kernel<PARTS, true, true> : split_kernel<PARTS, true, false>)
+                      : (vec_b ? split_kernel<PARTS, false, true> : split_kernel<PARTS, false, false>);
+  LAPIS_CUDA_TRY(launch_pdl(kernel, grid, SPLIT_THREADS, 0, st, A, B, sh, w));
+  CUtensorMap map_a, map_b;
+  const int64_t parts = PARTS * nb * sh.stretches;
+  const CUtensorMapDataType type = PARTS == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  LAPIS_TRY(tc::make_map(&map_a, type, w.a, parts, M, sh.kc, 2 * (int64_t)sh.kc, tc::BM, BK, CU_TENSOR_MAP_SWIZZLE_128B));
+  LAPIS_TRY(tc::make_map(&map_b, type, w.b, parts, sh.kc, sh.Np, 2 * (int64_t)sh.Np, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+  auto count = [&](int64_t rows, int64_t cols) { return ((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
+  if (PARTS == 3)  // six products of what a CTA loads: pairs, which load half of B each, are no faster (1000 x 1501 x 777 36.8, single 35.7 us)
+    return launch_gemm<Config<3, 1, 128>>(map_a, map_b, C, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st);
+  // rounds of tiles that the busiest SM works through, by what one takes
+  const int64_t sms = sm_count();
+  auto cost = [&](int64_t n, int64_t at_once, int64_t each) { return (n * group_b + at_once - 1) / at_once * each; };
+  const int64_t wide = cost(count(256, 256), sms / 2, 128), pair = cost(count(256, 128), sms / 2, 80), single = cost(count(128, 128), sms, 107);
+  if (wide < pair && wide < single)
+    return launch_gemm<Config<2, 2, 256>>(map_a, map_b, C, sh, w, flags, nb * count(256, 256), vec_c, error_flag, dev, st);
+  if (pair < single) return launch_gemm<Config<2, 2, 128>>(map_a, map_b, C, sh, w, flags, nb * count(256, 128), vec_c, error_flag, dev, st);
+  return launch_gemm<Config<2, 1, 128>>(map_a, map_b, C, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st);
+}
 
 }  // namespace split
 
@@ -669,7 +735,8 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
   sh.Np = (int)((N + GROUP_COLS - 1) / GROUP_COLS * GROUP_COLS);
   sh.panels_a = (int)((M + 127) / 128);
   sh.panels_b = (int)((N + 127) / 128);
-  sh.chain = exact_order ? std::min(KC / BK, std::max(2, (int)(std::sqrt((double)K) / 5))) : KC / BK;
+  sh.chain = exact_order ? std::min(KC, 64 * std::max(1, (int)(std::sqrt((double)K) / 7))) : KC;
+  const int parts = exact_order ? 3 : 2;
   int64_t all = 0;  // stretches of K
   size_t per = 0;   // bytes of a stretch: parts, scales, flags, each from a 256-byte boundary
   size_t bytes_a = 0, bytes_b = 0;
@@ -677,8 +744,8 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
     all = (K + longest - 1) / longest;
     sh.kc = (int)(((K + all - 1) / all + 63) / 64 * 64);
     all = (K + sh.kc - 1) / sh.kc;
-    bytes_a = (size_t)4 * M * sh.kc;
-    bytes_b = (size_t)4 * sh.kc * sh.Np;
+    bytes_a = (size_t)2 * parts * M * sh.kc;
+    bytes_b = (size_t)2 * parts * sh.kc * sh.Np;
     per = bytes_a + bytes_b + 4 * (size_t)(M + sh.Np) + 8 * (size_t)(sh.panels_a + sh.panels_b);
     if (per <= SPLIT_BYTES) break;
   }
@@ -695,15 +762,8 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
     return LAPIS_OK;
   }
   uint8_t *p = static_cast<uint8_t *>(buf.p);
-  Scratch w = {reinterpret_cast<__half *>(p), reinterpret_cast<__half *>(p + off_b), reinterpret_cast<float *>(p + off_sa),
+  Scratch w = {reinterpret_cast<uint16_t *>(p), reinterpret_cast<uint16_t *>(p + off_b), reinterpret_cast<float *>(p + off_sa),
                reinterpret_cast<float *>(p + off_sb), p + off_fa, p + off_fb};
-  const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, vec_b = N % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
-  const bool vec_c = N % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
-  auto count = [&](int64_t rows, int64_t cols) { return ((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
-  // rounds of tiles that the busiest SM works through, by what one takes
-  const int64_t sms = sm_count();
-  auto cost = [&](int64_t n, int64_t at_once, int64_t each) { return (n * group_b + at_once - 1) / at_once * each; };
-  const int64_t wide = cost(count(256, 256), sms / 2, 128), pair = cost(count(256, 128), sms / 2, 80), single = cost(count(128, 128), sms, 107);
   for (int64_t b0 = 0; b0 < batch; b0 += group_b) {
     const int64_t nb = std::min(group_b, batch - b0);
     const float *Ab = A + b0 * M * K, *Bb = B + b0 * K * N;
@@ -711,22 +771,10 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
     for (int64_t s0 = 0; s0 < all; s0 += group_s) {
       sh.first = (int)s0;
       sh.stretches = (int)std::min(group_s, all - s0);
-      const dim3 grid((unsigned)(8 * (sh.panels_a + sh.panels_b)), (unsigned)sh.stretches, (unsigned)nb);
-      auto kernel = vec_a ? (vec_b ? split_kernel<true, true> : split_kernel<true, false>)
-                          : (vec_b ? split_kernel<false, true> : split_kernel<false, false>);
-      LAPIS_CUDA_TRY(launch_pdl(kernel, grid, SPLIT_THREADS, 0, st, Ab, Bb, sh, w));
-      CUtensorMap map_a, map_b;
-      const int64_t parts = 2 * nb * sh.stretches;
-      LAPIS_TRY(tc::make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.a, parts, M, sh.kc, 2 * (int64_t)sh.kc, tc::BM, BK, CU_TENSOR_MAP_SWIZZLE_128B));
-      LAPIS_TRY(tc::make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, w.b, parts, sh.kc, sh.Np, 2 * (int64_t)sh.Np, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B));
       const PanelFlags flags = {reinterpret_cast<const unsigned long long *>(w.flag_a), reinterpret_cast<const unsigned long long *>(w.flag_b),
                                 sh.panels_a, sh.panels_b, sh.stretches, sh.kc};
-      if (wide < pair && wide < single)
-        LAPIS_TRY(launch_gemm<Wide>(map_a, map_b, Cb, sh, w, flags, nb * count(256, 256), vec_c, error_flag, dev, st));
-      else if (pair < single)
-        LAPIS_TRY(launch_gemm<Pair>(map_a, map_b, Cb, sh, w, flags, nb * count(256, 128), vec_c, error_flag, dev, st));
-      else
-        LAPIS_TRY(launch_gemm<Single>(map_a, map_b, Cb, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st));
+      LAPIS_TRY(parts == 2 ? launch_tiles<2>(M, N, group_b, nb, Ab, Bb, Cb, sh, w, flags, error_flag, dev, st)
+                           : launch_tiles<3>(M, N, group_b, nb, Ab, Bb, Cb, sh, w, flags, error_flag, dev, st));
       LAPIS_TRY(bgemm_unsplit_panels(nb, M, N, K, Ab, Bb, Cb, flags, (int)s0, st));
     }
   }
