@@ -72,152 +72,149 @@ constexpr int SG_STAGES = 3;  // slabs in shared memory
 // 16-byte boundaries the slabs travel in 4-byte copies (2000 x 2001 x 2002: 21 TFLOP/s).
 //
 // One block owns a BM x BN tile of C, a thread TM rows (BM / TM apart) by TN columns (groups of four, 4 BN / TN apart).
-template <int BM, int BN, int TM, int TN, int MINB>
+template <int BM, int BN, int TM, int TN, int MINB, bool MARKED>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB)
 bgemm_simt_kernel(int64_t batch, int64_t M, int64_t N, int64_t K, const float *__restrict__ A0,
-                  const float *__restrict__ B0, float *__restrict__ C0, bool vec_a, bool vec_b, uint64_t minus_zero, PanelFlags flags,
-                  int first) {
+                  const float *__restrict__ B0, float *__restrict__ C0, bool vec_a, bool vec_b, uint64_t minus_zero, PanelFlags flags) {
   constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY, PITCH = SG_K + 4;
   static_assert(TN % 4 == 0 && THREADS % 32 == 0 && THREADS >= BN / 4, "tile");
   __shared__ __align__(16) float sA[SG_STAGES][BM][PITCH];
   __shared__ __align__(16) float sB[SG_STAGES][SG_K][BN];
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int64_t row0 = (int64_t)blockIdx.y * BM, col0 = (int64_t)blockIdx.x * BN;
+  const int nslab = (int)((K + SG_K - 1) / SG_K);
   static_assert(128 % BM == 0 && 128 % BN == 0, "a tile lies in one panel of rows and one of columns");
-  // With marks of one stretch: the inputs and the marks were there before the kernel in front let this one start, and that
-  // kernel leaves the marked elements of C alone.  With several it adds the stretches that are not marked to them.
-  const bool beside = flags.a != nullptr && flags.stretches == 1;
-  if (!beside) pdl_wait();
-  const int stretches = flags.a != nullptr ? flags.stretches : 1;
+  if (!MARKED) pdl_wait();
   for (int64_t b = blockIdx.z; b < batch; b += gridDim.z) {
-    for (int s = 0; s < stretches; ++s) {
-      int64_t k_lo = 0, k_hi = K;
-      if (flags.a != nullptr) {  // only what is marked, a stretch at a time
-        if ((flags.row(b, s)[row0 / 128] | flags.col(b, s)[col0 / 128]) == 0) continue;
-        k_lo = (int64_t)(first + s) * flags.kc;
-        k_hi = K < k_lo + flags.kc ? K : k_lo + flags.kc;
-      }
-      const int nslab = (int)((k_hi - k_lo + SG_K - 1) / SG_K);
-      const float *A = A0 + b * M * K;
-      const float *B = B0 + b * K * N;
-      float *C = C0 + b * M * N;
-      auto load = [&](int slab) {
-        if (slab < nslab) {
-          const int st = slab % SG_STAGES;
-          const int64_t k0 = k_lo + (int64_t)slab * SG_K;
-          if (vec_a) {
-            constexpr int Q = SG_K / 4;
-            const int c = 4 * (tid % Q);
-#pragma unroll
-            for (int i = 0; i < (BM * Q + THREADS - 1) / THREADS; ++i) {
-              const int r = tid / Q + i * (THREADS / Q);
-              const bool in = row0 + r < M && k0 + c < k_hi;
-              if (BM * Q % THREADS == 0 || r < BM) copy_async<16>(&sA[st][r][c], in ? A + (row0 + r) * K + k0 + c : A, in);
-            }
-          } else {
-            const int c = tid % SG_K;
-#pragma unroll
-            for (int i = 0; i < BM * SG_K / THREADS; ++i) {
-              const int r = tid / SG_K + i * (THREADS / SG_K);
-              const bool in = row0 + r < M && k0 + c < k_hi;
-              copy_async<4>(&sA[st][r][c], in ? A + (row0 + r) * K + k0 + c : A, in);
-            }
-          }
-          if (vec_b) {
-            constexpr int Q = BN / 4;
-            const int c = 4 * (tid % Q);
-#pragma unroll
-            for (int i = 0; i < (SG_K * Q + THREADS - 1) / THREADS; ++i) {
-              const int r = tid / Q + i * (THREADS / Q);
-              const bool in = k0 + r < k_hi && col0 + c < N;
-              if (SG_K * Q % THREADS == 0 || r < SG_K) copy_async<16>(&sB[st][r][c], in ? B + (k0 + r) * N + col0 + c : B, in);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < SG_K * BN / THREADS; ++i) {
-              const int e = tid + i * THREADS, r = e / BN, c = e % BN;
-              const bool in = k0 + r < k_hi && col0 + c < N;
-              copy_async<4>(&sB[st][r][c], in ? B + (k0 + r) * N + col0 + c : B, in);
-            }
-          }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      };
-      uint64_t acc[TM][TN / 2];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
-#pragma unroll
-      for (int s = 0; s < SG_STAGES - 1; ++s) load(s);
-      for (int slab = 0; slab < nslab; ++slab) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(SG_STAGES - 2) : "memory");
-        __syncthreads();
-        load(slab + SG_STAGES - 1);  // into the stage that every thread has left
+    // MARKED: only what is marked in any stretch of K, over all of K.  The inputs and the marks were there before the kernel in
+    // front let this one start, and that kernel leaves the marked elements of C alone.
+    if (MARKED) {
+      bool any = false;
+      for (int s = tid; s < flags.stretches; s += THREADS) any |= (flags.row(b, s)[row0 / 128] | flags.col(b, s)[col0 / 128]) != 0;
+      if (!__syncthreads_or(any)) continue;
+    }
+    const float *A = A0 + b * M * K;
+    const float *B = B0 + b * K * N;
+    float *C = C0 + b * M * N;
+    auto load = [&](int slab) {
+      if (slab < nslab) {
         const int st = slab % SG_STAGES;
+        const int64_t k0 = (int64_t)slab * SG_K;
+        if (vec_a) {
+          constexpr int Q = SG_K / 4;
+          const int c = 4 * (tid % Q);
 #pragma unroll
-        for (int k4 = 0; k4 < SG_K; k4 += 4) {
-          float4 a[TM];
+          for (int i = 0; i < (BM * Q + THREADS - 1) / THREADS; ++i) {
+            const int r = tid / Q + i * (THREADS / Q);
+            const bool in = row0 + r < M && k0 + c < K;
+            if (BM * Q % THREADS == 0 || r < BM) copy_async<16>(&sA[st][r][c], in ? A + (row0 + r) * K + k0 + c : A, in);
+          }
+        } else {
+          const int c = tid % SG_K;
 #pragma unroll
-          for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4 *>(&sA[st][ty + i * TY][k4]);
+          for (int i = 0; i < BM * SG_K / THREADS; ++i) {
+            const int r = tid / SG_K + i * (THREADS / SG_K);
+            const bool in = row0 + r < M && k0 + c < K;
+            copy_async<4>(&sA[st][r][c], in ? A + (row0 + r) * K + k0 + c : A, in);
+          }
+        }
+        if (vec_b) {
+          constexpr int Q = BN / 4;
+          const int c = 4 * (tid % Q);
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            ulonglong2 bb[TN / 4];
+          for (int i = 0; i < (SG_K * Q + THREADS - 1) / THREADS; ++i) {
+            const int r = tid / Q + i * (THREADS / Q);
+            const bool in = k0 + r < K && col0 + c < N;
+            if (SG_K * Q % THREADS == 0 || r < SG_K) copy_async<16>(&sB[st][r][c], in ? B + (k0 + r) * N + col0 + c : B, in);
+          }
+        } else {
 #pragma unroll
-            for (int j = 0; j < TN / 4; ++j)
-              bb[j] = *reinterpret_cast<const ulonglong2 *>(&sB[st][k4 + kk][4 * tx + 4 * TX * j]);
-#pragma unroll
-            for (int i = 0; i < TM; ++i) {
-              const float av = kk == 0 ? a[i].x : kk == 1 ? a[i].y : kk == 2 ? a[i].z : a[i].w;
-              const uint64_t aa = pack2(av, av);
-#pragma unroll
-              for (int j = 0; j < TN / 4; ++j) {
-                acc[i][2 * j] = add2(acc[i][2 * j], mul2(aa, bb[j].x, minus_zero));
-                acc[i][2 * j + 1] = add2(acc[i][2 * j + 1], mul2(aa, bb[j].y, minus_zero));
-              }
-            }
+          for (int i = 0; i < SG_K * BN / THREADS; ++i) {
+            const int e = tid + i * THREADS, r = e / BN, c = e % BN;
+            const bool in = k0 + r < K && col0 + c < N;
+            copy_async<4>(&sB[st][r][c], in ? B + (k0 + r) * N + col0 + c : B, in);
           }
         }
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();  // the stages are free for the next problem
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint64_t acc[TM][TN / 2];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        const int64_t gr = row0 + ty + i * TY;
-        if (gr >= M) break;
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN / 4; ++j) {
-          const int64_t gc = col0 + 4 * tx + 4 * TX * j;
-          float o[4];
-          unpack2(acc[i][2 * j], o[0], o[1]);
-          unpack2(acc[i][2 * j + 1], o[2], o[3]);
-          float *c = C + gr * N + gc;
-          if (vec_b) {
-            if (gc < N) {
-              const float4 cin = *reinterpret_cast<const float4 *>(c);
-              *reinterpret_cast<float4 *>(c) =
-                  make_float4(__fadd_rn(o[0], cin.x), __fadd_rn(o[1], cin.y), __fadd_rn(o[2], cin.z), __fadd_rn(o[3], cin.w));
+      for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0;
+#pragma unroll
+    for (int s = 0; s < SG_STAGES - 1; ++s) load(s);
+    for (int slab = 0; slab < nslab; ++slab) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(SG_STAGES - 2) : "memory");
+      __syncthreads();
+      load(slab + SG_STAGES - 1);  // into the stage that every thread has left
+      const int st = slab % SG_STAGES;
+#pragma unroll
+      for (int k4 = 0; k4 < SG_K; k4 += 4) {
+        float4 a[TM];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4 *>(&sA[st][ty + i * TY][k4]);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          ulonglong2 bb[TN / 4];
+#pragma unroll
+          for (int j = 0; j < TN / 4; ++j)
+            bb[j] = *reinterpret_cast<const ulonglong2 *>(&sB[st][k4 + kk][4 * tx + 4 * TX * j]);
+#pragma unroll
+          for (int i = 0; i < TM; ++i) {
+            const float av = kk == 0 ? a[i].x : kk == 1 ? a[i].y : kk == 2 ? a[i].z : a[i].w;
+            const uint64_t aa = pack2(av, av);
+#pragma unroll
+            for (int j = 0; j < TN / 4; ++j) {
+              acc[i][2 * j] = add2(acc[i][2 * j], mul2(aa, bb[j].x, minus_zero));
+              acc[i][2 * j + 1] = add2(acc[i][2 * j + 1], mul2(aa, bb[j].y, minus_zero));
             }
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (gc + q < N) c[q] = __fadd_rn(o[q], c[q]);
           }
         }
       }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the stages are free for the next problem
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int64_t gr = row0 + ty + i * TY;
+      if (gr >= M) break;
+#pragma unroll
+      for (int j = 0; j < TN / 4; ++j) {
+        const int64_t gc = col0 + 4 * tx + 4 * TX * j;
+        float o[4];
+        unpack2(acc[i][2 * j], o[0], o[1]);
+        unpack2(acc[i][2 * j + 1], o[2], o[3]);
+        float *c = C + gr * N + gc;
+        if (vec_b) {
+          if (gc < N) {
+            const float4 cin = *reinterpret_cast<const float4 *>(c);
+            *reinterpret_cast<float4 *>(c) =
+                make_float4(__fadd_rn(o[0], cin.x), __fadd_rn(o[1], cin.y), __fadd_rn(o[2], cin.z), __fadd_rn(o[3], cin.w));
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (gc + q < N) c[q] = __fadd_rn(o[q], c[q]);
+        }
+      }
+    }
   }
-  if (beside && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();  // what follows in the stream waits for both
+  if (MARKED && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();  // what follows in the stream waits for both
 }
 
 template <int BM, int BN, int TM, int TN, int MINB>
 static cudaError_t launch_simt(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C,
-                               const PanelFlags &flags, int first, cudaStream_t st) {
+                               const PanelFlags &flags, cudaStream_t st) {
   const dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM), (unsigned)(batch < 65535 ? batch : 65535));
   const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0;
   const bool vec_b = N % 4 == 0 && (reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) % 16 == 0;
-  return launch_pdl(bgemm_simt_kernel<BM, BN, TM, TN, MINB>, grid, (BM / TM) * (BN / TN), 0, st, batch, M, N, K, A, B, C, vec_a, vec_b,
-                    0x8000000080000000ull, flags, first);
+  if (flags.a != nullptr)
+    return launch_pdl(bgemm_simt_kernel<BM, BN, TM, TN, MINB, true>, grid, (BM / TM) * (BN / TN), 0, st, batch, M, N, K, A, B, C, vec_a, vec_b,
+                      0x8000000080000000ull, flags);
+  return launch_pdl(bgemm_simt_kernel<BM, BN, TM, TN, MINB, false>, grid, (BM / TM) * (BN / TN), 0, st, batch, M, N, K, A, B, C, vec_a, vec_b,
+                    0x8000000080000000ull, flags);
 }
 
 // Tile by the time the busiest SM needs for a k-slab of its tiles: `slab` us each when it has several to overlap,
@@ -225,7 +222,7 @@ static cudaError_t launch_simt(int64_t batch, int64_t M, int64_t N, int64_t K, c
 struct GeneralTile {
   int bm, bn;
   float slab, alone;
-  cudaError_t (*launch)(int64_t, int64_t, int64_t, int64_t, const float *, const float *, float *, const PanelFlags &, int, cudaStream_t);
+  cudaError_t (*launch)(int64_t, int64_t, int64_t, int64_t, const float *, const float *, float *, const PanelFlags &, cudaStream_t);
 };
 static constexpr GeneralTile general_tiles[] = {{64, 64, 0.706f, 0.92f, launch_simt<64, 64, 4, 8, 4>},
                                                 {64, 32, 0.403f, 0.55f, launch_simt<64, 32, 4, 4, 5>},
@@ -247,8 +244,8 @@ static TileChoice general_tile(int64_t batch, int64_t M, int64_t N) {
 }
 
 static int launch_general(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
-                          int first, cudaStream_t st) {
-  LAPIS_CUDA_TRY(general_tile(batch, M, N).tile->launch(batch, M, N, K, A, B, C, flags, first, st));
+                          cudaStream_t st) {
+  LAPIS_CUDA_TRY(general_tile(batch, M, N).tile->launch(batch, M, N, K, A, B, C, flags, st));
   return LAPIS_OK;
 }
 
@@ -258,11 +255,15 @@ static bool whole_tiles(int64_t batch, int64_t M, int64_t N, int64_t K, const fl
          bgemm_tcgen05_supported(batch, M, N, K);
 }
 
-// What a product from split operands leaves out: the marked panels of `count` stretches of K from `first`.
+// What a product from split operands leaves out.  Whole tiles: the marked panels of the group of stretches of K from `first`.
+int bgemm_unsplit_stretches(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
+                            int first, cudaStream_t st) {
+  return bgemm_tcgen05_launch(batch, M, N, K, A, B, C, flags, first, st);
+}
+// Other shapes: the panels that are marked in any stretch.
 int bgemm_unsplit_panels(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
-                         int first, cudaStream_t st) {
-  if (whole_tiles(batch, M, N, K, A, B, C)) return bgemm_tcgen05_launch(batch, M, N, K, A, B, C, flags, first, st);
-  return launch_general(batch, M, N, K, A, B, C, flags, first, st);
+                         cudaStream_t st) {
+  return launch_general(batch, M, N, K, A, B, C, flags, st);
 }
 
 // Whether the product is left to gemm_split.cu: estimates of the time of both, in us, measured on one machine (split / other
@@ -313,5 +314,5 @@ extern "C" int lapis_b200_bgemm_f32(int64_t batch, int64_t M, int64_t N, int64_t
     if (done) return LAPIS_OK;
   }
   if (tiles) return bgemm_tcgen05_launch(batch, M, N, K, d_A, d_B, d_C, PanelFlags(), 0, st);
-  return launch_general(batch, M, N, K, d_A, d_B, d_C, PanelFlags(), 0, st);
+  return launch_general(batch, M, N, K, d_A, d_B, d_C, PanelFlags(), st);
 }

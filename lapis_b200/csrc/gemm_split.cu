@@ -12,10 +12,11 @@
 // a selection are exact, as they are there.  With two parts they were not (a quarter of the elements off by a bit).
 //
 //   split_kernel       reads A and B once, writes the parts as 16-bit matrices with 16-byte rows (so that TMA can load shapes
-//                      and pointers of any alignment), and the scales.  K is cut into stretches of at most 1024, each with
-//                      scales of its own.
+//                      and pointers of any alignment), and the scales of two parts.  K is cut into stretches of at most 1024,
+//                      each with scales of its own.
 //   gemm_split_kernel  a persistent GEMM over the parts: TMA -> tcgen05.mma.kind::f16 -> two accumulators in tensor memory
-//                      (the large product, and the mixed ones) -> scaled, joined, added to C.
+//                      (the large product, and the mixed ones) -> scaled, joined, added to C: two parts once a stretch, three
+//                      parts once, after all of K.
 //
 // 8192^3: 5.05 -> 2.70 ms where the clock holds (407 TFLOP/s, three products at 75 % of cuBLAS's bf16 rate), 5.91 -> 3.33 where
 // power caps it, with an error of 1.25e-6 against 64 bits (2-norm; TF32 split 8.0e-6).  Three parts cost 5 to 65 % more time
@@ -27,9 +28,9 @@
 // fp16 has 5 bits of exponent: the hi of an element below 2^-14 after scaling (2^-29 of the largest of its row or column)
 // would be subnormal and lo lo up to 2^-17 of a product of two such, and an infinity or NaN has no scale.  split_kernel marks
 // the 128-row and 128-column panels that hold such an element (three parts: below 2^-31); the products of those panels are left to
-// the kernels on unsplit operands (PanelFlags), which run behind this one and return at once where there are none.  In 8192 x
-// 8192 normally distributed numbers one is expected in every second matrix, in uniformly distributed ones (multiples of 2^-24)
-// none.
+// the kernels on unsplit operands (PanelFlags), which run behind this one and return at once where there are none.  Three
+// parts: with all of K, in the loop's order and bits.  In 8192 x 8192 normally distributed numbers one is expected in every
+// second matrix, in uniformly distributed ones (multiples of 2^-24) none.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -49,16 +50,22 @@ constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f;
 
 struct Shape {
   int M, N, Np, K;          // Np: columns of the split B, a multiple of GROUP_COLS
+  int ldn;                   // elements between rows of B and C
   int chain;                 // elements of K that are added in tensor memory, a multiple of 64
   int kc, first, stretches;  // stretches first .. first + stretches - 1, of kc (a multiple of 64) each, the last one shorter
   int panels_a, panels_b;
+  // Three parts, where the launches of several groups of stretches make one product: the sums of the groups in front (null: one
+  // group), element by element as the epilogue's threads hold them, whether there are any, and whether this is the last.
+  float *sums;
+  bool fresh, last;
   __host__ __device__ int length(int s) const { return K - (first + s) * kc < kc ? K - (first + s) * kc : kc; }
 };
 
 struct Scratch {
   uint16_t *a, *b;           // [batch][stretch][part][M][kc], [batch][stretch][part][kc][Np]: fp16 or bf16
   float *scale_a, *scale_b;  // [batch][stretch][M], [batch][stretch][Np]: 2^-e
-  unsigned char *flag_a, *flag_b;  // [batch][stretch][panels][8]: a byte for every 16 rows or columns
+  unsigned char *flag_a, *flag_b;  // a byte for every 16 rows or columns: [batch][stretch][panel][8], strides and place of
+  int flag_stretches, flag_first, flag_panels_a, flag_panels_b;  // the first stretch of the launch
 };
 
 // Exponent of the scale for a row or column whose largest magnitude has these bits: the largest power of two that keeps it
@@ -123,6 +130,7 @@ split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int s = blockIdx.y, kc = sh.length(s);
   const int64_t batch = blockIdx.z, at = batch * sh.stretches + s, k0 = (int64_t)(sh.first + s) * sh.kc;
+  const int64_t flags_at = batch * w.flag_stretches + w.flag_first + s;
   const int kpad = (kc + 63) & ~63;
   constexpr int STEPS = KC / 128;
   if ((int)blockIdx.x < 8 * sh.panels_a) {
@@ -166,23 +174,23 @@ split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
     }
     pdl_release();
     const int any = __syncthreads_or(bad);
-    if (tid == 0) w.flag_a[at * 8 * sh.panels_a + blockIdx.x] = any ? 1 : 0;
+    if (tid == 0) w.flag_a[flags_at * 8 * w.flag_panels_a + blockIdx.x] = any ? 1 : 0;
   } else {
     const int group = blockIdx.x - 8 * sh.panels_a, col = group * GROUP_COLS + 4 * (tid & 3), r0 = tid >> 2;
     bool bad = false;
     if (group * GROUP_COLS < sh.Np) {
-      const float *src = B + (batch * sh.K + k0) * sh.N + col;
+      const float *src = B + (batch * sh.K + k0) * sh.ldn + col;
       float v[STEPS][4];
       uint32_t m[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int i = 0; i < STEPS; ++i) {
         const int k = r0 + 128 * i;
         if (VEC_B) {
-          const float4 q = k < kc && col < sh.N ? load_now4(src + (int64_t)k * sh.N) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float4 q = k < kc && col < sh.N ? load_now4(src + (int64_t)k * sh.ldn) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           v[i][0] = q.x, v[i][1] = q.y, v[i][2] = q.z, v[i][3] = q.w;
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) v[i][j] = k < kc && col + j < sh.N ? load_now(src + (int64_t)k * sh.N + j) : 0.0f;
+          for (int j = 0; j < 4; ++j) v[i][j] = k < kc && col + j < sh.N ? load_now(src + (int64_t)k * sh.ldn + j) : 0.0f;
         }
       }
 #pragma unroll
@@ -234,7 +242,7 @@ split_kernel(const float *A, const float *B, Shape sh, Scratch w) {
     }
     pdl_release();
     const int any = __syncthreads_or(bad);
-    if (tid == 0) w.flag_b[at * 8 * sh.panels_b + group] = any ? 1 : 0;
+    if (tid == 0) w.flag_b[flags_at * 8 * w.flag_panels_b + group] = any ? 1 : 0;
   }
 }
 
@@ -246,8 +254,9 @@ constexpr int TILE_BYTES = 32 * 32 * 4;      // an epilogue warp's staging tile
 
 // CTAS CTAs own a tile of 128 CTAS x BN: each loads its 128 rows of A and its share of B's columns, the first one issues the
 // MMAs for all.  In tensor memory: hi hi and mixed products of a tile, 2 BN columns, once or twice.
-template <int PARTS_, int CTAS_, int BN_>
+template <int PARTS_, int CTAS_, int BN_, bool SUMS_ = false>
 struct Config {
+  static constexpr bool SUMS = SUMS_;  // in several launches, the sums kept in between
   static constexpr int PARTS = PARTS_, CTAS = CTAS_, BN = BN_, BUFS = 256 / BN, NB = BN / CTAS;
   static constexpr int A_BYTES = tc::BM * BK * 2, B_BYTES = NB * BK * 2;  // of a part
   static constexpr int STAGE_BYTES = PARTS * (A_BYTES + B_BYTES), STAGES = 196608 / STAGE_BYTES;
@@ -367,6 +376,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   constexpr int PARTS = C_::PARTS, CTAS = C_::CTAS, BN = C_::BN, BUFS = C_::BUFS, NB = C_::NB, A_BYTES = C_::A_BYTES, B_BYTES = C_::B_BYTES,
                 STAGE_BYTES = C_::STAGE_BYTES, STAGES = C_::STAGES, COLS = BN / 2;  // COLS: of an epilogue thread
   constexpr uint32_t IDESC = C_::IDESC;
+  constexpr bool SUMS = C_::SUMS;
   const int chain = sh.chain / BK;  // k blocks
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -407,7 +417,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
-  pdl_release();  // the kernel for the marked panels needs only the flags, unless there are several stretches
 
   // Nothing of the tile is computed here: every row panel or every column panel of it is left to the other kernel.
   auto skipped = [&](const tc::TileCoord &t, int s) {
@@ -424,6 +433,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     return !(row_in && col_in);
   };
+  // Three parts: the whole tile is left to the other kernel, which then adds all of K in the loop's order.  A mark of a later
+  // group of stretches is met by the launch for that group.
+  const int marks = w.flag_first + sh.stretches;
+  auto left_out = [&](const tc::TileCoord &t) {
+    unsigned long long any = 0;
+#pragma unroll 4
+    for (int s = 0; s < marks; ++s) any |= load_flag(flags.row(t.batch, s) + t.m0 / 128) | load_flag(flags.col(t.batch, s) + t.n0 / 128);
+    return any != 0;
+  };
   auto coord = [&](int t) { return tc::tile_coord(t, tm, tn, tc::BM * CTAS, BN); };
   bool ok = true;
 
@@ -433,8 +451,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       uint32_t g = 0;
       for (int t = unit0; t < tiles && ok; t += units) {
         const tc::TileCoord c = coord(t);
+        if (PARTS == 3 && left_out(c)) continue;
         for (int s = 0; s < sh.stretches && ok; ++s) {
-          if (skipped(c, s)) continue;
+          if (PARTS == 2 && skipped(c, s)) continue;
           const int z = PARTS * (c.batch * sh.stretches + s), nk = (sh.length(s) + BK - 1) / BK;
           for (int kb = 0; kb < nk; ++kb, ++g) {
             const int st = g % STAGES;
@@ -461,8 +480,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       uint32_t g = 0, it = 0;
       for (int t = unit0; t < tiles && ok; t += units) {
         const tc::TileCoord c = coord(t);
+        if (PARTS == 3 && left_out(c)) continue;
         for (int s = 0; s < sh.stretches && ok; ++s) {
-          if (skipped(c, s)) continue;
+          if (PARTS == 2 && skipped(c, s)) continue;
           const int nk = (sh.length(s) + BK - 1) / BK;
           for (int kb = 0; kb < nk && ok; ++it) {  // chains
             const int end = nk - kb < chain ? nk : kb + chain;
@@ -508,6 +528,26 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
       if (!ok) atomicExch(error_flag, 6);
     }
+  } else if (warp == 2) {
+    // The kernel for the marked panels may start: at once where this CTA's tiles have no mark, so that it looks at the marks
+    // beside this kernel; otherwise at the end, because blocks that come while SMs are taken are spread unevenly over them
+    // (1000 x 1501 x 777, all panels marked: 180 us, 147 now).
+    bool any = false;
+    for (int t = unit0; t < tiles && !any; t += units) {
+      const tc::TileCoord c = coord(t);
+      for (int s = lane; s < marks; s += 32) {
+        unsigned long long m = 0;
+#pragma unroll
+        for (int i = 0; i < CTAS; ++i)
+          if (c.m0 / 128 + i < sh.panels_a) m |= load_flag(flags.row(c.batch, s) + c.m0 / 128 + i);
+#pragma unroll
+        for (int i = 0; i < BN / 128; ++i)
+          if (c.n0 / 128 + i < sh.panels_b) m |= load_flag(flags.col(c.batch, s) + c.n0 / 128 + i);
+        any |= m != 0;
+      }
+      any = __any_sync(0xffffffffu, any);
+    }
+    if (!any) pdl_release();
   } else if (warp >= 4) {
     // ---------------- epilogue ----------------
     constexpr float MIXED = PARTS == 2 ? LO_UNSCALE : 1.0f;  // weight of the mixed products
@@ -518,34 +558,48 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     for (int t = unit0; t < tiles && ok; t += units) {
       const tc::TileCoord c = coord(t);
       const int m0 = c.m0 + 128 * rank, row0 = m0 + 32 * q, col0 = c.n0 + COLS * half;
+      if (PARTS == 3) {
+        bool any = false;
+        for (int s = lane; s < marks; s += 32)
+          any |= (load_flag(flags.row(c.batch, s) + m0 / 128) | load_flag(flags.col(c.batch, s) + c.n0 / 128)) != 0;
+        if (__any_sync(0xffffffffu, any)) continue;
+      }
+      float4 *sums = SUMS ? reinterpret_cast<float4 *>(sh.sums) + ((int64_t)t * 8 + warp - 4) * COLS / 4 * 32 + lane : nullptr;
+      uint32_t acc[COLS / 16][16];
       for (int s = 0; s < sh.stretches; ++s) {
-        // every load of this stretch at once: the marks, then the scales of this thread's row and columns
-        const bool row_in = m0 / 128 < sh.panels_a, col_in = col0 / 128 < sh.panels_b;
-        const int64_t at = (int64_t)c.batch * sh.stretches + s;
-        const float *scale_a = w.scale_a + at * sh.M, *scale_b = w.scale_b + at * sh.Np;
-        const unsigned long long mark_a = row_in ? load_flag(flags.row(c.batch, s) + m0 / 128) : 1;
-        const unsigned long long mark_b = col_in ? load_flag(flags.col(c.batch, s) + col0 / 128) : 1;
-        const float fa = PARTS == 3 ? 1.0f : row0 + lane < sh.M ? load_scale(scale_a + row0 + lane) : 0.0f;
-        float fb[COLS / 32];  // of the columns 32 ch + lane
+        float fa = 1.0f, fb[COLS / 32];  // scales of this thread's row, of the columns 32 ch + lane
+        bool mine = true;
+        if (PARTS == 2) {
+          // every load of this stretch at once: the marks, then the scales of this thread's row and columns
+          const bool row_in = m0 / 128 < sh.panels_a, col_in = col0 / 128 < sh.panels_b;
+          const int64_t at = (int64_t)c.batch * sh.stretches + s;
+          const float *scale_a = w.scale_a + at * sh.M, *scale_b = w.scale_b + at * sh.Np;
+          const unsigned long long mark_a = row_in ? load_flag(flags.row(c.batch, s) + m0 / 128) : 1;
+          const unsigned long long mark_b = col_in ? load_flag(flags.col(c.batch, s) + col0 / 128) : 1;
+          fa = row0 + lane < sh.M ? load_scale(scale_a + row0 + lane) : 0.0f;
 #pragma unroll
-        for (int ch = 0; ch < COLS / 32; ++ch)
-          fb[ch] = PARTS == 3 ? 1.0f : col0 + 32 * ch + lane < sh.N ? load_scale(scale_b + col0 + 32 * ch + lane) : 0.0f;
-        if (skipped(c, s)) continue;
-        const bool mine = (mark_a | mark_b) == 0;
-        if (s == 0 && mine && row0 + lane < sh.M) {  // C into L2 while the product is computed
-          const float *p = C + ((int64_t)c.batch * sh.M + row0 + lane) * sh.N + col0;
+          for (int ch = 0; ch < COLS / 32; ++ch) fb[ch] = col0 + 32 * ch + lane < sh.N ? load_scale(scale_b + col0 + 32 * ch + lane) : 0.0f;
+          if (skipped(c, s)) continue;
+          mine = (mark_a | mark_b) == 0;
+        } else {
+#pragma unroll
+          for (int ch = 0; ch < COLS / 32; ++ch) fb[ch] = 1.0f;
+        }
+        if (SUMS && s == 0 && !sh.fresh)
+          for (int i = lane & 7; i < COLS / 4; i += 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(sums + 32 * i - lane + (lane & 24)));
+        if (s == 0 && mine && (!SUMS || sh.last) && row0 + lane < sh.M) {  // C into L2 while the product is computed
+          const float *p = C + ((int64_t)c.batch * sh.M + row0 + lane) * sh.ldn + col0;
           const int cols = sh.N - col0 < COLS ? sh.N - col0 : COLS;
           for (int i = 0; i < cols; i += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
           if (cols > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + cols - 1));
         }
-        uint32_t acc[COLS / 16][16];
         for (int kb = 0, nk = (sh.length(s) + BK - 1) / BK; kb < nk; kb += chain, ++it) {
           const uint32_t buf = it % BUFS;
           ok = tc::mbar_wait(&acc_full[buf], (it / BUFS) & 1);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t addr = tmem + buf * 2 * BN + ((uint32_t)(32 * q) << 16) + COLS * half;
-          if (kb == 0) {
+          if (kb == 0 && (PARTS == 2 || s == 0)) {
 #pragma unroll
             for (int i = 0; i < COLS / 16; ++i) tmem_load16(addr + BN + 16 * i, acc[i]);
 #pragma unroll
@@ -582,14 +636,36 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
         if (!ok) break;
         if (!mine) continue;
+        if (PARTS == 3) {  // C is joined last and once
+          if (s + 1 < sh.stretches) continue;
+          if (SUMS && !sh.fresh) {
+#pragma unroll
+            for (int i = 0; i < COLS / 4; ++i) {
+              const float4 v = sums[32 * i];
+              uint32_t *a = &acc[i / 4][4 * (i & 3)];
+              a[0] = __float_as_uint(__fadd_rn(v.x, __uint_as_float(a[0])));
+              a[1] = __float_as_uint(__fadd_rn(v.y, __uint_as_float(a[1])));
+              a[2] = __float_as_uint(__fadd_rn(v.z, __uint_as_float(a[2])));
+              a[3] = __float_as_uint(__fadd_rn(v.w, __uint_as_float(a[3])));
+            }
+          }
+          if (SUMS && !sh.last) {
+#pragma unroll
+            for (int i = 0; i < COLS / 4; ++i) {
+              const uint32_t *a = &acc[i / 4][4 * (i & 3)];
+              sums[32 * i] = make_float4(__uint_as_float(a[0]), __uint_as_float(a[1]), __uint_as_float(a[2]), __uint_as_float(a[3]));
+            }
+            continue;
+          }
+        }
         const int rows = sh.M - row0 < 32 ? sh.M - row0 : 32;
-        const int64_t row4 = 4 * (int64_t)sh.N;
+        const int64_t row4 = 4 * (int64_t)sh.ldn;
         // 32 columns at a time through shared memory (float4 slots rotated by the row: no bank conflicts), so that C is
         // accessed by rows
 #pragma unroll
         for (int ch = 0; ch < COLS / 32; ++ch) {
           const int c0 = col0 + 32 * ch;
-          float *cp = C + ((int64_t)c.batch * sh.M + row0) * sh.N + c0;
+          float *cp = C + ((int64_t)c.batch * sh.M + row0) * sh.ldn + c0;
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -605,7 +681,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                                          __shfl_sync(0xffffffffu, fb[ch], 4 * qc + 2), __shfl_sync(0xffffffffu, fb[ch], 4 * qc + 3));
             if (col < sh.N) {
               int row = lane >> 3;
-              float *p = cp + (int64_t)row * sh.N + 4 * qc;
+              float *p = cp + (int64_t)row * sh.ldn + 4 * qc;
 #pragma unroll 1
               for (int pass = 0; pass < 8; pass += DEPTH) {
                 float4 cin[DEPTH];
@@ -632,13 +708,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               float cin[2 * DEPTH];
 #pragma unroll
               for (int i = 0; i < 2 * DEPTH; ++i)
-                if (row + i < rows) cin[i] = p[(int64_t)i * sh.N];
+                if (row + i < rows) cin[i] = p[(int64_t)i * sh.ldn];
 #pragma unroll
               for (int i = 0; i < 2 * DEPTH; ++i) {
                 const float a = stile[(row + i) * 32 + 4 * ((lane >> 2) ^ (i & 7)) + (lane & 3)];  // row is a multiple of 8
-                if (row + i < rows) p[(int64_t)i * sh.N] = __fadd_rn(__fmul_rn(a, f), cin[i]);
+                if (row + i < rows) p[(int64_t)i * sh.ldn] = __fadd_rn(__fmul_rn(a, f), cin[i]);
               }
-              p += 2 * DEPTH * (int64_t)sh.N;
+              p += 2 * DEPTH * (int64_t)sh.ldn;
             }
           }
         }
@@ -684,11 +760,11 @@ static int launch_gemm(const CUtensorMap &map_a, const CUtensorMap &map_b, float
 
 // With PARTS = 2 or 3.
 template <int PARTS>
-static int launch_tiles(int64_t M, int64_t N, int64_t group_b, int64_t nb, const float *A, const float *B, float *C, const Shape &sh,
+static int launch_tiles(int64_t group_b, int64_t nb, const float *A, const float *B, float *C, const Shape &sh,
                         const Scratch &w, const PanelFlags &flags, int *error_flag, int dev, cudaStream_t st) {
-  const int64_t K = sh.K;
-  const bool vec_a = K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, vec_b = N % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
-  const bool vec_c = N % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
+  const int64_t M = sh.M, N = sh.N;
+  const bool vec_a = sh.K % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0, vec_b = sh.ldn % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  const bool vec_c = sh.ldn % 4 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   const dim3 grid((unsigned)(8 * (sh.panels_a + sh.panels_b)), (unsigned)sh.stretches, (unsigned)nb);
   auto kernel = vec_a ? (vec_b ? split_kernel<PARTS, true, true> : split_kernel<PARTS, true, false>)
                       : (vec_b ? split_kernel<PARTS, false, true> : split_kernel<PARTS, false, false>);
@@ -700,7 +776,8 @@ static int launch_tiles(int64_t M, int64_t N, int64_t group_b, int64_t nb, const
   LAPIS_TRY(tc::make_map(&map_b, type, w.b, parts, sh.kc, sh.Np, 2 * (int64_t)sh.Np, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B));
   auto count = [&](int64_t rows, int64_t cols) { return ((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
   if (PARTS == 3)  // six products of what a CTA loads: pairs, which load half of B each, are no faster (1000 x 1501 x 777 36.8, single 35.7 us)
-    return launch_gemm<Config<3, 1, 128>>(map_a, map_b, C, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st);
+    return sh.sums != nullptr ? launch_gemm<Config<3, 1, 128, true>>(map_a, map_b, C, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st)
+                              : launch_gemm<Config<3, 1, 128>>(map_a, map_b, C, sh, w, flags, nb * count(128, 128), vec_c, error_flag, dev, st);
   // rounds of tiles that the busiest SM works through, by what one takes
   const int64_t sms = sm_count();
   auto cost = [&](int64_t n, int64_t at_once, int64_t each) { return (n * group_b + at_once - 1) / at_once * each; };
@@ -713,12 +790,21 @@ static int launch_tiles(int64_t M, int64_t N, int64_t group_b, int64_t nb, const
 
 }  // namespace split
 
+int bgemm_unsplit_stretches(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
+                            int first, cudaStream_t st);
 int bgemm_unsplit_panels(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, const PanelFlags &flags,
-                         int first, cudaStream_t st);
+                         cudaStream_t st);
 
 constexpr size_t SPLIT_BYTES = size_t(160) << 20;
 
 // *done: false where the caller has to use another kernel (no memory for the split operands).
+//
+// What does not fit into SPLIT_BYTES is worked on in groups of stretches of K.  Whole tiles add each group to C, as the kernel
+// that they replaced adds its segments.  Three parts keep the sums of the groups aside, so that C is joined last and once, as
+// in the loop (with |C| near 1000 and K = 8000 an addition for every 1024 of K had 2.8 times the loop's error), and take C in
+// blocks whose sums leave at least a third of SPLIT_BYTES to the operands, which are split again for every block beside theirs:
+// 8191^3 5.38 -> 5.59 ms, in four blocks; 2100 x 2099 x 8000 425 -> 407 us; 70,000 x 321 x 1300 1165 -> 643, where shorter
+// stretches had made room before.
 int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const float *A, const float *B, float *C, bool exact_order,
                        bool *done, cudaStream_t st) {
   using namespace split;
@@ -728,54 +814,95 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
   int *error_flag = bgemm_error_flag(dev);
   if (error_flag == nullptr) return LAPIS_ECUDA;
 
-  Shape sh = {};
-  sh.M = (int)M;
-  sh.N = (int)N;
-  sh.K = (int)K;
-  sh.Np = (int)((N + GROUP_COLS - 1) / GROUP_COLS * GROUP_COLS);
-  sh.panels_a = (int)((M + 127) / 128);
-  sh.panels_b = (int)((N + 127) / 128);
-  sh.chain = exact_order ? std::min(KC, 64 * std::max(1, (int)(std::sqrt((double)K) / 7))) : KC;
+  auto panels = [](int64_t extent) { return (extent + 127) / 128; };
+  auto padded = [](int64_t cols) { return (cols + GROUP_COLS - 1) / GROUP_COLS * GROUP_COLS; };
   const int parts = exact_order ? 3 : 2;
+  Shape sh = {};
+  sh.K = (int)K;
+  sh.ldn = (int)N;
+  sh.chain = exact_order ? std::min(KC, 64 * std::max(1, (int)(std::sqrt((double)K) / 7))) : KC;
   int64_t all = 0;  // stretches of K
-  size_t per = 0;   // bytes of a stretch: parts, scales, flags, each from a 256-byte boundary
-  size_t bytes_a = 0, bytes_b = 0;
+  int64_t block_m = M, block_n = N;
+  size_t sums = 0;  // bytes
+  auto per = [&] {  // bytes of a stretch: parts, scales, flags
+    return 2 * (size_t)parts * sh.kc * (block_m + padded(block_n)) + 4 * (size_t)(block_m + padded(block_n)) + 8 * (size_t)(panels(block_m) + panels(block_n));
+  };
   for (int longest = KC; longest >= 64; longest /= 2) {
     all = (K + longest - 1) / longest;
     sh.kc = (int)(((K + all - 1) / all + 63) / 64 * 64);
     all = (K + sh.kc - 1) / sh.kc;
-    bytes_a = (size_t)2 * parts * M * sh.kc;
-    bytes_b = (size_t)2 * parts * sh.kc * sh.Np;
-    per = bytes_a + bytes_b + 4 * (size_t)(M + sh.Np) + 8 * (size_t)(sh.panels_a + sh.panels_b);
-    if (per <= SPLIT_BYTES) break;
+    if (parts == 3 || per() <= SPLIT_BYTES) break;
   }
-  if (per > SPLIT_BYTES) return LAPIS_OK;
-  const int64_t group_s = std::min<int64_t>({all, (int64_t)(SPLIT_BYTES / per), 65535});
-  const int64_t group_b = std::min<int64_t>({batch, std::max<int64_t>(1, SPLIT_BYTES / (per * group_s)), 65535});
-  auto round = [](size_t x) { return (x + 255) & ~size_t(255); };
+  if (parts == 3 && per() * all > SPLIT_BYTES) {
+    for (int64_t cm = 1, cn = 1;;) {
+      block_m = cm == 1 ? M : 128 * panels((M + cm - 1) / cm);
+      block_n = cn == 1 ? N : 128 * panels((N + cn - 1) / cn);
+      sums = 4 * (size_t)(128 * panels(block_m)) * (size_t)(128 * panels(block_n));
+      if (per() <= SPLIT_BYTES && sums <= SPLIT_BYTES - std::max(per(), SPLIT_BYTES / 3)) break;
+      ++(block_m >= block_n ? cm : cn);
+    }
+  }
+  if (per() > SPLIT_BYTES) return LAPIS_OK;
+  const bool aside = sums != 0;
+  const int64_t group_s = std::min<int64_t>({all, (int64_t)((SPLIT_BYTES - sums) / per()), 65535});
+  const int64_t group_b = aside ? 1 : std::min<int64_t>({batch, std::max<int64_t>(1, SPLIT_BYTES / (per() * group_s)), 65535});
+  const int64_t marks = parts == 3 ? all : group_s;  // stretches whose marks are kept
+  size_t total = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = total;
+    total = (total + bytes + 255) & ~size_t(255);
+    return at;
+  };
   const size_t n = (size_t)(group_s * group_b);
-  const size_t off_b = round(n * bytes_a), off_sa = off_b + round(n * bytes_b), off_sb = off_sa + round(n * M * 4),
-               off_fa = off_sb + round(n * sh.Np * 4), off_fb = off_fa + round(n * 8 * sh.panels_a), total = off_fb + round(n * 8 * sh.panels_b);
+  const size_t off_a = take(n * 2 * parts * block_m * sh.kc), off_b = take(n * 2 * parts * sh.kc * padded(block_n)), off_sa = take(n * block_m * 4),
+               off_sb = take(n * padded(block_n) * 4), off_fa = take((size_t)(marks * group_b) * 8 * panels(M)),
+               off_fb = take((size_t)(marks * group_b) * 8 * panels(N)), off_sums = take(sums);
   PoolBuf buf;
   if (buf.alloc(total, st) != LAPIS_OK) {
     clear_error();
     return LAPIS_OK;
   }
   uint8_t *p = static_cast<uint8_t *>(buf.p);
-  Scratch w = {reinterpret_cast<uint16_t *>(p), reinterpret_cast<uint16_t *>(p + off_b), reinterpret_cast<float *>(p + off_sa),
-               reinterpret_cast<float *>(p + off_sb), p + off_fa, p + off_fb};
+  Scratch w = {reinterpret_cast<uint16_t *>(p + off_a), reinterpret_cast<uint16_t *>(p + off_b), reinterpret_cast<float *>(p + off_sa),
+               reinterpret_cast<float *>(p + off_sb)};
+  w.flag_panels_a = (int)panels(M);
+  w.flag_panels_b = (int)panels(N);
+  sh.sums = aside ? reinterpret_cast<float *>(p + off_sums) : nullptr;
+  PanelFlags flags = {nullptr, nullptr, w.flag_panels_a, w.flag_panels_b, 0, sh.kc};
   for (int64_t b0 = 0; b0 < batch; b0 += group_b) {
     const int64_t nb = std::min(group_b, batch - b0);
     const float *Ab = A + b0 * M * K, *Bb = B + b0 * K * N;
     float *Cb = C + b0 * M * N;
-    for (int64_t s0 = 0; s0 < all; s0 += group_s) {
-      sh.first = (int)s0;
-      sh.stretches = (int)std::min(group_s, all - s0);
-      const PanelFlags flags = {reinterpret_cast<const unsigned long long *>(w.flag_a), reinterpret_cast<const unsigned long long *>(w.flag_b),
-                                sh.panels_a, sh.panels_b, sh.stretches, sh.kc};
-      LAPIS_TRY(parts == 2 ? launch_tiles<2>(M, N, group_b, nb, Ab, Bb, Cb, sh, w, flags, error_flag, dev, st)
-                           : launch_tiles<3>(M, N, group_b, nb, Ab, Bb, Cb, sh, w, flags, error_flag, dev, st));
-      LAPIS_TRY(bgemm_unsplit_panels(nb, M, N, K, Ab, Bb, Cb, flags, (int)s0, st));
+    for (int64_t m0 = 0; m0 < M; m0 += block_m) {
+      for (int64_t n0 = 0; n0 < N; n0 += block_n) {
+        sh.M = (int)std::min(block_m, M - m0);
+        sh.N = (int)std::min(block_n, N - n0);
+        sh.Np = (int)padded(sh.N);
+        sh.panels_a = (int)panels(sh.M);
+        sh.panels_b = (int)panels(sh.N);
+        for (int64_t s0 = 0; s0 < all; s0 += group_s) {
+          sh.first = (int)s0;
+          sh.stretches = (int)std::min(group_s, all - s0);
+          sh.fresh = s0 == 0;
+          sh.last = parts == 2 || s0 + group_s >= all;
+          w.flag_a = p + off_fa + 8 * (m0 / 128);
+          w.flag_b = p + off_fb + 8 * (n0 / 128);
+          w.flag_stretches = flags.stretches = parts == 3 ? (int)all : sh.stretches;
+          w.flag_first = parts == 3 ? (int)s0 : 0;
+          flags.a = reinterpret_cast<const unsigned long long *>(w.flag_a);
+          flags.b = reinterpret_cast<const unsigned long long *>(w.flag_b);
+          const float *As = Ab + m0 * K, *Bs = Bb + n0;
+          float *Cs = Cb + m0 * N + n0;
+          LAPIS_TRY(parts == 2 ? launch_tiles<2>(group_b, nb, As, Bs, Cs, sh, w, flags, error_flag, dev, st)
+                               : launch_tiles<3>(group_b, nb, As, Bs, Cs, sh, w, flags, error_flag, dev, st));
+          if (parts == 2) LAPIS_TRY(bgemm_unsplit_stretches(nb, M, N, K, Ab, Bb, Cb, flags, (int)s0, st));
+        }
+      }
+    }
+    if (parts == 3) {
+      flags.a = reinterpret_cast<const unsigned long long *>(p + off_fa);
+      flags.b = reinterpret_cast<const unsigned long long *>(p + off_fb);
+      LAPIS_TRY(bgemm_unsplit_panels(nb, M, N, K, Ab, Bb, Cb, flags, st));
     }
   }
   *done = true;

@@ -92,8 +92,8 @@ int make_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64
 }  // namespace tc
 
 // Which operand panels of a product that is computed from split operands (gemm_split.cu) the split does not cover: a word
-// for every 128 rows of A and every 128 columns of B, for each of the stretches of `kc` that K is cut into.  Null: the
-// kernel computes everything.
+// for every 128 rows of A and every 128 columns of B, for each of the stretches of `kc` that K is cut into (whole tiles: that a
+// launch takes).  Null: the kernel computes everything.
 struct PanelFlags {
   const unsigned long long *a, *b;  // [batch][stretches][panels_a], [batch][stretches][panels_b]
   int panels_a, panels_b;
