@@ -13,10 +13,7 @@
 //
 // A row of 4096 entries walked U at a time is a chain of 4096 / U trips to memory, which outlasts everything else in a
 // skewed matrix.  Such rows go to a kernel of their own that runs beside this one (spmm_long_kernel): 50,021 rows with
-// a mean of 16 and rows up to 4096, k = 37, DCSR: 884 -> 218 to 283 us with the matrix drawn; 10,000 rows, mean 30,
-// k = 128: 839 -> 235.
-#include <cooperative_groups.h>
-
+// a mean of 16 and rows up to 4096, k = 37, DCSR: 884 -> 102 us.
 #include <algorithm>
 #include <cstdint>
 
@@ -30,9 +27,11 @@ constexpr int SPMM_PANEL = 64;                     // columns of a row that a bl
 constexpr int SPMM_ADDERS = 2, SPMM_FEEDERS = 10;  // warps that add and warps that gather and multiply
 constexpr int SPMM_LONG_THREADS = 32 * (SPMM_ADDERS + SPMM_FEEDERS);
 constexpr int SPMM_PER = 4, SPMM_TILE = 32 * SPMM_FEEDERS * SPMM_PER;  // products of a feeder, of a tile
-constexpr int SPMM_CLUSTER = 4;                       // blocks that share their long rows
+constexpr int SPMM_TEAM = 4;                          // blocks that share their long rows
+constexpr int SPMM_LOOK = 4;                          // neighbouring rows that a thread looks at together
+constexpr int64_t SPMM_TEAM_BYTES = 450000;           // offsets beyond which a block looks at its own rows only
 constexpr int SPMM_LIST = SPMM_LONG_THREADS + 64;     // long rows that a block notes before it works on them
-constexpr int SPMM_SHARED = 768;                      // pieces that a cluster divides among its blocks
+constexpr int SPMM_SHARED = 768;                      // pieces that a team divides by length; a block alone: SPMM_LIST
 
 template <int V>
 struct Columns;
@@ -166,28 +165,53 @@ spmm_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__r
 // count, because __syncthreads() in one branch of an if is undefined even where the other branch has as many.
 __device__ __forceinline__ void tile_barrier() { asm volatile("barrier.sync 1, %0;" ::"n"(SPMM_LONG_THREADS) : "memory"); }
 
-// The long rows.  A block notes those among its rows (eight neighbours, then the eight gridDim.x * 8 further on, so that
-// neighbouring long rows meet different blocks); at the end the blocks of a cluster divide what they noted, a piece being a row
-// and up to 64 columns: by length, the longest first, 0 1 2 3 3 2 1 0 0 1 .. (too many pieces: each block keeps its own).
+// Which of the rows r .. r + 3 are long: what spmm_row finds, but with loads that do not wait for each other.
+template <typename I, bool DCSR>
+__device__ __forceinline__ unsigned spmm_long_among(const I *__restrict__ rowno, const I *__restrict__ pos, int64_t nrows, int64_t k, int64_t r) {
+  I at[SPMM_LOOK + 1], no[SPMM_LOOK + 2];
+#pragma unroll
+  for (int i = 0; i <= SPMM_LOOK; ++i) at[i] = r + i <= nrows ? pos[r + i] : (I)0;
+  if (DCSR) {
+#pragma unroll
+    for (int i = 0; i <= SPMM_LOOK + 1; ++i) no[i] = r + i > 0 && r + i <= nrows ? rowno[r + i - 1] : (I)-1;
+  }
+  unsigned found = 0;
+#pragma unroll
+  for (int i = 0; i < SPMM_LOOK; ++i) {
+    if (r + i >= nrows || (DCSR && no[i] == no[i + 1])) continue;  // beyond the last, or not the first of its run
+    int64_t lo = (int64_t)at[i], hi = (int64_t)at[i + 1], out;
+    if (DCSR && no[i + 1] == no[i + 2]) spmm_row<I, DCSR>(rowno, pos, nrows, r + i, lo, hi, out);
+    if (spmm_is_long(hi - lo, pos, nrows, k)) found |= 1u << i;
+  }
+  return found;
+}
+
+// The long rows.  The blocks of a team note those among the team's rows (eight neighbours, then the eight further on by eight
+// for every team, so that neighbouring long rows meet different teams), all four alike, and divide them, a piece being a row
+// and up to 64 columns: by length, the longest first, 0 1 2 3 3 2 1 0 0 1 .. (too many pieces: whole rows in turn).  That each
+// block looks through four times as many rows costs less than an exchange: with one share of the rows for each block of a
+// cluster, passed round through shared memory, products without long rows took 2 to 4 us longer, the launch of clusters and its
+// barriers (10,844 stored rows of 25, k = 3, 12.3 us, now 8.3; 50,021 of 4, k = 37, 20.9 and 19.0).  It does so up to about one look of
+// every thread; beyond, blocks look at their own rows and share nothing: there are enough long rows for each (1,000,000 rows of 4, k = 2,
+// 64 us in teams, 47 alone, 54 in clusters; with skewed lengths 1,500,000 of 8, k = 8, 722, 684 and 697, but 100,000 of 16, k = 8, 81,
+// 117 and 79).
 // A block works through its pieces in tiles of SPMM_TILE products: ten warps gather and multiply, two tiles ahead of the one
 // they store, across the ends of pieces, and two warps add, a lane one column, in entry order out of shared memory.
-// One tile ahead, one row on an SM, a barrier for both, and now: 50,021 rows, k = 37 264 -> 104 us; 40,000, k = 130 374 -> 252;
-// 30,000 of 39, k = 100 476 -> 363; 200,000 of 30, k = 16 566 -> 274.
+// One tile ahead, one row on an SM, a barrier for both, and now: 50,021 rows of 16, k = 37 276 -> 102 us; 40,000 of 30, k = 130
+// 635 -> 438; 30,000 of 39, k = 100 426 -> 267; 200,000 of 30, k = 16 400 -> 273; 20,000 of 10, k = 3 94 -> 33.
 template <typename I, bool DCSR>
 __global__ void __launch_bounds__(SPMM_LONG_THREADS, 2)  // registers: the kernel beside this one needs half of them
 spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val,
-                 int64_t nrows, int64_t k, const double *__restrict__ B, double *__restrict__ C, int accumulate) {
-  namespace cg = cooperative_groups;
+                 int64_t nrows, int64_t k, int team, const double *__restrict__ B, double *__restrict__ C, int accumulate) {
   __shared__ double s_prod[2][SPMM_TILE];
   __shared__ int64_t s_lo[SPMM_LIST], s_out[SPMM_LIST];  // noted rows
   __shared__ int s_len[SPMM_LIST];
   __shared__ int64_t w_lo[SPMM_LIST], w_out[SPMM_LIST];  // pieces of work
   __shared__ int w_len[SPMM_LIST], w_c0[SPMM_LIST], w_c1[SPMM_LIST];
-  __shared__ int s_all[SPMM_SHARED];
-  __shared__ int s_n, s_count;
+  __shared__ int s_before[SPMM_LONG_THREADS / 32 + 1];
   pdl_release();  // the kernel for the other rows shares nothing with this one but inputs
-  cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, feeder = tid - 32 * SPMM_ADDERS;  // negative: an adder
+  const int member = blockIdx.x % team;
   const int64_t panels = (k + SPMM_PANEL - 1) / SPMM_PANEL;
   const int width = (int)((k + panels - 1) / panels), entries = SPMM_TILE / width;  // of a tile
   int je[SPMM_PER], ce[SPMM_PER];  // this feeder's products in a tile: entry (beyond any row: none) and column
@@ -197,77 +221,69 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
     je[i] = feeder >= 0 && at < entries * width ? at / width : 0x40000000;
     ce[i] = at - at / width * width;
   }
-  if (tid == 0) s_n = 0;
-  __syncthreads();
-  const int64_t turn = (int64_t)gridDim.x * SPMM_LONG_THREADS;
+  const int64_t teams = gridDim.x / team, turn = teams * SPMM_LONG_THREADS * SPMM_LOOK;
+  const int64_t mine = ((int64_t)(tid / (8 / SPMM_LOOK)) * teams + blockIdx.x / team) * 8 + tid % (8 / SPMM_LOOK) * SPMM_LOOK;
+  int seen = 0;  // rows of each thread's in this turn that are noted or worked on
   for (int64_t r0 = 0;;) {
     int noted = 0;
-    for (; r0 < nrows && noted <= SPMM_LIST - SPMM_LONG_THREADS; r0 += turn) {
-      int64_t lo = 0, hi = 0, out = 0;
-      const int64_t r = r0 + ((int64_t)(tid / 8) * gridDim.x + blockIdx.x) * 8 + tid % 8;
-      const bool found = spmm_row<I, DCSR>(rowno, pos, nrows, r, lo, hi, out) && spmm_is_long(hi - lo, pos, nrows, k);
-      if (found) {
-        const int at = atomicAdd(&s_n, 1);  // the order of the list does not matter: rows are independent
-        s_lo[at] = lo;
-        s_len[at] = (int)(hi - lo);
-        s_out[at] = out;
+    for (bool room = true; room && r0 < nrows;) {
+      const unsigned found = spmm_long_among<I, DCSR>(rowno, pos, nrows, k, r0 + mine);
+      if (__syncthreads_or(found != 0)) {
+        for (; seen < SPMM_LOOK; ++seen) {
+          const bool one = found >> seen & 1;
+          const int more = __syncthreads_count(one);
+          room = noted + more <= SPMM_LIST;
+          if (!room) break;
+          if (more == 0) continue;
+          // in the order of the threads, which is the same in every block of the team
+          const unsigned votes = __ballot_sync(0xffffffffu, one);
+          if (tid % 32 == 0) s_before[tid / 32] = __popc(votes);
+          __syncthreads();
+          if (one) {
+            int at = noted + __popc(votes & ((1u << tid % 32) - 1));
+            for (int q = 0; q < tid / 32; ++q) at += s_before[q];
+            int64_t lo, hi, out;
+            spmm_row<I, DCSR>(rowno, pos, nrows, r0 + mine + seen, lo, hi, out);
+            s_lo[at] = lo;
+            s_len[at] = (int)(hi - lo);
+            s_out[at] = out;
+          }
+          noted += more;
+        }
+        if (!room) break;
       }
-      noted += __syncthreads_count(found);
+      seen = 0;
+      r0 += turn;
     }
     const bool end = r0 >= nrows;
-    int n = 0;  // pieces
-    bool shared = false;
-    if (end) {
-      if (tid == 0) s_count = 0;
-      cluster.sync();
-      int all = 0, begin[SPMM_CLUSTER + 1];
-#pragma unroll
-      for (int c = 0; c < SPMM_CLUSTER; ++c) {
-        begin[c] = all;
-        all += *cluster.map_shared_rank(&s_n, c);
+    if (end && noted == 0) return;
+    __syncthreads();
+    // pieces of this block
+    const bool by_length = noted * panels <= (team == 1 ? SPMM_LIST : SPMM_SHARED);
+    const int np = by_length ? (int)panels : 1, pieces = noted * np;
+    const int rounds = pieces / team, turned = by_length && rounds % 2 != 0 ? team - 1 - member : member;
+    const int n = rounds + (turned < pieces % team ? 1 : 0);
+    for (int u = tid; u < pieces; u += SPMM_LONG_THREADS) {
+      const int row = u / np, len = s_len[row];
+      int at;
+      if (by_length) {
+        int rank = 0;  // longer ones, and equal ones in front
+        for (int v = 0; v < noted; ++v) rank += s_len[v] > len ? np : s_len[v] == len && v < row ? np : 0;
+        rank += u - row * np;
+        const int place = rank % (2 * team);
+        if ((place < team ? place : 2 * team - 1 - place) != member) continue;
+        at = rank / team;  // its turn in this block
+      } else {
+        if (u % team != member) continue;
+        at = u / team;
       }
-      begin[SPMM_CLUSTER] = all;
-      shared = all * panels <= SPMM_SHARED;
-      if (shared) {
-        const int np = (int)panels, pieces = all * np;
-        for (int u = tid; u < pieces; u += SPMM_LONG_THREADS) {
-          const int row = u / np;
-          int c = 0;
-          while (row >= begin[c + 1]) ++c;
-          s_all[u] = cluster.map_shared_rank(s_len, c)[row - begin[c]];
-        }
-        __syncthreads();
-        for (int u = tid; u < pieces; u += SPMM_LONG_THREADS) {
-          const int mine = s_all[u];
-          int rank = 0;  // longer ones, and equal ones in front
-          for (int v = 0; v < pieces; ++v) rank += s_all[v] > mine || (s_all[v] == mine && v < u);
-          const int place = rank % (2 * SPMM_CLUSTER);
-          if ((place < SPMM_CLUSTER ? place : 2 * SPMM_CLUSTER - 1 - place) != (int)cluster.block_rank()) continue;
-          const int row = u / np, at = rank / SPMM_CLUSTER;  // its turn in this block
-          int c = 0;
-          while (row >= begin[c + 1]) ++c;
-          w_lo[at] = cluster.map_shared_rank(s_lo, c)[row - begin[c]];
-          w_out[at] = cluster.map_shared_rank(s_out, c)[row - begin[c]];
-          w_len[at] = mine;
-          w_c0[at] = (u - row * np) * width;
-          w_c1[at] = min(w_c0[at] + width, (int)k);
-          atomicAdd(&s_count, 1);
-        }
-      }
-      cluster.sync();  // nobody reads another block's list any more
-      n = shared ? s_count : 0;
+      w_lo[at] = s_lo[row];
+      w_out[at] = s_out[row];
+      w_len[at] = len;
+      w_c0[at] = by_length ? (u - row * np) * width : 0;
+      w_c1[at] = by_length ? min(w_c0[at] + width, (int)k) : (int)k;
     }
-    if (!shared) {
-      n = noted;
-      for (int u = tid; u < n; u += SPMM_LONG_THREADS) {
-        w_lo[u] = s_lo[u];
-        w_out[u] = s_out[u];
-        w_len[u] = s_len[u];
-        w_c0[u] = 0;
-        w_c1[u] = (int)k;
-      }
-      __syncthreads();
-    }
+    __syncthreads();
     // a place in the sequence of tiles: piece, first column of the panel, first entry of the tile
     struct Place {
       int q, c0, j;
@@ -361,9 +377,7 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
       }
     }
     if (end) break;
-    __syncthreads();
-    if (tid == 0) s_n = 0;
-    __syncthreads();
+    __syncthreads();  // the lists are free
   }
 }
 
@@ -412,18 +426,11 @@ static cudaError_t launch_spmm_width(const SpmmArgs<I> &m, cudaStream_t st) {
 template <typename I, bool DCSR>
 static cudaError_t launch_spmm(const SpmmArgs<I> &m, cudaStream_t st) {
   if (m.long_rows) {
-    const int64_t clusters = std::min<int64_t>((m.nrows + 8 * SPMM_CLUSTER - 1) / (8 * SPMM_CLUSTER), sm_count() / SPMM_CLUSTER);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(clusters * SPMM_CLUSTER));
-    cfg.blockDim = dim3(SPMM_LONG_THREADS);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SPMM_CLUSTER;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, spmm_long_kernel<I, DCSR>, m.rowno, m.pos, m.crd, m.val, m.nrows, m.k, m.B, m.C, m.accumulate);
+    const int team = m.nrows * (int64_t)sizeof(I) <= SPMM_TEAM_BYTES ? SPMM_TEAM : 1;
+    const int64_t teams = std::min<int64_t>((m.nrows + 8 * team - 1) / (8 * team), std::max(1, sm_count() / team));
+    spmm_long_kernel<I, DCSR><<<(unsigned)(teams * team), SPMM_LONG_THREADS, 0, st>>>(m.rowno, m.pos, m.crd, m.val, m.nrows, m.k, team, m.B, m.C,
+                                                                                     m.accumulate);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   // pairs of columns travel as 16-byte accesses when k is even and B and C are aligned for it
