@@ -231,14 +231,14 @@ static constexpr GeneralTile general_tiles[] = {{64, 64, 0.706f, 0.92f, launch_s
                                                 {32, 32, 0.255f, 0.46f, launch_simt<32, 32, 2, 4, 6>}};
 struct TileChoice {
   const GeneralTile *tile;
-  float us;  // a k-slab
+  float us, all;  // a k-slab: what the choice goes by; what the busiest SM takes, a few tiles overlapping only in part
 };
 static TileChoice general_tile(int64_t batch, int64_t M, int64_t N) {
-  TileChoice best = {nullptr, 0.0f};
+  TileChoice best = {nullptr, 0.0f, 0.0f};
   for (const GeneralTile &t : general_tiles) {
     const int64_t count = batch * ((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn);
-    const float us = std::max(t.alone, t.slab * (float)((count + sm_count() - 1) / sm_count()));
-    if (best.tile == nullptr || us < best.us) best = {&t, us};
+    const float most = (float)((count + sm_count() - 1) / sm_count()), us = std::max(t.alone, t.slab * most);
+    if (best.tile == nullptr || us < best.us) best = {&t, us, t.alone + t.slab * (most - 1.0f)};
   }
   return best;
 }
@@ -267,11 +267,16 @@ int bgemm_unsplit_panels(int64_t batch, int64_t M, int64_t N, int64_t K, const f
 }
 
 // Whether the product is left to gemm_split.cu: estimates of the time of both, in us, measured on one machine (split / other
-// kernel): 8192^3 2700 / 5055, 2048^3 67 / 126, 1024^3 25 / 38, 128 x 128 x 1024 24 / 35 (whole tiles); 1000 x 1501 x 777 27 / 122,
-// 5000 x 3000 x 1999 208 / 2049, 129 x 4000 x 1000 28 / 95, 8191 x 8190 x 130 365 / 765, 100 problems of 200^3 72 / 93 (other
-// shapes).  Not for 512^3 20 / 21, 2048 x 2048 x 256 28 / 22, 64 of 256^3 60 / 22, 400 of 100 x 100 x 128 106 / 65, 300^3 17 / 10.
-// Below K = 128 the split would cost more precision than the sequential sum of the kernel for general shapes loses, and
-// with fewer than 64 rows or columns most of a tile is padding.
+// kernel).  Whole tiles, two parts: 8192^3 2700 / 5055, 2048^3 67 / 126, 1024^3 25 / 38, 128 x 128 x 1024 24 / 35; not for 512^3
+// 20 / 21, 2048 x 2048 x 256 28 / 22, 64 of 256^3 60 / 22.  Other shapes, three parts: 1000 x 1501 x 777 36 / 142, 5000 x 3000 x
+// 1999 310 / 2272, 129 x 4000 x 1000 35 / 100, 8191 x 8190 x 130 430 / 947, 100 problems of 200^3 74 / 97; not for 255 x 296 x
+// 719 24.7 / 23.1, 227 x 96 x 1016 28.4 / 27.0, 291 x 247 x 968 34.8 / 32.9, 400 of 100 x 100 x 128 111 / 68, 300^3 19 / 12.
+// Below K = 128 the chains in tensor memory would cost more precision than the sequential sum of the kernel for general shapes
+// loses, and with fewer than 64 rows or columns most of a tile is padding.
+//
+// What the estimates cannot see are the values: operands of which the split covers nothing (a range above 2^29 in every 128
+// rows or columns: graded matrices, exponentials) pay for the pass over them and for two more launches, 1000 x 1501 x 777 146.5
+// us, which it takes alone as well, 1024^3 44.5 for 36.9, 4096^3 786 for 705, 100 of 200^3 153 for 103.
 static bool split_pays(int64_t batch, int64_t M, int64_t N, int64_t K, bool tiles, bool vec_c) {
   if (M > (1 << 30) || N > (1 << 30) || K > (1 << 30) || batch * ((M + 127) / 128) * ((N + 127) / 128) >= (1ll << 31)) return false;
   if (M < 64 || N < 64 || (!tiles && K < 128)) return false;
@@ -279,19 +284,23 @@ static bool split_pays(int64_t batch, int64_t M, int64_t N, int64_t K, bool tile
   auto rounds = [&](int64_t rows, int64_t cols, double at_once) {
     return std::ceil(problems * (double)((M + rows - 1) / rows) * (double)((N + cols - 1) / cols) / at_once);
   };
-  double before;
-  if (tiles) {
-    const double wide = N % 256 == 0 ? rounds(128, 256, sms) : 1e30;
-    before = wide > 1 && wide < 1e30 ? wide * 0.0441 * depth : rounds(128, 128, sms) * 0.030 * depth;
-    before = 5.0 + std::max(before, 4.0 * problems * (depth * (double)(M + N) + 2.0 * (double)M * (double)N) / 5.3e6);
-  } else {
-    before = 4.0 + general_tile(batch, M, N).us * std::ceil(depth / SG_K);
+  const double c = vec_c ? 1.0 : 2.0, operands = 8.0 * problems * depth * (double)(M + N);  // bytes of the parts, about
+  if (!tiles) {
+    // Launches; the pass over the operands, by bytes and by blocks of 16 rows or columns, two on an SM; rounds of tiles, by the
+    // products or, where K is short, by the accesses to C.  Fitted to 700 shapes of 3e6 to 6e9 products: with it 4 of them take
+    // the kernel that is slower by more than 3 % (at most 11 %), with the estimate for two parts 51 (up to 62 %).
+    const double before = 4.0 + general_tile(batch, M, N).all * std::ceil(depth / SG_K);
+    const double blocks = 8.0 * problems * (double)((M + 127) / 128 + (N + 127) / 128) * std::ceil(depth / 1024.0);
+    const double now = 12.0 + 4.0 * (c - 1.0) + operands / 5.2e6 + 3.4 * blocks / (2.0 * sms) + rounds(128, 128, sms) * std::max(0.0163 * depth, 3.4 * c);
+    return 1.1 * now < before;
   }
+  const double wide = N % 256 == 0 ? rounds(128, 256, sms) : 1e30;
+  double before = wide > 1 && wide < 1e30 ? wide * 0.0441 * depth : rounds(128, 128, sms) * 0.030 * depth;
+  before = 5.0 + std::max(before, 4.0 * problems * (depth * (double)(M + N) + 2.0 * (double)M * (double)N) / 5.3e6);
   // a round of tiles: the MMAs, or the accesses to C where K is short
-  const double c = vec_c ? 1.0 : 2.0;
   const double product = std::min({rounds(256, 256, sms / 2) * std::max(0.0213 * depth, 12.0 * c), rounds(256, 128, sms / 2) * std::max(0.0133 * depth, 6.0 * c),
                                    rounds(128, 128, sms) * std::max(0.0178 * depth, 6.0 * c)});
-  const double now = std::max(16.0, 8.0 + 8.0 * problems * depth * (double)(M + N) / 4.5e6 + product);
+  const double now = std::max(16.0, 8.0 + operands / 4.5e6 + product);
   return before > 20.0 && 1.15 * now < before;
 }
 
