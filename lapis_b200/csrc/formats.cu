@@ -235,7 +235,7 @@ static int64_t bspmm_slice(int64_t n2, int64_t E) {
   if (4.0 * (double)n2 * (double)E <= 96e6) return E;
   int64_t width = 256;
   while (width > 32 && 4.0 * (double)n2 * (double)width > 72e6) width /= 2;
-  return width < E ? width : E;
+  return width < E && (E + width - 1) / width <= 65535 ? width : E;  // a slice is a row of the grid
 }
 
 template <typename I>
