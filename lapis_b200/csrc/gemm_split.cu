@@ -857,8 +857,13 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
   const size_t off_a = take(n * 2 * parts * block_m * sh.kc), off_b = take(n * 2 * parts * sh.kc * padded(block_n)), off_sa = take(n * block_m * 4),
                off_sb = take(n * padded(block_n) * 4), off_fa = take((size_t)(marks * group_b) * 8 * panels(M)),
                off_fb = take((size_t)(marks * group_b) * 8 * panels(N)), off_sums = take(sums);
+  // The pool is made by the first allocation, which belongs to no stream and may come while one is being captured.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  LAPIS_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
   PoolBuf buf;
-  if (buf.alloc(total, st) != LAPIS_OK) {
+  const int allocated = buf.alloc(total, st);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (allocated != LAPIS_OK) {
     clear_error();
     return LAPIS_OK;
   }

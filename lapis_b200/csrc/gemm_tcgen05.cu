@@ -30,6 +30,7 @@
 // Every mbarrier wait is bounded: after WAIT_LIMIT polls the thread records an error code
 // in a global flag and stops waiting, the block still frees its tensor memory and exits,
 // and the host turns the flag into LAPIS_ECUDA.
+#include <atomic>
 #include <cstdlib>
 
 #include "tcgen05.h"
@@ -429,23 +430,26 @@ int make_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, int64
 
 }  // namespace tc
 
-static int *error_flag[64] = {nullptr};
+// Part of the library's image on every device, so that a first call under stream capture has nothing to allocate.
+__device__ int g_bgemm_error;
+static std::atomic<int *> error_flag[64];  // where it lies on each device
 int *bgemm_error_flag(int dev) {
   if (dev < 0 || dev >= 64) {
     fail(LAPIS_EBADARG, "bgemm: device index %d not supported", dev);
     return nullptr;
   }
-  if (error_flag[dev] == nullptr) {
-    int *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p, 0, sizeof(int));
+  int *p = error_flag[dev].load(std::memory_order_relaxed);
+  if (p == nullptr) {
+    void *at = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&at, g_bgemm_error);
     if (e != cudaSuccess) {
       fail(LAPIS_ECUDA, "bgemm: %s", cudaGetErrorString(e));
       return nullptr;
     }
-    error_flag[dev] = p;
+    p = static_cast<int *>(at);
+    error_flag[dev].store(p, std::memory_order_relaxed);
   }
-  return error_flag[dev];
+  return p;
 }
 
 template <typename C_>
@@ -465,7 +469,7 @@ static int launch_cfg(int64_t batch, int64_t M, int64_t N, int64_t K, const floa
   const int64_t grid = total < sm_count() ? total : sm_count();  // persistent: one block per SM
   const int kseg = (flags.a != nullptr ? flags.kc : tc::K_SEGMENT) / C_::BK;
   LAPIS_CUDA_TRY(launch_pdl(tc::bgemm_tcgen05_kernel<C_>, (unsigned)grid, tc::THREADS, C_::SMEM_BYTES, st, map_a, map_b, C, (int)M,
-                            (int)N, (int)K, (int)total, kseg, flags, first, error_flag[dev]));
+                            (int)N, (int)K, (int)total, kseg, flags, first, bgemm_error_flag(dev)));
   return LAPIS_OK;
 }
 
@@ -501,18 +505,20 @@ int bgemm_tcgen05_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const f
 
 // Reads and clears the tensor-core kernel's error flag; synchronises `stream`.  A non-zero flag
 // means a bounded wait inside the kernel gave up (1 producer, 2 MMA issuer, 3 split warps,
-// 4 epilogue) and the output of that launch is not valid.
+// 4 epilogue; of the product from split operands 5 producer, 6 MMA issuer, 7 epilogue) and the output of that launch is not
+// valid.
 extern "C" int lapis_b200_bgemm_status(void *stream) {
   using namespace lapis_b200;
   clear_error();
   int dev = 0;
   LAPIS_CUDA_TRY(cudaGetDevice(&dev));
   LAPIS_CUDA_TRY(cudaStreamSynchronize(as_stream(stream)));
-  if (dev < 0 || dev >= 64 || error_flag[dev] == nullptr) return LAPIS_OK;
+  int *at = dev < 0 || dev >= 64 ? nullptr : error_flag[dev].load(std::memory_order_relaxed);
+  if (at == nullptr) return LAPIS_OK;
   int flag = 0;
-  LAPIS_CUDA_TRY(cudaMemcpy(&flag, error_flag[dev], sizeof(int), cudaMemcpyDeviceToHost));
+  LAPIS_CUDA_TRY(cudaMemcpy(&flag, at, sizeof(int), cudaMemcpyDeviceToHost));
   if (flag != 0) {
-    cudaMemset(error_flag[dev], 0, sizeof(int));
+    cudaMemset(at, 0, sizeof(int));
     return fail(LAPIS_ECUDA, "bgemm: tensor-core kernel gave up waiting (role %d)", flag);
   }
   return LAPIS_OK;
