@@ -35,7 +35,7 @@ int spmv_launch(const lapis_b200_csr *h, const double *x, double *y, int accumul
                 double *blk_partial, const int *skip_flag, cudaStream_t st);
 bool spmv_fuses_pcg_pass(const lapis_b200_csr *h);
 bool spmv_fits_small_pcg(const lapis_b200_csr *h);
-int pcg_small(const lapis_b200_csr *h, bool grid, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
+int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
               uint64_t *iters, double *relres, bool *solved, cudaStream_t st);
 bool spmv_fits_grid_pcg(const lapis_b200_csr *h);
 int pcg_grid(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
@@ -628,13 +628,11 @@ extern "C" int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const d
     if (relres) *relres = NAN;
     return LAPIS_OK;
   }
-  const bool grid = spmv_fits_grid_pcg(h);
   if (spmv_fits_small_pcg(h)) {
     bool solved = false;
-    LAPIS_TRY(pcg_small(h, grid, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
+    LAPIS_TRY(pcg_small(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
     if (solved) return LAPIS_OK;
-  }
-  if (grid) {
+  } else if (spmv_fits_grid_pcg(h)) {
     bool solved = false;
     LAPIS_TRY(pcg_grid(h, d_b, d_dinv, tol, maxiter, d_x, iters, relres, &solved, st));
     if (solved) return LAPIS_OK;

@@ -11,10 +11,9 @@
 // Bound by the chains of dependent additions and shuffles between the barriers.  5-point stencils, us an iteration, with
 // 512 to 1024 threads a CTA and the totals left to one warp, and now: 1024 rows 2.9 and 2.1, 4096 rows 3.5 and 3.3, 6400
 // rows 4.7 and 3.7, 16,384 rows 6.1 and 5.4 (the passes of pcg.cu 18); 2000 scattered rows of 10, 9.3 and 8.7.  With
-// scattered columns by the gathers from the other CTAs' memory, which the solve therefore counts first where there may be too
-// many.  us an iteration here, in one cooperative launch (pcg_grid.cu), in passes: 4000 rows of 9, 28,000 such gathers, 11.3, 13.0,
-// 19.7; of 13, 42,000, 16.7, 14.9, 21.7; 5500 of 7, 27,000, 13.4, 11.9, 21.5; 8000 of 5, 28,000, 10.3, 10.8, 21.4; of 11, 70,000,
-// 24.8, 13.9, 21.6.  Systems that are left go to pcg_grid.cu, or to the passes where that does not take them.
+// scattered columns by the gathers from the other CTAs' memory: 8000 rows of 11, 70,000 such gathers, 23.3 us,
+// passes 20 to 21.5.  The solve therefore counts them first where there may be too many, and leaves the system to the
+// passes.
 //
 // The recurrences are those of pcg.cu (examples/pcg_solve.py:65-98 in the LAPIS project), element by element; a row of A p
 // is added in entry order.  Results are identical from run to run; against the other passes they differ by the order of the
@@ -26,10 +25,8 @@
 
 namespace lapis_b200 {
 
-// Gathers from other CTAs' memory in an iteration, beyond which the passes are faster, and one cooperative launch, for up to
-// 4096 rows and for more.
-constexpr int SMALL_FAR_PASSES = 60000, SMALL_FAR_GRID[2] = {36000, 24000};
-constexpr int SMALL_LEFT = 2;       // FL_DONE of a system that is left to the others
+constexpr int SMALL_FAR = 60000;  // gathers from other CTAs' memory in an iteration, beyond which the passes are faster
+constexpr int SMALL_LEFT = 2;     // FL_DONE of a system that was left to the passes
 constexpr int SMALL_BUDGET = 4096;  // iterations per launch (a few milliseconds): the host looks at the outcome in between
 
 struct SmallSolve {
@@ -39,7 +36,7 @@ struct SmallSolve {
   long long *fl;
   double tol;
   unsigned long long maxiter;
-  int n, far;  // far: gathers from other CTAs that are solved here at most
+  int n;
   bool first, count_far;
 };
 
@@ -139,7 +136,7 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     small_barrier<CTAS>();  // every CTA of the cluster runs before its shared memory is written
     send(0, (double)far);
     small_barrier<CTAS>();
-    if (total(0) > s.far) {  // in all CTAs alike; nothing of theirs is read or written any more
+    if (total(0) > SMALL_FAR) {  // in all CTAs alike; nothing of theirs is read or written any more
       if (rank == 0 && tid == 0) s.fl[FL_DONE] = SMALL_LEFT;
       return;
     }
@@ -268,8 +265,8 @@ static cudaError_t launch_small_size(const lapis_b200_csr *h, const SmallSolve &
 }
 
 // Only for handles on which spmv_fits_small_pcg() is true (at most 16384 rows).  *solved: false where the system is left
-// to one cooperative launch (grid: which would take it) or to the passes.
-int pcg_small(const lapis_b200_csr *h, bool grid, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
+// to the passes.
+int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter, double *d_x,
               uint64_t *iters, double *relres, bool *solved, cudaStream_t st) {
   const int64_t n = h->nrows;
   PoolBuf buf;
@@ -286,8 +283,7 @@ int pcg_small(const lapis_b200_csr *h, bool grid, const double *d_b, const doubl
   s.maxiter = maxiter;
   s.n = (int)n;
   s.first = true;
-  s.far = !grid ? SMALL_FAR_PASSES : n <= 4096 ? SMALL_FAR_GRID[0] : SMALL_FAR_GRID[1];
-  s.count_far = h->nnz > s.far;
+  s.count_far = h->nnz > SMALL_FAR;
   const uint64_t limit = maxiter == 0 ? (1ull << 31) : maxiter;
   int done = 0;
   uint64_t it = 0;
