@@ -9,11 +9,17 @@
 // about 200 KB each and L2 beyond.
 //
 // Bound by the chains of dependent additions and shuffles between the barriers.  5-point stencils, us an iteration, with
-// 512 to 1024 threads a CTA and the totals left to one warp, and now: 1024 rows 2.9 and 2.1, 4096 rows 3.5 and 3.3, 6400
-// rows 4.7 and 3.7, 16,384 rows 6.1 and 5.4 (the passes of pcg.cu 18); 2000 scattered rows of 10, 9.3 and 8.7.  With
-// scattered columns by the gathers from the other CTAs' memory: 8000 rows of 11, 70,000 such gathers, 23.3 us,
-// passes 20 to 21.5.  The solve therefore counts them first where there may be too many, and leaves the system to the
-// passes.
+// 512 to 1024 threads a CTA and the totals left to one warp, and now, 32-bit indices (64-bit): 1024 rows 2.96 and 1.86 (2.25),
+// 4096 rows 3.50 and 3.28 (3.32), 6400 rows 4.6 and 4.0 (4.2), 16,384 rows 6.1 and 5.4 (6.3); the passes of pcg.cu 18.
+// With scattered columns by the gathers from the other CTAs' memory: 8000 rows of 9, 56,000 such gathers, 17.1 and 16.1 (15.5), of
+// 11, 70,000, 20.9, passes 20 to 21.5.  The solve therefore counts them first.  Where there are more than one in eight a thread
+// takes its rows one behind the other: side by side all wait for the longest of them, and rows of scattered matrices differ in
+// length (8000 rows of 9 20.0 (22.9), 16,000 of 5 19.5 (20.6) instead of 15.2 (15.3)), where those of a stencil gain by the
+// loads that are under way together (6400 rows 5.3 one behind the other); rows of up to four entries on average do, too, as long
+// as a CTA has no more than 1024.  Where there are too many the system is left to the passes.
+//
+// One CTA on an SM is said to the compiler: without that it keeps to half of the registers, and the loads of a step wait for each
+// other (3000 rows of 9 10.7 and 9.3, 900 of 9 4.3 and 3.9).
 //
 // The recurrences are those of pcg.cu (examples/pcg_solve.py:65-98 in the LAPIS project), element by element; a row of A p
 // is added in entry order.  Results are identical from run to run; against the other passes they differ by the order of the
@@ -26,6 +32,7 @@
 namespace lapis_b200 {
 
 constexpr int SMALL_FAR = 60000;  // gathers from other CTAs' memory in an iteration, beyond which the passes are faster
+constexpr int SMALL_SHARE = 8;    // one in so many entries far: a system with scattered columns
 constexpr int SMALL_LEFT = 2;     // FL_DONE of a system that was left to the passes
 constexpr int SMALL_BUDGET = 4096;  // iterations per launch (a few milliseconds): the host looks at the outcome in between
 
@@ -36,7 +43,7 @@ struct SmallSolve {
   long long *fl;
   double tol;
   unsigned long long maxiter;
-  int n;
+  int n, nnz;
   bool first, count_far;
 };
 
@@ -69,10 +76,12 @@ __device__ __forceinline__ double warp_total(double v) {
 // between them, and a total had to be formed by one warp and handed out behind another barrier, where eight can each form it
 // (the same additions, so the same bits) together with alpha, beta and the stop test.
 template <typename I, int CTAS, int THREADS, int R>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 1)
 pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const double *__restrict__ val, SmallSolve s) {
   constexpr int SLICE = THREADS * R, WARPS = THREADS / 32, PARTS = CTAS * WARPS;
-  constexpr int STEP = R >= 4 ? 2 : 4;  // entries of each row requested together
+  constexpr int STEP = R >= 4 && sizeof(I) == 4 ? 2 : 4;  // entries of each row requested together
+  constexpr bool TWO_FORMS = CTAS > 1 && R >= 4;           // scattered columns: the rows one behind the other
+  constexpr bool AHEAD = THREADS < 512 || sizeof(I) == 8;  // their columns asked for while the entries before are gathered
   static_assert(PARTS % 32 == 0 || 32 % PARTS == 0, "a warp adds whole rounds of parts, or has each of them in several lanes");
   __shared__ double s_p[SLICE];
   __shared__ double s_part[3][PARTS];
@@ -128,7 +137,8 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     z[i] = __dmul_rn(r[i], d[i]);
     s_p[tid + i * THREADS] = in ? (s.first ? z[i] : s.p[row]) : 0.0;
   }
-  if (CTAS > 1 && s.count_far) {
+  bool scattered = false;
+  if (TWO_FORMS || (CTAS > 1 && s.count_far)) {
     int far = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i)
@@ -136,10 +146,12 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     small_barrier<CTAS>();  // every CTA of the cluster runs before its shared memory is written
     send(0, (double)far);
     small_barrier<CTAS>();
-    if (total(0) > SMALL_FAR) {  // in all CTAs alike; nothing of theirs is read or written any more
+    const double all = total(0);
+    if (s.count_far && all > SMALL_FAR) {  // in all CTAs alike; nothing of theirs is read or written any more
       if (rank == 0 && tid == 0) s.fl[FL_DONE] = SMALL_LEFT;
       return;
     }
+    scattered = TWO_FORMS && SMALL_SHARE * all > (double)s.nnz && (SLICE > 1024 || s.nnz > 4 * s.n);
   }
   double initres = 0.0, rz = 0.0, relres = 0.0;
   unsigned long long iters = 0;
@@ -168,21 +180,53 @@ pcg_small_kernel(const I *__restrict__ pos, const I *__restrict__ crd, const dou
     double ap[R], pap = 0.0;
 #pragma unroll
     for (int i = 0; i < R; ++i) ap[i] = 0.0;
-    for (int j = 0; j < longest; j += STEP) {  // the rows side by side, each in entry order
-      double a[R][STEP], g[R][STEP];
+    if (TWO_FORMS && scattered) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
+      for (int i = 0; i < R; ++i) {
+        int col[4];
+        if (AHEAD) {
 #pragma unroll
-        for (int u = 0; u < STEP; ++u) {
-          const bool in = j + u < len[i];
-          a[i][u] = in ? __ldg(v[i] + j + u) : 0.0;
-          g[i][u] = in ? gather(__ldg(c[i] + j + u)) : 0.0;
+          for (int u = 0; u < 4; ++u) col[u] = u < len[i] ? (int)__ldg(c[i] + u) : 0;
         }
+        for (int j = 0; j < len[i]; j += 4) {
+          double a[4], g[4];
+          int next[4];
+          if (!AHEAD) {
 #pragma unroll
-      for (int i = 0; i < R; ++i)
+            for (int u = 0; u < 4; ++u) col[u] = j + u < len[i] ? (int)__ldg(c[i] + j + u) : 0;
+          }
 #pragma unroll
-        for (int u = 0; u < STEP; ++u)
-          if (j + u < len[i]) ap[i] = __dadd_rn(ap[i], __dmul_rn(a[i][u], g[i][u]));
+          for (int u = 0; u < 4; ++u) a[u] = j + u < len[i] ? __ldg(v[i] + j + u) : 0.0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) g[u] = j + u < len[i] ? gather((I)col[u]) : 0.0;
+          if (AHEAD) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) next[u] = j + 4 + u < len[i] ? (int)__ldg(c[i] + j + 4 + u) : 0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (j + u < len[i]) ap[i] = __dadd_rn(ap[i], __dmul_rn(a[u], g[u]));
+            if (AHEAD) col[u] = next[u];
+          }
+        }
+      }
+    } else {
+      for (int j = 0; j < longest; j += STEP) {  // the rows side by side, each in entry order
+        double a[R][STEP], g[R][STEP];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int u = 0; u < STEP; ++u) {
+            const bool in = j + u < len[i];
+            a[i][u] = in ? __ldg(v[i] + j + u) : 0.0;
+            g[i][u] = in ? gather(__ldg(c[i] + j + u)) : 0.0;
+          }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int u = 0; u < STEP; ++u)
+            if (j + u < len[i]) ap[i] = __dadd_rn(ap[i], __dmul_rn(a[i][u], g[i][u]));
+      }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i)
@@ -282,6 +326,7 @@ int pcg_small(const lapis_b200_csr *h, const double *d_b, const double *d_dinv, 
   s.tol = tol;
   s.maxiter = maxiter;
   s.n = (int)n;
+  s.nnz = (int)h->nnz;  // at most 131,072 (spmv_fits_small_pcg)
   s.first = true;
   s.count_far = h->nnz > SMALL_FAR;
   const uint64_t limit = maxiter == 0 ? (1ull << 31) : maxiter;
