@@ -29,7 +29,7 @@ constexpr int SPMM_LONG_THREADS = 32 * (SPMM_ADDERS + SPMM_FEEDERS);
 constexpr int SPMM_PER = 4, SPMM_TILE = 32 * SPMM_FEEDERS * SPMM_PER;  // products of a feeder, of a tile
 constexpr int SPMM_TEAM = 4;                          // blocks that share their long rows
 constexpr int SPMM_LOOK = 4;                          // neighbouring rows that a thread looks at together
-constexpr int64_t SPMM_TEAM_BYTES = 450000;           // offsets beyond which a block looks at its own rows only
+constexpr int64_t SPMM_TEAM_BYTES = 450000;           // offsets that a team looks through, for every eight columns
 constexpr int SPMM_LIST = SPMM_LONG_THREADS + 64;     // long rows that a block notes before it works on them
 constexpr int SPMM_SHARED = 768;                      // pieces that a team divides by length; a block alone: SPMM_LIST
 
@@ -191,10 +191,11 @@ __device__ __forceinline__ unsigned spmm_long_among(const I *__restrict__ rowno,
 // and up to 64 columns: by length, the longest first, 0 1 2 3 3 2 1 0 0 1 .. (too many pieces: whole rows in turn).  That each
 // block looks through four times as many rows costs less than an exchange: with one share of the rows for each block of a
 // cluster, passed round through shared memory, products without long rows took 2 to 4 us longer, the launch of clusters and its
-// barriers (10,844 stored rows of 25, k = 3, 12.3 us, now 8.3; 50,021 of 4, k = 37, 20.9 and 19.0).  It does so up to about one look of
-// every thread; beyond, blocks look at their own rows and share nothing: there are enough long rows for each (1,000,000 rows of 4, k = 2,
-// 64 us in teams, 47 alone, 54 in clusters; with skewed lengths 1,500,000 of 8, k = 8, 722, 684 and 697, but 100,000 of 16, k = 8, 81,
-// 117 and 79).
+// barriers (10,844 stored rows of 25, k = 3, 12.3 us, now 8.3; 50,021 of 4, k = 37, 20.9 and 19.0).  It does so while a
+// team's offsets are few beside the product's columns; otherwise blocks look at their own rows and share nothing: there are enough
+// long rows for each (1,000,000 rows of 4, k = 2, 64 us in teams, 47 alone, 54 in clusters; with skewed lengths 1,500,000 of 8,
+// k = 8, 722, 684 and 697; but 100,000 of 16, k = 8, 81, 117 and 79, 91,623 of 25, 64-bit, k = 153, 1103 and 1715).  Where a team has
+// fewer pieces than blocks they are of 32 or 16 columns (3465 rows, five of them long, k = 64, 14.4 us once, 16.4, 12.3 now).
 // A block works through its pieces in tiles of SPMM_TILE products: ten warps gather and multiply, two tiles ahead of the one
 // they store, across the ends of pieces, and two warps add, a lane one column, in entry order out of shared memory.
 // One tile ahead, one row on an SM, a barrier for both, and now: 50,021 rows of 16, k = 37 276 -> 102 us; 40,000 of 30, k = 130
@@ -212,15 +213,6 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
   pdl_release();  // the kernel for the other rows shares nothing with this one but inputs
   const int tid = threadIdx.x, feeder = tid - 32 * SPMM_ADDERS;  // negative: an adder
   const int member = blockIdx.x % team;
-  const int64_t panels = (k + SPMM_PANEL - 1) / SPMM_PANEL;
-  const int width = (int)((k + panels - 1) / panels), entries = SPMM_TILE / width;  // of a tile
-  int je[SPMM_PER], ce[SPMM_PER];  // this feeder's products in a tile: entry (beyond any row: none) and column
-#pragma unroll
-  for (int i = 0; i < SPMM_PER; ++i) {
-    const int at = feeder + 32 * SPMM_FEEDERS * i;
-    je[i] = feeder >= 0 && at < entries * width ? at / width : 0x40000000;
-    ce[i] = at - at / width * width;
-  }
   const int64_t teams = gridDim.x / team, turn = teams * SPMM_LONG_THREADS * SPMM_LOOK;
   const int64_t mine = ((int64_t)(tid / (8 / SPMM_LOOK)) * teams + blockIdx.x / team) * 8 + tid % (8 / SPMM_LOOK) * SPMM_LOOK;
   int seen = 0;  // rows of each thread's in this turn that are noted or worked on
@@ -258,7 +250,17 @@ spmm_long_kernel(const I *__restrict__ rowno, const I *__restrict__ pos, const I
     const bool end = r0 >= nrows;
     if (end && noted == 0) return;
     __syncthreads();
-    // pieces of this block
+    // pieces of this block: of up to 64 columns, or of up to 16 where the team has few rows, so that each block has one
+    int64_t panels = (k + SPMM_PANEL - 1) / SPMM_PANEL;
+    for (int most = SPMM_PANEL / 2; most >= 16 && noted * panels < team; most /= 2) panels = (k + most - 1) / most;
+    const int width = (int)((k + panels - 1) / panels), entries = SPMM_TILE / width;  // of a tile
+    int je[SPMM_PER], ce[SPMM_PER];  // this feeder's products in a tile: entry (beyond any row: none) and column
+#pragma unroll
+    for (int i = 0; i < SPMM_PER; ++i) {
+      const int at = feeder + 32 * SPMM_FEEDERS * i;
+      je[i] = feeder >= 0 && at < entries * width ? at / width : 0x40000000;
+      ce[i] = at - at / width * width;
+    }
     const bool by_length = noted * panels <= (team == 1 ? SPMM_LIST : SPMM_SHARED);
     const int np = by_length ? (int)panels : 1, pieces = noted * np;
     const int rounds = pieces / team, turned = by_length && rounds % 2 != 0 ? team - 1 - member : member;
@@ -426,7 +428,7 @@ static cudaError_t launch_spmm_width(const SpmmArgs<I> &m, cudaStream_t st) {
 template <typename I, bool DCSR>
 static cudaError_t launch_spmm(const SpmmArgs<I> &m, cudaStream_t st) {
   if (m.long_rows) {
-    const int team = m.nrows * (int64_t)sizeof(I) <= SPMM_TEAM_BYTES ? SPMM_TEAM : 1;
+    const int team = m.nrows * (int64_t)sizeof(I) <= SPMM_TEAM_BYTES * std::max<int64_t>(1, m.k / 8) ? SPMM_TEAM : 1;
     const int64_t teams = std::min<int64_t>((m.nrows + 8 * team - 1) / (8 * team), std::max(1, sm_count() / team));
     spmm_long_kernel<I, DCSR><<<(unsigned)(teams * team), SPMM_LONG_THREADS, 0, st>>>(m.rowno, m.pos, m.crd, m.val, m.nrows, m.k, team, m.B, m.C,
                                                                                      m.accumulate);

@@ -18,15 +18,17 @@ def _on(a):
 @pytest.mark.parametrize("idx", [np.int32, np.int64])
 @pytest.mark.parametrize("k", [1, 2, 5, 7, 16, 31, 33, 63, 64, 65, 128, 129, 200])
 def test_rows_that_end_at_a_tile(k, idx):
-    """One entry less and more than the first four whole numbers of tiles above 256 entries, each several times, in any order."""
+    """One entry less and more than the first four whole numbers of tiles above 256 entries, each several times, in any order; in panels of
+    up to 64 columns, or of up to 32 or 16 where a team has few rows."""
     from lapis_b200 import device
     panels = -(-k // 64)
-    entries = TILE // -(-k // panels)
-    tiles = LONG // entries + 1
-    marks = [e * entries + d for e in range(tiles, tiles + 4) for d in (-1, 0, 1)]
-    marks = [n for n in marks if n > LONG] * (2 if k < 16 else 6) + [LONG - 1, LONG, LONG + 1]
+    marks = [LONG - 1, LONG, LONG + 1]
+    for entries in {TILE // -(-k // -(-k // most)) for most in (64, 32, 16)}:
+        tiles = LONG // entries + 1
+        ends = [e * entries + d for e in range(tiles, tiles + 4) for d in (-1, 0, 1)]
+        marks += [n for n in ends if n > LONG] * (1 if k < 16 else 2)
     rng = np.random.default_rng(k)
-    rows, cols = 500, 300
+    rows, cols = 600, 300
     lens = rng.integers(0, 9, rows)
     lens[rng.choice(rows, len(marks), replace=False)] = marks
     assert np.sum(lens) * (k + 8) // panels >> 18 < LONG  # the kernel's rule on the length beside the whole product
