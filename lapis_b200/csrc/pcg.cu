@@ -883,7 +883,8 @@ extern "C" int lapis_b200_pcg_p2p_halo_wait(void *d_work, void *d_mbox, const vo
 // ---------------------------------------------------------------------------------------------
 // Hitting-time moments (examples/hitting_times.py:151-194 in the LAPIS project): two Jacobi-PCG solves
 // with the masked graph Laplacian y = M (D - alpha A) M x as the operator (@plpt, :73-92) and z = r / d
-// as the preconditioner (:113, :140).  Two passes per iteration where the one-thread-per-row SpMV serves the matrix:
+// as the preconditioner (:113, :140).  Two passes per iteration where the one-thread-per-row SpMV serves the matrix and its columns
+// allow it (mht_two_pass):
 //   A  p = z + beta p, at the own row and at every column of it; t = (alpha A)(mask p); Ap = (d mask p - t) mask;
 //      partial sums of (mask p).t and d (mask p)^2, whose difference is p.Ap; tail: alpha
 //   B  x, r, z updates; partial sums of r.r and r.z; tail: stop test, beta
@@ -1251,6 +1252,59 @@ static int mht_solve(const lapis_b200_csr *A, bool two_pass, double alpha, const
   return LAPIS_OK;
 }
 
+// Counts, for every sixteenth row, the entries that have one in the next row at the same place of it (count[1]), and those of
+// them whose columns are at most eight apart (count[0]): gathers that neighbouring threads share lines for.
+template <typename I>
+__global__ void __launch_bounds__(VEC_THREADS)
+mht_neighbours_kernel(const I *__restrict__ pos, const I *__restrict__ crd, int64_t n, unsigned long long *count) {
+  unsigned near = 0, all = 0;
+  for (int64_t r = 16 * ((int64_t)blockIdx.x * VEC_THREADS + threadIdx.x); r + 1 < n; r += 16 * (int64_t)gridDim.x * VEC_THREADS) {
+    const int64_t lo = (int64_t)pos[r], mid = (int64_t)pos[r + 1], hi = (int64_t)pos[r + 2];
+    const int64_t both = mid - lo < hi - mid ? mid - lo : hi - mid;
+    for (int64_t u = 0; u < both; ++u) {
+      const int64_t apart = (int64_t)crd[lo + u] - (int64_t)crd[mid + u];
+      near += apart >= -8 && apart <= 8;
+    }
+    all += (unsigned)both;
+  }
+  near = __reduce_add_sync(0xffffffffu, near);
+  all = __reduce_add_sync(0xffffffffu, all);
+  if (threadIdx.x % 32 == 0 && all != 0) {
+    atomicAdd(count, near);
+    atomicAdd(count + 1, all);
+  }
+}
+
+// Whether the solves of a matrix that the one-thread-per-row SpMV serves take two passes, which save launches and vectors but
+// gather three vectors at every entry where the SpMV gathers one.  us of two solves of 48 iterations, in four launches and in two
+// passes: neighbouring rows with neighbouring columns, 1000^2 grid 5710 and 4611, 10^6 rows of 6 in a band 5998 and 5218, of 12
+// 8599 and 7693, but of 30 13,400 and 15,700; scattered columns, 140,000 rows of 4 3188 and 2724, 300,000 of 6 4429 and 4333, but
+// 100,000 of 10 3530 and 3800, 700,000 of 4 5386 and 6378, 2,000,000 of 6 12,964 and 20,855.  Below 2^19 entries the launches
+// decide: 20,000 scattered rows of 10 3037 and 2078.
+static int mht_two_pass(const lapis_b200_csr *h, bool *two_pass, cudaStream_t st) {
+  constexpr int64_t FEW_ENTRIES = 1 << 19, FEW_ROWS = 300000;
+  *two_pass = spmv_fuses_pcg_pass(h);
+  const int64_t n = h->nrows, nnz = h->nnz;
+  const int64_t scattered = n <= FEW_ROWS ? 6 : 0, beside = n <= FEW_ROWS ? 32 : 16;  // entries of a row on average, at most
+  if (!*two_pass || nnz < FEW_ENTRIES || nnz <= scattered * n) return LAPIS_OK;
+  *two_pass = nnz <= beside * n;
+  if (!*two_pass) return LAPIS_OK;
+  PoolBuf buf;
+  LAPIS_TRY(buf.alloc(2 * sizeof(unsigned long long), st));
+  unsigned long long *count = static_cast<unsigned long long *>(buf.p), host[2];
+  LAPIS_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(host), st));
+  const unsigned blocks = vec_grid((n + 15) / 16);
+  if (h->idx_bytes == 4)
+    mht_neighbours_kernel<<<blocks, VEC_THREADS, 0, st>>>(static_cast<const int32_t *>(h->pos), static_cast<const int32_t *>(h->crd), n, count);
+  else
+    mht_neighbours_kernel<<<blocks, VEC_THREADS, 0, st>>>(static_cast<const int64_t *>(h->pos), static_cast<const int64_t *>(h->crd), n, count);
+  LAPIS_CUDA_TRY(cudaGetLastError());
+  LAPIS_CUDA_TRY(cudaMemcpyAsync(host, count, sizeof(host), cudaMemcpyDeviceToHost, st));
+  LAPIS_CUDA_TRY(cudaStreamSynchronize(st));
+  *two_pass = 2 * host[0] >= host[1];
+  return LAPIS_OK;
+}
+
 }  // namespace lapis_b200
 
 extern "C" int lapis_b200_mht_f64(lapis_b200_csr_t h, const double *d_mask, const double *d_d, double alpha, double tol,
@@ -1266,7 +1320,8 @@ extern "C" int lapis_b200_mht_f64(lapis_b200_csr_t h, const double *d_mask, cons
   cudaStream_t st = as_stream(stream);
   // two solves run the SpMV pass many times: pick the kernel variant for this matrix first
   if (h->tuned_threads == 0 && (maxiter == 0 || maxiter >= 16)) LAPIS_TRY(lapis_b200_csr_tune(h, st));
-  const bool two_pass = spmv_fuses_pcg_pass(h);  // one thread per row, which multiplies by alpha as it goes
+  bool two_pass = false;  // one thread per row, which multiplies by alpha as it goes
+  LAPIS_TRY(mht_two_pass(h, &two_pass, st));
   const unsigned G = vec_grid(n);
   // partials: three sums of G blocks, or two of at most eight blocks per SM
   const size_t partials = std::max<size_t>(3 * (size_t)G, 2 * 8 * (size_t)sm_count());
