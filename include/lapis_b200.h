@@ -247,7 +247,11 @@ int lapis_b200_axpby_f64(int64_t n, double a, const double *d_x, double b, const
 int lapis_b200_mult_f64(int64_t n, const double *d_x, const double *d_y, double *d_dst, void *stream);
 
 /* PCG with all state on the device (examples/pcg_solve.py:52-101).  d_x receives
- * the solution; *iters and *relres are host outputs.  Blocks until finished. */
+ * the solution; *iters and *relres are host outputs.  Blocks until finished.
+ * Systems of short rows that one launch solves (up to 16,384 rows, and up to 2048 for each SM with no more than 16 entries a
+ * row on average) leave the handle as it is; the others tune it first, as lapis_b200_csr_tune does, if nobody has and
+ * maxiter is 0 or at least 16.  A loop that solves and multiplies with one handle calls the tuner itself: products
+ * of 250,000 rows of 9 take 6.9 us tuned and 10 untuned. */
 int lapis_b200_pcg_f64(lapis_b200_csr_t h, const double *d_b, const double *d_dinv, double tol, uint64_t maxiter,
                        double *d_x, uint64_t *iters, double *relres, void *stream);
 

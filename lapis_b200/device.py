@@ -119,7 +119,8 @@ class CsrMatrix:
         return C
 
     def pcg(self, b: torch.Tensor, dinv: torch.Tensor, tol: float, maxiter: int):
-        """Returns (x, iters, relres); blocks until the solve has finished."""
+        """Returns (x, iters, relres); blocks until the solve has finished.  A solve does not always tune the handle: a loop that
+        also multiplies with it calls ``tune`` itself (lapis_b200.h)."""
         _f64(b, "b"), _f64(dinv, "dinv")
         x = torch.empty_like(b)
         iters, relres = c_u64(0), c_dbl(0.0)
