@@ -20,10 +20,10 @@
 //
 // 8192^3: 5.05 -> 2.70 ms where the clock holds (407 TFLOP/s, three products at 75 % of cuBLAS's bf16 rate), 5.91 -> 3.33 where
 // power caps it, with an error of 1.25e-6 against 64 bits (2-norm; TF32 split 8.0e-6).  Three parts cost 5 to 65 % more time
-// than two: 1000 x 1501 x 777 142 us in the kernel for general shapes, 30.6 with two parts, 35.7 with three; 5000 x 3000 x 1999
-// 2270, 260 and 361; 8191^3 46, 4.3 and 6.1 ms.  Their errors, that kernel's first: 1000 x 1501 x 777 uniform in [-1, 1) 5.0e-7,
-// 3.9e-7 and 1.6e-7, in [0, 1) 4.2e-7, 1.4e-6 and 2.4e-7, A with 1 % nonzeros 6.3e-8, 7.5e-8 and 4.7e-8, 100 x 200^3 2.6e-7,
-// 1.8e-7 and 9.8e-8.
+// than two: 1000 x 1501 x 777 142 us in the kernel for general shapes, 30.6 with two parts, 36.7 with three; 5000 x 3000 x 1999
+// 2270, 260 and 319; 8191^3 46, 4.3 and 5.8 ms.  Their errors, that kernel's first: 1000 x 1501 x 777 uniform in [-1, 1) 5.0e-7,
+// 3.9e-7 and 1.2e-7, in [0, 1) 4.2e-7, 1.4e-6 and 1.5e-7, A with 1 % nonzeros 6.3e-8, 7.5e-8 and 5.2e-8, 100 x 200^3 2.6e-7,
+// 1.8e-7 and 7.7e-8.
 //
 // fp16 has 5 bits of exponent: the hi of an element below 2^-14 after scaling (2^-29 of the largest of its row or column)
 // would be subnormal and lo lo up to 2^-17 of a product of two such, and an infinity or NaN has no scale.  split_kernel marks
@@ -367,8 +367,10 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
 //
 // The tensor core truncates when it adds to its accumulator, an error that grows with the length of the chain (chain / 16
 // additions, 2^-25 of the partial sum each on average); sh.chain of K are added there, the rest in registers, rounded.  For
-// operands of one sign that is the largest error: chains of 9 sqrt(K) keep it below the sequential sum's (K = 8189 1.08e-6 and
-// 1.19e-6, K = 777 2.4e-7 and 4.2e-7; with 13 sqrt(K) 1.70e-6 and 4.1e-7).
+// operands of one sign, or of so wide a range that few products make the sum, that is the largest error.  Chains of about 4.5 sqrt(K)
+// keep it below the sequential sum's: in [0, 1) K = 777 1.5e-7 and 4.2e-7, 8351 5.9e-7 and 1.23e-6; lognormal entries (sigma 2) 0.4 of
+// it in the median of 76 shapes, up to 1.5 where one element is the norm.  With 9 sqrt(K) 2.4e-7, 1.26e-6, 0.65 and up to 2.8; it
+// costs 2 to 5 % more time (1000 x 1501 x 777 35.9 -> 36.7 us, 8191^3 5.6 -> 5.7 to 5.9 ms).
 template <typename C_>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, float *__restrict__ C, Shape sh,
@@ -820,7 +822,7 @@ int bgemm_split_launch(int64_t batch, int64_t M, int64_t N, int64_t K, const flo
   Shape sh = {};
   sh.K = (int)K;
   sh.ldn = (int)N;
-  sh.chain = exact_order ? std::min(KC, 64 * std::max(1, (int)(std::sqrt((double)K) / 7))) : KC;
+  sh.chain = exact_order ? std::min(KC, 64 * std::max(1, (int)(std::sqrt((double)K) / 14 + 0.5))) : KC;
   int64_t all = 0;  // stretches of K
   int64_t block_m = M, block_n = N;
   size_t sums = 0;  // bytes
